@@ -1,6 +1,7 @@
 // ugks_lo.cuh -- device-side state of one Couette domain and the second-order (Van-Leer UGKS)
 // kernels' parameter blocks.
 #pragma once
+#include <algorithm>
 #include <cmath>
 
 #include "../../include/ugks_b200.h"
@@ -22,6 +23,8 @@ struct LoParams {
     double inv_area;         // 1/area when area is a power of two (then x/area == x*inv_area exactly), else 0
     // the research S2CN2 wall variants (ugks_params): kinetic walls, W1T midpoint walls, W1D, W2R
     int s2_kinetic, s2_midpoint, s2_face_time, s2_shared;
+    // a tensor-product velocity table (tensor_table): its abscissae per axis, nvel = tnu tnv; 0: none
+    int tnu, tnv;
 };
 
 // x / area, as a multiplication when that is exact (area a power of two: both operations round the
@@ -34,6 +37,7 @@ struct LoBuffers {
     const double* u;         // [nvel] velocity table, k = i + j*Nu
     const double* v;
     const double* w;
+    const double* tab;       // [4][64] the axes of a tensor table (LoParams::tnu > 0): u, wx, v, wy
     double* h;               // [nc][nvel] state, cell c = j*nx + i
     double* b;
     double* W;               // [nc][4] conservative variables
@@ -94,6 +98,54 @@ __device__ __forceinline__ Slot slot(int r, int nv) {
     s.ok = s.k < nv;
     s.kk = s.ok ? s.k : nv - 1;
     return s;
+}
+
+// Whether (u, v, w) is the tensor product of two rules of at most 64 abscissae each, k = i + j nu
+// (InitVelocityFromStructuredFile, mod_InitializeFlow.f90:480-509): u[k] = u_i and v[k] = v_j exactly, and
+// w[k] = wx_i wy_j to within 4 units in the last place, the rounding of a product whose factors are
+// themselves recovered from the products (the S2 closures use the factors: a table of rounded decimal weights that
+// misses this keeps the general kernels).  On success tab holds u, wx, v, wy, each padded to 64 with its last
+// abscissa and weight 0.  Host only.
+inline bool tensor_table(int nv, const double* u, const double* v, const double* w, int* nu_out, int* nv_out,
+                         double tab[256]) {
+    int nu = 1;
+    while (nu < nv && v[nu] == v[0]) ++nu;
+    if (nv % nu != 0) return false;
+    const int nj = nv / nu;
+    if (nu < 2 || nj < 2 || nu > 64 || nj > 64) return false;
+    for (int k = 0; k < nv; ++k) {
+        if (!(u[k] == u[k % nu] && v[k] == v[k - k % nu])) return false;
+        if (!(w[k] > 0.0) || !std::isfinite(w[k]) || !std::isfinite(u[k]) || !std::isfinite(v[k])) return false;
+    }
+    // factors up to their common scale: alternating weighted means of the ratios, each weight's rounding averaged out
+    long double fx[64], fy[64];
+    for (int j = 0; j < nj; ++j) fy[j] = (long double)w[j * nu] / (long double)w[0];
+    for (int it = 0; it < 2; ++it) {
+        for (int i = 0; i < nu; ++i) {
+            fx[i] = 0.0L;
+            for (int j = 0; j < nj; ++j) fx[i] += (long double)w[j * nu + i] / fy[j];
+            fx[i] /= (long double)nj;
+        }
+        for (int j = 0; j < nj; ++j) {
+            fy[j] = 0.0L;
+            for (int i = 0; i < nu; ++i) fy[j] += (long double)w[j * nu + i] / fx[i];
+            fy[j] /= (long double)nu;
+        }
+    }
+    for (int a = 0; a < 64; ++a) {
+        tab[a] = u[std::min(a, nu - 1)];
+        tab[64 + a] = a < nu ? (double)fx[a] : 0.0;
+        tab[128 + a] = v[(size_t)std::min(a, nj - 1) * nu];
+        tab[192 + a] = a < nj ? (double)fy[a] : 0.0;
+    }
+    for (int j = 0; j < nj; ++j)
+        for (int i = 0; i < nu; ++i) {
+            const double x = w[j * nu + i];
+            if (!(std::fabs(tab[64 + i] * tab[192 + j] - x) <= 4.0 * 2.220446049250313e-16 * x)) return false;
+        }
+    *nu_out = nu;
+    *nv_out = nj;
+    return true;
 }
 
 // The kernels' parameter block of a domain described by the C ABI's ugks_params, with U_MAX / V_MAX

@@ -24,7 +24,7 @@
 // those identical totals.  Per-velocity closure quantities (the Maxwellian, the Shakhov directions,
 // the slope directions) are recomputed from the closure's few scalars in each pass instead of being
 // stored.
-#include "ugks_s2_math.cuh"
+#include "ugks_s2_tensor.cuh"
 
 namespace ugks {
 
@@ -315,6 +315,128 @@ __global__ void __launch_bounds__(256) k_s2_target_sum(LoParams P, LoBuffers B, 
     }
     const size_t q = (size_t)cc * nv + k;
     SB.mh[q] = amh; SB.mb[q] = amb; SB.kxh[q] = akxh; SB.kxb[q] = akxb; SB.kyh[q] = akyh; SB.kyb[q] = akyb;
+}
+
+// build_targets on a tensor-product velocity table (LoParams::tnu > 0): the closures by 1-D sums, eight lanes a
+// (cell, volume node), four nodes a warp -> the same node scalars.  Bound by the latency of the Newton
+// chain (two exponentials, a butterfly, a 4x4 solve an evaluation).  With the sums below it took the S2CN2 step at
+// 8x64x32^2 from 0.869 to 0.704 ms and the 16-instance batch from 17.5 to 14.0 ms a step.  Eight lanes a
+// node share the uniform scalar work four ways a warp and still fill the chip with 1152 warps at that size.
+// A table that is no tensor product (tensor_table) takes the kernels above.
+template <int R>
+__global__ void __launch_bounds__(128, 3) k_s2_target_nodes_t(LoParams P, LoBuffers B, S2Buffers SB) {
+    if (eval_cached(B)) return;
+    __shared__ double s_jac[128 / kTG][17];
+    const int nn = P.nx * P.ny * 9, gl = threadIdx.x & (kTG - 1);
+    const int id = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kTG), node = min(id, nn - 1);
+    double w[4], td[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) w[m] = SB.wq[(size_t)node * 4 + m];
+    TClosure C;
+    C.jac = s_jac[threadIdx.x / kTG];
+    WMke M;
+    bool ok = t_closure<R>(P, B, w, id < nn, C);
+    ok = t_mke<R>(P, B, w, C, M, nullptr, td) && ok;
+    if (id >= nn) return;
+    if (!ok) {
+        if (gl == 0) set_status(B.status, ST_PROJECTION);
+        return;
+    }
+    double* o = SB.tscal + (size_t)node * kS2TScal;
+    if (gl == 0) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) { o[m] = C.th[m]; o[4 + m] = M.tdx[m]; o[8 + m] = M.tdy[m]; }
+        o[12] = M.ux; o[13] = M.vy; o[14] = M.lam; o[15] = M.coeff;
+    }
+    o[16 + gl] = C.jac[gl];
+    o[24 + gl] = C.jac[8 + gl];
+}
+
+// build_targets, sum part, on a tensor table: one CTA per cell and 1024 velocities.  The 9 nodes' Maxwellians are
+// products of two rows of exponentials (shared memory, the Gauss weight and rho / (pi T) folded into the x
+// row), and M, K_x, K_y the product times a cubic in the velocity whose coefficients are the node's.
+struct S2TargetC {   // one node: mean of theta, mean of the state, ck T / 2, the cubic's coefficients
+    double u, v, ux, vy, ckh, sl, s0, kb;   // Shakhov factor sl c^2 - s0; kb = 2 coeff / ck
+    double x[5], y[5];                      // direction polynomial 1, cx, cy, c^2 of K_x and K_y, and its b part
+};
+__global__ void __launch_bounds__(256) k_s2_target_sum_t(LoParams P, LoBuffers B, S2Buffers SB) {
+    if (eval_cached(B)) return;
+    __shared__ double ex[9][64], ey[9][64];
+    __shared__ S2TargetC sc[9];
+    const int nv = P.nvel, nu = P.tnu, nw = P.tnv, cc = blockIdx.y, tid = threadIdx.x;
+    const double gw[3] = {5.0 / 18.0, 4.0 / 9.0, 5.0 / 18.0};
+    if (tid < 9) {
+        double th[4];
+        WMke M;
+        w_load_scalars(SB.tscal + ((size_t)cc * 9 + tid) * kS2TScal, th, M);
+        const S2Th t = s2_th(th, P.ck);
+        S2TargetC& c = sc[tid];
+        c.u = t.u; c.v = t.v; c.ux = M.ux; c.vy = M.vy; c.ckh = t.ckh;
+        c.sl = 2.0 * M.lam * M.coeff; c.s0 = 4.0 * M.coeff; c.kb = 2.0 / (double)P.ck * M.coeff;
+        const double i2 = t.itw * t.itw;
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            const double* td = d ? M.tdy : M.tdx;
+            double* p = d ? c.y : c.x;
+            p[0] = td[0] * t.ir - td[3] * t.itw;
+            p[1] = 2.0 * t.itw * td[1];
+            p[2] = 2.0 * t.itw * td[2];
+            p[3] = td[3] * i2;
+            p[4] = td[3] * t.itw;
+        }
+    }
+    for (int q = tid; q < 9 * (nu + nw); q += blockDim.x) {
+        const int p = q / (nu + nw), a = q - p * (nu + nw);
+        const double* o = SB.tscal + ((size_t)cc * 9 + p) * kS2TScal;
+        const double itw = 1.0 / o[3];
+        if (a < nu) {
+            const double d = B.tab[a] - o[1];
+            ex[p][a] = gw[p % 3] * gw[p / 3] * (o[0] / (kPi * o[3])) * exp(-(d * d) * itw);
+        } else {
+            const double d = B.tab[128 + a - nu] - o[2];
+            ey[p][a - nu] = exp(-(d * d) * itw);
+        }
+    }
+    __syncthreads();
+    double a[4][6], uk[4], vk[4];
+    int iu[4], iv[4];
+    const int k0 = blockIdx.x * 1024 + tid;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int k = min(k0 + r * (int)blockDim.x, nv - 1);
+        iv[r] = k / nu;
+        iu[r] = k - iv[r] * nu;
+        uk[r] = B.tab[iu[r]];
+        vk[r] = B.tab[128 + iv[r]];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) a[r][m] = 0.0;
+    }
+#pragma unroll 1
+    for (int p = 0; p < 9; ++p) {
+        const S2TargetC& c = sc[p];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const double q = ex[p][iu[r]] * ey[p][iv[r]], qb = c.ckh * q;
+            const double cx = uk[r] - c.u, cy = vk[r] - c.v, px = uk[r] - c.ux, py = vk[r] - c.vy;
+            const double c2 = cx * cx + cy * cy, sh = c.sl * (px * px + py * py) - c.s0;
+            const double kx = px * sh - (c.x[0] + c.x[1] * cx + c.x[2] * cy + c.x[3] * c2);
+            const double ky = py * sh - (c.y[0] + c.y[1] * cx + c.y[2] * cy + c.y[3] * c2);
+            a[r][0] += q;
+            a[r][1] += qb;
+            a[r][2] += q * kx;
+            a[r][3] += qb * (kx + c.kb * px - c.x[4]);
+            a[r][4] += q * ky;
+            a[r][5] += qb * (ky + c.kb * py - c.y[4]);
+        }
+    }
+    double* out[6] = {SB.mh, SB.mb, SB.kxh, SB.kxb, SB.kyh, SB.kyb};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int k = k0 + r * (int)blockDim.x;
+        if (k < nv && k < (int)(blockIdx.x + 1) * 1024)
+#pragma unroll
+            for (int m = 0; m < 6; ++m) out[m][(size_t)cc * nv + k] = a[r][m];
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -846,12 +968,24 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
     }
     if (e == cudaSuccess && targets) {
         cudaStream_t ts = side_targets ? s2 : s;
-        const int qb = qrec_bytes(S, nv, 256, kQRecCap256x2);
-        k_s2_target_nodes<<<warps((long long)nc * 9), 256, qb, ts>>>(P, B, S, qb > 0);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) {
-            k_s2_target_sum<<<dim3((unsigned)((nv + 255) / 256), (unsigned)nc), 256, 0, ts>>>(P, B, S);
+        if (P.tnu > 0) {
+            const unsigned g = (unsigned)((nc * 9 * kTG + 127) / 128);
+            const int n = P.tnu > P.tnv ? P.tnu : P.tnv;
+            if (n <= 24) k_s2_target_nodes_t<3><<<g, 128, 0, ts>>>(P, B, S);
+            else if (n <= 32) k_s2_target_nodes_t<4><<<g, 128, 0, ts>>>(P, B, S);
+            else if (n <= 48) k_s2_target_nodes_t<6><<<g, 128, 0, ts>>>(P, B, S);
+            else k_s2_target_nodes_t<8><<<g, 128, 0, ts>>>(P, B, S);
+            const int nt = std::min(256, (nv + 127) / 128 * 32);
+            k_s2_target_sum_t<<<dim3((unsigned)((nv + 1023) / 1024), (unsigned)nc), nt, 0, ts>>>(P, B, S);
             e = cudaGetLastError();
+        } else {
+            const int qb = qrec_bytes(S, nv, 256, kQRecCap256x2);
+            k_s2_target_nodes<<<warps((long long)nc * 9), 256, qb, ts>>>(P, B, S, qb > 0);
+            e = cudaGetLastError();
+            if (e == cudaSuccess) {
+                k_s2_target_sum<<<dim3((unsigned)((nv + 255) / 256), (unsigned)nc), 256, 0, ts>>>(P, B, S);
+                e = cudaGetLastError();
+            }
         }
     }
     if (e != cudaSuccess || which == 3) return e;

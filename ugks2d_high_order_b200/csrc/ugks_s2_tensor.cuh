@@ -1,0 +1,231 @@
+// ugks_s2_tensor.cuh -- the discrete closure and make_mke on tensor-product velocity tables.
+//
+// A structured velocity table (k = i + j Nu, u depending on i alone, v on j alone, weight = wx_i wy_j) makes
+// the closure Maxwellian a product, exp(-cx^2 / T) exp(-cy^2 / T), so every velocity sum of it times a
+// polynomial is a combination of products of 1-D sums: about 2 (Nu + Nv) terms and 2 exponential rows instead of
+// Nu Nv terms with one exponential each.  The sums are taken about the Maxwellian's (or the state's) mean,
+// so no term cancels against another of larger size.  Eight lanes own one node (four nodes a warp): each
+// lane takes every eighth abscissa of both axes, the sums are joined by a butterfly, and the node's scalar
+// logic runs on the group's lanes alike, except where several right-hand sides of one 4x4 system are
+// wanted: there each lane solves its own.
+#pragma once
+#include "ugks_s2_math.cuh"
+
+namespace ugks {
+namespace {
+
+constexpr int kTG = 8;   // lanes per node
+
+// xor-butterfly sums over the node's lanes: every lane returns the same totals
+template <int N>
+__device__ __forceinline__ void t_sum(double* v) {
+#pragma unroll
+    for (int o = kTG / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int m = 0; m < N; ++m) v[m] += __shfl_xor_sync(0xffffffffu, v[m], o);
+}
+__device__ __forceinline__ double t_min(double v) {
+#pragma unroll
+    for (int o = kTG / 2; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+// lane `src` of the node's group
+__device__ __forceinline__ double t_get(double v, int src) {
+    return __shfl_sync(0xffffffffu, v, ((threadIdx.x & 31) & ~(kTG - 1)) + src);
+}
+
+// this lane's part of the 1-D sums s[a] = sum_i w_i c_i^a exp(-(x_i - mean)^2 itw), c_i = x_i - center, over an
+// axis of the table (LoBuffers::tab: padded to 64 abscissae with weight 0).  R >= abscissae / 8.
+template <int R, int N>
+__device__ __forceinline__ void t_axis(const double* __restrict__ pos, const double* __restrict__ wt, double mean,
+                                       double itw, double center, double* s, double& emin) {
+    const int gl = threadIdx.x & (kTG - 1);
+#pragma unroll
+    for (int a = 0; a < N; ++a) s[a] = 0.0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const double x = __ldg(pos + gl + kTG * r), d = x - mean, c = x - center;
+        const double e = exp(-(d * d) * itw);
+        emin = fmin(emin, e);
+        double t = __ldg(wt + gl + kTG * r) * e;
+        s[0] += t;
+#pragma unroll
+        for (int a = 1; a < N; ++a) { t = t * c; s[a] += t; }
+    }
+}
+
+struct TClosure {
+    double th[4];   // converged (rho, u, v, T_native)
+    double res;     // scaled residual of the moments at th (make_mke's gate)
+    double* jac;    // [16] moment Jacobian at th, row-major, in the group's slice of shared memory
+};
+
+// solve_q_first (mod_CorrectedWF2DClosure.f90:331-426) for the target moments w: the accept / backtrack / stop
+// logic of w_closure on the 1-D sums.  Every lane of the warp calls it; a group whose `act` is false
+// (no node) or whose iteration has ended idles through the others' evaluations.
+template <int R>
+__device__ bool t_closure(const LoParams& P, const LoBuffers& B, const double w[4], bool act, TClosure& C) {
+    const int ck = P.ck;
+    const bool lead = (threadIdx.x & (kTG - 1)) == 0;
+    double trial[4];
+    bool done = !act, ok = false;
+    {   // primitive_from_conserved_2d (mod_CorrectedWF2DEquilibrium.f90:25-41)
+        const double u = w[1] / w[0], v = w[2] / w[0];
+        const double kin = 0.5 * (u * u + v * v), ein = w[3] / w[0] - kin;
+        const double temp = 4.0 * ein / (double)(ck + 2);
+        if (!(isfinite(w[0]) && isfinite(w[1]) && isfinite(w[2]) && isfinite(w[3]) && w[0] > 0.0 && isfinite(u) &&
+              isfinite(v) && isfinite(temp) && temp > 0.0))
+            done = true;
+        trial[0] = done ? 1.0 : w[0]; trial[1] = done ? 0.0 : u; trial[2] = done ? 0.0 : v; trial[3] = done ? 1.0 : temp;
+    }
+    WClosure Cw;   // th and the Jacobian slice w_newton_next works on
+    Cw.jac = C.jac;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) Cw.th[m] = trial[m];
+    double res[4] = {0.0, 0.0, 0.0, 0.0}, step[4] = {0.0, 0.0, 0.0, 0.0}, alpha = 1.0, norm = 0.0;
+    int iter = 0;
+    bool first = true;
+    for (int guard = 0; guard < 1024; ++guard) {
+        if (__all_sync(0xffffffffu, done)) break;
+        double s[10], ex = INFINITY, ey = INFINITY;   // A_a = sum wx cx^a e_x (0..4), then B_b
+        const S2Th t = s2_th(trial, ck);
+        t_axis<R, 5>(B.tab, B.tab + 64, t.u, t.itw, t.u, s, ex);
+        t_axis<R, 5>(B.tab + 128, B.tab + 192, t.v, t.itw, t.v, s + 5, ey);
+        t_sum<10>(s);
+        ex = t_min(ex);
+        ey = t_min(ey);
+        const double *A = s, *Bq = s + 5;
+        auto S = [&](int a, int b) { return t.pref * A[a] * Bq[b]; };
+        const double s00 = S(0, 0), s10 = S(1, 0), s01 = S(0, 1), s11 = S(1, 1), s20 = S(2, 0), s02 = S(0, 2);
+        const double c20 = s20 + s02;                          // sums of c^2, c^2 cx, c^2 cy, c^4
+        const double c30 = S(3, 0) + S(1, 2), c03 = S(2, 1) + S(0, 3);
+        const double c40 = S(4, 0) + 2.0 * S(2, 2) + S(0, 4);
+        const double u2 = 0.5 * (t.u * t.u + t.v * t.v), hb = 0.5 * t.ckh;
+        // moments (1, u, v, |c|^2 / 2 + b) of q f from f's sums with 1, cx, cy, c^2 and the b part
+        auto mom = [&](double f0, double fx, double fy, double f2, double fb, double* m, int st) {
+            m[0] = f0;
+            m[st] = t.u * f0 + fx;
+            m[2 * st] = t.v * f0 + fy;
+            m[3 * st] = u2 * f0 + t.u * fx + t.v * fy + 0.5 * f2 + hb * fb;
+        };
+        double J[16], q[4];
+        const double i1 = t.itw, i2 = t.itw * t.itw, d1 = 2.0 * t.itw;
+        mom(s00, s10, s01, c20, s00, q, 1);
+        mom(t.ir * s00, t.ir * s10, t.ir * s01, t.ir * c20, t.ir * s00, J, 4);
+        mom(d1 * s10, d1 * s20, d1 * s11, d1 * c30, d1 * s10, J + 1, 4);
+        mom(d1 * s01, d1 * s11, d1 * s02, d1 * c03, d1 * s01, J + 2, 4);
+        mom(i2 * c20 - i1 * s00, i2 * c30 - i1 * s10, i2 * c03 - i1 * s01, i2 * c40 - i1 * c20, i2 * c20, J + 3, 4);
+        bool fin = true;
+#pragma unroll
+        for (int m = 0; m < 16; ++m) fin = fin && isfinite(J[m]);
+        double nres[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) { fin = fin && isfinite(q[m]); nres[m] = q[m] - w[m]; }
+        // the Maxwellian is positive at every velocity (its smallest value is the product of the axes' smallest)
+        const double qmin = t.pref * ex * ey;
+        const bool pos = qmin > 0.0 && t.ckh * qmin > 0.0;
+        const double nn = fin ? s2_scaled(nres, w) : INFINITY;
+        const bool accept = !done && (first ? fin : (fin && (nn < norm || nn <= 5.0e-13)));
+        if (accept && lead)
+#pragma unroll
+            for (int m = 0; m < 16; ++m) C.jac[m] = J[m];
+        __syncwarp();
+        if (!done) {
+            int a;
+            if (accept) {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) { Cw.th[m] = trial[m]; res[m] = nres[m]; }
+                norm = nn;
+                iter = first ? 1 : iter + 1;
+                a = w_newton_next(true, Cw, res, norm, iter, step, alpha, trial);
+                if (a == W_DONE && !pos) a = W_FAIL;
+            } else if (first) {
+                a = W_FAIL;
+            } else {
+                alpha = 0.5 * alpha;
+                a = w_newton_next(false, Cw, res, norm, iter, step, alpha, trial);
+            }
+            first = false;
+            if (a != W_TRIAL) { done = true; ok = a == W_DONE; }
+        }
+        __syncwarp();
+    }
+    double rs = 0.0, sc = 1.0;   // make_mke's gate on the moments of M
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        C.th[m] = Cw.th[m];
+        rs = fmax(rs, fabs(res[m]));
+        sc = fmax(sc, fabs(w[m]));
+    }
+    C.res = rs / sc;
+    return ok;
+}
+
+// J x - rhs in the largest component (the moments left by a direction of the closure)
+__device__ __forceinline__ double t_left(const double* jac, const double x[4], const double rhs[4]) {
+    double mx = 0.0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        double s = -rhs[r];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) s = s + jac[r * 4 + a] * x[a];
+        mx = fmax(mx, fabs(s));
+    }
+    return mx;
+}
+
+// make_mke_prepared (mod_S2D1.f90:111-151) at the closure C of w: the primitive scalars and the closure
+// directions of the raw Shakhov terms, whose moments come from 1-D sums about the state's mean.  Lane 0
+// of the group solves for K_x, lane 1 (the axes exchanged) for K_y; lanes 2..4 solve for three further
+// right-hand sides extra[0..11] when given (the macro slopes of a face node) and return their own solution
+// in td.  Returns the gates: M's moments equal w, every direction's moments are met to 2e-12, all finite.
+template <int R>
+__device__ bool t_mke(const LoParams& P, const LoBuffers& B, const double w[4], const TClosure& C, WMke& M,
+                      const double* extra, double td[4]) {
+    const int ck = P.ck, gl = threadIdx.x & (kTG - 1);
+    double rho, th;
+    const bool pok = s2_primitive(w, ck, rho, M.ux, M.vy, th);
+    M.lam = 0.5 / th;
+    M.coeff = 0.8 * (1.0 - P.pr) * M.lam * M.lam / rho;
+    const S2Th t = s2_th(C.th, ck);
+    double s[12], em = INFINITY;
+    t_axis<R, 6>(B.tab, B.tab + 64, t.u, t.itw, M.ux, s, em);
+    t_axis<R, 6>(B.tab + 128, B.tab + 192, t.v, t.itw, M.vy, s + 6, em);
+    t_sum<12>(s);
+    const bool sw = gl & 1;   // the axis of K is the first of (N, O)
+    double N[6], O[6];
+#pragma unroll
+    for (int a = 0; a < 6; ++a) { N[a] = sw ? s[6 + a] : s[a]; O[a] = sw ? s[a] : s[6 + a]; }
+    const double un = sw ? M.vy : M.ux, uo = sw ? M.ux : M.vy, l2 = 2.0 * M.lam, pc = t.pref * M.coeff;
+    // f = cn (2 lam c^2 - 4): its sums with 1, cn, co, c^2; b adds (2 / ck) cn
+    const double s10 = N[1] * O[0];
+    const double m0 = l2 * (N[3] * O[0] + N[1] * O[2]) - 4.0 * s10;
+    const double mn = l2 * (N[4] * O[0] + N[2] * O[2]) - 4.0 * (N[2] * O[0]);
+    const double mo = l2 * (N[3] * O[1] + N[1] * O[3]) - 4.0 * (N[1] * O[1]);
+    const double m2 = l2 * (N[5] * O[0] + 2.0 * (N[3] * O[2]) + N[1] * O[4]) - 4.0 * (N[3] * O[0] + N[1] * O[2]);
+    const double cn = pc * (un * m0 + mn), co = pc * (uo * m0 + mo);
+    double rhs[4];
+    rhs[0] = pc * m0;
+    rhs[1] = sw ? co : cn;
+    rhs[2] = sw ? cn : co;
+    rhs[3] = pc * (0.5 * (un * un + uo * uo) * m0 + un * mn + uo * mo + 0.5 * m2 +
+                   0.5 * t.ckh * (m0 + 2.0 / (double)ck * s10));
+    const bool mine = extra != nullptr && gl >= 2 && gl < 5;
+    if (mine)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) rhs[m] = extra[(gl - 2) * 4 + m];
+    bool ok = s2_solve4(C.jac, rhs, td);
+    double sc = 1.0;
+    if (mine)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) sc = fmax(sc, fabs(rhs[m]));
+    ok = ok && t_left(C.jac, td, rhs) / sc <= 2.0e-12;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) { M.tdx[m] = t_get(td[m], 0); M.tdy[m] = t_get(td[m], 1); }
+    const unsigned grp = 0xffu << ((threadIdx.x & 31) & ~(kTG - 1));
+    ok = (__ballot_sync(0xffffffffu, !ok) & grp) == 0u;
+    return pok && ok && C.res <= 2.0e-12;
+}
+
+}  // namespace
+}  // namespace ugks
