@@ -655,6 +655,307 @@ __global__ void __launch_bounds__(256, 3) k_s2_face_flux(LoParams P, LoBuffers B
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// interior faces on a tensor-product velocity table, in three kernels:
+//   k_s2_face_moments : one warp a node, the sums of the upwind face values that W0 and q0 need, taken
+//                       about the lower cell's velocity -> fscal[1..9] (the only pass over the velocities
+//                       that the node's scalars need; bound by the face cache's values, 16 KB a node at 32^2)
+//   k_s2_face_nodes_t : eight lanes a node, W0's closure, make_mke, q0, the directions and Mt by 1-D sums
+//                       -> the node scalars of k_s2_face_nodes
+//   k_s2_face_flux_t  : one CTA a face, its three nodes' micro fluxes and their Gauss sum -> the face arrays
+// Against k_s2_face_nodes, k_s2_face_flux and k_s2_combine, which other tables and the wall variants' coefficient
+// outputs keep, the S2CN2 step at 8x64x32^2 went from 0.704 to 0.565 ms and the 16-instance batch from
+// 14.0 to 10.6 ms a step.
+__global__ void __launch_bounds__(256) k_s2_face_moments(LoParams P, LoBuffers B, S2Buffers SB) {
+    if (eval_cached(B)) return;
+    const int nv = P.nvel, nx = P.nx, ny = P.ny, lane = threadIdx.x & 31;
+    const int nfx = nx * ny, nf = nfx + nx * (ny - 1);
+    const int wid = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (wid >= nf * 3) return;
+    const int fi = wid / 3, g = wid % 3;
+    const int axis = fi < nfx ? 0 : 1, cl = axis == 0 ? fi : fi - nfx;
+    const int i = cl % nx, j = cl / nx;
+    const int cr = axis == 0 ? j * nx + (i + 1) % nx : (j + 1) * nx + i;
+    const double iw = 1.0 / B.W[cl * 4], ur = B.W[cl * 4 + 1] * iw, vr = B.W[cl * 4 + 2] * iw;
+    const double* rl = SB.rec + rec_cell(cl, axis, 0, g, nv);
+    const double* rr = SB.rec + rec_cell(cr, axis, 0, g, nv);
+    double a[9];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) a[m] = 0.0;
+#pragma unroll 4
+    for (int k = lane; k < nv; k += 32) {
+        const double uk = B.u[k], vk = B.v[k], wk = B.w[k];
+        const double* rc = ((axis == 0 ? uk : vk) >= 0.0 ? rl : rr) + k;
+        const double h = wk * rc[0], b = wk * rc[(size_t)3 * nv];
+        const double cx = uk - ur, cy = vk - vr, xx = cx * cx, yy = cy * cy, e = (xx + yy) * h + b;
+        a[0] += h;
+        a[1] += cx * h;
+        a[2] += cy * h;
+        a[3] += xx * h;
+        a[4] += cx * cy * h;
+        a[5] += yy * h;
+        a[6] += b;
+        a[7] += cx * e;
+        a[8] += cy * e;
+    }
+    const double t = warp_halving<9, false>(a);   // the total of sum lane / 2
+    if ((lane & 1) == 0 && lane < 18) SB.fscal[(size_t)wid * kS2FScal + 1 + (lane >> 1)] = t;
+}
+
+template <int R>
+__global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffers B, S2Buffers SB) {
+    if (eval_cached(B)) return;
+    __shared__ double s_jac[128 / kTG][17];
+    const int nx = P.nx, ny = P.ny, ck = P.ck, gl = threadIdx.x & (kTG - 1);
+    const int nfx = nx * ny, nn = (nfx + nx * (ny - 1)) * 3;
+    const int id = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kTG), node = min(id, nn - 1);
+    const int fi = node / 3, axis = fi < nfx ? 0 : 1, cl = axis == 0 ? fi : fi - nfx;
+    const double dt = B.dt[0];
+    const double* mac = SB.mac + (size_t)node * 12;   // [nl | nr | t][component] of this node
+    double* o = SB.fscal + (size_t)node * kS2FScal;
+    // W0: the moments of the upwind face values, from the sums about the lower cell's velocity (ur, vr)
+    const double iw = 1.0 / B.W[cl * 4], ur = B.W[cl * 4 + 1] * iw, vr = B.W[cl * 4 + 2] * iw;
+    double f[9];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) f[m] = o[1 + m];
+    const double w0[4] = {f[0], ur * f[0] + f[1], vr * f[0] + f[2],
+                          0.5 * (ur * ur + vr * vr) * f[0] + ur * f[1] + vr * f[2] + 0.5 * (f[3] + f[5] + f[6])};
+    TClosure C;
+    C.jac = s_jac[threadIdx.x / kTG];
+    WMke M;
+    double td[4];
+    bool ok = t_closure<R>(P, B, w0, id < nn, C);
+    ok = t_mke<R>(P, B, w0, C, M, mac, td) && ok;
+    // q0 = heat(w0, f0 - analytic Maxwellian of w0) about (ux, vy): f0's part shifted from (ur, vr)
+    double q0x, q0y;
+    {
+        const double temp = 4.0 * (w0[3] / w0[0] - 0.5 * (M.ux * M.ux + M.vy * M.vy)) / (double)(ck + 2), lamn = 1.0 / temp;
+        const double dx = M.ux - ur, dy = M.vy - vr, d2 = dx * dx + dy * dy, e2 = f[3] + f[5], dp = dx * f[1] + dy * f[2];
+        const double hx = 0.5 * (f[7] - dx * (e2 + f[6]) + d2 * f[1] - d2 * dx * f[0]) - (dx * f[3] + dy * f[4]) + dx * dp;
+        const double hy = 0.5 * (f[8] - dy * (e2 + f[6]) + d2 * f[2] - d2 * dy * f[0]) - (dx * f[4] + dy * f[5]) + dy * dp;
+        double s[8], em = INFINITY;
+        t_axis<R, 4>(B.tab, B.tab + 64, M.ux, lamn, M.ux, s, em);
+        t_axis<R, 4>(B.tab + 128, B.tab + 192, M.vy, lamn, M.vy, s + 4, em);
+        t_sum<8>(s);
+        const double pr = 0.5 * w0[0] * lamn / kPi, cb = 0.5 * (double)ck * temp;
+        q0x = hx - pr * (s[3] * s[4] + s[1] * s[6] + cb * s[1] * s[4]);
+        q0y = hy - pr * (s[7] * s[0] + s[5] * s[2] + cb * s[5] * s[0]);
+    }
+    // wt = -moments of vn (left ? dl : dr) + vt dt: lane 2 sums the left half of the normal axis with the left
+    // direction, lane 3 the right half with the right one, lane 4 the other axis with the tangential one
+    const S2Th t = s2_th(C.th, ck);
+    double wt[4], tdm[4];
+    {
+        const double* tn = B.tab + (axis == 0 ? 0 : 128);
+        const double* to = B.tab + (axis == 0 ? 128 : 0);
+        const double un0 = axis == 0 ? t.u : t.v, uo0 = axis == 0 ? t.v : t.u;
+        double s[18], em = INFINITY;   // normal axis: vn >= 0, vn < 0; other axis
+#pragma unroll
+        for (int a = 0; a < 12; ++a) s[a] = 0.0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const double x = __ldg(tn + gl + kTG * r), d = x - un0;
+            double p = __ldg(tn + 64 + gl + kTG * r) * exp(-(d * d) * t.itw);
+            double pl = x >= 0.0 ? p : 0.0, pr = x >= 0.0 ? 0.0 : p;
+#pragma unroll
+            for (int a = 0; a < 6; ++a) { s[a] += pl; s[6 + a] += pr; pl = pl * d; pr = pr * d; }
+        }
+        t_axis<R, 6>(to, to + 64, uo0, t.itw, uo0, s + 12, em);
+        t_sum<18>(s);
+        double N[6], O[5];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) N[a] = gl == 4 ? s[12 + a] : (gl == 3 ? s[6 + a] : s[a]);
+#pragma unroll
+        for (int a = 0; a < 5; ++a) O[a] = gl == 4 ? s[a] + s[6 + a] : s[12 + a];
+        const bool nisx = (axis == 0) != (gl == 4);   // this lane's normal component is x
+        const double un = gl == 4 ? uo0 : un0, uo = gl == 4 ? un0 : uo0;
+        const double d0 = td[0] * t.ir - td[3] * t.itw, d3 = td[3] * t.itw * t.itw, db = td[3] * t.itw;
+        const double dn = 2.0 * t.itw * (nisx ? td[1] : td[2]), dco = 2.0 * t.itw * (nisx ? td[2] : td[1]);
+        // f = (un + cn)(d0 + dn cn + do co + d3 c^2): its sums with 1, cn, co, c^2 by rows of equal cn power
+        const double p00 = un * d0, p10 = d0 + un * dn, p20 = dn + un * d3, p01 = un * dco, p02 = un * d3;
+        double F[4][3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            F[0][b] = p00 * O[b] + p01 * O[b + 1] + p02 * O[b + 2];
+            F[1][b] = p10 * O[b] + dco * O[b + 1] + d3 * O[b + 2];
+            F[2][b] = p20 * O[b];
+            F[3][b] = d3 * O[b];
+        }
+        double m0 = 0.0, mn = 0.0, mo = 0.0, m2 = 0.0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            m0 += N[a] * F[a][0];
+            mn += N[a + 1] * F[a][0];
+            mo += N[a] * F[a][1];
+            m2 += N[a + 2] * F[a][0] + N[a] * F[a][2];
+        }
+        const double mb = m0 + db * O[0] * (un * N[0] + N[1]);
+        const double cn = t.pref * (un * m0 + mn), co = t.pref * (uo * m0 + mo);
+        double c[4] = {t.pref * m0, nisx ? cn : co, nisx ? co : cn,
+                       t.pref * (0.5 * (un * un + uo * uo) * m0 + un * mn + uo * mo + 0.5 * m2 + 0.5 * t.ckh * mb)};
+#pragma unroll
+        for (int m = 0; m < 4; ++m) wt[m] = -(t_get(c[m], 2) + t_get(c[m], 3) + t_get(c[m], 4));
+        ok = s2_solve4(C.jac, wt, tdm) && ok;
+        double sc = 1.0;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) sc = fmax(sc, fabs(wt[m]));
+        ok = ok && t_left(C.jac, tdm, wt) / sc <= 2.0e-12;
+    }
+    double tau = 0.0, mt[5];
+    ok = ok && s2_tau(P, w0, tau) && isfinite(q0x) && isfinite(q0y);
+    const double ex = exp(-dt / tau);   // Mt (mod_Evolution.f90:346-350)
+    mt[3] = tau * (1.0 - ex);
+    mt[4] = -tau * dt * ex + tau * mt[3];
+    mt[0] = dt - mt[3];
+    mt[1] = -tau * mt[0] + mt[4];
+    mt[2] = 0.5 * dt * dt - tau * mt[0];
+    if (id >= nn) return;
+    if (!ok) {
+        if (gl == 0) { o[0] = 0.0; set_status(B.status, ST_NONFINITE_FLUX); }
+        return;
+    }
+    if (gl == 0) {
+        o[0] = 1.0;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            o[1 + m] = C.th[m]; o[5 + m] = M.tdx[m]; o[9 + m] = M.tdy[m]; o[31 + m] = tdm[m]; o[40 + m] = wt[m];
+        }
+        o[13] = M.ux; o[14] = M.vy; o[15] = M.lam; o[16] = M.coeff; o[17] = q0x; o[18] = q0y;
+#pragma unroll
+        for (int m = 0; m < 5; ++m) o[35 + m] = mt[m];
+        o[60] = tau;
+    } else if (gl >= 2 && gl < 5) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) o[19 + (gl - 2) * 4 + m] = td[m];
+    }
+    o[44 + gl] = C.jac[gl];
+    o[52 + gl] = C.jac[8 + gl];
+}
+
+// The flux of a face: at each node, per velocity, the Maxwellian (a product of two rows of exponentials in
+// shared memory) times a cubic in the velocity, whose coefficients join s0, the slope and the time directions
+// with their Mt, plus the face values' part (ugks_node, mod_S2D1.f90:486-507).  The three nodes' Gauss sum
+// goes straight to the face arrays and its velocity moments are the face's macro flux, so no node flux is
+// stored.  Bound by the face cache: 18 values a (face, velocity), 151 MB at 8x64x32^2.
+struct S2FluxC {
+    double u, v, ux, vy, ckh, l2, kq, kb, qx, qy, mt0, mt3, mt4;   // means, ck T / 2, 2 lam, mt0 coeff, kq 2 / ck, q0, Mt
+    double e[5], t[5], d[2][5];   // polynomials 1, cx, cy, c^2 and b part: mt2 dm - mt0 K dirs; mt1 tangential; mt1 left, right
+};
+__global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers B, S2Buffers SB) {
+    if (eval_cached(B)) return;
+    __shared__ double ex[3][64], ey[3][64];
+    __shared__ S2FluxC sc[3];
+    __shared__ double red[8 * 8], rout[kRedSlots];
+    const int nv = P.nvel, nu = P.tnu, nw = P.tnv, nx = P.nx, ny = P.ny, nfx = nx * ny, tid = threadIdx.x;
+    const int fi = blockIdx.x, axis = fi < nfx ? 0 : 1, cl = axis == 0 ? fi : fi - nfx, i = cl % nx, j = cl / nx;
+    const int cr = axis == 0 ? j * nx + (i + 1) % nx : (j + 1) * nx + i;
+    const double* fs = SB.fscal + (size_t)fi * 3 * kS2FScal;
+    if (fs[0] == 0.0 || fs[kS2FScal] == 0.0 || fs[2 * kS2FScal] == 0.0) return;   // a failed node (status set there)
+    if (tid < 3) {
+        const double* o = fs + tid * kS2FScal;
+        const double th[4] = {o[1], o[2], o[3], o[4]};
+        const S2Th t = s2_th(th, P.ck);
+        S2FluxC& c = sc[tid];
+        c.u = t.u; c.v = t.v; c.ux = o[13]; c.vy = o[14]; c.ckh = t.ckh; c.l2 = 2.0 * o[15];
+        c.qx = o[17]; c.qy = o[18]; c.mt0 = o[35]; c.mt3 = o[38]; c.mt4 = o[39];
+        c.kq = o[35] * o[16]; c.kb = c.kq * (2.0 / (double)P.ck);
+        auto poly = [&](const double td[4], double* p) {
+            p[0] = td[0] * t.ir - td[3] * t.itw;
+            p[1] = 2.0 * t.itw * td[1];
+            p[2] = 2.0 * t.itw * td[2];
+            p[3] = td[3] * (t.itw * t.itw);
+            p[4] = td[3] * t.itw;
+        };
+        double x[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) x[m] = o[37] * o[31 + m] - o[35] * (o[17] * o[5 + m] + o[18] * o[9 + m]);
+        poly(x, c.e);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) x[m] = o[36] * o[27 + m];
+        poly(x, c.t);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) x[m] = o[36] * o[19 + m];
+        poly(x, c.d[0]);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) x[m] = o[36] * o[23 + m];
+        poly(x, c.d[1]);
+    }
+    for (int q = tid; q < 3 * (nu + nw); q += blockDim.x) {
+        const int g = q / (nu + nw), a = q - g * (nu + nw);
+        const double* o = fs + g * kS2FScal + 1;
+        const double itw = 1.0 / o[3];
+        if (a < nu) {
+            const double d = B.tab[a] - o[1];
+            ex[g][a] = o[0] / (kPi * o[3]) * exp(-(d * d) * itw);
+        } else {
+            const double d = B.tab[128 + a - nu] - o[2];
+            ey[g][a - nu] = exp(-(d * d) * itw);
+        }
+    }
+    __syncthreads();
+    const double gw[3] = {5.0 / 18.0, 4.0 / 9.0, 5.0 / 18.0};
+    const double len = axis == 0 ? P.dy : P.dx;
+    const size_t out = axis == 0 ? (size_t)j * nx + (i + 1) % nx : (size_t)(j + 1) * nx + i;
+    double* Fh = (axis == 0 ? B.fxh : B.fyh) + out * nv;
+    double* Fb = (axis == 0 ? B.fxb : B.fyb) + out * nv;
+    double* Fw = (axis == 0 ? B.fxw : B.fyw) + out * 4;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    int bad = 0;
+    for (int k0 = tid; k0 < nv; k0 += 4 * (int)blockDim.x) {
+        double fh[4], fb[4], uk[4], vk[4];
+        int iu[4], iv[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int k = min(k0 + r * (int)blockDim.x, nv - 1);
+            iv[r] = k / nu;
+            iu[r] = k - iv[r] * nu;
+            uk[r] = B.tab[iu[r]];
+            vk[r] = B.tab[128 + iv[r]];
+            fh[r] = fb[r] = 0.0;
+        }
+#pragma unroll 1
+        for (int g = 0; g < 3; ++g) {
+            const S2FluxC& c = sc[g];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const double vn = axis == 0 ? uk[r] : vk[r], vt = axis == 0 ? vk[r] : uk[r];
+                const bool left = vn >= 0.0;
+                const double* rc = SB.rec + rec_cell(left ? cl : cr, axis, 0, g, nv) + min(k0 + r * (int)blockDim.x, nv - 1);
+                const double f0h = rc[0], f0b = rc[(size_t)3 * nv], nh = rc[(size_t)6 * nv], th = rc[(size_t)9 * nv];
+                const double nb = rc[(size_t)12 * nv], tb = rc[(size_t)15 * nv];
+                const double* d = c.d[left ? 0 : 1];
+                const double q = ex[g][iu[r]] * ey[g][iv[r]];
+                const double cx = uk[r] - c.u, cy = vk[r] - c.v, px = uk[r] - c.ux, py = vk[r] - c.vy;
+                const double c2 = cx * cx + cy * cy, qd = c.qx * px + c.qy * py;
+                const double pe = c.e[0] + c.e[1] * cx + c.e[2] * cy + c.e[3] * c2;
+                const double pd = d[0] + d[1] * cx + d[2] * cy + d[3] * c2;
+                const double pt = c.t[0] + c.t[1] * cx + c.t[2] * cy + c.t[3] * c2;
+                const double vh = c.mt0 + c.kq * qd * (c.l2 * (px * px + py * py) - 4.0) + pe + vn * pd + vt * pt;
+                const double vb = vh + c.kb * qd + c.e[4] + vn * d[4] + vt * c.t[4];
+                const double wn = gw[g] * vn;
+                fh[r] += wn * (q * vh + c.mt3 * f0h - c.mt4 * (vn * nh + vt * th));
+                fb[r] += wn * (c.ckh * q * vb + c.mt3 * f0b - c.mt4 * (vn * nb + vt * tb));
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int k = k0 + r * (int)blockDim.x;
+            if (k < nv) {
+                fh[r] = fh[r] * len;
+                fb[r] = fb[r] * len;
+                Fh[k] = fh[r];
+                Fb[k] = fb[r];
+                moment_add(B.w[k], uk[r], vk[r], fh[r], fb[r], acc);
+                if (!(isfinite(fh[r]) && isfinite(fb[r]))) bad = 1;
+            }
+        }
+    }
+    block_reduce_smem<4, 0>(acc, red, rout);
+    bad = __syncthreads_or(bad);
+    if (tid < 4) Fw[tid] = rout[tid];
+    if (tid == 0 && bad) set_status(B.status, ST_NONFINITE_FLUX);
+}
+
 // wall face nodes (s2w2_wall_node, mod_S2MultiscaleWall.f90:45-184): one warp per (wall face,
 // Gauss node); bottom faces of row 0, then top faces of row ny-1.  Node fluxes go to the node
 // buffers after the interior faces.
@@ -1004,7 +1305,19 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
         }
     }
     if (e == cudaSuccess) e = cudaEventRecord(join, s2);
-    if (e == cudaSuccess) {
+    // a tensor table's faces: the fused flux, unless a wall variant wants the nodes' fluxes and coefficients
+    const bool tensor = P.tnu > 0, fused = tensor && S.coef == nullptr;
+    if (e == cudaSuccess && tensor) {
+        const unsigned g = (unsigned)((nf * 3 * kTG + 127) / 128);
+        const int n = P.tnu > P.tnv ? P.tnu : P.tnv;
+        k_s2_face_moments<<<warps((long long)nf * 3), 256, 0, s>>>(P, B, S);
+        if (n <= 24) k_s2_face_nodes_t<3><<<g, 128, 0, s>>>(P, B, S);
+        else if (n <= 32) k_s2_face_nodes_t<4><<<g, 128, 0, s>>>(P, B, S);
+        else if (n <= 48) k_s2_face_nodes_t<6><<<g, 128, 0, s>>>(P, B, S);
+        else k_s2_face_nodes_t<8><<<g, 128, 0, s>>>(P, B, S);
+        if (fused) k_s2_face_flux_t<<<(unsigned)nf, std::min(256, (nv + 127) / 128 * 32), 0, s>>>(P, B, S);
+        e = cudaGetLastError();
+    } else if (e == cudaSuccess) {
         if (S.concurrent) {
             const int qb = qrec_bytes(S, nv, 256, kQRecCap256x2);
             k_s2_face_nodes<256, 2><<<warps((long long)nf * 3), 256, qb, s>>>(P, B, S, qb > 0);
@@ -1014,13 +1327,13 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
         }
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && !fused) {
         if (nv <= 1024) k_s2_face_flux<4><<<(unsigned)(nf * 3), 256, 0, s>>>(P, B, S);
         else k_s2_face_flux<10><<<(unsigned)(nf * 3), 256, 0, s>>>(P, B, S);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join, 0);
-    if (e == cudaSuccess) e = launch_s2_combine(P, B, S, 0, nf + 2 * nx, s);
+    if (e == cudaSuccess) e = launch_s2_combine(P, B, S, fused ? nf : 0, fused ? 2 * nx : nf + 2 * nx, s);
     return e;
 }
 
