@@ -1149,6 +1149,201 @@ __global__ void __launch_bounds__(256, 2) k_s2_wall_nodes(LoParams P, LoBuffers 
     if (!ok && lane == 0) set_status(B.status, ST_NONFINITE_FLUX);
 }
 
+// The multiscale wall on a tensor-product velocity table: one CTA per wall face, its three Gauss nodes at once.
+// The nodes share the wall state, so one closure (warp 0, by 1-D sums) serves them while the other warps
+// sum the incident state's moments; three lanes then form the nodes' slopes, and each velocity's
+// incident flux is taken once, kept in registers until the wall density is known, and summed over the nodes
+// into the face arrays (no node flux is stored; nodew keeps the nodes' macro fluxes).  16 CTAs at nx = 8, beside
+// the interior faces on the side stream: bound by the chain closure -> slopes -> two block reductions (54 us alone,
+// 136 us for k_s2_wall_nodes, one warp a node).  S2CN2 step 8x64x32^2 527 -> 500 us, 7x21x20^2 166 -> 138 us,
+// HighOrderImplicit pseudo-step 701 -> 644 us; the batch, whose other instances hid it, 9.18 -> 9.24 ms.
+struct S2WallC {
+    double n[4], t[4], m[4], hx, hy;   // normal, tangential, time slopes (half of the energy slope last); heat of the incident state
+};
+template <int VPT, int NT>
+__global__ void __launch_bounds__(NT) k_s2_walls_t(LoParams P, LoBuffers B, S2Buffers SB, int rows) {
+    if (eval_cached(B)) return;
+    __shared__ double red[(NT / 32) * 32], rout[kRedSlots];
+    __shared__ double ex[64], ey[64], s_jac[4][17], s_th[4];
+    __shared__ S2WallC sc[3];
+    __shared__ double s_mt[5];
+    __shared__ int s_ok;
+    const int nv = P.nvel, nu = P.tnu, nw = P.tnv, nx = P.nx, ny = P.ny, ck = P.ck, tid = threadIdx.x;
+    const int wf = blockIdx.x, top = wf >= nx ? 1 : 0, i = wf - top * nx, cc = top ? (ny - 1) * nx + i : i;
+    const double side = top ? 1.0 : -1.0, ux = P.wall_ux[top], theta = 0.5 / P.wall_lam[top], dt = B.dt[0];
+    const double* wcell = B.W + cc * 4;
+    const double pp = (2.0 / (double)(ck + 2)) * (wcell[3] - 0.5 * (wcell[1] * wcell[1] + wcell[2] * wcell[2]) / wcell[0]);
+    const double lambda = 0.5 / theta, rho = pp / theta;
+    const double* rec = SB.rec + rec_wall(nx, ny, top, i, 0, 0, nv);   // [field][node][nvel]
+    auto at = [&](int field, int g, int k) { return rec[((size_t)field * 3 + g) * nv + k]; };
+    if (tid < 32) {   // wall_equilibrium: the discrete closure of the wall state
+        const double wwall[4] = {rho, rho * ux, 0.0, rho * ((double)(ck + 2) * theta / 2.0 + ux * ux / 2.0)};
+        TClosure C;
+        C.jac = s_jac[tid / kTG];
+        bool ok;
+        switch (rows) {
+            case 3: ok = t_closure<3>(P, B, wwall, true, C); break;
+            case 4: ok = t_closure<4>(P, B, wwall, true, C); break;
+            case 6: ok = t_closure<6>(P, B, wwall, true, C); break;
+            default: ok = t_closure<8>(P, B, wwall, true, C); break;
+        }
+        if (tid == 0) {
+            s_ok = ok && pp > 0.0 && isfinite(pp);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) s_th[m] = C.th[m];
+        }
+    } else {   // the tangential slope's moments and the heat of the incident state, per node
+        double a[18];
+#pragma unroll
+        for (int m = 0; m < 18; ++m) a[m] = 0.0;
+        for (int k = tid - 32; k < nv; k += NT - 32) {
+            const double wk = B.w[k], vn = B.v[k], vt = -B.u[k], v2 = vn * vn + vt * vt, vt2 = vt + ux, w2 = vn * vn + vt2 * vt2;
+#pragma unroll
+            for (int g = 0; g < 3; ++g) {
+                const double ht = wk * at(3, g, k), q = 0.5 * wk * (w2 * at(0, g, k) + at(1, g, k));
+                a[6 * g] -= ht;
+                a[6 * g + 1] -= vn * ht;
+                a[6 * g + 2] -= vt * ht;
+                a[6 * g + 3] -= 0.5 * (v2 * ht + wk * at(5, g, k));
+                a[6 * g + 4] += vn * q;
+                a[6 * g + 5] += vt2 * q;
+            }
+        }
+        red[(tid >> 5) * 32 + (tid & 31)] = warp_halving<18, false>(a);   // lane m: the warp's total of sum m
+    }
+    __syncthreads();
+    if (tid < 3) {   // the slopes of node tid and the time coefficients
+        const double prim_g[4] = {rho, 0.0, -ux, lambda};
+        const double wc[4] = {wcell[0], wcell[2], -wcell[1], wcell[3]};
+        const double wg[4] = {rho, 0.0, -rho * ux, rho * ((double)(ck + 2) / (4.0 * lambda) + 0.5 * ux * ux)};
+        double a[6], sw[4], an[4], atn[4], am[4], Mu[7], Mv[6], Mxi[3], m1[4], m2[4], mt[5], tau = 1.0;
+        for (int m = 0; m < 6; ++m) {
+            a[m] = 0.0;
+            for (int w = 1; w < NT / 32; ++w) a[m] += red[w * 32 + 6 * tid + m];
+        }
+        for (int m = 0; m < 4; ++m) sw[m] = (wg[m] - wc[m]) / (side * 0.5 * P.dy);
+        s2w_micro_slope(ck, prim_g, sw, an);
+        s2w_micro_slope(ck, prim_g, a, atn);
+        s2w_moments(ck, prim_g, Mu, Mv, Mxi);
+        s2w_auvxi(an, Mu, Mv, Mxi, 1, 0, m1);
+        s2w_auvxi(atn, Mu, Mv, Mxi, 0, 1, m2);
+        for (int m = 0; m < 4; ++m) sw[m] = -rho * (m1[m] + m2[m]);
+        s2w_micro_slope(ck, prim_g, sw, am);
+        const double wgg[4] = {wg[0], -wg[2], wg[1], wg[3]};
+        const bool ok = s2_tau(P, wgg, tau);
+        s2w_time_coeffs(dt, tau, mt);
+        S2WallC& c = sc[tid];
+        for (int m = 0; m < 4; ++m) { const double f = m < 3 ? 1.0 : 0.5; c.n[m] = f * an[m]; c.t[m] = f * atn[m]; c.m[m] = f * am[m]; }
+        c.hx = a[4];
+        c.hy = a[5];
+        if (tid == 0) {
+            for (int m = 0; m < 5; ++m) s_mt[m] = mt[m];
+            if (!ok) s_ok = 0;
+        }
+    }
+    const S2Th t = s2_th(s_th, ck);
+    for (int q = tid - 32; q >= 0 && q < nu + nw; q += NT - 32) {
+        const double d = q < nu ? B.tab[q] - t.u : B.tab[128 + q - nu] - t.v;
+        const double e = exp(-(d * d) * t.itw);
+        if (q < nu) ex[q] = t.pref * e;
+        else ey[q - nu] = e;
+    }
+    __syncthreads();
+    if (!s_ok) {
+        if (tid == 0) set_status(B.status, ST_NONFINITE_FLUX);
+        return;
+    }
+    const double coeff = P.pr != 1.0 ? 0.8 * (1.0 - P.pr) * lambda * lambda / rho : 0.0;
+    const double mxi2 = (double)ck * ((double)ck + 2.0) / (4.0 * (lambda * lambda)), c2ck = 2.0 / (double)ck, irho = 1.0 / rho;
+    const double mt0 = s_mt[0], mt1 = s_mt[1], mt2 = s_mt[2], mt3 = s_mt[3], mt4 = s_mt[4];
+    double fh[3][VPT], fb[3][VPT], acc[12];   // toward the wall: v times the incident flux; away: dt v times the unit wall Maxwellian
+#pragma unroll
+    for (int m = 0; m < 6; ++m) acc[m] = 0.0;
+#pragma unroll
+    for (int r = 0; r < VPT; ++r) {
+        const Slot s = slot(r, nv);
+        const int k = s.kk, jv = k / nu;
+        const double u = B.u[k], v = B.v[k], wk = s.ok ? B.w[k] : 0.0, mh = ex[k - jv * nu] * ey[jv], mb = t.ckh * mh;
+        const bool toward = side * v > 0.0;
+        const double vn = v, vt = -u, v2 = vn * vn + vt * vt, vt2 = vt + ux, sh = 2.0 * lambda * (vn * vn + vt2 * vt2) - 4.0;
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+            const S2WallC& c = sc[g];
+            const double qd = coeff * (vn * c.hx + vt2 * c.hy);
+            const double ln = c.n[0] + c.n[1] * vn + c.n[2] * vt + c.n[3] * v2, lt = c.t[0] + c.t[1] * vn + c.t[2] * vt + c.t[3] * v2;
+            const double lm = c.m[0] + c.m[1] * vn + c.m[2] * vt + c.m[3] * v2;
+            const double L = mt1 * (vn * ln + vt * lt) + mt2 * lm, E = mt1 * (vn * c.n[3] + vt * c.t[3]) + mt2 * c.m[3];
+            const double gh = mh * (mt0 * (1.0 + qd * sh) + L + t.ckh * E) + mt3 * at(0, g, k) - mt4 * (vn * at(2, g, k) + u * at(3, g, k));
+            const double gb = mh * (t.ckh * (mt0 * (1.0 + qd * (sh + c2ck)) + L) + mxi2 * E) + mt3 * at(1, g, k) -
+                              mt4 * (vn * at(4, g, k) + u * at(5, g, k));
+            fh[g][r] = toward ? v * gh : dt * v * (mh * irho);
+            fb[g][r] = toward ? v * gb : dt * v * (mb * irho);
+            acc[2 * g] += toward ? wk * fh[g][r] : 0.0;
+            acc[2 * g + 1] += toward ? 0.0 : wk * fh[g][r];
+        }
+    }
+    block_reduce<6, 0>(acc, red, rout);   // incidence and reflection of the nodes -> wall densities
+    double rw[3], inc[3];
+    bool ok = true;
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+        inc[g] = acc[2 * g];
+        const double refl = acc[2 * g + 1];
+        rw[g] = -inc[g] / refl;
+        ok = ok && isfinite(refl) && fabs(refl) > DBL_MIN && isfinite(rw[g]) && rw[g] > 0.0;
+    }
+    const double gw[3] = {5.0 / 18.0, 4.0 / 9.0, 5.0 / 18.0};
+    const size_t o = top ? (size_t)ny * nx + i : (size_t)i;
+#pragma unroll
+    for (int m = 0; m < 12; ++m) acc[m] = 0.0;
+#pragma unroll
+    for (int r = 0; r < VPT; ++r) {
+        const Slot s = slot(r, nv);
+        const double u = B.u[s.kk], v = B.v[s.kk], wk = s.ok ? B.w[s.kk] : 0.0;
+        const bool toward = side * v > 0.0;
+        double ah = 0.0, ab = 0.0;
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+            const double f = toward ? 1.0 : rw[g], h = f * fh[g][r], b = f * fb[g][r];
+            moment_add(wk, u, v, h, b, acc + 4 * g);
+            ah += gw[g] * h;
+            ab += gw[g] * b;
+        }
+        if (s.ok) {
+            B.fyh[o * nv + s.k] = ah * P.dx;
+            B.fyb[o * nv + s.k] = ab * P.dx;
+            ok = ok && isfinite(ah) && isfinite(ab);
+        }
+    }
+    block_reduce_smem<12, 0>(acc, red, rout);
+    const int bad = __syncthreads_or(!ok);
+    if (tid == 0) {
+        bool fine = !bad;
+        double rate[4] = {0.0, 0.0, 0.0, 0.0};
+        const size_t node = (size_t)(nx * ny + nx * (ny - 1) + wf) * 3;
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+            const double mass = rout[4 * g];
+            fine = fine && isfinite(mass) && fabs(mass) <= 2.0e-12 * fmax(1.0, fabs(inc[g]));
+#pragma unroll
+            for (int m = 0; m < 4; ++m) { SB.nodew[(node + g) * 4 + m] = rout[4 * g + m]; rate[m] += gw[g] * rout[4 * g + m]; }
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            B.fyw[o * 4 + m] = rate[m] * P.dx;
+            if (SB.wall_raw != nullptr) SB.wall_raw[(size_t)wf * 4 + m] = rate[m];
+            rate[m] = rate[m] / dt;
+        }
+        // PublishWallDiagnostics (mod_S2NativeAdapter.f90:1075-1097): native frame n = +y, t = -x; the heat removes
+        // the moving wall's mechanical work
+        double* a = B.wall_aero + (size_t)wf * 3;
+        a[0] = rate[2];
+        a[1] = -rate[1];
+        a[2] = rate[3] - ux * rate[1];
+        if (!fine) set_status(B.status, ST_NONFINITE_FLUX);
+    }
+}
+
 // Gauss-weighted sum of the node fluxes of every face (interior, then the walls) times the face
 // length, into the face arrays ComputeResidual reads; the walls' macro fluxes also unscaled into
 // SB.wall_raw, and the walls' (pnn, pnt, qn) into B.wall_aero.  One thread per (face, velocity);
@@ -1290,6 +1485,8 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
         }
     }
     if (e != cudaSuccess || which == 3) return e;
+    // a tensor table's faces and walls: the fused fluxes, unless a wall variant wants the nodes' fluxes and coefficients
+    const bool tensor = P.tnu > 0, fused = tensor && S.coef == nullptr;
     const dim3 grid((unsigned)((nv + 31) / 32), (unsigned)nc);
     k_s2_recon1<<<grid, 128, 0, s>>>(P, B, S);
     e = cudaGetLastError();
@@ -1298,15 +1495,18 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s2, fork, 0);
     if (e == cudaSuccess) {
         if (P.s2_kinetic) e = launch_s2_w1_walls(P, B, S, s2);
-        else {
+        else if (fused) {
+            const int n = P.tnu > P.tnv ? P.tnu : P.tnv, rows = n <= 24 ? 3 : n <= 32 ? 4 : n <= 48 ? 6 : 8;
+            if (nv <= 1024) k_s2_walls_t<4, 256><<<2 * nx, 256, 0, s2>>>(P, B, S, rows);
+            else k_s2_walls_t<5, 512><<<2 * nx, 512, 0, s2>>>(P, B, S, rows);
+            e = cudaGetLastError();
+        } else {
             const int qb = qrec_bytes(S, nv, 256, kQRecCapWall);
             k_s2_wall_nodes<<<warps(2LL * nx * 3), 256, qb, s2>>>(P, B, S, qb > 0);
             e = cudaGetLastError();
         }
     }
     if (e == cudaSuccess) e = cudaEventRecord(join, s2);
-    // a tensor table's faces: the fused flux, unless a wall variant wants the nodes' fluxes and coefficients
-    const bool tensor = P.tnu > 0, fused = tensor && S.coef == nullptr;
     if (e == cudaSuccess && tensor) {
         const unsigned g = (unsigned)((nf * 3 * kTG + 127) / 128);
         const int n = P.tnu > P.tnv ? P.tnu : P.tnv;
@@ -1333,7 +1533,9 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join, 0);
-    if (e == cudaSuccess) e = launch_s2_combine(P, B, S, fused ? nf : 0, fused ? 2 * nx : nf + 2 * nx, s);
+    // the node fluxes that were stored: all faces', or a kinetic wall's alone
+    if (e == cudaSuccess && !fused) e = launch_s2_combine(P, B, S, 0, nf + 2 * nx, s);
+    else if (e == cudaSuccess && P.s2_kinetic) e = launch_s2_combine(P, B, S, nf, 2 * nx, s);
     return e;
 }
 
