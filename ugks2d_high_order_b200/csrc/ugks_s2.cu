@@ -49,104 +49,93 @@ __global__ void __launch_bounds__(128) k_s2_recon1(LoParams P, LoBuffers B, S2Bu
     const int cc = blockIdx.y, i = cc % nx, j = cc / nx;
     if (dir == 1 && s2_near_wall(j, ny)) return;   // walls use one-sided quartics instead
     const S2Field F{(f == 0 ? B.h : B.b) + k, nv, nx, ny};
-    double q[5];
-    S2Weno ww;
+    double q[5], fw[4], c[5];
 #pragma unroll
     for (int s = -2; s <= 2; ++s) q[s + 2] = dir == 0 ? F.at(i + s, j) : F.at(i, j + s);
-    const bool ok = s2_weno(q, ww);
+    const S2Diff d = s2_diff(q);
+    s2_weights(q, d, fw);
+    s2_power(q[2], d, fw, c);
     double* o = S.l1 + ((size_t)cc * 22 + f * 11 + (dir == 0 ? 0 : 7)) * nv + k;
-    double v0, d0, v1, d1;
-    s2_at(ww, S2_XM, v0, d0);
-    s2_at(ww, S2_XP, v1, d1);
+    const double e = c[0] + (0.25 * c[2] + 0.0625 * c[4]), odd = 0.5 * c[1] + 0.125 * c[3];
+    const double de = c[1] + 0.75 * c[3], dodd = c[2] + 0.5 * c[4];
     if (kok) {
-        o[0] = v0; o[(size_t)nv] = d0; o[2 * (size_t)nv] = v1; o[3 * (size_t)nv] = d1;
-        if (dir == 0)
+        o[0] = e - odd; o[(size_t)nv] = de - dodd; o[2 * (size_t)nv] = e + odd; o[3 * (size_t)nv] = de + dodd;
+        if (dir == 0) {
+            double v[3];
+            s2_gauss_values(c, v);
 #pragma unroll
-            for (int a = 0; a < 3; ++a) o[(size_t)(4 + a) * nv] = s2_at_v(ww, S2_G0 + a);
-        if (!ok) set_status(B.status, ST_NONFINITE_FLUX);
+            for (int a = 0; a < 3; ++a) o[(size_t)(4 + a) * nv] = v[a];
+        }
+        if (!(isfinite(e) && isfinite(odd) && isfinite(de) && isfinite(dodd))) set_status(B.status, ST_NONFINITE_FLUX);
     }
 }
 
 // k_s2_recon2, the second layer (tensor_velocity_tile, :723-792; reconstruct_wall_tile, :918-971) and
-// limit_cell_outputs (mod_S2D1.f90:315-345): CTA = 8 warps (field f = warp / 4, part p = warp % 4)
-// over 32 velocities of one cell.  Part p reconstructs face side p (x left, x right, y bottom, y top)
-// at its 3 Gauss nodes with value, normal and tangential derivative, and parts 0..2 also the volume
-// Gauss row p; the positivity factor theta is the minimum over the 8 warps (both fields, all face and
-// volume samples), then each warp writes its side's limited values.
-__global__ void __launch_bounds__(256, 3) k_s2_recon2(LoParams P, LoBuffers B, S2Buffers S) {
-    if (eval_cached(B)) return;
-    __shared__ double s_th[8][32];
+// limit_cell_outputs (mod_S2D1.f90:315-345).  A cell has four face sides (x left, x right, y bottom, y top) at 3 Gauss
+// nodes with value, normal and tangential derivative, and three volume Gauss rows, for h and b; the
+// positivity factor theta is the minimum over all their values.  The face cache keeps, per velocity, the sides it
+// leaves the cell through, so along each axis only that side needs its derivatives: the other side's
+// values enter theta alone.
+//
+// Cells away from the walls: a thread takes one field of one velocity through both axes and the three
+// rows and keeps the two leaving sides until theta is known; CTA = 8 warps, warp pairs (h, b) over 4 x 32 velocities.
+// Cells in the three rows next to a wall (one-sided quartics across y; the wall sides for every velocity): CTA = 8
+// warps (field f = warp / 4, side and row p = warp % 4) over 32 velocities.
+// Bound by FP64 arithmetic (about 1,700 operations a cell-velocity; all four sides in the tables' form took about
+// 3,100).  At 8x64x32^2 this kernel went from 220 to 146 us and k_s2_recon1 from 42 to 33 (ncu, cold), the S2CN2 step
+// from 500 to 427 us, 48^2 velocities from 1011 to 845 us, the 16-instance batch from 9.24 to 7.61 ms a step.
+__device__ __forceinline__ double s2_limit(double cand, double x, double mf) {
+    return x < 0.0 ? fmin(cand, (1.0 - 64.0 * kEps) * mf / (mf - x)) : cand;
+}
+
+__device__ __forceinline__ void s2_recon2_wall(const LoParams& P, const LoBuffers& B, const S2Buffers& S, int cc, int kgroup,
+                                               double (*s_th)[32]) {
     const int nv = P.nvel, nx = P.nx, ny = P.ny, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int f = warp >> 2, p = warp & 3;
-    const int k0 = blockIdx.x * 32 + lane;
+    const int k0 = kgroup * 32 + lane;
     const bool kok = k0 < nv;
     const int k = kok ? k0 : nv - 1;
-    const int cc = blockIdx.y, i = cc % nx, j = cc / nx;
-    const bool nw = s2_near_wall(j, ny);
-    const int first = nw ? s2_wall_first(j, ny) : j - 2;   // rows of the x first layer
+    const int i = cc % nx, j = cc / nx;
+    const int first = s2_wall_first(j, ny);   // rows of the x first layer
     const double* L1 = S.l1 + (size_t)f * 11 * nv + k;
     auto X = [&](int r, int q) { return L1[((size_t)((first + r) * nx + i) * 22 + q) * nv]; };
     double face[3], dn[3], dt[3], vol[3];
     bool ok = true;
     if (p < 2) {   // x face p
-        double a5[5], b5[5];
+        double a5[5], b5[5], dummy;
 #pragma unroll
         for (int r = 0; r < 5; ++r) { a5[r] = X(r, 2 * p); b5[r] = X(r, 2 * p + 1); }
-        if (!nw) ok = s2_companion3(a5, b5, face, dt, dn);
-        else {
-            double dummy;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                s2_wall_eval(a5, j, ny, c_s2.gnode[a], face[a], dt[a]);
-                s2_wall_eval(b5, j, ny, c_s2.gnode[a], dn[a], dummy);
-            }
+        for (int a = 0; a < 3; ++a) {
+            s2_wall_eval(a5, j, ny, c_s2.gnode[a], face[a], dt[a]);
+            s2_wall_eval(b5, j, ny, c_s2.gnode[a], dn[a], dummy);
         }
     } else {       // y face p - 2
-        const int s = p - 2;
         double a5[5], b5[5];
-        if (!nw) {
+        const S2Field F{(f == 0 ? B.h : B.b) + k, nv, nx, ny};
 #pragma unroll
-            for (int r = 0; r < 5; ++r) {
-                const double* y = L1 + ((size_t)(j * nx + wrapx(i + r - 2, nx)) * 22 + 7 + 2 * s) * nv;
-                a5[r] = y[0];
-                b5[r] = y[(size_t)nv];
-            }
-        } else {
-            const S2Field F{(f == 0 ? B.h : B.b) + k, nv, nx, ny};
+        for (int r = -2; r <= 2; ++r) {
+            double q[5];
 #pragma unroll
-            for (int r = -2; r <= 2; ++r) {
-                double q[5];
-#pragma unroll
-                for (int t = 0; t < 5; ++t) q[t] = F.at(i + r, first + t);
-                s2_wall_eval(q, j, ny, s == 0 ? -0.5 : 0.5, a5[r + 2], b5[r + 2]);
-            }
+            for (int t = 0; t < 5; ++t) q[t] = F.at(i + r, first + t);
+            s2_wall_eval(q, j, ny, p == 2 ? -0.5 : 0.5, a5[r + 2], b5[r + 2]);
         }
-        ok = s2_companion3(a5, b5, face, dt, dn);
+        s2_power_companion3(a5, b5, face, dt, dn);
     }
     if (p < 3) {   // volume Gauss row p
-        double a5[5];
+        double a5[5], dummy;
 #pragma unroll
         for (int r = 0; r < 5; ++r) a5[r] = X(r, 4 + p);
-        if (!nw) {
-            S2Weno ww;
-            ok = ok && s2_weno(a5, ww);
 #pragma unroll
-            for (int b = 0; b < 3; ++b) vol[b] = s2_at_v(ww, S2_G0 + b);
-        } else {
-            double dummy;
-#pragma unroll
-            for (int b = 0; b < 3; ++b) s2_wall_eval(a5, j, ny, c_s2.gnode[b], vol[b], dummy);
-        }
+        for (int b = 0; b < 3; ++b) s2_wall_eval(a5, j, ny, c_s2.gnode[b], vol[b], dummy);
     }
-    // positivity factor (limit_cell_outputs): min over both fields' face and volume samples
     const double hm = B.h[(size_t)cc * nv + k], bm = B.b[(size_t)cc * nv + k];
     const double mf = f == 0 ? hm : bm;
-    const double margin = 64.0 * kEps;
     double cand = 1.0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        if (face[a] < 0.0) cand = fmin(cand, (1.0 - margin) * mf / (mf - face[a]));
-        if (p < 3 && vol[a] < 0.0) cand = fmin(cand, (1.0 - margin) * mf / (mf - vol[a]));
+        cand = s2_limit(cand, face[a], mf);
+        if (p < 3) cand = s2_limit(cand, vol[a], mf);
     }
     s_th[warp][lane] = cand;
     __syncthreads();
@@ -157,7 +146,6 @@ __global__ void __launch_bounds__(256, 3) k_s2_recon2(LoParams P, LoBuffers B, S
     // the derivatives are divided by the cell sizes (limit_cell_outputs): multiplied by the reciprocals
     // here, exact when dx and dy are powers of two (the delivered meshes), within an ulp otherwise
     const double ind = 1.0 / (p < 2 ? P.dx : P.dy), itd = 1.0 / (p < 2 ? P.dy : P.dx);
-    // the side this velocity leaves the cell through (the face cache's upwind half), and the wall sides
     const int fv = f == 0 ? 0 : 1, fn = f == 0 ? 2 : 4, ft = f == 0 ? 3 : 5;
     const bool store = kok && rec_leaves(p, B.u[k], B.v[k]);
     const bool wall = kok && ((p == 2 && j == 0) || (p == 3 && j == ny - 1));
@@ -177,6 +165,92 @@ __global__ void __launch_bounds__(256, 3) k_s2_recon2(LoParams P, LoBuffers B, S
         ok = ok && isfinite(v) && isfinite(n) && isfinite(t);
     }
     if (!ok && kok) set_status(B.status, ST_NONFINITE_FLUX);
+}
+
+__global__ void __launch_bounds__(256, 2) k_s2_recon2(LoParams P, LoBuffers B, S2Buffers S) {
+    if (eval_cached(B)) return;
+    __shared__ double s_th[8][32];
+    const int nv = P.nvel, nx = P.nx, ny = P.ny, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // CTAs: the wall rows' (row, i, 32 velocities), then the other cells' (cell, 4 x 32 velocities)
+    const int ng = (nv + 31) >> 5, nq = (ng + 3) >> 2, wrows = min(ny, 6), nwall = wrows * nx * ng;
+    int id = (int)blockIdx.x;
+    if (id < nwall) {
+        const int c = id / ng, row = c / nx;
+        s2_recon2_wall(P, B, S, (row < 3 ? row : ny - wrows + row) * nx + c % nx, id % ng, s_th);
+        return;
+    }
+    id -= nwall;
+    const int c0 = id / nq, i = c0 % nx, j = 3 + c0 / nx, cc = j * nx + i, f = warp & 1;
+    const int k0 = ((id % nq) * 4 + (warp >> 1)) * 32 + lane;
+    const bool kok = k0 < nv;
+    const int k = kok ? k0 : nv - 1;
+    const size_t st = (size_t)22 * nv, rowst = st * nx;
+    const double* L1 = S.l1 + (size_t)f * 11 * nv + k + (size_t)cc * st;
+    const double hm = B.h[(size_t)cc * nv + k], bm = B.b[(size_t)cc * nv + k], mf = f == 0 ? hm : bm;
+    double face[2][3], dn[2][3], dt[2][3], cand = 1.0, sum = 0.0;   // sum: of the values that only theta sees, for their finiteness
+    int col[5];
+#pragma unroll
+    for (int r = -2; r <= 2; ++r) col[r + 2] = wrapx(i + r, nx) - i;
+#pragma unroll
+    for (int axis = 0; axis < 2; ++axis) {
+        const bool hi = (axis == 0 ? B.u[k] : B.v[k]) >= 0.0;   // the upper side is the leaving one
+        const double* L = L1 + (size_t)(axis == 0 ? 0 : 7) * nv;
+        const double *Lv = L + (size_t)(hi ? 2 : 0) * nv, *Lo = L + (size_t)(hi ? 0 : 2) * nv;
+        double a5[5], b5[5], o5[5], ov[3];
+#pragma unroll
+        for (int r = 0; r < 5; ++r) {
+            const long long off = axis == 0 ? (long long)(r - 2) * (long long)rowst : (long long)col[r] * (long long)st;
+            a5[r] = Lv[off];
+            b5[r] = Lv[off + nv];
+            o5[r] = Lo[off];
+        }
+        s2_power_companion3(a5, b5, face[axis], dt[axis], dn[axis]);
+        s2_power_values3(o5, ov);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) cand = s2_limit(s2_limit(cand, face[axis][a], mf), ov[a], mf);
+        sum += (ov[0] + ov[1]) + ov[2];
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {   // volume Gauss row p
+        double a5[5], vol[3];
+#pragma unroll
+        for (int r = 0; r < 5; ++r) a5[r] = L1[(long long)(r - 2) * (long long)rowst + (size_t)(4 + p) * nv];
+        s2_power_values3(a5, vol);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) cand = s2_limit(cand, vol[a], mf);
+        sum += (vol[0] + vol[1]) + vol[2];
+    }
+    s_th[warp][lane] = cand;
+    __syncthreads();
+    double theta = fmin(cand, s_th[warp ^ 1][lane]);
+    theta = (hm <= 0.0 || bm <= 0.0) ? 0.0 : fmax(0.0, fmin(1.0, theta));
+    bool ok = isfinite(sum);
+    const int fv = f == 0 ? 0 : 1, fn = f == 0 ? 2 : 4, ft = f == 0 ? 3 : 5;
+#pragma unroll
+    for (int axis = 0; axis < 2; ++axis) {
+        const double ind = 1.0 / (axis == 0 ? P.dx : P.dy), itd = 1.0 / (axis == 0 ? P.dy : P.dx);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const double v = mf + theta * (face[axis][a] - mf), n = theta * dn[axis][a] * ind, t = theta * dt[axis][a] * itd;
+            if (kok) {
+                S.rec[rec_cell(cc, axis, fv, a, nv) + k] = v;
+                S.rec[rec_cell(cc, axis, fn, a, nv) + k] = n;
+                S.rec[rec_cell(cc, axis, ft, a, nv) + k] = t;
+            }
+            ok = ok && isfinite(v) && isfinite(n) && isfinite(t);
+        }
+    }
+    if (!ok && kok) set_status(B.status, ST_NONFINITE_FLUX);
+}
+
+// first and second layer of all cells
+static cudaError_t launch_recon(const LoParams& P, const LoBuffers& B, const S2Buffers& S, cudaStream_t s) {
+    const int ng = (P.nvel + 31) / 32, inner = P.ny > 6 ? P.ny - 6 : 0, wall = P.ny - inner;
+    k_s2_recon1<<<dim3((unsigned)ng, (unsigned)(P.nx * P.ny)), 128, 0, s>>>(P, B, S);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_s2_recon2<<<(unsigned)(P.nx * (wall * ng + inner * ((ng + 3) / 4))), 256, 0, s>>>(P, B, S);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1444,11 +1518,7 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
         return cudaGetLastError();
     }
     if (which == 4) {
-        const dim3 grid((unsigned)((nv + 31) / 32), (unsigned)nc);
-        k_s2_recon1<<<grid, 128, 0, s>>>(P, B, S);
-        cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess) { k_s2_recon2<<<grid, 256, 0, s>>>(P, B, S); e = cudaGetLastError(); }
-        return e;
+        return launch_recon(P, B, S, s);
     }
     const int faces = which != 3, targets = which != 2;
     const long long nmacw = (faces ? (long long)nf * 2 : 0) + (targets ? (long long)nc : 0);   // warps
@@ -1487,10 +1557,7 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
     if (e != cudaSuccess || which == 3) return e;
     // a tensor table's faces and walls: the fused fluxes, unless a wall variant wants the nodes' fluxes and coefficients
     const bool tensor = P.tnu > 0, fused = tensor && S.coef == nullptr;
-    const dim3 grid((unsigned)((nv + 31) / 32), (unsigned)nc);
-    k_s2_recon1<<<grid, 128, 0, s>>>(P, B, S);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) { k_s2_recon2<<<grid, 256, 0, s>>>(P, B, S); e = cudaGetLastError(); }
+    e = launch_recon(P, B, S, s);
     if (e == cudaSuccess) e = cudaEventRecord(fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s2, fork, 0);
     if (e == cudaSuccess) {

@@ -128,6 +128,100 @@ __device__ __forceinline__ void s2_at(const S2Weno& w, int p, double& val, doubl
 }
 __device__ __forceinline__ double s2_at_v(const S2Weno& w, int p) { return s2_cand_sum(w.fw, w.q, c_s2p.E[p]); }
 
+// The same interpolant in power form about the cell centre, for the per-velocity reconstruction (k_s2_recon1/2).  Every
+// candidate is the polynomial with the stencil's cell averages, so its coefficients are differences of the
+// stencil: with t the second difference of a three-cell candidate and l its slope, q3 - t/24, l, t/2.  The smoothness
+// indicators are quadratic forms in the same differences; beta_4 splits into an even form in (a, b) and an
+// odd one in (d1, d2), where the mean has already cancelled.
+struct S2Diff {
+    double a, b, d1, d2, t0, t2, u0, u2;   // q2 - 2 q3 + q4, q1 - 2 q3 + q5, q4 - q2, q5 - q1, the outer t's, 2 l's
+};
+__device__ __forceinline__ S2Diff s2_diff(const double q[5]) {
+    S2Diff d;
+    d.a = (q[1] + q[3]) - 2.0 * q[2];
+    d.b = (q[0] + q[4]) - 2.0 * q[2];
+    d.d1 = q[3] - q[1];
+    d.d2 = q[4] - q[0];
+    d.t0 = (q[0] + q[2]) - 2.0 * q[1];
+    d.t2 = (q[4] + q[2]) - 2.0 * q[3];
+    d.u0 = d.t0 + 2.0 * (q[2] - q[1]);
+    d.u2 = d.t2 + 2.0 * (q[2] - q[3]);
+    return d;
+}
+// the weights of s2_weno (weno_coefficients, :168-204) by one division: alpha_c times the squared product D of the four
+// denominators is gam_c (D^2 + (tau D / d_c)^2).  D^2 leaves the normal range only for stencils beyond
+// about 1e19, where s2_weno takes over.
+__device__ __noinline__ void s2_weights_far(double q1, double q2, double q3, double q4, double q5, double fw[4]) {
+    const double q[5] = {q1, q2, q3, q4, q5};
+    S2Weno w;
+    s2_weno(q, w);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) fw[c] = w.fw[c];
+}
+__device__ __forceinline__ void s2_weights(const double q[5], const S2Diff& d, double fw[4]) {
+    const double k = 13.0 / 12.0;
+    const double b0 = k * (d.t0 * d.t0) + 0.25 * (d.u0 * d.u0), b1 = k * (d.a * d.a) + 0.25 * (d.d1 * d.d1);
+    const double b2 = k * (d.t2 * d.t2) + 0.25 * (d.u2 * d.u2);
+    const double b3 = d.a * ((97256.0 / 5040.0) * d.a - (44974.0 / 5040.0) * d.b) + (5506.25 / 5040.0) * (d.b * d.b) +
+                      (d.d1 * ((7707.0 / 5040.0) * d.d1 - (6027.0 / 5040.0) * d.d2) + (1401.75 / 5040.0) * (d.d2 * d.d2));
+    const double tau = (fabs(b3 - b0) + fabs(b3 - b1) + fabs(b3 - b2)) * (1.0 / 3.0);
+    const double d0 = b0 + 1.0e-8, d1 = b1 + 1.0e-8, d2 = b2 + 1.0e-8, d3 = b3 + 1.0e-8;
+    const double p01 = d0 * d1, p23 = d2 * d3, D = p01 * p23, D2 = D * D, t01 = tau * p01, t23 = tau * p23;
+    const double r0 = d1 * t23, r1 = d0 * t23, r2 = d3 * t01, r3 = d2 * t01;
+    const double a0 = 0.01125 * (D2 + r0 * r0), a1 = 0.1275 * (D2 + r1 * r1), a2 = 0.01125 * (D2 + r2 * r2);
+    const double a3 = D2 + r3 * r3, S = (a0 + a2) + (a1 + 0.85 * a3);   // a3 without its 0.85, which fw[3] divides by
+    if (S > 1.0e-280 && S < 1.0e280) {
+        const double is = 1.0 / S;
+        fw[3] = a3 * is;
+        fw[0] = a0 * is - 0.01125 * fw[3];
+        fw[1] = a1 * is - 0.1275 * fw[3];
+        fw[2] = a2 * is - 0.01125 * fw[3];
+    } else {
+        s2_weights_far(q[0], q[1], q[2], q[3], q[4], fw);
+    }
+}
+// coefficients of the weighted interpolant of the stencil v (differences d) with weights fw, whose sum is one
+__device__ __forceinline__ void s2_power(double v3, const S2Diff& d, const double fw[4], double c[5]) {
+    const double lo = 0.5 * (fw[0] * d.t0 + fw[1] * d.a + fw[2] * d.t2);
+    c[0] = v3 + (fw[3] * ((9.0 / 1920.0) * d.b - (116.0 / 1920.0) * d.a) - lo * (1.0 / 12.0));
+    c[1] = 0.5 * (fw[0] * d.u0 + fw[1] * d.d1 - fw[2] * d.u2) + fw[3] * ((34.0 / 48.0) * d.d1 - (5.0 / 48.0) * d.d2);
+    c[2] = lo + fw[3] * (0.75 * d.a - 0.0625 * d.b);
+    c[3] = fw[3] * ((1.0 / 12.0) * d.d2 - (1.0 / 6.0) * d.d1);
+    c[4] = fw[3] * ((1.0 / 24.0) * d.b - (1.0 / 6.0) * d.a);
+}
+constexpr double kS2G = 0.38729833462074168852;   // the outer Gauss node, sqrt(3/5) / 2; its square is 0.15
+__device__ __forceinline__ void s2_gauss_values(const double c[5], double val[3]) {
+    const double e = c[0] + (0.15 * c[2] + 0.0225 * c[4]), o = kS2G * (c[1] + 0.15 * c[3]);
+    val[0] = e - o;
+    val[1] = c[0];
+    val[2] = e + o;
+}
+__device__ __forceinline__ void s2_gauss_slopes(const double c[5], double der[3]) {
+    const double e = c[1] + 0.45 * c[3], o = 2.0 * kS2G * (c[2] + 0.3 * c[4]);
+    der[0] = e - o;
+    der[1] = c[1];
+    der[2] = e + o;
+}
+// companion_eval3 (:287-318) in this form, and the interpolant's Gauss values alone
+__device__ __forceinline__ void s2_power_companion3(const double q[5], const double comp[5], double val[3], double der[3],
+                                                    double cval[3]) {
+    double fw[4], c[5];
+    const S2Diff d = s2_diff(q);
+    s2_weights(q, d, fw);
+    s2_power(q[2], d, fw, c);
+    s2_gauss_values(c, val);
+    s2_gauss_slopes(c, der);
+    s2_power(comp[2], s2_diff(comp), fw, c);
+    s2_gauss_values(c, cval);
+}
+__device__ __forceinline__ void s2_power_values3(const double q[5], double val[3]) {
+    double fw[4], c[5];
+    const S2Diff d = s2_diff(q);
+    s2_weights(q, d, fw);
+    s2_power(q[2], d, fw, c);
+    s2_gauss_values(c, val);
+}
+
 // companion_eval3 (:287-318): the weights of q applied to the companion samples comp as well
 __device__ __forceinline__ bool s2_companion3(const double q[5], const double comp[5], double val[3], double der[3],
                                               double cval[3]) {
