@@ -77,21 +77,27 @@ __global__ void __launch_bounds__(128) k_s2_recon1(LoParams P, LoBuffers B, S2Bu
 // leaves the cell through, so along each axis only that side needs its derivatives: the other side's
 // values enter theta alone.
 //
-// Cells away from the walls: a thread takes one field of one velocity through both axes and the three
-// rows and keeps the two leaving sides until theta is known; CTA = 8 warps, warp pairs (h, b) over 4 x 32 velocities.
-// Cells in the three rows next to a wall (one-sided quartics across y; the wall sides for every velocity): CTA = 8
-// warps (field f = warp / 4, side and row p = warp % 4) over 32 velocities.
-// Bound by FP64 arithmetic (about 1,700 operations a cell-velocity; all four sides in the tables' form took about
-// 3,100).  At 8x64x32^2 this kernel went from 220 to 146 us and k_s2_recon1 from 42 to 33 (ncu, cold), the S2CN2 step
-// from 500 to 427 us, 48^2 velocities from 1011 to 845 us, the 16-instance batch from 9.24 to 7.61 ms a step.
-__device__ __forceinline__ double s2_limit(double cand, double x, double mf) {
-    return x < 0.0 ? fmin(cand, (1.0 - 64.0 * kEps) * mf / (mf - x)) : cand;
+// Cells away from the walls: a thread takes one field of one velocity through both axes and the three rows; CTA = 4
+// warps, warp pairs (h, b) over 2 x 32 velocities.  Each side is stored as soon as it is known, as if
+// theta were 1, and drawn towards the mean afterwards where the limiter acts, so no result waits in registers.
+// Cells in the three rows next to a wall (one-sided quartics across y; the wall sides for every velocity): CTA = 4
+// warps (field, axis) over 32 velocities, both sides of the axis held until theta is known.
+// Bound by FP64 arithmetic and issue slots (about 930 FP64 operations a thread, two threads a cell-velocity;
+// 56 % and 63 % busy).  Residency pays: at 8x64x32^2 the S2CN2 step took 392, 384, 382 and 380 us with 5, 6, 7 and 8
+// CTAs an SM (94 to 64 registers).  All four sides in the tables' form took 220 us here and this form 110 (ncu,
+// cold), k_s2_recon1 42 and 33; the step went from 500 to 380 us, at 48^2 velocities from 1011 to 748 us, and the
+// 16-instance batch from 9.24 to 6.63 ms a step.
+// The limiter's candidate of a sample x < 0, (1 - margin) m / (m - x), falls with x (m > 0; theta is 0 otherwise): the
+// smallest sample gives the smallest candidate.
+__device__ __forceinline__ double s2_limit(double xmin, double mf) {
+    return xmin < 0.0 ? fmin(1.0, (1.0 - 64.0 * kEps) * mf / (mf - xmin)) : 1.0;
 }
+__device__ __forceinline__ double s2_min(double a, double b) { return b < a ? b : a; }
 
 __device__ __forceinline__ void s2_recon2_wall(const LoParams& P, const LoBuffers& B, const S2Buffers& S, int cc, int kgroup,
                                                double (*s_th)[32]) {
     const int nv = P.nvel, nx = P.nx, ny = P.ny, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int f = warp >> 2, p = warp & 3;
+    const int f = warp >> 1, axis = warp & 1;
     const int k0 = kgroup * 32 + lane;
     const bool kok = k0 < nv;
     const int k = kok ? k0 : nv - 1;
@@ -99,80 +105,86 @@ __device__ __forceinline__ void s2_recon2_wall(const LoParams& P, const LoBuffer
     const int first = s2_wall_first(j, ny);   // rows of the x first layer
     const double* L1 = S.l1 + (size_t)f * 11 * nv + k;
     auto X = [&](int r, int q) { return L1[((size_t)((first + r) * nx + i) * 22 + q) * nv]; };
-    double face[3], dn[3], dt[3], vol[3];
-    bool ok = true;
-    if (p < 2) {   // x face p
-        double a5[5], b5[5], dummy;
-#pragma unroll
-        for (int r = 0; r < 5; ++r) { a5[r] = X(r, 2 * p); b5[r] = X(r, 2 * p + 1); }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            s2_wall_eval(a5, j, ny, c_s2.gnode[a], face[a], dt[a]);
-            s2_wall_eval(b5, j, ny, c_s2.gnode[a], dn[a], dummy);
-        }
-    } else {       // y face p - 2
-        double a5[5], b5[5];
-        const S2Field F{(f == 0 ? B.h : B.b) + k, nv, nx, ny};
-#pragma unroll
-        for (int r = -2; r <= 2; ++r) {
-            double q[5];
-#pragma unroll
-            for (int t = 0; t < 5; ++t) q[t] = F.at(i + r, first + t);
-            s2_wall_eval(q, j, ny, p == 2 ? -0.5 : 0.5, a5[r + 2], b5[r + 2]);
-        }
-        s2_power_companion3(a5, b5, face, dt, dn);
-    }
-    if (p < 3) {   // volume Gauss row p
-        double a5[5], dummy;
-#pragma unroll
-        for (int r = 0; r < 5; ++r) a5[r] = X(r, 4 + p);
-#pragma unroll
-        for (int b = 0; b < 3; ++b) s2_wall_eval(a5, j, ny, c_s2.gnode[b], vol[b], dummy);
-    }
     const double hm = B.h[(size_t)cc * nv + k], bm = B.b[(size_t)cc * nv + k];
     const double mf = f == 0 ? hm : bm;
-    double cand = 1.0;
+    double face[2][3], dn[2][3], dt[2][3], xmin = 0.0, sum = 0.0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        cand = s2_limit(cand, face[a], mf);
-        if (p < 3) cand = s2_limit(cand, vol[a], mf);
+    for (int s = 0; s < 2; ++s) {
+        double a5[5], b5[5], dummy;
+        if (axis == 0) {
+#pragma unroll
+            for (int r = 0; r < 5; ++r) { a5[r] = X(r, 2 * s); b5[r] = X(r, 2 * s + 1); }
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                s2_wall_eval(a5, j, ny, c_s2.gnode[a], face[s][a], dt[s][a]);
+                s2_wall_eval(b5, j, ny, c_s2.gnode[a], dn[s][a], dummy);
+            }
+        } else {
+            const S2Field F{(f == 0 ? B.h : B.b) + k, nv, nx, ny};
+#pragma unroll
+            for (int r = -2; r <= 2; ++r) {
+                double q[5];
+#pragma unroll
+                for (int t = 0; t < 5; ++t) q[t] = F.at(i + r, first + t);
+                s2_wall_eval(q, j, ny, s == 0 ? -0.5 : 0.5, a5[r + 2], b5[r + 2]);
+            }
+            s2_power_companion3(a5, b5, face[s], dt[s], dn[s]);
+        }
+        const int row = axis == 0 ? s : 2;   // volume Gauss rows 0, 1 by the x warp, 2 by the y warp
+        if (axis == 0 || s == 0) {
+#pragma unroll
+            for (int r = 0; r < 5; ++r) a5[r] = X(r, 4 + row);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                double vol;
+                s2_wall_eval(a5, j, ny, c_s2.gnode[b], vol, dummy);
+                xmin = s2_min(xmin, vol);
+                sum += vol;
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            xmin = s2_min(xmin, face[s][a]);
+            sum += face[s][a] + dn[s][a] + dt[s][a];
+        }
     }
-    s_th[warp][lane] = cand;
+    s_th[warp][lane] = s2_limit(xmin, mf);
     __syncthreads();
-    double theta = s_th[0][lane];
-#pragma unroll
-    for (int w = 1; w < 8; ++w) theta = fmin(theta, s_th[w][lane]);
+    double theta = fmin(fmin(s_th[0][lane], s_th[1][lane]), fmin(s_th[2][lane], s_th[3][lane]));
     theta = (hm <= 0.0 || bm <= 0.0) ? 0.0 : fmax(0.0, fmin(1.0, theta));
     // the derivatives are divided by the cell sizes (limit_cell_outputs): multiplied by the reciprocals
     // here, exact when dx and dy are powers of two (the delivered meshes), within an ulp otherwise
-    const double ind = 1.0 / (p < 2 ? P.dx : P.dy), itd = 1.0 / (p < 2 ? P.dy : P.dx);
+    const double ind = 1.0 / (axis == 0 ? P.dx : P.dy), itd = 1.0 / (axis == 0 ? P.dy : P.dx);
     const int fv = f == 0 ? 0 : 1, fn = f == 0 ? 2 : 4, ft = f == 0 ? 3 : 5;
-    const bool store = kok && rec_leaves(p, B.u[k], B.v[k]);
-    const bool wall = kok && ((p == 2 && j == 0) || (p == 3 && j == ny - 1));
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const double v = mf + theta * (face[a] - mf), n = theta * dn[a] * ind, t = theta * dt[a] * itd;
-        if (store) {
-            S.rec[rec_cell(cc, p >> 1, fv, a, nv) + k] = v;
-            S.rec[rec_cell(cc, p >> 1, fn, a, nv) + k] = n;
-            S.rec[rec_cell(cc, p >> 1, ft, a, nv) + k] = t;
+    for (int s = 0; s < 2; ++s) {
+        const bool store = kok && rec_leaves(2 * axis + s, B.u[k], B.v[k]);
+        const bool wall = kok && axis == 1 && ((s == 0 && j == 0) || (s == 1 && j == ny - 1));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const double v = mf + theta * (face[s][a] - mf), n = theta * dn[s][a] * ind, t = theta * dt[s][a] * itd;
+            if (store) {
+                S.rec[rec_cell(cc, axis, fv, a, nv) + k] = v;
+                S.rec[rec_cell(cc, axis, fn, a, nv) + k] = n;
+                S.rec[rec_cell(cc, axis, ft, a, nv) + k] = t;
+            }
+            if (wall) {
+                S.rec[rec_wall(nx, ny, s, i, fv, a, nv) + k] = v;
+                S.rec[rec_wall(nx, ny, s, i, fn, a, nv) + k] = n;
+                S.rec[rec_wall(nx, ny, s, i, ft, a, nv) + k] = t;
+            }
         }
-        if (wall) {
-            S.rec[rec_wall(nx, ny, p - 2, i, fv, a, nv) + k] = v;
-            S.rec[rec_wall(nx, ny, p - 2, i, fn, a, nv) + k] = n;
-            S.rec[rec_wall(nx, ny, p - 2, i, ft, a, nv) + k] = t;
-        }
-        ok = ok && isfinite(v) && isfinite(n) && isfinite(t);
     }
-    if (!ok && kok) set_status(B.status, ST_NONFINITE_FLUX);
+    if (kok && !(isfinite(sum) && isfinite(theta))) set_status(B.status, ST_NONFINITE_FLUX);
 }
 
-__global__ void __launch_bounds__(256, 2) k_s2_recon2(LoParams P, LoBuffers B, S2Buffers S) {
+constexpr int kRecon2Threads = 128;
+__global__ void __launch_bounds__(kRecon2Threads, 8) k_s2_recon2(LoParams P, LoBuffers B, S2Buffers S) {
     if (eval_cached(B)) return;
-    __shared__ double s_th[8][32];
+    __shared__ double s_th[kRecon2Threads / 32][32];
     const int nv = P.nvel, nx = P.nx, ny = P.ny, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // CTAs: the wall rows' (row, i, 32 velocities), then the other cells' (cell, 4 x 32 velocities)
-    const int ng = (nv + 31) >> 5, nq = (ng + 3) >> 2, wrows = min(ny, 6), nwall = wrows * nx * ng;
+    // CTAs: the wall rows' (row, i, 32 velocities), then the other cells' (cell, 2 x 32 velocities)
+    const int ng = (nv + 31) >> 5, nq = (ng + 1) >> 1, wrows = min(ny, 6), nwall = wrows * nx * ng;
     int id = (int)blockIdx.x;
     if (id < nwall) {
         const int c = id / ng, row = c / nx;
@@ -181,34 +193,44 @@ __global__ void __launch_bounds__(256, 2) k_s2_recon2(LoParams P, LoBuffers B, S
     }
     id -= nwall;
     const int c0 = id / nq, i = c0 % nx, j = 3 + c0 / nx, cc = j * nx + i, f = warp & 1;
-    const int k0 = ((id % nq) * 4 + (warp >> 1)) * 32 + lane;
+    const int k0 = ((id % nq) * 2 + (warp >> 1)) * 32 + lane;
     const bool kok = k0 < nv;
     const int k = kok ? k0 : nv - 1;
     const size_t st = (size_t)22 * nv, rowst = st * nx;
     const double* L1 = S.l1 + (size_t)f * 11 * nv + k + (size_t)cc * st;
     const double hm = B.h[(size_t)cc * nv + k], bm = B.b[(size_t)cc * nv + k], mf = f == 0 ? hm : bm;
-    double face[2][3], dn[2][3], dt[2][3], cand = 1.0, sum = 0.0;   // sum: of the values that only theta sees, for their finiteness
-    int col[5];
-#pragma unroll
-    for (int r = -2; r <= 2; ++r) col[r + 2] = wrapx(i + r, nx) - i;
+    const int fv = f == 0 ? 0 : 1, fn = f == 0 ? 2 : 4, ft = f == 0 ? 3 : 5;
+    double xmin = 0.0, sum = 0.0;   // sum: a value of every template with all its coefficients, for their finiteness
 #pragma unroll
     for (int axis = 0; axis < 2; ++axis) {
         const bool hi = (axis == 0 ? B.u[k] : B.v[k]) >= 0.0;   // the upper side is the leaving one
         const double* L = L1 + (size_t)(axis == 0 ? 0 : 7) * nv;
         const double *Lv = L + (size_t)(hi ? 2 : 0) * nv, *Lo = L + (size_t)(hi ? 0 : 2) * nv;
-        double a5[5], b5[5], o5[5], ov[3];
+        double a5[5], b5[5], o5[5], face[3], dn[3], dt[3], ov[3];
 #pragma unroll
         for (int r = 0; r < 5; ++r) {
-            const long long off = axis == 0 ? (long long)(r - 2) * (long long)rowst : (long long)col[r] * (long long)st;
+            const long long off = axis == 0 ? (long long)(r - 2) * (long long)rowst
+                                            : (long long)(wrapx(i + r - 2, nx) - i) * (long long)st;
             a5[r] = Lv[off];
             b5[r] = Lv[off + nv];
             o5[r] = Lo[off];
         }
-        s2_power_companion3(a5, b5, face[axis], dt[axis], dn[axis]);
+        s2_power_companion3(a5, b5, face, dt, dn);
         s2_power_values3(o5, ov);
+        // the derivatives are divided by the cell sizes (limit_cell_outputs): multiplied by the reciprocals
+        // here, exact when dx and dy are powers of two (the delivered meshes), within an ulp otherwise
+        const double ind = 1.0 / (axis == 0 ? P.dx : P.dy), itd = 1.0 / (axis == 0 ? P.dy : P.dx);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) cand = s2_limit(s2_limit(cand, face[axis][a], mf), ov[a], mf);
-        sum += (ov[0] + ov[1]) + ov[2];
+        for (int a = 0; a < 3; ++a) {
+            xmin = s2_min(s2_min(xmin, face[a]), ov[a]);
+            const double n = dn[a] * ind, t = dt[a] * itd;
+            if (a == 2) sum += (face[a] + n) + (t + ov[a]);
+            if (kok) {   // unlimited: theta is 1 but for a few cells and velocities
+                S.rec[rec_cell(cc, axis, fv, a, nv) + k] = face[a];
+                S.rec[rec_cell(cc, axis, fn, a, nv) + k] = n;
+                S.rec[rec_cell(cc, axis, ft, a, nv) + k] = t;
+            }
+        }
     }
 #pragma unroll
     for (int p = 0; p < 3; ++p) {   // volume Gauss row p
@@ -217,30 +239,27 @@ __global__ void __launch_bounds__(256, 2) k_s2_recon2(LoParams P, LoBuffers B, S
         for (int r = 0; r < 5; ++r) a5[r] = L1[(long long)(r - 2) * (long long)rowst + (size_t)(4 + p) * nv];
         s2_power_values3(a5, vol);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) cand = s2_limit(cand, vol[a], mf);
-        sum += (vol[0] + vol[1]) + vol[2];
+        for (int a = 0; a < 3; ++a) xmin = s2_min(xmin, vol[a]);
+        sum += vol[2];
     }
+    const double cand = s2_limit(xmin, mf);
     s_th[warp][lane] = cand;
     __syncthreads();
     double theta = fmin(cand, s_th[warp ^ 1][lane]);
     theta = (hm <= 0.0 || bm <= 0.0) ? 0.0 : fmax(0.0, fmin(1.0, theta));
-    bool ok = isfinite(sum);
-    const int fv = f == 0 ? 0 : 1, fn = f == 0 ? 2 : 4, ft = f == 0 ? 3 : 5;
-#pragma unroll
-    for (int axis = 0; axis < 2; ++axis) {
-        const double ind = 1.0 / (axis == 0 ? P.dx : P.dy), itd = 1.0 / (axis == 0 ? P.dy : P.dx);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const double v = mf + theta * (face[axis][a] - mf), n = theta * dn[axis][a] * ind, t = theta * dt[axis][a] * itd;
-            if (kok) {
-                S.rec[rec_cell(cc, axis, fv, a, nv) + k] = v;
-                S.rec[rec_cell(cc, axis, fn, a, nv) + k] = n;
-                S.rec[rec_cell(cc, axis, ft, a, nv) + k] = t;
+    if (!kok) return;
+    if (theta < 1.0) {   // the limiter acts: the values this thread stored, drawn towards the mean
+#pragma unroll 1
+        for (int axis = 0; axis < 2; ++axis)
+#pragma unroll 1
+            for (int a = 0; a < 3; ++a) {
+                double* v = S.rec + rec_cell(cc, axis, fv, a, nv) + k;
+                *v = mf + theta * (*v - mf);
+                S.rec[rec_cell(cc, axis, fn, a, nv) + k] *= theta;
+                S.rec[rec_cell(cc, axis, ft, a, nv) + k] *= theta;
             }
-            ok = ok && isfinite(v) && isfinite(n) && isfinite(t);
-        }
     }
-    if (!ok && kok) set_status(B.status, ST_NONFINITE_FLUX);
+    if (!isfinite(sum)) set_status(B.status, ST_NONFINITE_FLUX);
 }
 
 // first and second layer of all cells
@@ -249,7 +268,7 @@ static cudaError_t launch_recon(const LoParams& P, const LoBuffers& B, const S2B
     k_s2_recon1<<<dim3((unsigned)ng, (unsigned)(P.nx * P.ny)), 128, 0, s>>>(P, B, S);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_s2_recon2<<<(unsigned)(P.nx * (wall * ng + inner * ((ng + 3) / 4))), 256, 0, s>>>(P, B, S);
+    k_s2_recon2<<<(unsigned)(P.nx * (wall * ng + inner * ((ng + 1) / 2))), kRecon2Threads, 0, s>>>(P, B, S);
     return cudaGetLastError();
 }
 

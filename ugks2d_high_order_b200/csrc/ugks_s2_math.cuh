@@ -133,6 +133,15 @@ __device__ __forceinline__ double s2_at_v(const S2Weno& w, int p) { return s2_ca
 // stencil: with t the second difference of a three-cell candidate and l its slope, q3 - t/24, l, t/2.  The smoothness
 // indicators are quadratic forms in the same differences; beta_4 splits into an even form in (a, b) and an
 // odd one in (d1, d2), where the mean has already cancelled.
+constexpr double kS2G = 0.38729833462074168852;   // the outer Gauss node, sqrt(3/5) / 2; its square is 0.15
+#define S2_POWER_CONSTANTS                                                                                         \
+    3.0 / 13.0, 97256.0 / 5460.0, 44974.0 / 5460.0, 5506.25 / 5460.0, 7707.0 / 5460.0, 6027.0 / 5460.0,              \
+        1401.75 / 5460.0, 12.0e-8 / 13.0, 34.0 / 3.0, 680.0 / 9.0, 800.0 / 9.0, 0.01125, 0.1275, 9.0 / 1920.0,       \
+        116.0 / 1920.0, 1.0 / 24.0, 34.0 / 48.0, 5.0 / 48.0, 1.0 / 12.0, 1.0 / 6.0, 0.15, 0.0225, kS2G, 0.15 * kS2G, \
+        0.45, 2.0 * kS2G, 0.6 * kS2G
+// in constant memory: an operand of the arithmetic itself instead of two moves a use
+__constant__ double c_s2k[27] = {S2_POWER_CONSTANTS};
+#define S2K(i) c_s2k[i]
 struct S2Diff {
     double a, b, d1, d2, t0, t2, u0, u2;   // q2 - 2 q3 + q4, q1 - 2 q3 + q5, q4 - q2, q5 - q1, the outer t's, 2 l's
 };
@@ -159,45 +168,45 @@ __device__ __noinline__ void s2_weights_far(double q1, double q2, double q3, dou
     for (int c = 0; c < 4; ++c) fw[c] = w.fw[c];
 }
 __device__ __forceinline__ void s2_weights(const double q[5], const S2Diff& d, double fw[4]) {
-    const double k = 13.0 / 12.0;
-    const double b0 = k * (d.t0 * d.t0) + 0.25 * (d.u0 * d.u0), b1 = k * (d.a * d.a) + 0.25 * (d.d1 * d.d1);
-    const double b2 = k * (d.t2 * d.t2) + 0.25 * (d.u2 * d.u2);
-    const double b3 = d.a * ((97256.0 / 5040.0) * d.a - (44974.0 / 5040.0) * d.b) + (5506.25 / 5040.0) * (d.b * d.b) +
-                      (d.d1 * ((7707.0 / 5040.0) * d.d1 - (6027.0 / 5040.0) * d.d2) + (1401.75 / 5040.0) * (d.d2 * d.d2));
-    const double tau = (fabs(b3 - b0) + fabs(b3 - b1) + fabs(b3 - b2)) * (1.0 / 3.0);
-    const double d0 = b0 + 1.0e-8, d1 = b1 + 1.0e-8, d2 = b2 + 1.0e-8, d3 = b3 + 1.0e-8;
-    const double p01 = d0 * d1, p23 = d2 * d3, D = p01 * p23, D2 = D * D, t01 = tau * p01, t23 = tau * p23;
+    // the indicators and the 1e-8 beside them times 12/13, and tau times 36/13: the ratios keep their values up to a
+    // factor of 3, which 9 D^2 takes up
+    const double b0 = d.t0 * d.t0 + S2K(0) * (d.u0 * d.u0), b1 = d.a * d.a + S2K(0) * (d.d1 * d.d1);
+    const double b2 = d.t2 * d.t2 + S2K(0) * (d.u2 * d.u2);
+    const double b3 = d.a * (S2K(1) * d.a - S2K(2) * d.b) + (S2K(3) * (d.b * d.b) +
+                      (d.d1 * (S2K(4) * d.d1 - S2K(5) * d.d2) + S2K(6) * (d.d2 * d.d2)));
+    const double tau = fabs(b3 - b0) + fabs(b3 - b1) + fabs(b3 - b2);
+    const double d0 = b0 + S2K(7), d1 = b1 + S2K(7), d2 = b2 + S2K(7), d3 = b3 + S2K(7);
+    const double p01 = d0 * d1, p23 = d2 * d3, D = p01 * p23, N = 9.0 * (D * D), t01 = tau * p01, t23 = tau * p23;
     const double r0 = d1 * t23, r1 = d0 * t23, r2 = d3 * t01, r3 = d2 * t01;
-    const double a0 = 0.01125 * (D2 + r0 * r0), a1 = 0.1275 * (D2 + r1 * r1), a2 = 0.01125 * (D2 + r2 * r2);
-    const double a3 = D2 + r3 * r3, S = (a0 + a2) + (a1 + 0.85 * a3);   // a3 without its 0.85, which fw[3] divides by
+    const double a0 = N + r0 * r0, a1 = N + r1 * r1, a2 = N + r2 * r2, a3 = N + r3 * r3;
+    const double S = (a0 + a2) + (S2K(8) * a1 + S2K(9) * a3);   // sum of the alphas over gam_1
     if (S > 1.0e-280 && S < 1.0e280) {
         const double is = 1.0 / S;
-        fw[3] = a3 * is;
-        fw[0] = a0 * is - 0.01125 * fw[3];
-        fw[1] = a1 * is - 0.1275 * fw[3];
-        fw[2] = a2 * is - 0.01125 * fw[3];
+        fw[3] = a3 * (S2K(10) * is);
+        fw[0] = a0 * is - S2K(11) * fw[3];
+        fw[1] = a1 * (S2K(8) * is) - S2K(12) * fw[3];
+        fw[2] = a2 * is - S2K(11) * fw[3];
     } else {
         s2_weights_far(q[0], q[1], q[2], q[3], q[4], fw);
     }
 }
 // coefficients of the weighted interpolant of the stencil v (differences d) with weights fw, whose sum is one
 __device__ __forceinline__ void s2_power(double v3, const S2Diff& d, const double fw[4], double c[5]) {
-    const double lo = 0.5 * (fw[0] * d.t0 + fw[1] * d.a + fw[2] * d.t2);
-    c[0] = v3 + (fw[3] * ((9.0 / 1920.0) * d.b - (116.0 / 1920.0) * d.a) - lo * (1.0 / 12.0));
-    c[1] = 0.5 * (fw[0] * d.u0 + fw[1] * d.d1 - fw[2] * d.u2) + fw[3] * ((34.0 / 48.0) * d.d1 - (5.0 / 48.0) * d.d2);
-    c[2] = lo + fw[3] * (0.75 * d.a - 0.0625 * d.b);
-    c[3] = fw[3] * ((1.0 / 12.0) * d.d2 - (1.0 / 6.0) * d.d1);
-    c[4] = fw[3] * ((1.0 / 24.0) * d.b - (1.0 / 6.0) * d.a);
+    const double lo = fw[0] * d.t0 + fw[1] * d.a + fw[2] * d.t2;
+    c[0] = v3 + (fw[3] * (S2K(13) * d.b - S2K(14) * d.a) - S2K(15) * lo);
+    c[1] = 0.5 * (fw[0] * d.u0 + fw[1] * d.d1 - fw[2] * d.u2) + fw[3] * (S2K(16) * d.d1 - S2K(17) * d.d2);
+    c[2] = 0.5 * lo + fw[3] * (0.75 * d.a - 0.0625 * d.b);
+    c[3] = fw[3] * (S2K(18) * d.d2 - S2K(19) * d.d1);
+    c[4] = fw[3] * (S2K(15) * d.b - S2K(19) * d.a);
 }
-constexpr double kS2G = 0.38729833462074168852;   // the outer Gauss node, sqrt(3/5) / 2; its square is 0.15
 __device__ __forceinline__ void s2_gauss_values(const double c[5], double val[3]) {
-    const double e = c[0] + (0.15 * c[2] + 0.0225 * c[4]), o = kS2G * (c[1] + 0.15 * c[3]);
+    const double e = c[0] + (S2K(20) * c[2] + S2K(21) * c[4]), o = S2K(22) * c[1] + S2K(23) * c[3];
     val[0] = e - o;
     val[1] = c[0];
     val[2] = e + o;
 }
 __device__ __forceinline__ void s2_gauss_slopes(const double c[5], double der[3]) {
-    const double e = c[1] + 0.45 * c[3], o = 2.0 * kS2G * (c[2] + 0.3 * c[4]);
+    const double e = c[1] + S2K(24) * c[3], o = S2K(25) * c[2] + S2K(26) * c[4];
     der[0] = e - o;
     der[1] = c[1];
     der[2] = e + o;
