@@ -1541,18 +1541,22 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
     }
     const int faces = which != 3, targets = which != 2;
     const long long nmacw = (faces ? (long long)nf * 2 : 0) + (targets ? (long long)nc : 0);   // warps
-    k_s2_macro<<<(unsigned)((nmacw * 32 + 127) / 128), 128, 0, s>>>(P, B, S, faces, targets);
-    cudaError_t e = cudaGetLastError();
-    // which 1: the targets need only the macro pass and are first read after the face combine, so
-    // they run on the side stream beside the reconstruction and the face nodes (the wall nodes
-    // follow them there); which 3: on the main stream
-    const bool side_targets = targets && faces;
-    if (e == cudaSuccess && side_targets) {
+    // The macro pass feeds the targets and the face nodes, the reconstruction neither of them: with an evolution it runs on
+    // the side stream beside the reconstruction (S2CN2 step 381 -> 378 us, HighOrderImplicit pseudo-step 519 -> 510
+    // at 8x64x32^2), followed there by the targets of which 1 (first read after the face
+    // arrays) and, after the reconstruction, the wall nodes; which 3: everything on the main stream
+    cudaStream_t ts = faces ? s2 : s;
+    cudaError_t e = cudaSuccess;
+    if (faces) {
         e = cudaEventRecord(fork, s);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s2, fork, 0);
     }
+    if (e == cudaSuccess) {
+        k_s2_macro<<<(unsigned)((nmacw * 32 + 127) / 128), 128, 0, ts>>>(P, B, S, faces, targets);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess && faces) e = cudaEventRecord(join, s2);
     if (e == cudaSuccess && targets) {
-        cudaStream_t ts = side_targets ? s2 : s;
         if (P.tnu > 0) {
             const unsigned g = (unsigned)((nc * 9 * kTG + 127) / 128);
             const int n = P.tnu > P.tnv ? P.tnu : P.tnv;
@@ -1577,6 +1581,7 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
     // a tensor table's faces and walls: the fused fluxes, unless a wall variant wants the nodes' fluxes and coefficients
     const bool tensor = P.tnu > 0, fused = tensor && S.coef == nullptr;
     e = launch_recon(P, B, S, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join, 0);   // the macro pass
     if (e == cudaSuccess) e = cudaEventRecord(fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s2, fork, 0);
     if (e == cudaSuccess) {
