@@ -502,12 +502,12 @@ extern "C" int ugks_init_freestream(ugks_ctx* c, double rho, double U, double V,
     c->launches += 1;
     if (c->imem && c->Q.high_order) {   // S2NativeInitializeState cold start: h, b := closure Maxwellian of W
         UGKS_CK(s2_enqueue(0, c->P, c->B, c->I.s2, c->stream, c->stream2, c->ev_fork, c->ev_join));
-        c->launches += s2_enqueue_kernels(0);
+        c->launches += 1;
     }
     if (c->cmem) {   // the same cold start, then the S2CN2 ledger and the targets of the state
         UGKS_CK(s2_enqueue(0, c->P, c->B, c->T[0], c->stream, c->stream2, c->ev_fork, c->ev_join));
         UGKS_CK(enqueue_s2cn2_prepare(c->P, c->Bs[0], c->T[0], c->C, c->stream, &c->launches));
-        c->launches += s2_enqueue_kernels(0);
+        c->launches += 1;
         c->cn_ready = true;
     }
     int r = kernel_timestep(c);
@@ -541,7 +541,7 @@ static int s2_evolution(ugks_ctx* c, bool rebuild_targets) {
         c->cn_reject_at = 0;
         const int which = rebuild_targets ? 1 : 2;
         UGKS_CK(s2_enqueue(which, c->P, c->Bs[0], c->T[0], c->stream, c->stream2, c->ev_fork, c->ev_join));
-        c->launches += s2_enqueue_kernels(which);
+        c->launches += s2_enqueue_kernels(which, c->P, c->T[0]);
         if (c->has_var) {   // the wall variant's part of S2NativeEvolution (mod_S2NativeAdapter.f90:491-540)
             UGKS_CK(enqueue_s2cn2_variant(c->P, c->Bs[0], c->T[0], c->V, c->stream, c->stream2, c->ev_fork,
                                           c->ev_join));
@@ -553,7 +553,7 @@ static int s2_evolution(ugks_ctx* c, bool rebuild_targets) {
         return r;
     }
     UGKS_CK(s2_enqueue(1, c->P, c->B, c->I.s2, c->stream, c->stream2, c->ev_fork, c->ev_join));
-    c->launches += s2_enqueue_kernels(1);
+    c->launches += s2_enqueue_kernels(1, c->P, c->I.s2);
     return collect_status(c);
 }
 
@@ -606,7 +606,7 @@ static int s2cn2_apply(ugks_ctx* c) {
     if (c->cn_stage != 2) return UGKS_EINVAL;
     c->cn_stage = 0;
     UGKS_CK(enqueue_cn_apply(c->P, c->Bs[0], c->Bs[1], c->T[1], c->C, c->stream));
-    c->launches += 1 + s2_enqueue_kernels(3);
+    c->launches += cn_apply_kernels(c->P, c->T[1]);
     unsigned acc = 0;
     UGKS_CK(cudaMemcpyAsync(&acc, c->C.accepted, sizeof acc, cudaMemcpyDeviceToHost, c->stream));
     const int r = collect_status(c);
@@ -820,7 +820,7 @@ extern "C" int ugks_implicit_init(ugks_ctx* c) {
     UGKS_CK(cudaSetDevice(c->device));
     UGKS_CK(launch_im_init(c->P, c->B, c->Q, c->I, c->stream));
     // + the first pseudo-step's pre-update S2 evaluation and residual (in graphs a conditional body)
-    c->launches += 1 + (c->Q.high_order ? 1 + s2_enqueue_kernels(1) : 0);
+    c->launches += 1 + (c->Q.high_order ? 1 + s2_enqueue_kernels(1, c->P, c->I.s2) : 0);
     c->implicit_ready = true;
     return collect_status(c);
 }
@@ -835,7 +835,7 @@ extern "C" int ugks_implicit_restore(ugks_ctx* c, double m0, double reference_h,
     UGKS_CK(cudaSetDevice(c->device));
     UGKS_CK(launch_im_init(c->P, c->B, c->Q, c->I, c->stream));
     // + the first pseudo-step's pre-update S2 evaluation and residual (in graphs a conditional body)
-    c->launches += 1 + (c->Q.high_order ? 1 + s2_enqueue_kernels(1) : 0);
+    c->launches += 1 + (c->Q.high_order ? 1 + s2_enqueue_kernels(1, c->P, c->I.s2) : 0);
     static_assert(IS_REF_H == IS_M0 + 1 && IS_REF_B == IS_M0 + 2 && IS_REF_INIT == IS_M0 + 3,
                   "M0 and the residual references are contiguous state words");
     const double v[4] = {m0, have_reference ? reference_h : 0.0, have_reference ? reference_b : 0.0,
@@ -1167,7 +1167,7 @@ extern "C" int ugks_s2cn2_steps(ugks_ctx* c, int nsteps, int* steps_done, double
         for (int q = 0; q < pairs; ++q) UGKS_CK(cudaGraphLaunch(c->cgraph, c->stream));
     }
     if (nsteps % 2) UGKS_CK(enqueue_cn_step(c, 0));
-    c->launches += (long long)(kCnStepKernels - 1 + (c->has_var ? s2cn2_variant_kernels(c->P) : 0)) * nsteps;
+    c->launches += (long long)(cn_step_kernels(c->P, c->T[0]) - 1 + (c->has_var ? s2cn2_variant_kernels(c->P) : 0)) * nsteps;
     unsigned acc = 0;
     UGKS_CK(cudaMemcpyAsync(&acc, c->C.accepted, sizeof acc, cudaMemcpyDeviceToHost, c->stream));
     if (report) UGKS_CK(cudaMemcpyAsync(report, c->C.report, kCnReport * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1538,7 +1538,7 @@ extern "C" int ugks_s2cn2_backward(ugks_ctx* c, const double* seed, double* grad
             UGKS_CK(copy_state(c, s0, ck.h, ck.b, ck.W));
             UGKS_CK(copy_ledger(c, s0.ledger, ck.ledger));
             UGKS_CK(s2_enqueue(3, c->P, slot_lo(c, s0), slot_targets(c, s0), c->stream, c->stream, nullptr, nullptr));
-            c->launches += s2_enqueue_kernels(3);
+            c->launches += s2_enqueue_kernels(3, c->P, c->T[0]);
         }
         if (records) {
             // the segment recomputed once from its checkpoint, each step leaving its record; then the
@@ -1588,7 +1588,7 @@ extern "C" int ugks_s2cn2_backward(ugks_ctx* c, const double* seed, double* grad
         UGKS_CK(s2_enqueue(3, c->P, slot_lo(c, s0), c->T[1], c->stream, c->stream, nullptr, nullptr));
         const AdjBuffers A = adj_bind(c, 1 - cur, nullptr);
         UGKS_CK(enqueue_targets_adjoint(c->P, slot_lo(c, s0), c->T[0], g.T, g.W, A, c->stream));
-        c->launches += s2_enqueue_kernels(3) + 2;
+        c->launches += s2_enqueue_kernels(3, c->P, c->T[1]) + 2;
         if (int r = adj_status(c)) return r;
     }
     return adj_download(c, g, gh0, gb0, gW0, grad);
@@ -1618,7 +1618,7 @@ extern "C" int ugks_s2cn2_step_vjp(ugks_ctx* c, const double* gh, const double* 
     UGKS_CK(enqueue_s2cn2_adjoint(c->P, B0, c->T[0], c->T[0], c->T[1], rerun_cn(c), A, c->stream, c->stream2, c->adj_ev));
     UGKS_CK(s2_enqueue(3, c->P, B0, c->T[1], c->stream, c->stream, nullptr, nullptr));   // W's targets, for their adjoint
     UGKS_CK(enqueue_targets_adjoint(c->P, B0, c->T[0], in.T, in.W, A, c->stream));
-    c->launches += kAdjStepKernels + s2_enqueue_kernels(3) + 2;
+    c->launches += kAdjStepKernels + s2_enqueue_kernels(3, c->P, c->T[1]) + 2;
     if (int r = adj_status(c)) return r;
     return adj_download(c, in, gh_in, gb_in, gW_in, grad);
 }

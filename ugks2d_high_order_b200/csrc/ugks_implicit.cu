@@ -1620,7 +1620,7 @@ cudaError_t enqueue_implicit_step(const LoParams& P, const LoBuffers& B, const I
     // conditional body, not counted here: it runs only when no accepted-state evaluation applies
     // (counted once per sequence by ugks_implicit_init / ugks_implicit_restore); the gate replaces the
     // pre-update residual in the count
-    const int evaluation = Q.high_order ? s2_enqueue_kernels(1) : 3;
+    const int evaluation = Q.high_order ? s2_enqueue_kernels(1, P, I.s2) : 3;
     if (launches) *launches += 10 + (cond ? evaluation : 2 * evaluation);
     return e;
 }

@@ -445,83 +445,16 @@ __global__ void __launch_bounds__(128, 3) k_s2_target_nodes_t(LoParams P, LoBuff
     o[24 + gl] = C.jac[8 + gl];
 }
 
-// build_targets, sum part, on a tensor table: one CTA per cell and 1024 velocities.  The 9 nodes' Maxwellians are
-// products of two rows of exponentials (shared memory, the Gauss weight and rho / (pi T) folded into the x
-// row), and M, K_x, K_y the product times a cubic in the velocity whose coefficients are the node's.
-struct S2TargetC {   // one node: mean of theta, mean of the state, ck T / 2, the cubic's coefficients
-    double u, v, ux, vy, ckh, sl, s0, kb;   // Shakhov factor sl c^2 - s0; kb = 2 coeff / ck
-    double x[5], y[5];                      // direction polynomial 1, cx, cy, c^2 of K_x and K_y, and its b part
-};
+// build_targets, sum part, on a tensor table: one CTA per cell and 1024 velocities (STargets, ugks_s2_tensor.cuh)
 __global__ void __launch_bounds__(256) k_s2_target_sum_t(LoParams P, LoBuffers B, S2Buffers SB) {
     if (eval_cached(B)) return;
-    __shared__ double ex[9][64], ey[9][64];
-    __shared__ S2TargetC sc[9];
-    const int nv = P.nvel, nu = P.tnu, nw = P.tnv, cc = blockIdx.y, tid = threadIdx.x;
-    const double gw[3] = {5.0 / 18.0, 4.0 / 9.0, 5.0 / 18.0};
-    if (tid < 9) {
-        double th[4];
-        WMke M;
-        w_load_scalars(SB.tscal + ((size_t)cc * 9 + tid) * kS2TScal, th, M);
-        const S2Th t = s2_th(th, P.ck);
-        S2TargetC& c = sc[tid];
-        c.u = t.u; c.v = t.v; c.ux = M.ux; c.vy = M.vy; c.ckh = t.ckh;
-        c.sl = 2.0 * M.lam * M.coeff; c.s0 = 4.0 * M.coeff; c.kb = 2.0 / (double)P.ck * M.coeff;
-        const double i2 = t.itw * t.itw;
-#pragma unroll
-        for (int d = 0; d < 2; ++d) {
-            const double* td = d ? M.tdy : M.tdx;
-            double* p = d ? c.y : c.x;
-            p[0] = td[0] * t.ir - td[3] * t.itw;
-            p[1] = 2.0 * t.itw * td[1];
-            p[2] = 2.0 * t.itw * td[2];
-            p[3] = td[3] * i2;
-            p[4] = td[3] * t.itw;
-        }
-    }
-    for (int q = tid; q < 9 * (nu + nw); q += blockDim.x) {
-        const int p = q / (nu + nw), a = q - p * (nu + nw);
-        const double* o = SB.tscal + ((size_t)cc * 9 + p) * kS2TScal;
-        const double itw = 1.0 / o[3];
-        if (a < nu) {
-            const double d = B.tab[a] - o[1];
-            ex[p][a] = gw[p % 3] * gw[p / 3] * (o[0] / (kPi * o[3])) * exp(-(d * d) * itw);
-        } else {
-            const double d = B.tab[128 + a - nu] - o[2];
-            ey[p][a - nu] = exp(-(d * d) * itw);
-        }
-    }
+    __shared__ STargets st;
+    const int nv = P.nvel, cc = blockIdx.y;
+    st.fill(P, B, SB, cc);
     __syncthreads();
-    double a[4][6], uk[4], vk[4];
-    int iu[4], iv[4];
-    const int k0 = blockIdx.x * 1024 + tid;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int k = min(k0 + r * (int)blockDim.x, nv - 1);
-        iv[r] = k / nu;
-        iu[r] = k - iv[r] * nu;
-        uk[r] = B.tab[iu[r]];
-        vk[r] = B.tab[128 + iv[r]];
-#pragma unroll
-        for (int m = 0; m < 6; ++m) a[r][m] = 0.0;
-    }
-#pragma unroll 1
-    for (int p = 0; p < 9; ++p) {
-        const S2TargetC& c = sc[p];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const double q = ex[p][iu[r]] * ey[p][iv[r]], qb = c.ckh * q;
-            const double cx = uk[r] - c.u, cy = vk[r] - c.v, px = uk[r] - c.ux, py = vk[r] - c.vy;
-            const double c2 = cx * cx + cy * cy, sh = c.sl * (px * px + py * py) - c.s0;
-            const double kx = px * sh - (c.x[0] + c.x[1] * cx + c.x[2] * cy + c.x[3] * c2);
-            const double ky = py * sh - (c.y[0] + c.y[1] * cx + c.y[2] * cy + c.y[3] * c2);
-            a[r][0] += q;
-            a[r][1] += qb;
-            a[r][2] += q * kx;
-            a[r][3] += qb * (kx + c.kb * px - c.x[4]);
-            a[r][4] += q * ky;
-            a[r][5] += qb * (ky + c.kb * py - c.y[4]);
-        }
-    }
+    double a[4][6];
+    const int k0 = blockIdx.x * 1024 + threadIdx.x;
+    st.at<4>(P, B, k0, blockDim.x, a);
     double* out[6] = {SB.mh, SB.mb, SB.kxh, SB.kxb, SB.kyh, SB.kyb};
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -1526,7 +1459,7 @@ static int qrec_bytes(const S2Buffers& S, int nv, int threads, int cap) {
 
 
 // which 0: the S2 cold start; 1: the S2 Evolution of one pseudo-step (targets, reconstruction,
-// faces, walls); 2: the Evolution with the targets kept (S2CN2); 3: the targets of B.W only
+// faces, walls); 2: the Evolution with the targets kept (S2CN2); 3: the targets of B.W only; 5: their node scalars alone
 cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S2Buffers& S, cudaStream_t s,
                        cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join) {
     const int nx = P.nx, ny = P.ny, nv = P.nvel, nc = nx * ny, nf = nx * ny + nx * (ny - 1);
@@ -1539,12 +1472,12 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
     if (which == 4) {
         return launch_recon(P, B, S, s);
     }
-    const int faces = which != 3, targets = which != 2;
+    const int faces = which < 3, targets = which != 2;
     const long long nmacw = (faces ? (long long)nf * 2 : 0) + (targets ? (long long)nc : 0);   // warps
     // The macro pass feeds the targets and the face nodes, the reconstruction neither of them: with an evolution it runs on
     // the side stream beside the reconstruction (S2CN2 step 381 -> 378 us, HighOrderImplicit pseudo-step 519 -> 510
     // at 8x64x32^2), followed there by the targets of which 1 (first read after the face
-    // arrays) and, after the reconstruction, the wall nodes; which 3: everything on the main stream
+    // arrays) and, after the reconstruction, the wall nodes; which 3 and 5: everything on the main stream
     cudaStream_t ts = faces ? s2 : s;
     cudaError_t e = cudaSuccess;
     if (faces) {
@@ -1565,7 +1498,7 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
             else if (n <= 48) k_s2_target_nodes_t<6><<<g, 128, 0, ts>>>(P, B, S);
             else k_s2_target_nodes_t<8><<<g, 128, 0, ts>>>(P, B, S);
             const int nt = std::min(256, (nv + 127) / 128 * 32);
-            k_s2_target_sum_t<<<dim3((unsigned)((nv + 1023) / 1024), (unsigned)nc), nt, 0, ts>>>(P, B, S);
+            if (which != 5) k_s2_target_sum_t<<<dim3((unsigned)((nv + 1023) / 1024), (unsigned)nc), nt, 0, ts>>>(P, B, S);
             e = cudaGetLastError();
         } else {
             const int qb = qrec_bytes(S, nv, 256, kQRecCap256x2);
@@ -1577,7 +1510,7 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
             }
         }
     }
-    if (e != cudaSuccess || which == 3) return e;
+    if (e != cudaSuccess || !faces) return e;
     // a tensor table's faces and walls: the fused fluxes, unless a wall variant wants the nodes' fluxes and coefficients
     const bool tensor = P.tnu > 0, fused = tensor && S.coef == nullptr;
     e = launch_recon(P, B, S, s);

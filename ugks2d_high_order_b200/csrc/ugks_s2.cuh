@@ -105,14 +105,19 @@ __device__ __forceinline__ bool s2_primitive(const double w[4], int ck, double& 
 cudaError_t prepare_s2();
 // which 0: S2 cold start (h, b := discrete closure Maxwellian of W); 1: S2 Evolution (targets of B.W,
 // reconstruction, faces, walls); 2: S2 Evolution with the targets in S kept; 3: targets of B.W into S;
-// 4: the reconstruction of B's h, b into S.rec only
+// 4: the reconstruction of B's h, b into S.rec only; 5: the node scalars of the targets of B.W into S only
 cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S2Buffers& S, cudaStream_t s,
                        cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join);
 // kernels s2_enqueue(which, ...) launches: the cold start 1; the macro pass, then 2 for the targets
-// (volume nodes, sum) and 6 for the evolution (reconstruction x2, wall nodes, face nodes, face flux,
-// combine); the reconstruction alone 2
-constexpr int s2_enqueue_kernels(int which) {
-    return which == 0 ? 1 : which == 4 ? 2 : 1 + (which != 2 ? 2 : 0) + (which != 3 ? 6 : 0);
+// (volume nodes, sum; 5: the nodes alone) and 6 for the evolution (reconstruction x2, walls, and for the faces
+// nodes, flux, combine or, on a tensor table, moments, nodes, flux), with one more combine on a tensor table for the
+// wall variants that store node fluxes; the reconstruction alone 2
+inline int s2_enqueue_kernels(int which, const LoParams& P, const S2Buffers& S) {
+    if (which == 0) return 1;
+    if (which == 4) return 2;
+    if (which == 5) return 2;
+    const int faces = which == 3 ? 0 : 6 + (P.tnu > 0 && (S.coef != nullptr || P.s2_kinetic) ? 1 : 0);
+    return 1 + (which != 2 ? 2 : 0) + faces;
 }
 // the wall nodes of the kinetic (FluxWall_type 0) wall into S.node / S.nodew (ugks_s2_walls.cu)
 cudaError_t launch_s2_w1_walls(const LoParams& P, const LoBuffers& B, const S2Buffers& S, cudaStream_t s);

@@ -227,5 +227,89 @@ __device__ bool t_mke(const LoParams& P, const LoBuffers& B, const double w[4], 
     return pok && ok && C.res <= 2.0e-12;
 }
 
+// build_targets' sums (mod_S2D1.f90:1246-1300) of one cell in shared memory: its 9 nodes' Maxwellians as products of two
+// rows of exponentials (the Gauss weight and rho / (pi T) folded into the x row), and M, K_x, K_y the product times a
+// cubic in the velocity whose coefficients are the node's.
+struct STargetNode {   // mean of theta, mean of the state, ck T / 2, the cubic's coefficients
+    double u, v, ux, vy, ckh, sl, s0, kb;   // Shakhov factor sl c^2 - s0; kb = 2 coeff / ck
+    double x[5], y[5];                      // direction polynomial 1, cx, cy, c^2 of K_x and K_y, and its b part
+};
+struct STargets {
+    double ex[9][64], ey[9][64];
+    STargetNode n[9];
+    // by the whole CTA, from the node scalars; followed by a barrier
+    __device__ __forceinline__ void fill(const LoParams& P, const LoBuffers& B, const S2Buffers& SB, int cc) {
+        const int nu = P.tnu, nw = P.tnv, tid = threadIdx.x;
+        const double gw[3] = {5.0 / 18.0, 4.0 / 9.0, 5.0 / 18.0};
+        if (tid < 9) {
+            double th[4];
+            WMke M;
+            w_load_scalars(SB.tscal + ((size_t)cc * 9 + tid) * kS2TScal, th, M);
+            const S2Th t = s2_th(th, P.ck);
+            STargetNode& c = n[tid];
+            c.u = t.u; c.v = t.v; c.ux = M.ux; c.vy = M.vy; c.ckh = t.ckh;
+            c.sl = 2.0 * M.lam * M.coeff; c.s0 = 4.0 * M.coeff; c.kb = 2.0 / (double)P.ck * M.coeff;
+            const double i2 = t.itw * t.itw;
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+                const double* td = d ? M.tdy : M.tdx;
+                double* p = d ? c.y : c.x;
+                p[0] = td[0] * t.ir - td[3] * t.itw;
+                p[1] = 2.0 * t.itw * td[1];
+                p[2] = 2.0 * t.itw * td[2];
+                p[3] = td[3] * i2;
+                p[4] = td[3] * t.itw;
+            }
+        }
+        for (int q = tid; q < 9 * (nu + nw); q += blockDim.x) {
+            const int p = q / (nu + nw), a = q - p * (nu + nw);
+            const double* o = SB.tscal + ((size_t)cc * 9 + p) * kS2TScal;
+            const double itw = 1.0 / o[3];
+            if (a < nu) {
+                const double d = B.tab[a] - o[1];
+                ex[p][a] = gw[p % 3] * gw[p / 3] * (o[0] / (kPi * o[3])) * exp(-(d * d) * itw);
+            } else {
+                const double d = B.tab[128 + a - nu] - o[2];
+                ey[p][a - nu] = exp(-(d * d) * itw);
+            }
+        }
+    }
+    // M, K_x, K_y (h and b each) of the velocities k0, k0 + step, ... (those past the table take its last one)
+    template <int VPT>
+    __device__ __forceinline__ void at(const LoParams& P, const LoBuffers& B, int k0, int step, double a[VPT][6]) const {
+        const int nu = P.tnu;
+        double uk[VPT], vk[VPT];
+        int iu[VPT], iv[VPT];
+#pragma unroll
+        for (int r = 0; r < VPT; ++r) {
+            const int k = min(k0 + r * step, P.nvel - 1);
+            iv[r] = k / nu;
+            iu[r] = k - iv[r] * nu;
+            uk[r] = B.tab[iu[r]];
+            vk[r] = B.tab[128 + iv[r]];
+#pragma unroll
+            for (int m = 0; m < 6; ++m) a[r][m] = 0.0;
+        }
+#pragma unroll 1
+        for (int p = 0; p < 9; ++p) {
+            const STargetNode& c = n[p];
+#pragma unroll
+            for (int r = 0; r < VPT; ++r) {
+                const double q = ex[p][iu[r]] * ey[p][iv[r]], qb = c.ckh * q;
+                const double cx = uk[r] - c.u, cy = vk[r] - c.v, px = uk[r] - c.ux, py = vk[r] - c.vy;
+                const double c2 = cx * cx + cy * cy, sh = c.sl * (px * px + py * py) - c.s0;
+                const double kx = px * sh - (c.x[0] + c.x[1] * cx + c.x[2] * cy + c.x[3] * c2);
+                const double ky = py * sh - (c.y[0] + c.y[1] * cx + c.y[2] * cy + c.y[3] * c2);
+                a[r][0] += q;
+                a[r][1] += qb;
+                a[r][2] += q * kx;
+                a[r][3] += qb * (kx + c.kb * px - c.x[4]);
+                a[r][4] += q * ky;
+                a[r][5] += qb * (ky + c.kb * py - c.y[4]);
+            }
+        }
+    }
+};
+
 }  // namespace
 }  // namespace ugks

@@ -318,9 +318,9 @@ __global__ void __launch_bounds__(256) k_w2r_walls(LoParams P, LoBuffers B, cons
 int s2cn2_variant_kernels(const LoParams& P) {
     int n = 0;
     if (P.s2_midpoint)
-        n += 1 + s2_enqueue_kernels(2) + 1 + 1 + s2_enqueue_kernels(3) + s2_enqueue_kernels(4) + 1 +
+        n += 1 + s2_enqueue_kernels(2, P, S2Buffers{}) + 1 + cn_apply_kernels(P, S2Buffers{}) + s2_enqueue_kernels(4, P, S2Buffers{}) + 1 +
              (P.s2_face_time ? 1 : 0) + 1;
-    if (P.s2_shared) n += 1 + s2_enqueue_kernels(4) + 1 + 1;
+    if (P.s2_shared) n += 1 + s2_enqueue_kernels(4, P, S2Buffers{}) + 1 + 1;
     return n;
 }
 

@@ -21,6 +21,7 @@
 //                    stays in its set).
 // The state and the targets are double-buffered: a step reads set p and writes set 1-p, so a
 // rejected proposal never touches the accepted state and nothing is copied on acceptance.
+#include "ugks_s2_tensor.cuh"
 #include "ugks_s2cn2.cuh"
 
 namespace ugks {
@@ -123,41 +124,69 @@ __global__ void __launch_bounds__(NT) k_cn_stream(LoParams P, LoBuffers B, S2Buf
 
 // ------------------------------------------------------------------------------------------
 // the CN collision of advance_step (mod_S2D1.f90:1376-1421): one CTA per cell, then the step's
-// acceptance in the last CTA
-template <int VPT, int NT>
-__global__ void __launch_bounds__(NT) k_cn_collide(LoParams P, LoBuffers B, S2Buffers Tn, CnBuffers C, LoBuffers Bo) {
+// acceptance in the last CTA.  The targets of the stream state stay in registers through both passes; on a tensor
+// velocity table the CTA also forms them from the node scalars (STargets) and writes them for the next step, instead of
+// reading what a kernel of its own stored.  Bound by the barriers around its three reductions at 16 warps an SM; with
+// 6 maxima instead of 11 in the last one the S2CN2 step at 8x64x32^2 went from 378 to 372 us and the 16-instance
+// batch from 6.6 to 6.5 ms a step.  512 threads (2 velocities each, 64 registers) took 390 us, 128 threads (8) 387,
+// three CTAs an SM (80 registers) 404.
+template <int VPT, int NT, bool TENSOR>
+__global__ void __launch_bounds__(NT, 512 / NT) k_cn_collide(LoParams P, LoBuffers B, S2Buffers Tn, CnBuffers C, LoBuffers Bo) {
     if (halted(B)) return;
     __shared__ double red[16 * 64];
     __shared__ double rout[kRedSlots];
     __shared__ double sc[8];   // [0] beta [1] ux [2] vy [3] ok [4] max 2 beta [5..6] q_new [7] solve ok
     __shared__ unsigned s_last;
+    __shared__ double s_targets[TENSOR ? sizeof(STargets) / sizeof(double) : 1];
     const int nv = P.nvel, tid = threadIdx.x, c = blockIdx.x;
     const double dt = B.dt[0];
     const double* wn = C.ws + c * 4;
-    if (tid == 0) {
+    if (tid == NT - 1) {
         double tau_o = 1.0, tau_n = 1.0, rho, ux = 0.0, vy = 0.0, th;
         const bool ok = s2_tau(P, B.W + c * 4, tau_o) && s2_tau(P, wn, tau_n) && s2_primitive(wn, P.ck, rho, ux, vy, th);
         const double beta_old = dt / (2.0 * tau_o), beta = dt / (2.0 * tau_n);
         sc[0] = ok ? beta : 0.0; sc[1] = ux; sc[2] = vy; sc[3] = ok ? 1.0 : 0.0;
         sc[4] = fmax(2.0 * beta_old, 2.0 * beta);
     }
-    __syncthreads();
+    double rh[VPT], rb[VPT], T[VPT][6], acc[16];   // T: M, K_x, K_y
+#pragma unroll
+    for (int r = 0; r < VPT; ++r) {
+        const size_t q = (size_t)c * nv + slot(r, nv).kk;
+        rh[r] = C.rh[q];
+        rb[r] = C.rb[q];
+        if (!TENSOR) {
+            T[r][0] = Tn.mh[q]; T[r][1] = Tn.mb[q]; T[r][2] = Tn.kxh[q];
+            T[r][3] = Tn.kxb[q]; T[r][4] = Tn.kyh[q]; T[r][5] = Tn.kyb[q];
+        }
+    }
+    if (TENSOR) {
+        STargets& st = *reinterpret_cast<STargets*>(s_targets);
+        st.fill(P, B, Tn, c);
+        __syncthreads();
+        st.at<VPT>(P, B, tid, NT, T);
+        double* out[6] = {Tn.mh, Tn.mb, Tn.kxh, Tn.kxb, Tn.kyh, Tn.kyb};
+#pragma unroll
+        for (int r = 0; r < VPT; ++r) {
+            const Slot s = slot(r, nv);
+            if (s.ok)
+#pragma unroll
+                for (int m = 0; m < 6; ++m) out[m][(size_t)c * nv + s.k] = T[r][m];
+        }
+    } else {
+        __syncthreads();
+    }
     const double beta = sc[0], ux = sc[1], vy = sc[2];
-    double rh[VPT], rb[VPT], acc[17];
 #pragma unroll
     for (int m = 0; m < 8; ++m) acc[m] = 0.0;
 #pragma unroll
     for (int r = 0; r < VPT; ++r) {
         const Slot s = slot(r, nv);
-        const size_t q = (size_t)c * nv + s.kk;
         const double uk = B.u[s.kk], vk = B.v[s.kk], wk = s.ok ? B.w[s.kk] : 0.0;
         const double cx = uk - ux, cy = vk - vy;
-        rh[r] = C.rh[q];
-        rb[r] = C.rb[q];
         heat_add(wk, cx, cy, rh[r], rb[r], acc);
-        heat_add(wk, cx, cy, Tn.mh[q], Tn.mb[q], acc + 2);
-        heat_add(wk, cx, cy, Tn.kxh[q], Tn.kxb[q], acc + 4);   // kappa(:,1) of build_targets
-        heat_add(wk, cx, cy, Tn.kyh[q], Tn.kyb[q], acc + 6);   // kappa(:,2)
+        heat_add(wk, cx, cy, T[r][0], T[r][1], acc + 2);
+        heat_add(wk, cx, cy, T[r][2], T[r][3], acc + 4);   // kappa(:,1) of build_targets
+        heat_add(wk, cx, cy, T[r][4], T[r][5], acc + 6);   // kappa(:,2)
     }
     block_reduce_smem<8, 0>(acc, red, rout);
     if (tid == 0) {
@@ -175,49 +204,48 @@ __global__ void __launch_bounds__(NT) k_cn_collide(LoParams P, LoBuffers B, S2Bu
     }
     __syncthreads();
     const double r0 = sc[5], r1 = sc[6], opb = 1.0 + beta;
-    // sums: [0..1] heat(hn - M_new), [2..5] moments(hn, bn); maxima: [6..9] |rh| |rb| |hn| |bn|,
-    // [10..11] CN equation residuals, [12..15] -min hn, max hn, -min bn, max bn, [16] nonfinite
+    // sums: [0..1] heat(hn - M_new), [2..5] moments(hn, bn); maxima: [6] |rh|, |rb|, [7] the CN equation's
+    // residuals, [8..11] -min hn, max hn, -min bn, max bn (|hn|, |bn| follow from them)
+    const double iopb = 1.0 / opb;
+    int bad = 0;
 #pragma unroll
     for (int m = 0; m < 6; ++m) acc[m] = 0.0;
 #pragma unroll
-    for (int m = 6; m < 17; ++m) acc[m] = -INFINITY;
+    for (int m = 6; m < 12; ++m) acc[m] = -INFINITY;
 #pragma unroll
     for (int r = 0; r < VPT; ++r) {
         const Slot s = slot(r, nv);
-        const size_t q = (size_t)c * nv + s.kk;
         const double uk = B.u[s.kk], vk = B.v[s.kk], wk = s.ok ? B.w[s.kk] : 0.0;
-        const double mh = Tn.mh[q], mb = Tn.mb[q];
-        const double eqh = mh + Tn.kxh[q] * r0 + Tn.kyh[q] * r1;
-        const double eqb = mb + Tn.kxb[q] * r0 + Tn.kyb[q] * r1;
-        const double hn = (rh[r] + beta * eqh) / opb;
-        const double bn = (rb[r] + beta * eqb) / opb;
+        const double mh = T[r][0], mb = T[r][1];
+        const double eqh = mh + T[r][2] * r0 + T[r][4] * r1;
+        const double eqb = mb + T[r][3] * r0 + T[r][5] * r1;
+        const double hn = (rh[r] + beta * eqh) * iopb;
+        const double bn = (rb[r] + beta * eqb) * iopb;
         heat_add(wk, uk - ux, vk - vy, hn - mh, bn - mb, acc);
         moment_add(wk, uk, vk, hn, bn, acc + 2);
+        // a slot past the table repeats its last velocity, which changes no maximum
+        acc[6] = fmax(acc[6], fmax(fabs(rh[r]), fabs(rb[r])));
+        acc[7] = fmax(acc[7], fmax(fabs(opb * hn - rh[r] - beta * eqh), fabs(opb * bn - rb[r] - beta * eqb)));
+        acc[8] = fmax(acc[8], -hn);
+        acc[9] = fmax(acc[9], hn);
+        acc[10] = fmax(acc[10], -bn);
+        acc[11] = fmax(acc[11], bn);
+        if (!(isfinite(hn) && isfinite(bn))) bad = 1;
         if (s.ok) {
-            acc[6] = fmax(acc[6], fabs(rh[r]));
-            acc[7] = fmax(acc[7], fabs(rb[r]));
-            acc[8] = fmax(acc[8], fabs(hn));
-            acc[9] = fmax(acc[9], fabs(bn));
-            acc[10] = fmax(acc[10], fabs(opb * hn - rh[r] - beta * eqh));
-            acc[11] = fmax(acc[11], fabs(opb * bn - rb[r] - beta * eqb));
-            acc[12] = fmax(acc[12], -hn);
-            acc[13] = fmax(acc[13], hn);
-            acc[14] = fmax(acc[14], -bn);
-            acc[15] = fmax(acc[15], bn);
-            acc[16] = fmax(acc[16], (isfinite(hn) && isfinite(bn)) ? 0.0 : 1.0);
             Bo.h[(size_t)c * nv + s.k] = hn;
             Bo.b[(size_t)c * nv + s.k] = bn;
         }
     }
-    block_reduce_smem<6, 11>(acc, red, rout);
+    block_reduce_smem<6, 6>(acc, red, rout);
+    bad = __syncthreads_or(bad);
     if (tid == 0) {
-        const double scale = fmax(fmax(fmax(fmax(1.0, rout[6]), rout[7]), rout[8]), rout[9]);
-        double cres = fmax(rout[10], rout[11]) / scale;
+        const double scale = fmax(fmax(fmax(1.0, rout[6]), fmax(rout[8], rout[9])), fmax(rout[10], rout[11]));
+        double cres = rout[7] / scale;
         const double rh0 = rout[0], rh1 = rout[1];
         cres = fmax(cres, fmax(fabs(rh0 - r0), fabs(rh1 - r1)) /
                               fmax(fmax(1.0, fmax(fabs(rh0), fabs(rh1))), fmax(fabs(r0), fabs(r1))));
         double mx = 0.0, ws = 1.0;
-        bool fin = sc[7] != 0.0 && rout[16] == 0.0;
+        bool fin = sc[7] != 0.0 && !bad;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             mx = fmax(mx, fabs(rout[2 + m] - wn[m]));
@@ -229,7 +257,7 @@ __global__ void __launch_bounds__(NT) k_cn_collide(LoParams P, LoBuffers B, S2Bu
         d[0] = sc[4];
         d[1] = isfinite(cres) ? cres : INFINITY;
         d[2] = isfinite(mx / ws) ? mx / ws : INFINITY;
-        d[3] = -rout[12]; d[4] = rout[13]; d[5] = -rout[14]; d[6] = rout[15];
+        d[3] = -rout[8]; d[4] = rout[9]; d[5] = -rout[10]; d[6] = rout[11];
         d[7] = fin ? 0.0 : 1.0;
         if (!C.predict) {   // the proposal's dt_local: the next step's TimeStep when the step is accepted
             bool okd;
@@ -348,9 +376,11 @@ static cudaError_t cn_apply_launch(const LoParams& P, const LoBuffers& B, const 
                                    const CnBuffers& C, cudaStream_t s) {
     LoBuffers Bw = B;   // the targets of the stream state
     Bw.W = C.ws;
-    cudaError_t e = s2_enqueue(3, P, Bw, To, s, s, nullptr, nullptr);
+    const bool tensor = P.tnu > 0;   // the collision forms the targets from their node scalars
+    cudaError_t e = s2_enqueue(tensor ? 5 : 3, P, Bw, To, s, s, nullptr, nullptr);
     if (e != cudaSuccess) return e;
-    k_cn_collide<VPT, NT><<<P.nx * P.ny, NT, 0, s>>>(P, B, To, C, Bo);
+    if (tensor) k_cn_collide<VPT, NT, true><<<P.nx * P.ny, NT, 0, s>>>(P, B, To, C, Bo);
+    else k_cn_collide<VPT, NT, false><<<P.nx * P.ny, NT, 0, s>>>(P, B, To, C, Bo);
     return cudaGetLastError();
 }
 
@@ -361,7 +391,7 @@ cudaError_t enqueue_cn_stream(const LoParams& P, const LoBuffers& B, const S2Buf
 
 cudaError_t enqueue_cn_apply(const LoParams& P, const LoBuffers& B, const LoBuffers& Bo, const S2Buffers& To,
                              const CnBuffers& C, cudaStream_t s) {
-    return P.nvel <= 1024 ? cn_apply_launch<4, 256>(P, B, Bo, To, C, s) : cn_apply_launch<10, 256>(P, B, Bo, To, C, s);
+    return P.nvel <= 1024 ? cn_apply_launch<4, 256>(P, B, Bo, To, C, s) : cn_apply_launch<5, 512>(P, B, Bo, To, C, s);
 }
 
 // Report (C.report) of the step: [0] dt, [1] cnres, [2] mmerr, [3] max 2 beta, [4] transport CFL,
@@ -376,7 +406,7 @@ cudaError_t enqueue_s2cn2_step(const LoParams& P, const LoBuffers& B, const S2Bu
     if (e == cudaSuccess && V) e = enqueue_s2cn2_variant(P, B, T, *V, s, s2, fork, join);
     if (e == cudaSuccess) e = enqueue_cn_stream(P, B, T, C, s);
     if (e == cudaSuccess) e = enqueue_cn_apply(P, B, Bo, To, C, s);
-    if (launches) *launches += kCnStepKernels - (timestep ? 0 : 1) + (V ? s2cn2_variant_kernels(P) : 0);
+    if (launches) *launches += cn_step_kernels(P, T) - (timestep ? 0 : 1) + (V ? s2cn2_variant_kernels(P) : 0);
     return e;
 }
 
@@ -385,7 +415,7 @@ cudaError_t enqueue_s2cn2_prepare(const LoParams& P, const LoBuffers& B, const S
     k_cn_ledger<<<1, 256, 0, s>>>(P, B, C);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = s2_enqueue(3, P, B, T, s, s, nullptr, nullptr);
-    if (launches) *launches += 1 + s2_enqueue_kernels(3);
+    if (launches) *launches += 1 + s2_enqueue_kernels(3, P, T);
     return e;
 }
 

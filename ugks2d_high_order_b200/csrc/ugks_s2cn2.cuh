@@ -6,10 +6,12 @@ namespace ugks {
 
 constexpr int kCnCell = 8;     // per-cell advance diagnostics
 constexpr int kCnReport = 24;  // report of the last step (layout at enqueue_s2cn2_step)
-// kernels of one S2CN2 step: timestep, the evolution keeping the targets, k_cn_stream, the targets of
-// the stream state, k_cn_collide
-constexpr int kCnStepKernels = 1 + s2_enqueue_kernels(2) + 1 + s2_enqueue_kernels(3) + 1;
-static_assert(kCnStepKernels == 13, "one S2CN2 step launches 13 kernels");
+// kernels of the second half of a step (the targets of the stream state and k_cn_collide, which forms the targets itself
+// on a tensor table), and of a whole step: timestep, the evolution keeping the targets, k_cn_stream, that half
+inline int cn_apply_kernels(const LoParams& P, const S2Buffers& T) { return s2_enqueue_kernels(P.tnu > 0 ? 5 : 3, P, T) + 1; }
+inline int cn_step_kernels(const LoParams& P, const S2Buffers& T) {
+    return 1 + s2_enqueue_kernels(2, P, T) + 1 + cn_apply_kernels(P, T);
+}
 
 struct CnBuffers {
     double* ws;          // [nc][4]    stream state W + res_w (the proposal's W)
