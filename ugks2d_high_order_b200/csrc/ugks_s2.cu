@@ -29,8 +29,8 @@
 namespace ugks {
 
 // ------------------------------------------------------------------------------------------
-// reconstruction + limiter in two passes into the face cache (rec_cell / rec_wall, ugks_s2.cuh; fields: h,
-// b, h_n, h_t, b_n, b_t; sides: x left, x right, y bottom, y top).
+// reconstruction + limiter in two passes into the face cache (rec_cell / rec_wall, ugks_s2.cuh; sides: x left, x right,
+// y bottom, y top).
 //
 // k_s2_recon1, the first layer (prepare_first_layer_plane, mod_S2D1Reconstruction.f90:501-578):
 // per (cell, velocity, field) the 1-D WENO along x of the cell's own row -- values and derivatives
@@ -156,17 +156,17 @@ __device__ __forceinline__ void s2_recon2_wall(const LoParams& P, const LoBuffer
     // here, exact when dx and dy are powers of two (the delivered meshes), within an ulp otherwise
     const double ind = 1.0 / (axis == 0 ? P.dx : P.dy), itd = 1.0 / (axis == 0 ? P.dy : P.dx);
     const int fv = f == 0 ? 0 : 1, fn = f == 0 ? 2 : 4, ft = f == 0 ? 3 : 5;
+    const double uk = B.u[k], vk = B.v[k];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-        const bool store = kok && rec_leaves(2 * axis + s, B.u[k], B.v[k]);
+        const bool store = kok && rec_leaves(2 * axis + s, uk, vk);
         const bool wall = kok && axis == 1 && ((s == 0 && j == 0) || (s == 1 && j == ny - 1));
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const double v = mf + theta * (face[s][a] - mf), n = theta * dn[s][a] * ind, t = theta * dt[s][a] * itd;
             if (store) {
-                S.rec[rec_cell(cc, axis, fv, a, nv) + k] = v;
-                S.rec[rec_cell(cc, axis, fn, a, nv) + k] = n;
-                S.rec[rec_cell(cc, axis, ft, a, nv) + k] = t;
+                S.rec[rec_cell(cc, axis, f, a, nv) + k] = v;
+                S.rec[rec_cell(cc, axis, 2 + f, a, nv) + k] = axis == 0 ? uk * n + vk * t : vk * n + uk * t;
             }
             if (wall) {
                 S.rec[rec_wall(nx, ny, s, i, fv, a, nv) + k] = v;
@@ -199,11 +199,11 @@ __global__ void __launch_bounds__(kRecon2Threads, 8) k_s2_recon2(LoParams P, LoB
     const size_t st = (size_t)22 * nv, rowst = st * nx;
     const double* L1 = S.l1 + (size_t)f * 11 * nv + k + (size_t)cc * st;
     const double hm = B.h[(size_t)cc * nv + k], bm = B.b[(size_t)cc * nv + k], mf = f == 0 ? hm : bm;
-    const int fv = f == 0 ? 0 : 1, fn = f == 0 ? 2 : 4, ft = f == 0 ? 3 : 5;
     double xmin = 0.0, sum = 0.0;   // sum: a value of every template with all its coefficients, for their finiteness
 #pragma unroll
     for (int axis = 0; axis < 2; ++axis) {
-        const bool hi = (axis == 0 ? B.u[k] : B.v[k]) >= 0.0;   // the upper side is the leaving one
+        const double vn = axis == 0 ? B.u[k] : B.v[k], vt = axis == 0 ? B.v[k] : B.u[k];
+        const bool hi = vn >= 0.0;   // the upper side is the leaving one
         const double* L = L1 + (size_t)(axis == 0 ? 0 : 7) * nv;
         const double *Lv = L + (size_t)(hi ? 2 : 0) * nv, *Lo = L + (size_t)(hi ? 0 : 2) * nv;
         double a5[5], b5[5], o5[5], face[3], dn[3], dt[3], ov[3];
@@ -219,16 +219,15 @@ __global__ void __launch_bounds__(kRecon2Threads, 8) k_s2_recon2(LoParams P, LoB
         s2_power_values3(o5, ov);
         // the derivatives are divided by the cell sizes (limit_cell_outputs): multiplied by the reciprocals
         // here, exact when dx and dy are powers of two (the delivered meshes), within an ulp otherwise
-        const double ind = 1.0 / (axis == 0 ? P.dx : P.dy), itd = 1.0 / (axis == 0 ? P.dy : P.dx);
+        const double in = vn * (1.0 / (axis == 0 ? P.dx : P.dy)), it = vt * (1.0 / (axis == 0 ? P.dy : P.dx));
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             xmin = s2_min(s2_min(xmin, face[a]), ov[a]);
-            const double n = dn[a] * ind, t = dt[a] * itd;
-            if (a == 2) sum += (face[a] + n) + (t + ov[a]);
+            const double path = in * dn[a] + it * dt[a];
+            if (a == 2) sum += (face[a] + path) + ov[a];
             if (kok) {   // unlimited: theta is 1 but for a few cells and velocities
-                S.rec[rec_cell(cc, axis, fv, a, nv) + k] = face[a];
-                S.rec[rec_cell(cc, axis, fn, a, nv) + k] = n;
-                S.rec[rec_cell(cc, axis, ft, a, nv) + k] = t;
+                S.rec[rec_cell(cc, axis, f, a, nv) + k] = face[a];
+                S.rec[rec_cell(cc, axis, 2 + f, a, nv) + k] = path;
             }
         }
     }
@@ -253,10 +252,9 @@ __global__ void __launch_bounds__(kRecon2Threads, 8) k_s2_recon2(LoParams P, LoB
         for (int axis = 0; axis < 2; ++axis)
 #pragma unroll 1
             for (int a = 0; a < 3; ++a) {
-                double* v = S.rec + rec_cell(cc, axis, fv, a, nv) + k;
+                double* v = S.rec + rec_cell(cc, axis, f, a, nv) + k;
                 *v = mf + theta * (*v - mf);
-                S.rec[rec_cell(cc, axis, fn, a, nv) + k] *= theta;
-                S.rec[rec_cell(cc, axis, ft, a, nv) + k] *= theta;
+                S.rec[rec_cell(cc, axis, 2 + f, a, nv) + k] *= theta;
             }
     }
     if (!isfinite(sum)) set_status(B.status, ST_NONFINITE_FLUX);
@@ -648,12 +646,11 @@ __global__ void __launch_bounds__(256, 3) k_s2_face_flux(LoParams P, LoBuffers B
         const double vn = axis == 0 ? uk : vk, vt = axis == 0 ? vk : uk;
         const bool left = vn >= 0.0;
         const double* rc = SB.rec + rec_cell(left ? cl : cr, axis, 0, g, nv) + k;   // fields 3 nv apart
-        const double f0h = rc[0], f0b = rc[(size_t)3 * nv], nh = rc[(size_t)6 * nv], th_ = rc[(size_t)9 * nv];
-        const double nb = rc[(size_t)12 * nv], tb_ = rc[(size_t)15 * nv];
+        const double f0h = rc[0], f0b = rc[(size_t)3 * nv], ph = rc[(size_t)6 * nv], pb = rc[(size_t)9 * nv];
         const double sh = vn * (left ? dlh : drh) + vt * dth;
         const double sb = vn * (left ? dlb : drb) + vt * dtb;
-        const double fhv = vn * (mt[0] * s0h + mt[1] * sh + mt[2] * mth + mt[3] * f0h - mt[4] * (vn * nh + vt * th_));
-        const double fbv = vn * (mt[0] * s0b + mt[1] * sb + mt[2] * mtb + mt[3] * f0b - mt[4] * (vn * nb + vt * tb_));
+        const double fhv = vn * (mt[0] * s0h + mt[1] * sh + mt[2] * mth + mt[3] * f0h - mt[4] * ph);
+        const double fbv = vn * (mt[0] * s0b + mt[1] * sb + mt[2] * mtb + mt[3] * f0b - mt[4] * pb);
         moment_add(wk, uk, vk, fhv, fbv, acc + 4);
         if (sl_.ok) {
             outh[sl_.k] = fhv;
@@ -664,8 +661,8 @@ __global__ void __launch_bounds__(256, 3) k_s2_face_flux(LoParams P, LoBuffers B
                 const double tau = sc[60];
                 cf[0] = vn * f0h;
                 cf[(size_t)nv] = vn * f0b;
-                cf[2 * (size_t)nv] = vn * ((s0h - f0h) / tau - vn * nh - vt * th_);
-                cf[3 * (size_t)nv] = vn * ((s0b - f0b) / tau - vn * nb - vt * tb_);
+                cf[2 * (size_t)nv] = vn * ((s0h - f0h) / tau - ph);
+                cf[3 * (size_t)nv] = vn * ((s0b - f0b) / tau - pb);
             }
         }
     }
@@ -862,7 +859,7 @@ __global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffer
 // shared memory) times a cubic in the velocity, whose coefficients join s0, the slope and the time directions
 // with their Mt, plus the face values' part (ugks_node, mod_S2D1.f90:486-507).  The three nodes' Gauss sum
 // goes straight to the face arrays and its velocity moments are the face's macro flux, so no node flux is
-// stored.  Bound by the face cache: 18 values a (face, velocity), 151 MB at 8x64x32^2.
+// stored.  Bound by the face cache: 12 values a (face, velocity), 100 MB at 8x64x32^2.
 struct S2FluxC {
     double u, v, ux, vy, ckh, l2, kq, kb, qx, qy, mt0, mt3, mt4;   // means, ck T / 2, 2 lam, mt0 coeff, kq 2 / ck, q0, Mt
     double e[5], t[5], d[2][5];   // polynomials 1, cx, cy, c^2 and b part: mt2 dm - mt0 K dirs; mt1 tangential; mt1 left, right
@@ -947,8 +944,7 @@ __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers
                 const double vn = axis == 0 ? uk[r] : vk[r], vt = axis == 0 ? vk[r] : uk[r];
                 const bool left = vn >= 0.0;
                 const double* rc = SB.rec + rec_cell(left ? cl : cr, axis, 0, g, nv) + min(k0 + r * (int)blockDim.x, nv - 1);
-                const double f0h = rc[0], f0b = rc[(size_t)3 * nv], nh = rc[(size_t)6 * nv], th = rc[(size_t)9 * nv];
-                const double nb = rc[(size_t)12 * nv], tb = rc[(size_t)15 * nv];
+                const double f0h = rc[0], f0b = rc[(size_t)3 * nv], ph = rc[(size_t)6 * nv], pb = rc[(size_t)9 * nv];
                 const double* d = c.d[left ? 0 : 1];
                 const double q = ex[g][iu[r]] * ey[g][iv[r]];
                 const double cx = uk[r] - c.u, cy = vk[r] - c.v, px = uk[r] - c.ux, py = vk[r] - c.vy;
@@ -959,8 +955,8 @@ __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers
                 const double vh = c.mt0 + c.kq * qd * (c.l2 * (px * px + py * py) - 4.0) + pe + vn * pd + vt * pt;
                 const double vb = vh + c.kb * qd + c.e[4] + vn * d[4] + vt * c.t[4];
                 const double wn = gw[g] * vn;
-                fh[r] += wn * (q * vh + c.mt3 * f0h - c.mt4 * (vn * nh + vt * th));
-                fb[r] += wn * (c.ckh * q * vb + c.mt3 * f0b - c.mt4 * (vn * nb + vt * tb));
+                fh[r] += wn * (q * vh + c.mt3 * f0h - c.mt4 * ph);
+                fb[r] += wn * (c.ckh * q * vb + c.mt3 * f0b - c.mt4 * pb);
             }
         }
 #pragma unroll

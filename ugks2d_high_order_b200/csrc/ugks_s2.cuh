@@ -13,20 +13,22 @@ struct S2Maps {
     double gnode[3];
 };
 
-// The face cache (S2Buffers::rec): the limited face values and normal / tangential derivatives of h and b
-// (fields 0..5: h, b, h_n, h_t, b_n, b_t) at the 3 Gauss nodes of a cell's sides.  Per velocity a cell
-// keeps, along each axis, only the side that velocity leaves it through (x: the right side when u >= 0,
-// else the left; y: the top when v >= 0, else the bottom) -- the upwind side, the only one an interior face
+// The face cache (S2Buffers::rec): the limited face values of h and b and their derivatives along the particle path,
+// vn h_n + vt h_t (the faces use them only so), at the 3 Gauss nodes of a cell's sides: fields 0..3 h, b, path h, path b.
+// Per velocity a cell keeps, along each axis, only the side that velocity leaves it through (x: the right side when
+// u >= 0, else the left; y: the top when v >= 0, else the bottom) -- the upwind side, the only one an interior face
 // reads: [cell][axis][field][node][nvel].  The wall rows' wall sides follow for every velocity (the wall
-// node reads both halves): [wall: bottom, top][i][field][node][nvel].
+// node reads both halves and uses the derivatives apart: fields h, b, h_n, h_t, b_n, b_t):
+// [wall: bottom, top][i][field][node][nvel].
+constexpr int kRecFields = 4;
 __host__ __device__ __forceinline__ size_t s2_rec_doubles(int nx, int ny, int nv) {
-    return ((size_t)nx * ny * 36 + (size_t)2 * nx * 18) * (size_t)nv;
+    return ((size_t)nx * ny * (2 * kRecFields * 3) + (size_t)2 * nx * 18) * (size_t)nv;
 }
 __host__ __device__ __forceinline__ size_t rec_cell(int cell, int axis, int field, int node, int nv) {
-    return ((((size_t)cell * 2 + axis) * 6 + field) * 3 + node) * (size_t)nv;
+    return ((((size_t)cell * 2 + axis) * kRecFields + field) * 3 + node) * (size_t)nv;
 }
 __host__ __device__ __forceinline__ size_t rec_wall(int nx, int ny, int wall, int i, int field, int node, int nv) {
-    return ((size_t)nx * ny * 36 + (((size_t)wall * nx + i) * 6 + field) * 3 + node) * (size_t)nv;
+    return ((size_t)nx * ny * (2 * kRecFields * 3) + (((size_t)wall * nx + i) * 6 + field) * 3 + node) * (size_t)nv;
 }
 // whether velocity (u, v) leaves a cell through side p (0 x left, 1 x right, 2 y bottom, 3 y top): the
 // upwind selector of the faces, vn >= 0 taking the lower cell's upper side

@@ -823,13 +823,12 @@ __global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers
         const double s0h = v.qh + kxh * q0x + kyh * q0y, s0b = v.qb + kxb * q0x + kyb * q0y;
         const double sh = vn * lr_h + vt * t_h, sb = vn * lr_b + vt * t_b;
         const double f0h = rec_at(cell, 0, s.k), f0b = rec_at(cell, 1, s.k);
-        const double nh = rec_at(cell, 2, s.k), th_ = rec_at(cell, 3, s.k);
-        const double nb = rec_at(cell, 4, s.k), tb_ = rec_at(cell, 5, s.k);
+        const double ph = rec_at(cell, 2, s.k), pb = rec_at(cell, 3, s.k);
         acc[0] += ah * s0h + ab * s0b;
         acc[1] += ah * sh + ab * sb;
         acc[2] += ah * m_h + ab * m_b;
         acc[3] += ah * f0h + ab * f0b;
-        acc[4] += -(ah * (vn * nh + vt * th_) + ab * (vn * nb + vt * tb_));
+        acc[4] += -(ah * ph + ab * pb);
         acc[5] += mt[0] * (ah * kxh + ab * kxb);
         acc[6] += mt[0] * (ah * kyh + ab * kyb);
 #pragma unroll
@@ -1012,17 +1011,17 @@ __global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers
     for (int r = 0; r < nr; ++r) {
         const WVel s = wvel(B, nv, r);
         if (!s.ok) continue;
-        const double vn = axis == 0 ? s.u : s.v, vt = axis == 0 ? s.v : s.u;
+        const double vn = axis == 0 ? s.u : s.v;
         const bool left = vn >= 0.0;
         double ah, ab;
         flux_cot(s, vn, ah, ab);
         const double cx = s.u - M.ux, cy = s.v - M.vy, c2 = cx * cx + cy * cy;
         const double gh0 = ah * mt[3] + psi_h(s.w, s.u, s.v, gW0) + 0.5 * s.w * c2 * (cx * gq0x + cy * gq0y);
         const double gb0 = ab * mt[3] + psi_b(s.w, gW0) + 0.5 * s.w * (cx * gq0x + cy * gq0y);
-        const double gv[6] = {gh0, gb0, -ah * mt[4] * vn, -ah * mt[4] * vt, -ab * mt[4] * vn, -ab * mt[4] * vt};
+        const double gv[kRecFields] = {gh0, gb0, -ah * mt[4], -ab * mt[4]};
         double* up = A.grec + rec_cell(left ? cl : cr, axis, 0, g, nv) + s.k;
 #pragma unroll
-        for (int fld = 0; fld < 6; ++fld) up[(size_t)fld * 3 * nv] = gv[fld];
+        for (int fld = 0; fld < kRecFields; ++fld) up[(size_t)fld * 3 * nv] = gv[fld];
     }
 }
 
@@ -1541,9 +1540,11 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2(LoParams P, LoBuffers B, 
     double gface[3], gdn[3], gdt[3], gvol[3] = {0.0, 0.0, 0.0}, gmf = 0.0, gth = 0.0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+        // an interior side's derivatives enter along the particle path, vn n + vt t
         const double gv = held ? gr[(size_t)(fv * 3 + a) * nv] : 0.0;
-        const double gn = held ? gr[(size_t)(fn * 3 + a) * nv] : 0.0;
-        const double gt = held ? gr[(size_t)(ft * 3 + a) * nv] : 0.0;
+        const double gp = held && !wside ? gr[(size_t)((2 + f) * 3 + a) * nv] : 0.0;
+        const double gn = wside ? (held ? gr[(size_t)(fn * 3 + a) * nv] : 0.0) : (p < 2 ? B.u[k] : B.v[k]) * gp;
+        const double gt = wside ? (held ? gr[(size_t)(ft * 3 + a) * nv] : 0.0) : (p < 2 ? B.v[k] : B.u[k]) * gp;
         gface[a] = theta * gv;
         gmf += (1.0 - theta) * gv;
         gth += (face[a] - mf) * gv + dn[a] * ind * gn + dt[a] * itd * gt;

@@ -28,7 +28,7 @@ struct AdjBuffers {
     double *grh, *grb;       // [nc][nvel] the CN right-hand side
     double* gws;             // [nc][4]    the stream state (= W')
     double* gwq;             // [nc][9][4] the volume node states of the stream state
-    double* grec;            // [nc][72][nvel] the face cache
+    double* grec;            // the face cache's layout (s2_rec_doubles)
     double* gl1;             // [nc][22][nvel] the first layer (zeroed by its consumer)
     double* gmac;            // [interior face][3][12] the macro slopes
     double* gpar;            // [GP_COUNT] parameter cotangents, accumulated over the steps
