@@ -680,49 +680,53 @@ __global__ void __launch_bounds__(256, 3) k_s2_face_flux(LoParams P, LoBuffers B
 
 // ------------------------------------------------------------------------------------------
 // interior faces on a tensor-product velocity table, in three kernels:
-//   k_s2_face_moments : one warp a node, the sums of the upwind face values that W0 and q0 need, taken
-//                       about the lower cell's velocity -> fscal[1..9] (the only pass over the velocities
-//                       that the node's scalars need; bound by the face cache's values, 16 KB a node at 32^2)
+//   k_s2_face_moments : one CTA a face, the sums of the upwind face values that W0 and q0 of its three nodes need,
+//                       taken about the lower cell's velocity -> fscal[1..9] (the only pass over the velocities
+//                       that the node's scalars need; bound by the latency of the face cache's values, 48 KB
+//                       a face at 32^2: 12 loads in flight a thread.  One warp a node took the S2CN2 step to 357 us
+//                       instead of 347, 6 loads in flight to 363, 24 to 348)
 //   k_s2_face_nodes_t : eight lanes a node, W0's closure, make_mke, q0, the directions and Mt by 1-D sums
 //                       -> the node scalars of k_s2_face_nodes
 //   k_s2_face_flux_t  : one CTA a face, its three nodes' micro fluxes and their Gauss sum -> the face arrays
 // Against k_s2_face_nodes, k_s2_face_flux and k_s2_combine, which other tables and the wall variants' coefficient
 // outputs keep, the S2CN2 step at 8x64x32^2 went from 0.704 to 0.565 ms and the 16-instance batch from
 // 14.0 to 10.6 ms a step.
-__global__ void __launch_bounds__(256) k_s2_face_moments(LoParams P, LoBuffers B, S2Buffers SB) {
+__global__ void __launch_bounds__(128) k_s2_face_moments(LoParams P, LoBuffers B, S2Buffers SB) {
     if (eval_cached(B)) return;
-    const int nv = P.nvel, nx = P.nx, ny = P.ny, lane = threadIdx.x & 31;
-    const int nfx = nx * ny, nf = nfx + nx * (ny - 1);
-    const int wid = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (wid >= nf * 3) return;
-    const int fi = wid / 3, g = wid % 3;
+    __shared__ double red[4][32];
+    const int nv = P.nvel, nx = P.nx, ny = P.ny, tid = threadIdx.x;
+    const int nfx = nx * ny, fi = blockIdx.x;
     const int axis = fi < nfx ? 0 : 1, cl = axis == 0 ? fi : fi - nfx;
     const int i = cl % nx, j = cl / nx;
     const int cr = axis == 0 ? j * nx + (i + 1) % nx : (j + 1) * nx + i;
     const double iw = 1.0 / B.W[cl * 4], ur = B.W[cl * 4 + 1] * iw, vr = B.W[cl * 4 + 2] * iw;
-    const double* rl = SB.rec + rec_cell(cl, axis, 0, g, nv);
-    const double* rr = SB.rec + rec_cell(cr, axis, 0, g, nv);
-    double a[9];
+    const double* rl = SB.rec + rec_cell(cl, axis, 0, 0, nv);   // [field][node][nvel]
+    const double* rr = SB.rec + rec_cell(cr, axis, 0, 0, nv);
+    double a[27];
 #pragma unroll
-    for (int m = 0; m < 9; ++m) a[m] = 0.0;
-#pragma unroll 4
-    for (int k = lane; k < nv; k += 32) {
+    for (int m = 0; m < 27; ++m) a[m] = 0.0;
+#pragma unroll 2
+    for (int k = tid; k < nv; k += 128) {
         const double uk = B.u[k], vk = B.v[k], wk = B.w[k];
         const double* rc = ((axis == 0 ? uk : vk) >= 0.0 ? rl : rr) + k;
-        const double h = wk * rc[0], b = wk * rc[(size_t)3 * nv];
-        const double cx = uk - ur, cy = vk - vr, xx = cx * cx, yy = cy * cy, e = (xx + yy) * h + b;
-        a[0] += h;
-        a[1] += cx * h;
-        a[2] += cy * h;
-        a[3] += xx * h;
-        a[4] += cx * cy * h;
-        a[5] += yy * h;
-        a[6] += b;
-        a[7] += cx * e;
-        a[8] += cy * e;
+        const double cx = uk - ur, cy = vk - vr, xx = cx * cx, yy = cy * cy, xy = cx * cy, c2 = xx + yy;
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+            const double h = wk * rc[(size_t)g * nv], b = wk * rc[(size_t)(3 + g) * nv], e = c2 * h + b;
+            a[9 * g] += h;
+            a[9 * g + 1] += cx * h;
+            a[9 * g + 2] += cy * h;
+            a[9 * g + 3] += xx * h;
+            a[9 * g + 4] += xy * h;
+            a[9 * g + 5] += yy * h;
+            a[9 * g + 6] += b;
+            a[9 * g + 7] += cx * e;
+            a[9 * g + 8] += cy * e;
+        }
     }
-    const double t = warp_halving<9, false>(a);   // the total of sum lane / 2
-    if ((lane & 1) == 0 && lane < 18) SB.fscal[(size_t)wid * kS2FScal + 1 + (lane >> 1)] = t;
+    red[tid >> 5][tid & 31] = warp_halving<27, false>(a);   // lane m: the warp's total of sum m
+    __syncthreads();
+    if (tid < 27) SB.fscal[((size_t)fi * 3 + tid / 9) * kS2FScal + 1 + tid % 9] = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
 }
 
 template <int R>
@@ -859,7 +863,8 @@ __global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffer
 // shared memory) times a cubic in the velocity, whose coefficients join s0, the slope and the time directions
 // with their Mt, plus the face values' part (ugks_node, mod_S2D1.f90:486-507).  The three nodes' Gauss sum
 // goes straight to the face arrays and its velocity moments are the face's macro flux, so no node flux is
-// stored.  Bound by the face cache: 12 values a (face, velocity), 100 MB at 8x64x32^2.
+// stored.  Bound by the latency of the face cache's 12 values a (face, velocity), 100 MB at 8x64x32^2.  Nodes unrolled
+// took 379 to 410 us a step instead of 347 (instruction fetch), 2 velocities a thread at four CTAs an SM 350.
 struct S2FluxC {
     double u, v, ux, vy, ckh, l2, kq, kb, qx, qy, mt0, mt3, mt4;   // means, ck T / 2, 2 lam, mt0 coeff, kq 2 / ck, q0, Mt
     double e[5], t[5], d[2][5];   // polynomials 1, cx, cy, c^2 and b part: mt2 dm - mt0 K dirs; mt1 tangential; mt1 left, right
@@ -1530,7 +1535,7 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
     if (e == cudaSuccess && tensor) {
         const unsigned g = (unsigned)((nf * 3 * kTG + 127) / 128);
         const int n = P.tnu > P.tnv ? P.tnu : P.tnv;
-        k_s2_face_moments<<<warps((long long)nf * 3), 256, 0, s>>>(P, B, S);
+        k_s2_face_moments<<<(unsigned)nf, 128, 0, s>>>(P, B, S);
         if (n <= 24) k_s2_face_nodes_t<3><<<g, 128, 0, s>>>(P, B, S);
         else if (n <= 32) k_s2_face_nodes_t<4><<<g, 128, 0, s>>>(P, B, S);
         else if (n <= 48) k_s2_face_nodes_t<6><<<g, 128, 0, s>>>(P, B, S);
