@@ -19,11 +19,11 @@ int main() {
     while (std::scanf("%d", &n) == 1) {
         std::vector<double> t(3 * (size_t)n);
         for (double& x : t) if (std::scanf("%la", &x) != 1) return 1;
-        double tab[256];
+        double tab[ugks::kTensorTab];
         int nu = 0, nv = 0;
         const bool ok = ugks::tensor_table(n, t.data(), t.data() + n, t.data() + 2 * n, &nu, &nv, tab);
         std::printf("%d %d %d", ok, nu, nv);
-        for (int a = 0; ok && a < 256; ++a) std::printf(" %a", tab[a]);
+        for (int a = 0; ok && a < ugks::kTensorTab; ++a) std::printf(" %a", tab[a]);
         std::printf("\n");
     }
 }
@@ -77,7 +77,7 @@ def test_tensor_table(tmp_path):
             continue
         nu, nv = shape
         assert (int(f[1]), int(f[2])) == shape, name
-        tab = np.array([float.fromhex(x) for x in f[3:]]).reshape(4, 64)
+        tab = np.array([float.fromhex(x) for x in f[3:]]).reshape(8, 64)
         assert np.array_equal(np.tile(tab[0, :nu], nv), u) and np.array_equal(np.repeat(tab[2, :nv], nu), v), name
         wk = np.tile(tab[1, :nu], nv) * np.repeat(tab[3, :nv], nu)
         assert np.abs(wk / w - 1).max() <= 4 * np.finfo(float).eps, name

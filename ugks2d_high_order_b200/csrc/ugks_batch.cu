@@ -169,16 +169,16 @@ extern "C" int ugks_batch_create(int n, const ugks_instance_desc* desc, int devi
         I.S = S;
         per_slot = std::max(per_slot, scratch_doubles(nx, ny, nv));
         // persistent: u v w | h b W (x2) | targets (x2) | dt | ledger | report | wall_aero
-        double tab[256];
+        double tab[kTensorTab];
         if (!tensor_table(nv, desc[i].u, desc[i].v, desc[i].w, &P.tnu, &P.tnv, tab)) P.tnu = P.tnv = 0;
-        const size_t tot = 3 * rnd(nv) + rnd(256) + 2 * (2 * rnd(S) + rnd(nc * 4)) + 12 * rnd(S) + rnd(2) + rnd(16) +
+        const size_t tot = 3 * rnd(nv) + rnd(kTensorTab) + 2 * (2 * rnd(S) + rnd(nc * 4)) + 12 * rnd(S) + rnd(2) + rnd(16) +
                            rnd(kCnReport) + rnd((size_t)2 * nx * 3);
         e = cudaMalloc(&I.mem, tot * sizeof(double));
         if (e == cudaSuccess) e = cudaMemsetAsync(I.mem, 0, tot * sizeof(double), b->origin);
         if (e != cudaSuccess) break;
         double* m = I.mem;
         auto take = [&](size_t k) { double* q = m; m += rnd(k); return q; };
-        double *u = take(nv), *v = take(nv), *w = take(nv), *dtab = take(256);
+        double *u = take(nv), *v = take(nv), *w = take(nv), *dtab = take(kTensorTab);
         if (P.tnu > 0) e = cudaMemcpyAsync(dtab, tab, sizeof tab, cudaMemcpyHostToDevice, b->origin);
         if (e == cudaSuccess) e = cudaMemcpyAsync(u, desc[i].u, nv * sizeof(double), cudaMemcpyHostToDevice, b->origin);
         if (e == cudaSuccess) e = cudaMemcpyAsync(v, desc[i].v, nv * sizeof(double), cudaMemcpyHostToDevice, b->origin);

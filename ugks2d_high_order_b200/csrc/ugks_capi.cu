@@ -202,7 +202,7 @@ extern "C" int ugks_ctx_create(const ugks_params* p, const double* u, const doub
     const size_t S = (size_t)nc * nv, SY = (size_t)(ny + 1) * nx * nv;
     size_t off = 0;
     auto take = [&](size_t n) { size_t o = off; off += (n + 31) / 32 * 32; return o; };
-    const size_t o_u = take(nv), o_v = take(nv), o_w = take(nv), o_tab = take(256);
+    const size_t o_u = take(nv), o_v = take(nv), o_w = take(nv), o_tab = take(kTensorTab);
     const size_t o_h = take(S), o_b = take(S), o_W = take((size_t)nc * 4);
     const size_t o_sxh = take(S), o_syh = take(S), o_sxb = take(S), o_syb = take(S);
     const size_t o_fxh = take(S), o_fxb = take(S), o_fxw = take((size_t)nc * 4);
@@ -232,7 +232,7 @@ extern "C" int ugks_ctx_create(const ugks_params* p, const double* u, const doub
     B.peq_h = d + o_eh; B.peq_b = d + o_eb; B.pcol_h = d + o_ch; B.pcol_b = d + o_cb;
     B.dtl = d + o_dtl; B.dt = d + o_dt; B.cell_diag = d + o_cd; B.diag = d + o_dg; B.wall_aero = d + o_wa;
     B.counter = c->dflags; B.status = c->dflags + 1;
-    double tab[256];
+    double tab[kTensorTab];
     if (tensor_table(nv, u, v, w, &c->P.tnu, &c->P.tnv, tab))
         e = cudaMemcpyAsync(d + o_tab, tab, sizeof tab, cudaMemcpyHostToDevice, c->stream);
     else

@@ -37,7 +37,8 @@ struct LoBuffers {
     const double* u;         // [nvel] velocity table, k = i + j*Nu
     const double* v;
     const double* w;
-    const double* tab;       // [4][64] the axes of a tensor table (LoParams::tnu > 0): u, wx, v, wy
+    const double* tab;       // [8][64] the axes of a tensor table (LoParams::tnu > 0): u, wx, v, wy, then wx for u >= 0,
+                             // u < 0 and wy for v >= 0, v < 0
     double* h;               // [nc][nvel] state, cell c = j*nx + i
     double* b;
     double* W;               // [nc][4] conservative variables
@@ -105,9 +106,10 @@ __device__ __forceinline__ Slot slot(int r, int nv) {
 // w[k] = wx_i wy_j to within 4 units in the last place, the rounding of a product whose factors are
 // themselves recovered from the products (the S2 closures use the factors: a table of rounded decimal weights that
 // misses this keeps the general kernels).  On success tab holds u, wx, v, wy, each padded to 64 with its last
-// abscissa and weight 0.  Host only.
+// abscissa and weight 0, and the weights of the axes' halves (LoBuffers::tab).  Host only.
+constexpr int kTensorTab = 8 * 64;
 inline bool tensor_table(int nv, const double* u, const double* v, const double* w, int* nu_out, int* nv_out,
-                         double tab[256]) {
+                         double tab[kTensorTab]) {
     int nu = 1;
     while (nu < nv && v[nu] == v[0]) ++nu;
     if (nv % nu != 0) return false;
@@ -137,6 +139,10 @@ inline bool tensor_table(int nv, const double* u, const double* v, const double*
         tab[64 + a] = a < nu ? (double)fx[a] : 0.0;
         tab[128 + a] = v[(size_t)std::min(a, nj - 1) * nu];
         tab[192 + a] = a < nj ? (double)fy[a] : 0.0;
+        tab[256 + a] = tab[a] >= 0.0 ? tab[64 + a] : 0.0;
+        tab[320 + a] = tab[a] >= 0.0 ? 0.0 : tab[64 + a];
+        tab[384 + a] = tab[128 + a] >= 0.0 ? tab[192 + a] : 0.0;
+        tab[448 + a] = tab[128 + a] >= 0.0 ? 0.0 : tab[192 + a];
     }
     for (int j = 0; j < nj; ++j)
         for (int i = 0; i < nu; ++i) {

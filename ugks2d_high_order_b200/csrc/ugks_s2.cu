@@ -760,13 +760,11 @@ __global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffer
         const double dx = M.ux - ur, dy = M.vy - vr, d2 = dx * dx + dy * dy, e2 = f[3] + f[5], dp = dx * f[1] + dy * f[2];
         const double hx = 0.5 * (f[7] - dx * (e2 + f[6]) + d2 * f[1] - d2 * dx * f[0]) - (dx * f[3] + dy * f[4]) + dx * dp;
         const double hy = 0.5 * (f[8] - dy * (e2 + f[6]) + d2 * f[2] - d2 * dy * f[0]) - (dx * f[4] + dy * f[5]) + dy * dp;
-        double s[8], em = INFINITY;
-        t_axis<R, 4>(B.tab, B.tab + 64, M.ux, lamn, M.ux, s, em);
-        t_axis<R, 4>(B.tab + 128, B.tab + 192, M.vy, lamn, M.vy, s + 4, em);
-        t_sum<8>(s);
+        TAxes ax;
+        t_sums<R>(B.tab, B.tab + 64, B.tab + 128, B.tab + 192, M.ux, M.vy, lamn, M.ux, M.vy, &ax);
         const double pr = 0.5 * w0[0] * lamn / kPi, cb = 0.5 * (double)ck * temp;
-        q0x = hx - pr * (s[3] * s[4] + s[1] * s[6] + cb * s[1] * s[4]);
-        q0y = hy - pr * (s[7] * s[0] + s[5] * s[2] + cb * s[5] * s[0]);
+        q0x = hx - pr * (ax.x[3] * ax.y[0] + ax.x[1] * ax.y[2] + cb * ax.x[1] * ax.y[0]);
+        q0y = hy - pr * (ax.y[3] * ax.x[0] + ax.y[1] * ax.x[2] + cb * ax.y[1] * ax.x[0]);
     }
     // wt = -moments of vn (left ? dl : dr) + vt dt: lane 2 sums the left half of the normal axis with the left
     // direction, lane 3 the right half with the right one, lane 4 the other axis with the tangential one
@@ -776,24 +774,15 @@ __global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffer
         const double* tn = B.tab + (axis == 0 ? 0 : 128);
         const double* to = B.tab + (axis == 0 ? 128 : 0);
         const double un0 = axis == 0 ? t.u : t.v, uo0 = axis == 0 ? t.v : t.u;
-        double s[18], em = INFINITY;   // normal axis: vn >= 0, vn < 0; other axis
-#pragma unroll
-        for (int a = 0; a < 12; ++a) s[a] = 0.0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const double x = __ldg(tn + gl + kTG * r), d = x - un0;
-            double p = __ldg(tn + 64 + gl + kTG * r) * exp(-(d * d) * t.itw);
-            double pl = x >= 0.0 ? p : 0.0, pr = x >= 0.0 ? 0.0 : p;
-#pragma unroll
-            for (int a = 0; a < 6; ++a) { s[a] += pl; s[6 + a] += pr; pl = pl * d; pr = pr * d; }
-        }
-        t_axis<R, 6>(to, to + 64, uo0, t.itw, uo0, s + 12, em);
-        t_sum<18>(s);
+        const double* h = B.tab + (axis == 0 ? 256 : 384);   // weights of the normal axis's halves
+        TAxes l, rt;   // (normal half vn >= 0, other axis), (normal half vn < 0, other axis)
+        t_sums<R>(tn, h, to, to + 64, un0, uo0, t.itw, un0, uo0, &l);
+        t_sums<R>(tn, h + 64, to, to + 64, un0, uo0, t.itw, un0, uo0, &rt);
         double N[6], O[5];
 #pragma unroll
-        for (int a = 0; a < 6; ++a) N[a] = gl == 4 ? s[12 + a] : (gl == 3 ? s[6 + a] : s[a]);
+        for (int a = 0; a < 6; ++a) N[a] = gl == 4 ? l.y[a] : (gl == 3 ? rt.x[a] : l.x[a]);
 #pragma unroll
-        for (int a = 0; a < 5; ++a) O[a] = gl == 4 ? s[a] + s[6 + a] : s[12 + a];
+        for (int a = 0; a < 5; ++a) O[a] = gl == 4 ? l.x[a] + rt.x[a] : l.y[a];
         const bool nisx = (axis == 0) != (gl == 4);   // this lane's normal component is x
         const double un = gl == 4 ? uo0 : un0, uo = gl == 4 ? un0 : uo0;
         const double d0 = td[0] * t.ir - td[3] * t.itw, d3 = td[3] * t.itw * t.itw, db = td[3] * t.itw;
@@ -822,7 +811,7 @@ __global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffer
                        t.pref * (0.5 * (un * un + uo * uo) * m0 + un * mn + uo * mo + 0.5 * m2 + 0.5 * t.ckh * mb)};
 #pragma unroll
         for (int m = 0; m < 4; ++m) wt[m] = -(t_get(c[m], 2) + t_get(c[m], 3) + t_get(c[m], 4));
-        ok = s2_solve4(C.jac, wt, tdm) && ok;
+        ok = t_solve(C.jac, wt, tdm) && ok;
         double sc = 1.0;
 #pragma unroll
         for (int m = 0; m < 4; ++m) sc = fmax(sc, fabs(wt[m]));

@@ -34,24 +34,90 @@ __device__ __forceinline__ double t_get(double v, int src) {
     return __shfl_sync(0xffffffffu, v, ((threadIdx.x & 31) & ~(kTG - 1)) + src);
 }
 
-// this lane's part of the 1-D sums s[a] = sum_i w_i c_i^a exp(-(x_i - mean)^2 itw), c_i = x_i - center, over an
-// axis of the table (LoBuffers::tab: padded to 64 abscissae with weight 0).  R >= abscissae / 8.
-template <int R, int N>
-__device__ __forceinline__ void t_axis(const double* __restrict__ pos, const double* __restrict__ wt, double mean,
-                                       double itw, double center, double* s, double& emin) {
+// The 1-D sums of both axes: x[a] = sum_i w_i c_i^a exp(-(x_i - mean)^2 itw), c_i = x_i - center, for a = 0..5, over the
+// abscissae (pos) and weights (wt) of an axis of the table (LoBuffers::tab: rows of 64, padded with weight 0), and
+// the smallest exponential of each.  R >= abscissae / 8.  A function of its own, as is t_solve: a node runs through it
+// six to eight times, and in line the nodes' kernels spent more time fetching instructions than waiting on them
+// (stalls 3.0 against 2.1 an issue).  S2CN2 step 8x64x32^2 347 -> 344.5 us, HighOrderImplicit pseudo-step 490 -> 486,
+// 16-instance batch 6.23 -> 6.14 ms a step.
+struct TAxes {
+    double x[6], y[6], ex, ey;
+};
+template <int R>
+__device__ __noinline__ void t_sums(const double* __restrict__ tu, const double* __restrict__ wu, const double* __restrict__ tv,
+                                    const double* __restrict__ wv, double mu, double mv, double itw, double cu, double cv,
+                                    TAxes* out) {
     const int gl = threadIdx.x & (kTG - 1);
+    double s[12], ex = INFINITY, ey = INFINITY;
 #pragma unroll
-    for (int a = 0; a < N; ++a) s[a] = 0.0;
+    for (int a = 0; a < 12; ++a) s[a] = 0.0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const double x = __ldg(pos + gl + kTG * r), d = x - mean, c = x - center;
-        const double e = exp(-(d * d) * itw);
-        emin = fmin(emin, e);
-        double t = __ldg(wt + gl + kTG * r) * e;
-        s[0] += t;
+        const double xu = __ldg(tu + gl + kTG * r), xv = __ldg(tv + gl + kTG * r);
+        const double du = xu - mu, dv = xv - mv, pu = xu - cu, pv = xv - cv;
+        const double eu = exp(-(du * du) * itw), ev = exp(-(dv * dv) * itw);
+        ex = fmin(ex, eu);
+        ey = fmin(ey, ev);
+        double a = __ldg(wu + gl + kTG * r) * eu, b = __ldg(wv + gl + kTG * r) * ev;
+        s[0] += a;
+        s[6] += b;
 #pragma unroll
-        for (int a = 1; a < N; ++a) { t = t * c; s[a] += t; }
+        for (int m = 1; m < 6; ++m) { a = a * pu; b = b * pv; s[m] += a; s[6 + m] += b; }
     }
+    t_sum<12>(s);
+#pragma unroll
+    for (int a = 0; a < 6; ++a) { out->x[a] = s[a]; out->y[a] = s[6 + a]; }
+    out->ex = t_min(ex);
+    out->ey = t_min(ey);
+}
+
+// solve_dense_4x4 (mod_CorrectedWF2DClosure.f90:631-661) as s2_solve4, the pivots' divisions taken as one reciprocal each
+__device__ __noinline__ bool t_solve(const double* m, const double* rhs, double* out) {
+    double a[4][5], x[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a[r][c] = m[r * 4 + c];
+        a[r][4] = rhs[r];
+    }
+    double ip[4];
+    bool ok = true;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        int row = p;
+        double best = fabs(a[p][p]);
+#pragma unroll
+        for (int i = p + 1; i < 4; ++i) if (fabs(a[i][p]) > best) { best = fabs(a[i][p]); row = i; }
+        ok = ok && best > 100.0 * DBL_MIN && isfinite(best);
+#pragma unroll
+        for (int i = p + 1; i < 4; ++i) {
+            const bool sw = row == i;
+#pragma unroll
+            for (int c = p; c < 5; ++c) {
+                const double t = a[p][c];
+                a[p][c] = sw ? a[i][c] : t;
+                a[i][c] = sw ? t : a[i][c];
+            }
+        }
+        ip[p] = 1.0 / a[p][p];
+#pragma unroll
+        for (int i = p + 1; i < 4; ++i) {
+            const double f = a[i][p] * ip[p];
+#pragma unroll
+            for (int c = p + 1; c < 5; ++c) a[i][c] = a[i][c] - f * a[p][c];
+        }
+    }
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+        double v = a[i][4];
+#pragma unroll
+        for (int c = i + 1; c < 4; ++c) v = v - a[i][c] * x[c];
+        x[i] = v * ip[i];
+        ok = ok && isfinite(x[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] = ok ? x[i] : 0.0;
+    return ok;
 }
 
 struct TClosure {
@@ -59,6 +125,31 @@ struct TClosure {
     double res;     // scaled residual of the moments at th (make_mke's gate)
     double* jac;    // [16] moment Jacobian at th, row-major, in the group's slice of shared memory
 };
+
+// w_newton_next with t_solve
+__device__ __forceinline__ int t_newton_next(bool new_iter, const WClosure& C, const double res[4], double norm, int iter,
+                                             double step[4], double& alpha, double trial[4]) {
+    const double tol = 5.0e-13, floor_a = 9.5367431640625e-07;   // 2^-20
+    if (new_iter) {
+        if (norm <= tol) return W_DONE;
+        if (iter > 12) return W_FAIL;
+        const double mr[4] = {-res[0], -res[1], -res[2], -res[3]};
+        if (!t_solve(C.jac, mr, step)) return W_FAIL;
+        alpha = 1.0;
+    }
+    while (alpha >= floor_a) {
+        double nt[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) nt[m] = C.th[m] + alpha * step[m];
+        if (nt[0] > 0.0 && nt[3] > 0.0 && isfinite(nt[0]) && isfinite(nt[1]) && isfinite(nt[2]) && isfinite(nt[3])) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) trial[m] = nt[m];
+            return W_TRIAL;
+        }
+        alpha = 0.5 * alpha;
+    }
+    return W_FAIL;
+}
 
 // solve_q_first (mod_CorrectedWF2DClosure.f90:331-426) for the target moments w: the accept / backtrack / stop
 // logic of w_closure on the 1-D sums.  Every lane of the warp calls it; a group whose `act` is false
@@ -87,15 +178,10 @@ __device__ bool t_closure(const LoParams& P, const LoBuffers& B, const double w[
     bool first = true;
     for (int guard = 0; guard < 1024; ++guard) {
         if (__all_sync(0xffffffffu, done)) break;
-        double s[10], ex = INFINITY, ey = INFINITY;   // A_a = sum wx cx^a e_x (0..4), then B_b
+        TAxes ax;   // sum wx cx^a e_x, sum wy cy^b e_y
         const S2Th t = s2_th(trial, ck);
-        t_axis<R, 5>(B.tab, B.tab + 64, t.u, t.itw, t.u, s, ex);
-        t_axis<R, 5>(B.tab + 128, B.tab + 192, t.v, t.itw, t.v, s + 5, ey);
-        t_sum<10>(s);
-        ex = t_min(ex);
-        ey = t_min(ey);
-        const double *A = s, *Bq = s + 5;
-        auto S = [&](int a, int b) { return t.pref * A[a] * Bq[b]; };
+        t_sums<R>(B.tab, B.tab + 64, B.tab + 128, B.tab + 192, t.u, t.v, t.itw, t.u, t.v, &ax);
+        auto S = [&](int a, int b) { return t.pref * ax.x[a] * ax.y[b]; };
         const double s00 = S(0, 0), s10 = S(1, 0), s01 = S(0, 1), s11 = S(1, 1), s20 = S(2, 0), s02 = S(0, 2);
         const double c20 = s20 + s02;                          // sums of c^2, c^2 cx, c^2 cy, c^4
         const double c30 = S(3, 0) + S(1, 2), c03 = S(2, 1) + S(0, 3);
@@ -115,14 +201,14 @@ __device__ bool t_closure(const LoParams& P, const LoBuffers& B, const double w[
         mom(d1 * s10, d1 * s20, d1 * s11, d1 * c30, d1 * s10, J + 1, 4);
         mom(d1 * s01, d1 * s11, d1 * s02, d1 * c03, d1 * s01, J + 2, 4);
         mom(i2 * c20 - i1 * s00, i2 * c30 - i1 * s10, i2 * c03 - i1 * s01, i2 * c40 - i1 * c20, i2 * c20, J + 3, 4);
-        bool fin = true;
+        double nres[4], all = 0.0;   // finite if every sum is (magnitudes, so that nothing cancels)
 #pragma unroll
-        for (int m = 0; m < 16; ++m) fin = fin && isfinite(J[m]);
-        double nres[4];
+        for (int m = 0; m < 16; ++m) all += fabs(J[m]);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) { fin = fin && isfinite(q[m]); nres[m] = q[m] - w[m]; }
+        for (int m = 0; m < 4; ++m) { all += fabs(q[m]); nres[m] = q[m] - w[m]; }
+        const bool fin = isfinite(all);
         // the Maxwellian is positive at every velocity (its smallest value is the product of the axes' smallest)
-        const double qmin = t.pref * ex * ey;
+        const double qmin = t.pref * ax.ex * ax.ey;
         const bool pos = qmin > 0.0 && t.ckh * qmin > 0.0;
         const double nn = fin ? s2_scaled(nres, w) : INFINITY;
         const bool accept = !done && (first ? fin : (fin && (nn < norm || nn <= 5.0e-13)));
@@ -137,13 +223,13 @@ __device__ bool t_closure(const LoParams& P, const LoBuffers& B, const double w[
                 for (int m = 0; m < 4; ++m) { Cw.th[m] = trial[m]; res[m] = nres[m]; }
                 norm = nn;
                 iter = first ? 1 : iter + 1;
-                a = w_newton_next(true, Cw, res, norm, iter, step, alpha, trial);
+                a = t_newton_next(true, Cw, res, norm, iter, step, alpha, trial);
                 if (a == W_DONE && !pos) a = W_FAIL;
             } else if (first) {
                 a = W_FAIL;
             } else {
                 alpha = 0.5 * alpha;
-                a = w_newton_next(false, Cw, res, norm, iter, step, alpha, trial);
+                a = t_newton_next(false, Cw, res, norm, iter, step, alpha, trial);
             }
             first = false;
             if (a != W_TRIAL) { done = true; ok = a == W_DONE; }
@@ -188,14 +274,12 @@ __device__ bool t_mke(const LoParams& P, const LoBuffers& B, const double w[4], 
     M.lam = 0.5 / th;
     M.coeff = 0.8 * (1.0 - P.pr) * M.lam * M.lam / rho;
     const S2Th t = s2_th(C.th, ck);
-    double s[12], em = INFINITY;
-    t_axis<R, 6>(B.tab, B.tab + 64, t.u, t.itw, M.ux, s, em);
-    t_axis<R, 6>(B.tab + 128, B.tab + 192, t.v, t.itw, M.vy, s + 6, em);
-    t_sum<12>(s);
+    TAxes ax;
+    t_sums<R>(B.tab, B.tab + 64, B.tab + 128, B.tab + 192, t.u, t.v, t.itw, M.ux, M.vy, &ax);
     const bool sw = gl & 1;   // the axis of K is the first of (N, O)
     double N[6], O[6];
 #pragma unroll
-    for (int a = 0; a < 6; ++a) { N[a] = sw ? s[6 + a] : s[a]; O[a] = sw ? s[a] : s[6 + a]; }
+    for (int a = 0; a < 6; ++a) { N[a] = sw ? ax.y[a] : ax.x[a]; O[a] = sw ? ax.x[a] : ax.y[a]; }
     const double un = sw ? M.vy : M.ux, uo = sw ? M.ux : M.vy, l2 = 2.0 * M.lam, pc = t.pref * M.coeff;
     // f = cn (2 lam c^2 - 4): its sums with 1, cn, co, c^2; b adds (2 / ck) cn
     const double s10 = N[1] * O[0];
@@ -214,7 +298,7 @@ __device__ bool t_mke(const LoParams& P, const LoBuffers& B, const double w[4], 
     if (mine)
 #pragma unroll
         for (int m = 0; m < 4; ++m) rhs[m] = extra[(gl - 2) * 4 + m];
-    bool ok = s2_solve4(C.jac, rhs, td);
+    bool ok = t_solve(C.jac, rhs, td);
     double sc = 1.0;
     if (mine)
 #pragma unroll
