@@ -135,3 +135,56 @@ def test_tensor_path_matches_oracle_and_general_path(shape):
     p = rng.permutation(len(t[0]))
     ph, pb, pW = gpu(tuple(a[p] for a in t), (h[..., p], b[..., p]))
     close((got[0][..., p], got[1][..., p], got[2]), (ph, pb, pW))
+
+
+# Tolerance: the two paths sum the same terms in other orders and leave out projection weights below 1e-16 of the
+# equilibrium: a few roundings of the largest value a step, 1e-12 over three steps with a wide margin for the walls'
+# density, a quotient of two sums.
+EXPLICIT_TOL = 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,grid", [((8, 4), (4, 3)), ((16, 16), (1, 5)), ((24, 24), (7, 9)), ((20, 28), (3, 4)),
+                                        ((32, 32), (2, 11)), ((64, 36), (5, 7)), ((50, 50), (4, 6))])
+def test_explicit_tensor_path_matches_oracle_and_general_path(shape, grid):
+    """Explicit steps on a tensor table, fused and operator by operator, against the oracle and against the same
+    table in another order, which takes the general kernels."""
+    from oracle.oracle import Oracle
+    from ugks2d_high_order_b200.case import reference_case
+    from ugks2d_high_order_b200.solver import Solver
+    t, (nx, ny) = rectangle(*shape), grid
+    c = reference_case("Explicit").with_(nx=nx, ny=ny, dx=1 / nx, dy=1 / ny, omega=0.81, wall_ux=(-2.0, 3.0), wall_tnative=(1.8, 2.1))
+    rng = np.random.default_rng(7)
+    rho, U, V, T = 1 + 0.05 * rng.uniform(-1, 1, (ny, nx)), *(0.2 * rng.uniform(-1, 1, (2, ny, nx))), 2 + 0.1 * rng.uniform(-1, 1, (ny, nx))
+    h = (rho / (np.pi * T))[..., None] * np.exp(-((t[0] - U[..., None]) ** 2 + (t[1] - V[..., None]) ** 2) / T[..., None])
+    h *= 1 + 0.05 * rng.uniform(-1, 1, h.shape)
+    b = 0.5 * T[..., None] * h
+    W = np.stack([h @ t[2], h @ (t[2] * t[0]), h @ (t[2] * t[1]), 0.5 * (h @ (t[2] * (t[0] ** 2 + t[1] ** 2)) + b @ t[2])], -1)
+
+    def gpu(table, hb, operators=False):
+        s = Solver(c, *table)
+        try:
+            s.upload(hb[0], hb[1], W)
+            for _ in range(3):
+                if operators:
+                    s.time_step(), s.evolution(), s.compute_residual(), s.apply_explicit_update()
+                else:
+                    s.step_explicit(1)
+            return s.download() + (s.wall_aero(),)
+        finally:
+            s.close()
+
+    def close(a, b):
+        for x, y in zip(a, b):
+            assert np.abs(np.asarray(x).reshape(-1) - np.asarray(y).reshape(-1)).max() <= EXPLICIT_TOL * np.abs(y).max()
+
+    got = gpu(t, (h, b))
+    o = Oracle(c, *t)
+    o.set_state(h, b, W)
+    for _ in range(3):
+        o.explicit_step()
+    close(got, o.get_state())
+    close(gpu(t, (h, b), operators=True), got)
+    p = rng.permutation(len(t[0]))
+    ph, pb, pW, aero = gpu(tuple(a[p] for a in t), (h[..., p], b[..., p]))
+    close((got[0][..., p], got[1][..., p], got[2], got[3]), (ph, pb, pW, aero))

@@ -19,6 +19,8 @@ cudaError_t launch_lo_slopes(const LoParams& P, const LoBuffers& B, cudaStream_t
 cudaError_t launch_lo_faces(const LoParams& P, const LoBuffers& B, cudaStream_t s);
 cudaError_t launch_lo_walls(const LoParams& P, const LoBuffers& B, cudaStream_t s);
 cudaError_t launch_lo_cells(const LoParams& P, const LoBuffers& B, int mode, bool collision, cudaStream_t s);
+cudaError_t launch_lo_fluxes_t(const LoParams& P, const LoBuffers& B, cudaStream_t s);
+cudaError_t launch_lo_cells_t(const LoParams& P, const LoBuffers& B, int mode, cudaStream_t s);
 cudaError_t launch_lo_timestep(const LoParams& P, const LoBuffers& B, cudaStream_t s);
 cudaError_t launch_lo_macro_fields(const LoParams& P, const LoBuffers& B, double* out, cudaStream_t s);
 cudaError_t launch_lo_init(const LoParams& P, const LoBuffers& B, double rho, double U, double V, double tn,
@@ -561,11 +563,19 @@ static bool is_s2(const ugks_ctx* c) {
     return c->prm.method == UGKS_METHOD_S2CN2 || c->prm.method == UGKS_METHOD_HIGH_ORDER_IMPLICIT;
 }
 
+// the second-order kernels of tensor-product velocity tables (ugks_lo_tensor.cu), on Explicit contexts
+static bool lo_tensor(const ugks_ctx* c) { return c->P.tnu > 0 && c->prm.method == UGKS_METHOD_EXPLICIT; }
+
 extern "C" int ugks_evolution(ugks_ctx* c) {
     if (!c) return UGKS_EINVAL;
     UGKS_CK(cudaSetDevice(c->device));
     if (int r = invalidate_eval(c)) return r;
     if (is_s2(c)) return s2_evolution(c, c->prm.method == UGKS_METHOD_HIGH_ORDER_IMPLICIT);
+    if (lo_tensor(c)) {
+        UGKS_CK(launch_lo_fluxes_t(c->P, c->B, c->stream));
+        c->launches += 1;
+        return collect_status(c);
+    }
     UGKS_CK(launch_lo_slopes(c->P, c->B, c->stream));
     UGKS_CK(launch_lo_faces(c->P, c->B, c->stream));
     UGKS_CK(launch_lo_walls(c->P, c->B, c->stream));
@@ -594,7 +604,8 @@ extern "C" int ugks_compute_residual(ugks_ctx* c, int with_collision) {
         c->cn_stage = r == UGKS_OK ? 2 : 0;
         return r;
     }
-    UGKS_CK(launch_lo_cells(c->P, c->B, 1, with_collision != 0, c->stream));
+    if (lo_tensor(c) && !with_collision) UGKS_CK(launch_lo_cells_t(c->P, c->B, 1, c->stream));
+    else UGKS_CK(launch_lo_cells(c->P, c->B, 1, with_collision != 0, c->stream));
     c->launches += 1;
     return collect_status(c);
 }
@@ -640,7 +651,8 @@ extern "C" int ugks_apply_explicit_update(ugks_ctx* c, double* res_out) {
     UGKS_CK(cudaSetDevice(c->device));
     if (int r = invalidate_eval(c)) return r;
     if (c->cmem) return s2cn2_apply(c);
-    UGKS_CK(launch_lo_cells(c->P, c->B, 2, false, c->stream));
+    if (lo_tensor(c)) UGKS_CK(launch_lo_cells_t(c->P, c->B, 2, c->stream));
+    else UGKS_CK(launch_lo_cells(c->P, c->B, 2, false, c->stream));
     c->launches += 1;
     return read_step_outputs(c, nullptr, res_out);
 }
@@ -650,6 +662,12 @@ extern "C" int ugks_apply_explicit_update(ugks_ctx* c, double* res_out) {
 // cell update.  The fork/join is recorded into the CUDA graph as two parallel branches.
 static cudaError_t enqueue_explicit_steps(ugks_ctx* c, int n) {
     for (int s = 0; s < n; ++s) {
+        if (lo_tensor(c)) {   // slopes, faces and walls in one launch, then the cells
+            cudaError_t e = launch_lo_fluxes_t(c->P, c->B, c->stream);
+            if (e == cudaSuccess) e = launch_lo_cells_t(c->P, c->B, 3, c->stream);
+            if (e != cudaSuccess) return e;
+            continue;
+        }
         cudaError_t e = launch_lo_slopes(c->P, c->B, c->stream);
         if (e == cudaSuccess) e = cudaEventRecord(c->ev_fork, c->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream2, c->ev_fork, 0);
@@ -686,14 +704,15 @@ extern "C" int ugks_step_explicit(ugks_ctx* c, int nsteps, double* dt_out, doubl
     if (nsteps == 0) return UGKS_OK;
     if (c->profile) {
         for (int s = 0; s < nsteps; ++s) {
+            const bool t = lo_tensor(c);   // "faces" holds the slopes and the walls there
             UGKS_CK(cudaEventRecord(c->ev[4], c->stream));
-            UGKS_CK(launch_lo_slopes(c->P, c->B, c->stream));
+            if (!t) UGKS_CK(launch_lo_slopes(c->P, c->B, c->stream));
             UGKS_CK(cudaEventRecord(c->ev[0], c->stream));
-            UGKS_CK(launch_lo_faces(c->P, c->B, c->stream));
+            UGKS_CK(t ? launch_lo_fluxes_t(c->P, c->B, c->stream) : launch_lo_faces(c->P, c->B, c->stream));
             UGKS_CK(cudaEventRecord(c->ev[1], c->stream));
-            UGKS_CK(launch_lo_walls(c->P, c->B, c->stream));
+            if (!t) UGKS_CK(launch_lo_walls(c->P, c->B, c->stream));
             UGKS_CK(cudaEventRecord(c->ev[2], c->stream));
-            UGKS_CK(launch_lo_cells(c->P, c->B, 3, false, c->stream));
+            UGKS_CK(t ? launch_lo_cells_t(c->P, c->B, 3, c->stream) : launch_lo_cells(c->P, c->B, 3, false, c->stream));
             UGKS_CK(cudaEventRecord(c->ev[3], c->stream));
             UGKS_CK(cudaEventSynchronize(c->ev[3]));
             float a = 0.f, w = 0.f, b = 0.f, sl = 0.f;
@@ -706,7 +725,7 @@ extern "C" int ugks_step_explicit(ugks_ctx* c, int nsteps, double* dt_out, doubl
             c->t_walls.total_ms += w; c->t_walls.launches += 1;
             c->t_cells.total_ms += b; c->t_cells.launches += 1;
         }
-        c->launches += 4LL * nsteps;
+        c->launches += (lo_tensor(c) ? 2LL : 4LL) * nsteps;
     } else {
         const int G = 16;
         int full = nsteps / G, rem = nsteps % G;
@@ -716,7 +735,7 @@ extern "C" int ugks_step_explicit(ugks_ctx* c, int nsteps, double* dt_out, doubl
             for (int i = 0; i < full; ++i) UGKS_CK(cudaGraphLaunch(c->graph, c->stream));
         }
         UGKS_CK(enqueue_explicit_steps(c, rem));
-        c->launches += 4LL * nsteps;
+        c->launches += (lo_tensor(c) ? 2LL : 4LL) * nsteps;
     }
     if (dt_out) UGKS_CK(cudaMemcpyAsync(dt_out, c->B.dt + 1, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     return read_step_outputs(c, dt_out, res_out);

@@ -771,44 +771,6 @@ __global__ void __launch_bounds__(NTMAX) k_lo_walls(LoParams P, LoBuffers B) {
                       B.wall_aero + ((side < 0 ? 0 : 1) * nx + i) * 3, red, rout);
 }
 
-// Last-CTA epilogue: dt_global = min(dt_local) (MPI_AllReduce MIN, mod_Solve.f90:409-418) and
-// the residual-norm sums (mod_TimeIntegrator.f90:102-106), reduced in a fixed order.
-__device__ void last_cta_epilogue(const LoParams& P, const LoBuffers& B, bool write_dt, bool write_diag,
-                                  double* red, double* rout) {
-    __shared__ unsigned s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(B.counter, 1u) == (unsigned)(gridDim.x - 1)) ? 1u : 0u;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    const int nc = P.nx * P.ny;
-    double acc[14];
-#pragma unroll
-    for (int m = 0; m < 13; ++m) acc[m] = 0.0;
-    acc[13] = -INFINITY;   // max of -dt_local == -min(dt_local)
-    for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-        if (write_dt) acc[13] = fmax(acc[13], -__ldcg(B.dtl + c));
-        if (write_diag) {
-#pragma unroll
-            for (int m = 0; m < 9; ++m) acc[m] += __ldcg(B.cell_diag + (size_t)c * kNDiag + m);
-#pragma unroll
-            for (int m = 0; m < 4; ++m) acc[9 + m] = fmax(acc[9 + m], __ldcg(B.cell_diag + (size_t)c * kNDiag + 9 + m));
-        }
-    }
-    block_reduce<9, 5>(acc, red, rout);
-    if (threadIdx.x == 0) {
-        if (write_diag) {
-            for (int m = 0; m < 13; ++m) B.diag[m] = acc[m];
-        }
-        if (write_dt) {
-            B.dt[1] = B.dt[0];   // dt_global of the step that just completed
-            B.dt[0] = P.fixed_dt > 0.0 ? P.fixed_dt : -acc[13];
-        }
-        *B.counter = 0u;
-    }
-}
-
 __global__ void __launch_bounds__(256) k_lo_timestep(LoParams P, LoBuffers B) {
     if (halted(B)) return;
     __shared__ double red[8 * 64];
