@@ -18,8 +18,8 @@
 //     process exits.
 //   * The first call on a device looks the array's device address up (cudaGetSymbolAddress) with
 //     that device current.
-//   * Every call synchronises its stream twice: once after copying the velocity table to the host
-//     (U_MAX / V_MAX set the time step) and once after reading the status and the outputs.  The
+//   * Every call synchronises its stream twice: once after scanning the velocity table (U_MAX / V_MAX set the
+//     time step, its structure the kernels) and once after reading the status and the outputs.  The
 //     call therefore cannot be captured in a CUDA graph.
 //   * Every call uses the same array and it keeps the previous call's contents; this call clears
 //     what must start at zero (the last-CTA counter and the status word).  Calls that overlap on
@@ -31,6 +31,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 
 #include "../../include/ugks_b200.h"
 #include "ugks_lo.cuh"
@@ -41,6 +42,8 @@ cudaError_t launch_lo_faces(const LoParams& P, const LoBuffers& B, cudaStream_t 
 cudaError_t launch_lo_walls(const LoParams& P, const LoBuffers& B, cudaStream_t s);
 cudaError_t launch_lo_cells(const LoParams& P, const LoBuffers& B, int mode, bool collision, cudaStream_t s);
 cudaError_t launch_lo_timestep(const LoParams& P, const LoBuffers& B, cudaStream_t s);
+cudaError_t launch_lo_fluxes_t(const LoParams& P, const LoBuffers& B, cudaStream_t s);
+cudaError_t launch_lo_cells_t(const LoParams& P, const LoBuffers& B, int mode, cudaStream_t s);
 }  // namespace ugks
 
 using namespace ugks;
@@ -54,6 +57,8 @@ constexpr int kMaxDevices = 64;
 // The scratch.  Host code must not use this name as an address: in host code it names a
 // host-side shadow, so only the address returned by cudaGetSymbolAddress is passed to kernels.
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
+// the axes of a tensor-product velocity table (LoBuffers::tab), beside the working set, whose limit stays as it was
+static __device__ __align__(256) double g_noalloc_tab[kTensorTab];
 
 // Device address of the scratch per device, filled on the first call on that device.  Every lookup of
 // one device yields the same address, so two host threads filling one entry at once store the same
@@ -61,7 +66,7 @@ static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
 std::atomic<double*> g_scratch_addr[kMaxDevices];
 
 struct Plan {
-    size_t flags, sxh, syh, sxb, syb, fxh, fxb, fxw, fyh, fyb, fyw, dtl, dt, cd, dg, wa, total;
+    size_t flags, dt, dg, scan, sxh, syh, sxb, syb, fxh, fxb, fxw, fyh, fyb, fyw, dtl, cd, wa, total;
 };
 
 Plan plan_for(int nx, int ny, int nv) {
@@ -69,14 +74,81 @@ Plan plan_for(int nx, int ny, int nv) {
     size_t off = 0;
     auto take = [&](size_t n) { size_t o = off; off += (n + 31) / 32 * 32; return o; };   // 256-byte aligned
     const size_t nc = (size_t)nx * ny, S = nc * nv, SY = (size_t)(ny + 1) * nx * nv;
-    p.flags = take(4);
+    p.flags = take(4); p.dt = take(2); p.dg = take(kNDiag);   // read back together
+    p.scan = 0;   // the table scan's result, in the words the steps then use: read before they start
     p.sxh = take(S); p.syh = take(S); p.sxb = take(S); p.syb = take(S);
     p.fxh = take(S); p.fxb = take(S); p.fxw = take(nc * 4);
     p.fyh = take(SY); p.fyb = take(SY); p.fyw = take((size_t)(ny + 1) * nx * 4);
-    p.dtl = take(nc); p.dt = take(2); p.cd = take(nc * kNDiag); p.dg = take(kNDiag);
+    p.dtl = take(nc); p.cd = take(nc * kNDiag);
     p.wa = take((size_t)2 * nx * 3);
     p.total = off;
     return p;
+}
+
+// One CTA over the velocity table: U_MAX and V_MAX (InitVelocityFromStructuredFile, mod_InitializeFlow.f90:508), and
+// whether it is a tensor product, by tensor_table's rule (the factors as means of the ratios, two alternations): then
+// out[2], out[3] are its abscissae per axis and tab its axes.  One launch and one small copy instead of two copies of the table.
+constexpr int kScanThreads = 256;
+__global__ void __launch_bounds__(kScanThreads) k_table_scan(const double* u, const double* v, const double* w, int nv, double* out,
+                                                             double* tab) {
+    __shared__ double mx[2][kScanThreads / 32], fx[64], fy[64];
+    __shared__ int s_nu, s_bad;
+    const int tid = threadIdx.x;
+    if (tid == 0) { s_nu = nv; s_bad = 0; }
+    __syncthreads();
+    double m[2] = {-INFINITY, -INFINITY};
+    for (int k = tid; k < nv; k += kScanThreads) {
+        m[0] = fmax(m[0], u[k]);
+        m[1] = fmax(m[1], v[k]);
+        if (v[k] != v[0]) atomicMin(&s_nu, k);
+    }
+    warp_max_all<2>(m);
+    if ((tid & 31) == 0) { mx[0][tid >> 5] = m[0]; mx[1][tid >> 5] = m[1]; }
+    __syncthreads();
+    const int nu = s_nu, nj = nv / nu;
+    bool ok = nv % nu == 0 && nu >= 2 && nj >= 2 && nu <= 64 && nj <= 64;
+    if (ok) {   // uniform over the CTA
+        for (int k = tid; k < nv; k += kScanThreads) {
+            const int i = k % nu;
+            if (!(u[k] == u[i] && v[k] == v[k - i] && w[k] > 0.0 && isfinite(w[k]) && isfinite(u[k]) && isfinite(v[k]))) s_bad = 1;
+        }
+        if (tid < nj) fy[tid] = w[tid * nu] / w[0];
+        // compensated means: the factors to an ulp, as the rule's 4 ulp for their product needs
+        for (int it = 0; it < 2; ++it) {
+            __syncthreads();
+            if (tid < nu) {
+                double t = 0.0, c = 0.0;
+                for (int j = 0; j < nj; ++j) comp_add(t, c, w[j * nu + tid] / fy[j]);
+                fx[tid] = (t + c) / (double)nj;
+            }
+            __syncthreads();
+            if (tid < nj) {
+                double t = 0.0, c = 0.0;
+                for (int i = 0; i < nu; ++i) comp_add(t, c, w[tid * nu + i] / fx[i]);
+                fy[tid] = (t + c) / (double)nu;
+            }
+        }
+        __syncthreads();
+        for (int k = tid; k < nv; k += kScanThreads) {
+            const int i = k % nu, j = k / nu;
+            if (!(fabs(fx[i] * fy[j] - w[k]) <= 4.0 * kEps * w[k])) s_bad = 1;
+        }
+        if (tid < 64) {
+            const double xu = u[min(tid, nu - 1)], xv = v[min(tid, nj - 1) * nu], a = tid < nu ? fx[tid] : 0.0, b = tid < nj ? fy[tid] : 0.0;
+            tab[tid] = xu; tab[64 + tid] = a; tab[128 + tid] = xv; tab[192 + tid] = b;
+            tab[256 + tid] = xu >= 0.0 ? a : 0.0; tab[320 + tid] = xu >= 0.0 ? 0.0 : a;
+            tab[384 + tid] = xv >= 0.0 ? b : 0.0; tab[448 + tid] = xv >= 0.0 ? 0.0 : b;
+        }
+        __syncthreads();
+        ok = s_bad == 0;
+    }
+    if (tid == 0) {
+        for (int t = 1; t < kScanThreads / 32; ++t) { mx[0][0] = fmax(mx[0][0], mx[0][t]); mx[1][0] = fmax(mx[1][0], mx[1][t]); }
+        out[0] = mx[0][0];
+        out[1] = mx[1][0];
+        out[2] = ok ? (double)nu : 0.0;
+        out[3] = ok ? (double)nj : 0.0;
+    }
 }
 
 int fail(cudaError_t e) {
@@ -116,20 +188,22 @@ extern "C" int ugks_step_explicit_noalloc(const ugks_params* prm, const double* 
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-    // U_MAX, V_MAX of the table (InitVelocityFromStructuredFile, mod_InitializeFlow.f90:508), staged in
-    // this call's own stack buffers (40 KB at the largest table), so concurrent calls from other host
-    // threads share no host memory
-    double hu[kMaxVel], hv[kMaxVel];
-    e = cudaMemcpyAsync(hu, u, nv * sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hv, v, nv * sizeof(double), cudaMemcpyDeviceToHost, s);
+    // U_MAX, V_MAX of the table and its axes when it is a tensor product; the host reads four numbers
+    void* tab = nullptr;
+    e = cudaGetSymbolAddress(&tab, g_noalloc_tab);
+    if (e != cudaSuccess) return fail(e);
+    k_table_scan<<<1, kScanThreads, 0, s>>>(u, v, w, nv, base + pl.scan, static_cast<double*>(tab));
+    double scan[4];
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(scan, base + pl.scan, sizeof scan, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(e);
-    double umax = -INFINITY, vmax = -INFINITY;
-    for (int k = 0; k < nv; ++k) { umax = std::fmax(umax, hu[k]); vmax = std::fmax(vmax, hv[k]); }
-    const LoParams P = make_lo_params(*prm, umax, vmax);
+    LoParams P = make_lo_params(*prm, scan[0], scan[1]);
+    P.tnu = (int)scan[2];
+    P.tnv = (int)scan[3];
 
     LoBuffers B{};
-    B.u = u; B.v = v; B.w = w; B.h = h; B.b = b; B.W = W;
+    B.u = u; B.v = v; B.w = w; B.tab = static_cast<double*>(tab); B.h = h; B.b = b; B.W = W;
     B.sxh = base + pl.sxh; B.syh = base + pl.syh; B.sxb = base + pl.sxb; B.syb = base + pl.syb;
     B.fxh = base + pl.fxh; B.fxb = base + pl.fxb; B.fxw = base + pl.fxw;
     B.fyh = base + pl.fyh; B.fyb = base + pl.fyb; B.fyw = base + pl.fyw;
@@ -145,19 +219,26 @@ extern "C" int ugks_step_explicit_noalloc(const ugks_params* prm, const double* 
     e = cudaMemsetAsync(base + pl.flags, 0, 4 * sizeof(double), s);
     if (e == cudaSuccess) e = launch_lo_timestep(P, B, s);
     for (int k = 0; k < nsteps && e == cudaSuccess; ++k) {
+        if (P.tnu > 0) {
+            e = launch_lo_fluxes_t(P, B, s);
+            if (e == cudaSuccess) e = launch_lo_cells_t(P, B, 3, s);
+            continue;
+        }
         e = launch_lo_slopes(P, B, s);
         if (e == cudaSuccess) e = launch_lo_faces(P, B, s);
         if (e == cudaSuccess) e = launch_lo_walls(P, B, s);
         if (e == cudaSuccess) e = launch_lo_cells(P, B, 3, false, s);
     }
     if (e != cudaSuccess) return fail(e);
-    unsigned status = 0;
-    double dt2[2] = {0.0, 0.0}, dg[kNDiag];
-    e = cudaMemcpyAsync(&status, B.status, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dt2, B.dt, sizeof dt2, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dg, B.diag, sizeof dg, cudaMemcpyDeviceToHost, s);
+    double back[96];   // status word, dt and norms, one copy
+    static_assert(kNDiag <= 32, "flags, dt and dg are the scratch's first three blocks of 32 doubles");
+    e = cudaMemcpyAsync(back, base + pl.flags, sizeof back, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(e);
+    unsigned words[2];
+    std::memcpy(words, back, sizeof words);
+    const unsigned status = words[1];
+    const double *dt2 = back + (pl.dt - pl.flags), *dg = back + (pl.dg - pl.flags);
     if (dt_out) *dt_out = nsteps > 0 ? dt2[1] : dt2[0];
     if (res_out && nsteps > 0) finish_explicit_res(nx, ny, dg, res_out);
     return status ? UGKS_ENUMERIC : UGKS_OK;
