@@ -1650,7 +1650,10 @@ __device__ __forceinline__ void adj_first_layer(const LoParams& P, const LoBuffe
 // each warp sums the five that land on its own cell into the state cotangent -- a plain read-modify-write
 // per (cell, velocity), nothing else writing the state cotangents meanwhile; the y stencil cotangents go to
 // yq ([cell][field][5][nvel], the face-cache cotangent's storage, free once k_adj_recon2 has read it).
-__global__ void __launch_bounds__(512) k_adj_recon1_xy(LoParams P, LoBuffers B, AdjBuffers A, double* yq) {
+// 32 warps an SM (64 registers, some spills): it waits on its loads, and at 8x64x32^2 16 warps took 273 us, 24 152,
+// 32 135 and 40 151 (ncu, cold).
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_adj_recon1_xy(LoParams P, LoBuffers B, AdjBuffers A, double* yq) {
     extern __shared__ double s_gq[];   // [cell][5][32]
     const int nv = P.nvel, nx = P.nx, ny = P.ny, lane = threadIdx.x & 31, i = threadIdx.x >> 5;
     const int k = blockIdx.x * 32 + lane, j = blockIdx.y, f = blockIdx.z, cc = j * nx + i;
@@ -1802,8 +1805,10 @@ static cudaError_t adj_launch(const LoParams& P, const LoBuffers& B, const S2Buf
         k_adj_recon2<<<grid, 256, 0, s>>>(P, B, S, A);
         const unsigned kb = (unsigned)((nv + 31) / 32);
         if (nx <= 16) {   // one row per CTA
-            k_adj_recon1_xy<<<dim3(kb, (unsigned)ny, 2), 32 * nx, (size_t)nx * 5 * 32 * sizeof(double), s>>>(P, B, A,
-                                                                                                         A.grec);
+            const dim3 g(kb, (unsigned)ny, 2);
+            const size_t sm = (size_t)nx * 5 * 32 * sizeof(double);
+            if (nx <= 8) k_adj_recon1_xy<256><<<g, 32 * nx, sm, s>>>(P, B, A, A.grec);
+            else k_adj_recon1_xy<512><<<g, 32 * nx, sm, s>>>(P, B, A, A.grec);
             k_adj_recon1_yg<<<dim3((unsigned)((nv + 255) / 256), (unsigned)nc, 2), 256, 0, s>>>(P, A, A.grec);
         } else {
             k_adj_recon1<<<grid, 128, 0, s>>>(P, B, A, 0);
