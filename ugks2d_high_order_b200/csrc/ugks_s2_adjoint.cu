@@ -1444,11 +1444,12 @@ __global__ void __launch_bounds__(256) k_adj_macro_faces(LoParams P, const doubl
 }
 
 // ---------------------------------------------------------------------------------------------
-// the second layer and the positivity limiter (k_s2_recon2), transposed: CTA = 8 warps (field, part)
-// over 32 velocities of one cell, as the forward kernel.  grec (this cell's face-cache entries) -> gl1 of the rows /
-// columns the templates read, and the state (the limiter's cell means, the wall rows' direct samples).
-// Three CTAs per SM (80 registers with spills): measured 2.3 % faster over the backward than two at 128.
-__global__ void __launch_bounds__(256, 3) k_adj_recon2(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
+// the second layer and the positivity limiter (k_s2_recon2), transposed.  grec (this cell's face-cache entries) -> gl1
+// of the rows / columns the templates read, and the state (the limiter's cell means, the wall rows' direct samples).
+//
+// k_adj_recon2_wall: the cells in the three rows next to a wall; CTA = 8 warps (field, part) over 32 velocities of one
+// cell.  Three CTAs per SM (80 registers with spills): measured 2.3 % faster over the backward than two at 128.
+__global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
     __shared__ double s_th[8][32];
     __shared__ double s_gth[8][32];
     const int nv = P.nvel, nx = P.nx, ny = P.ny, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1456,7 +1457,7 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2(LoParams P, LoBuffers B, 
     const int k0 = blockIdx.x * 32 + lane;
     const bool kok = k0 < nv;
     const int k = kok ? k0 : nv - 1;
-    const int cc = blockIdx.y, i = cc % nx, j = cc / nx;
+    const int wrows = min(ny, 6), row = blockIdx.y / nx, i = blockIdx.y % nx, j = row < 3 ? row : ny - wrows + row, cc = j * nx + i;
     const bool nw = s2_near_wall(j, ny);
     const int first = nw ? s2_wall_first(j, ny) : j - 2;
     const double* L1 = S.l1 + (size_t)f * 11 * nv + k;
@@ -1613,6 +1614,119 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2(LoParams P, LoBuffers B, 
         }
 #pragma unroll
         for (int r = 0; r < 5; ++r) atomic_add(gX(r, 4 + p), gc5[r]);
+    }
+}
+
+// k_adj_recon2: the other cells; CTA = 4 warps (field, axis) over 32 velocities of one cell.  Only the side a velocity
+// leaves through carries cotangents (the face cache keeps no other), so a thread runs that side's template and its
+// transpose; the other side and the volume rows enter the limiter's minimum with their values, and a transpose of theirs
+// runs only where one of them is the smallest sample of a limited cell.
+// At 8x64x32^2 188 us and 62 for the wall rows, which run beside it, against 482 for all cells in the wall rows' form
+// (ncu, cold); 3, 4 and 6 CTAs an SM took 216, 191 and 195.
+__global__ void __launch_bounds__(128, 5) k_adj_recon2(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
+    __shared__ double s_th[4][32], s_gth[4][32];
+    const int nv = P.nvel, nx = P.nx, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, f = warp >> 1, axis = warp & 1;
+    const int k0 = blockIdx.x * 32 + lane;
+    const bool kok = k0 < nv;
+    const int k = kok ? k0 : nv - 1;
+    const int cc = 3 * nx + (int)blockIdx.y, i = cc % nx;
+    const double vn = axis == 0 ? B.u[k] : B.v[k], vt = axis == 0 ? B.v[k] : B.u[k];
+    const int q0 = axis * 7 + (vn >= 0.0 ? 2 : 0), q1 = axis * 7 + (vn >= 0.0 ? 0 : 2);   // l1 entries of the two sides
+    const size_t field = (size_t)f * 11 * nv + k, cell = (size_t)22 * nv;
+    // the cell whose first layer is sample r of a face template, and of a volume row
+    auto fc = [&](int r) { return (size_t)(axis == 0 ? cc + (r - 2) * nx : cc - i + wrapx(i + r - 2, nx)) * cell + field; };
+    auto vc = [&](int r) { return (size_t)(cc + (r - 2) * nx) * cell + field; };
+    const double hm = B.h[(size_t)cc * nv + k], bm = B.b[(size_t)cc * nv + k], mf = f == 0 ? hm : bm;
+    const double margin = 64.0 * kEps;
+    double face[3], dn[3], dt[3], b5[5];
+    S2Weno wf;    // the template's weights and their intermediates, for its transpose
+    S2WenoX xf;
+    double xmin = 0.0;
+    int arg = -1;   // the smallest sample: a (face), 3 + a (other side), 6 + 3 row + a (volume)
+    auto sample = [&](double x, int id) {
+        if (x < xmin) { xmin = x; arg = id; }
+    };
+    {
+        double a5[5], o5[5], v3[3];
+#pragma unroll
+        for (int r = 0; r < 5; ++r) {
+            const double* l = S.l1 + fc(r);
+            a5[r] = l[(size_t)q0 * nv];
+            b5[r] = l[(size_t)(q0 + 1) * nv];
+            o5[r] = l[(size_t)q1 * nv];
+        }
+        companion3_fwd(a5, b5, face, dt, dn, wf, xf);
+        s2_power_values3(o5, v3);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) { sample(face[a], a); sample(v3[a], 3 + a); }
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {   // volume rows 0, 1 by the x warp, 2 by the y warp
+            const int row = axis == 0 ? p : 2;
+            if (axis == 1 && p == 1) break;
+#pragma unroll
+            for (int r = 0; r < 5; ++r) o5[r] = S.l1[vc(r) + (size_t)(4 + row) * nv];
+            s2_power_values3(o5, v3);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) sample(v3[a], 6 + 3 * row + a);
+        }
+    }
+    const double cand = xmin < 0.0 ? fmin(1.0, (1.0 - margin) * mf / (mf - xmin)) : 1.0;
+    s_th[warp][lane] = cand;
+    __syncthreads();
+    double tmin = s_th[0][lane];
+    int wmin = 0;
+#pragma unroll
+    for (int w = 1; w < 4; ++w) if (s_th[w][lane] < tmin) { tmin = s_th[w][lane]; wmin = w; }
+    const bool zero = hm <= 0.0 || bm <= 0.0;
+    const double theta = zero ? 0.0 : fmax(0.0, fmin(1.0, tmin));
+    const double ind = 1.0 / (axis == 0 ? P.dx : P.dy), itd = 1.0 / (axis == 0 ? P.dy : P.dx);
+    const double* gr = A.grec + rec_cell(cc, axis, f, 0, nv) + k;   // the path derivative two fields on
+    double gface[3], gdn[3], gdt[3], gmf = 0.0, gth = 0.0, gx = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double gv = gr[(size_t)a * nv], gp = gr[(size_t)(6 + a) * nv], gn = vn * gp * ind, gt = vt * gp * itd;
+        gface[a] = theta * gv;
+        gmf += (1.0 - theta) * gv;
+        gth += (face[a] - mf) * gv + dn[a] * gn + dt[a] * gt;
+        gdn[a] = theta * gn;
+        gdt[a] = theta * gt;
+    }
+    s_gth[warp][lane] = gth;
+    __syncthreads();
+    // theta = min over the 4 warps' candidates when it is below 1: the smallest sample carries its cotangent, gx
+    if (!zero && tmin < 1.0 && warp == wmin && arg >= 0) {
+        const double all = (s_gth[0][lane] + s_gth[1][lane]) + (s_gth[2][lane] + s_gth[3][lane]);
+        const double den = mf - xmin;
+        gx = all * ((1.0 - margin) * mf / (den * den));
+        gmf += all * (-(1.0 - margin) * xmin / (den * den));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) gface[a] += arg == a ? gx : 0.0;
+    }
+    if (!kok) return;
+    atomic_add((f == 0 ? A.ghi : A.gbi) + (size_t)cc * nv + k, gmf);
+    {
+        double ga5[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, gb5[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        companion3_vjp(wf, xf, b5, gface, gdt, gdn, ga5, gb5);
+#pragma unroll
+        for (int r = 0; r < 5; ++r) {
+            double* g = A.gl1 + fc(r);
+            atomic_add(g + (size_t)q0 * nv, ga5[r]);
+            atomic_add(g + (size_t)(q0 + 1) * nv, gb5[r]);
+        }
+    }
+    if (gx != 0.0 && arg >= 3) {   // a sample that only the limiter sees
+        const bool other = arg < 6;
+        const int q = other ? q1 : 4 + (arg - 6) / 3;
+        const int pts[3] = {S2_G0, S2_G0 + 1, S2_G0 + 2};
+        const double zero3[3] = {0.0, 0.0, 0.0};
+        double c5[5], gc5[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, gv[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) gv[a] = arg % 3 == a ? gx : 0.0;
+#pragma unroll
+        for (int r = 0; r < 5; ++r) c5[r] = S.l1[(other ? fc(r) : vc(r)) + (size_t)q * nv];
+        weno_points_vjp<3>(c5, pts, gv, zero3, gc5);
+#pragma unroll
+        for (int r = 0; r < 5; ++r) atomic_add(A.gl1 + (other ? fc(r) : vc(r)) + (size_t)q * nv, gc5[r]);
     }
 }
 
@@ -1788,21 +1902,24 @@ static cudaError_t adj_launch(const LoParams& P, const LoBuffers& B, const S2Buf
     }
     if (e == cudaSuccess) {
         k_adj_wall_nodes<<<warps(2LL * nx * 3, 256), 256, 0, sw>>>(P, B, S, A);
-        if (side) e = cudaEventRecord(ev[1], s2);
     }
     if (e == cudaSuccess) {
         k_adj_face_nodes<<<warps((long long)nf * 3, 128), 128, 0, s>>>(P, B, S, A);
         if (side) e = cudaEventRecord(ev[2], s);
     }
     if (e == cudaSuccess && side) e = cudaStreamWaitEvent(s2, ev[2], 0);
+    const dim3 grid((unsigned)((nv + 31) / 32), (unsigned)nc);
     if (e == cudaSuccess) {
         k_adj_macro_faces<<<(unsigned)((nf * 8 + 255) / 256), 256, 0, sw>>>(P, B.W, A.gmac, A.gWi);
+        // the wall rows' cells after the wall nodes, whose sides they read, beside the others
+        k_adj_recon2_wall<<<dim3(grid.x, (unsigned)((ny < 6 ? ny : 6) * nx)), 256, 0, sw>>>(P, B, S, A);
         if (side) e = cudaEventRecord(ev[3], s2);
     }
-    if (e == cudaSuccess && side) e = cudaStreamWaitEvent(s, ev[1], 0);   // recon2 reads the wall sides
     if (e == cudaSuccess) {
-        const dim3 grid((unsigned)((nv + 31) / 32), (unsigned)nc);
-        k_adj_recon2<<<grid, 256, 0, s>>>(P, B, S, A);
+        if (ny > 6) k_adj_recon2<<<dim3(grid.x, (unsigned)((ny - 6) * nx)), 128, 0, s>>>(P, B, S, A);
+        if (side) e = cudaStreamWaitEvent(s, ev[3], 0);   // the wall rows; and gWi complete before the next step
+    }
+    if (e == cudaSuccess) {
         const unsigned kb = (unsigned)((nv + 31) / 32);
         if (nx <= 16) {   // one row per CTA
             const dim3 g(kb, (unsigned)ny, 2);
@@ -1815,7 +1932,6 @@ static cudaError_t adj_launch(const LoParams& P, const LoBuffers& B, const S2Buf
             k_adj_recon1<<<grid, 128, 0, s>>>(P, B, A, 1);
         }
     }
-    if (e == cudaSuccess && side) e = cudaStreamWaitEvent(s, ev[3], 0);   // gWi complete before the next step
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
