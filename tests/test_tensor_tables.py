@@ -188,3 +188,39 @@ def test_explicit_tensor_path_matches_oracle_and_general_path(shape, grid):
     p = rng.permutation(len(t[0]))
     ph, pb, pW, aero = gpu(tuple(a[p] for a in t), (h[..., p], b[..., p]))
     close((got[0][..., p], got[1][..., p], got[2], got[3]), (ph, pb, pW, aero))
+
+
+# Tolerance: the two paths' closures meet their moments to 5e-13 each, and the closure systems they enter amplify that by
+# their condition, of order 1e2 in these units: 1e-10 of the largest cotangent.
+VJP_TOL = 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,grid", [((14, 14), (5, 9)), ((12, 20), (8, 12)), ((24, 10), (3, 9)), ((32, 32), (4, 9)),
+                                        ((34, 28), (18, 10)), ((64, 36), (3, 11))])
+def test_adjoint_tensor_path_matches_general_path(shape, grid):
+    """One S2CN2 step's vector-Jacobian product on a tensor table against the same table in another order."""
+    from ugks2d_high_order_b200.case import reference_case
+    from ugks2d_high_order_b200.solver import Solver
+    t, (nx, ny) = rectangle(*shape), grid
+    c = reference_case("S2CN2").with_(nx=nx, ny=ny, dx=1 / nx, dy=1 / ny, wall_ux=(-2.0, 3.0), wall_tnative=(1.8, 2.1))
+    rng = np.random.default_rng(7)
+    rho, U, V, T = (a + s * rng.uniform(-1, 1, (ny, nx, 1)) for a, s in ((1, 0.05), (0.1, 0.2), (0, 0.2), (2, 0.1)))
+    h = rho / (np.pi * T) * np.exp(-((t[0] - U) ** 2 + (t[1] - V) ** 2) / T) * (1 + 0.02 * np.tanh(t[0] * t[1]))
+    b = 0.5 * c.ck * T * h
+    W = np.stack([h @ t[2], h @ (t[2] * t[0]), h @ (t[2] * t[1]), 0.5 * (h @ (t[2] * (t[0] ** 2 + t[1] ** 2)) + b @ t[2])], -1)
+    gh, gb, gW, seed = rng.normal(size=h.shape), rng.normal(size=h.shape), rng.normal(size=W.shape), rng.normal(size=4)
+
+    def vjp(p):
+        s = Solver(c, *(np.ascontiguousarray(a[p]) for a in t))
+        try:
+            s.upload(h[..., p], b[..., p], W)
+            s.s2cn2_init()
+            return s.s2cn2_step_vjp(gh[..., p], gb[..., p], gW, seed)
+        finally:
+            s.close()
+
+    p = rng.permutation(len(t[0]))
+    got, want = vjp(np.arange(len(p))), vjp(p)
+    for x, y in zip((got[0][..., p], got[1][..., p], got[2], got[3]), want):
+        assert np.isfinite(y).all() and np.abs(x - y).max() <= VJP_TOL * np.abs(y).max()

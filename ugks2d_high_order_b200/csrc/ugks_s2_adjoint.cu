@@ -1561,7 +1561,8 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffer
         for (int w = 0; w < 8; ++w) gt_all += s_gth[w][lane];
         const double smp = arg < 3 ? face[arg] : vol[arg - 3];
         const double den = mf - smp;
-        const double dsmp = (1.0 - margin) * mf / (den * den), dmf = -(1.0 - margin) * smp / (den * den);
+        // (den times den is 0 below 1e-154, where velocities far from the mean lie)
+        const double dsmp = (1.0 - margin) * mf / den / den, dmf = -(1.0 - margin) * smp / den / den;
         if (arg < 3) gface[arg] += gt_all * dsmp;
         else gvol[arg - 3] += gt_all * dsmp;
         gmf += gt_all * dmf;
@@ -1697,8 +1698,8 @@ __global__ void __launch_bounds__(128, 5) k_adj_recon2(LoParams P, LoBuffers B, 
     if (!zero && tmin < 1.0 && warp == wmin && arg >= 0) {
         const double all = (s_gth[0][lane] + s_gth[1][lane]) + (s_gth[2][lane] + s_gth[3][lane]);
         const double den = mf - xmin;
-        gx = all * ((1.0 - margin) * mf / (den * den));
-        gmf += all * (-(1.0 - margin) * xmin / (den * den));
+        gx = all * ((1.0 - margin) * mf / den / den);   // den times den is 0 below 1e-154
+        gmf += all * (-(1.0 - margin) * xmin / den / den);
 #pragma unroll
         for (int a = 0; a < 3; ++a) gface[a] += arg == a ? gx : 0.0;
     }
