@@ -28,6 +28,8 @@
 #include "ugks_s2_adjoint.cuh"
 #include "ugks_s2_math.cuh"
 
+#include <utility>
+
 namespace ugks {
 namespace {
 
@@ -152,9 +154,8 @@ __device__ __forceinline__ void face_chain(const LoParams& P, double dt, const T
 struct QV {
     double qh, qb, ld[4], ldb[4], du, dv, c2;
 };
-__device__ __forceinline__ QV qv_at(const S2Th& t, double u, double v) {
+__device__ __forceinline__ QV qv_of(const S2Th& t, const S2Q& s, double u, double v) {
     QV q;
-    const S2Q s = s2_q(t, u, v);
     q.qh = s.qh;
     q.qb = s.qb;
 #pragma unroll
@@ -164,6 +165,7 @@ __device__ __forceinline__ QV qv_at(const S2Th& t, double u, double v) {
     q.c2 = q.du * q.du + q.dv * q.dv;
     return q;
 }
+__device__ __forceinline__ QV qv_at(const S2Th& t, double u, double v) { return qv_of(t, s2_q(t, u, v), u, v); }
 // out[b] = sum_a V[a] d(q ld_a)/d theta_b for the h field (hb = 0) or the b field (hb = 1):
 // d(q ld_a)/d theta_b = q (ld_a ld_b + d ld_a / d theta_b), theta = (rho, u, v, T_native)
 __device__ __forceinline__ void vhess(const S2Th& t, const QV& q, int hb, const double V[4], double out[4]) {
@@ -201,6 +203,120 @@ __device__ __forceinline__ void heat_shift_adj(double w, double cx, double cy, d
     gux += gx * (0.5 * w * (-base - 2.0 * cx * cx * fh)) - gy * xy;
     gvy += -gx * xy + gy * (0.5 * w * (-base - 2.0 * cy * cy * fh));
 }
+
+// make_mke's raw moments and the Jacobian, transposed at one velocity of weight w: cotangents gax, gay of the moments of
+// K_x and K_y, gJ of the moment Jacobian; g accumulates those of (coeff, lam, ux, vy, theta[4])
+__device__ __forceinline__ void mke_vjp(const S2Th& th, const QV& v, const WMke& M, double w, double u, double vv,
+                                        double shb_add, const double gax[4], const double gay[4], const double gJ[16],
+                                        double g[8]) {
+    const double cx = u - M.ux, cy = vv - M.vy, c2 = cx * cx + cy * cy;
+    const double shh = 2.0 * M.lam * c2 - 4.0, shb = shh + shb_add;
+    const double kxh = psi_h(w, u, vv, gax), kxb = psi_b(w, gax), kyh = psi_h(w, u, vv, gay), kyb = psi_b(w, gay);
+    const double xh = kxh * v.qh, xb = kxb * v.qb, yh = kyh * v.qh, yb = kyb * v.qb;
+    g[0] += cx * (xh * shh + xb * shb) + cy * (yh * shh + yb * shb);
+    g[1] += M.coeff * 2.0 * c2 * (cx * (xh + xb) + cy * (yh + yb));
+    g[2] += M.coeff * (xh * (-shh - 4.0 * M.lam * cx * cx) + xb * (-shb - 4.0 * M.lam * cx * cx) +
+                       (yh + yb) * (-4.0 * M.lam * cx * cy));
+    g[3] += M.coeff * (yh * (-shh - 4.0 * M.lam * cy * cy) + yb * (-shb - 4.0 * M.lam * cy * cy) +
+                       (xh + xb) * (-4.0 * M.lam * cx * cy));
+    const double Ah = M.coeff * shh * (cx * kxh + cy * kyh), Ab = M.coeff * shb * (cx * kxb + cy * kyb);
+    double Vh[4], Vb[4], hh[4], hb[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        Vh[a] = w * (gJ[a] + u * gJ[4 + a] + vv * gJ[8 + a] + 0.5 * (u * u + vv * vv) * gJ[12 + a]);
+        Vb[a] = 0.5 * w * gJ[12 + a];
+    }
+    vhess(th, v, 0, Vh, hh);
+    vhess(th, v, 1, Vb, hb);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) g[4 + a] += Ah * v.qh * v.ld[a] + Ab * v.qb * v.ldb[a] + hh[a] + hb[a];
+}
+
+// ---------------------------------------------------------------------------------------------
+// Polynomial nodes, for tensor-product velocity tables.  Every transposed closure sum is
+//   sum_k a_k e_x(u_i) e_y(v_j) p(u_i, v_j)
+// with e the exponential rows of a Maxwellian, a_k data (or the table's weights) and p a polynomial of degree < K along
+// an axis, whatever its coefficients.  Interpolating p along that axis at K points y_m (exact: sum_m l_m(v) p(y_m) = p(v))
+// turns an axis into K nodes of weight sum_j a_j e_y(v_j) l_m(v_j), and the long expressions p, 150 to 300 operations
+// each, run at the nodes instead of at the velocities.  The points follow the Maxwellian (its mean, times its
+// thermal width; near the Gauss-Hermite points), so no node's value is large against the sum; any K points are exact.
+template <int K>
+__host__ __device__ constexpr double pn_x(int m) {   // in thermal widths
+    return m >= K / 2 ? -pn_x<K>(K - 1 - m)
+           : K == 6   ? (m == 0 ? -2.35 : m == 1 ? -1.34 : -0.44)
+                      : (m == 0 ? -2.93 : m == 1 ? -1.98 : m == 2 ? -1.16 : -0.38);
+}
+template <int K>
+__host__ __device__ constexpr double pn_c(int m) {
+    double d = 1.0;
+    for (int n = 0; n < K; ++n)
+        if (n != m) d *= pn_x<K>(m) - pn_x<K>(n);
+    return 1.0 / d;
+}
+__constant__ double c_pn6[6] = {pn_x<6>(0), pn_x<6>(1), pn_x<6>(2), pn_x<6>(3), pn_x<6>(4), pn_x<6>(5)};
+__constant__ double c_pn8[8] = {pn_x<8>(0), pn_x<8>(1), pn_x<8>(2), pn_x<8>(3),
+                                pn_x<8>(4), pn_x<8>(5), pn_x<8>(6), pn_x<8>(7)};
+template <int K, int... I>
+__device__ __forceinline__ void pn_basis_i(double x, double f, double* l, std::integer_sequence<int, I...>) {
+    constexpr double xs[K] = {pn_x<K>(I)...}, cs[K] = {pn_c<K>(I)...};
+    double p = f;
+#pragma unroll
+    for (int m = 0; m < K; ++m) { l[m] = p * cs[m]; p *= x - xs[m]; }
+    p = 1.0;
+#pragma unroll
+    for (int m = K - 1; m >= 0; --m) { l[m] *= p; p *= x - xs[m]; }
+}
+// l[m] = f l_m(x)
+template <int K>
+__device__ __forceinline__ void pn_basis(double x, double f, double* l) {
+    pn_basis_i<K>(x, f, l, std::make_integer_sequence<int, K>{});
+}
+// node weights of an axis, out[m] = sum_j w_j exp(-(x_j - mean)^2 itw) l_m, by the warp; split: the abscissae >= 0 to
+// out[0..7], the others to out[8..15]
+template <bool SPLIT>
+__device__ __forceinline__ void pn_weights(const double* tab, const double* wt, int n, double mean, double itw, double iw,
+                                           double* out) {
+    const int lane = threadIdx.x & 31;
+    constexpr int N = SPLIT ? 16 : 8;
+    double a[N];
+#pragma unroll
+    for (int m = 0; m < N; ++m) a[m] = 0.0;
+    for (int j = lane; j < n; j += 32) {
+        const double d = tab[j] - mean;
+        double l[8];
+        pn_basis<8>(d * iw, wt[j] * exp(-(d * d) * itw), l);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            if (SPLIT) {
+                a[m] += tab[j] >= 0.0 ? l[m] : 0.0;
+                a[N - 8 + m] += tab[j] >= 0.0 ? 0.0 : l[m];
+            } else {
+                a[m] += l[m];
+            }
+        }
+    }
+    warp_sum_all<N>(a);
+    __syncwarp();
+    if (lane == 0)
+#pragma unroll
+        for (int m = 0; m < N; ++m) out[m] = a[m];
+    __syncwarp();
+}
+// the warp's shared scalars are read anew in every iteration: kept in registers across the long bodies they spilled
+__device__ __forceinline__ void pn_reload() { asm volatile("" ::: "memory"); }
+// A warp's columns of a table: lanes take a velocity column each, G lanes the rows of one where it is narrow
+struct PnCols {
+    int cw, G, c, g;
+    bool act;
+    __device__ __forceinline__ PnCols(int nu) {
+        const int lane = threadIdx.x & 31;
+        cw = min(nu, 32);
+        G = 32 / cw;
+        g = lane / cw;
+        c = lane - g * cw;
+        act = g < G;
+    }
+};
 
 // ---------------------------------------------------------------------------------------------
 // WENO-AO(5,3) weights: the transpose of fw(q) (weno_coefficients, mod_S2D1Reconstruction.f90:168-204),
@@ -468,13 +584,61 @@ __global__ void __launch_bounds__(NT) k_adj_collide(LoParams P, LoBuffers B, S2B
     }
 }
 
+// build_targets' six sums of a node, transposed at one velocity (or polynomial node): acc[0..3], [4..7] the directions
+// K_x, K_y, [8..11] coeff, lam, ux, vy, [12..15] theta
+__device__ __forceinline__ void target_vjp(const S2Th& th, const QV& v, const WMke& M, double u, double vv, double wt2,
+                                           double shb_add, double gmh, double gmb, double gkxh, double gkxb, double gkyh,
+                                           double gkyb, double acc[16]) {
+    const double cx = u - M.ux, cy = vv - M.vy, c2 = cx * cx + cy * cy;
+    const double shh = 2.0 * M.lam * c2 - 4.0, shb = shh + shb_add;
+    double Dh[4], Db[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) { Dh[a] = v.qh * v.ld[a]; Db[a] = v.qb * v.ldb[a]; }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        acc[a] += -wt2 * (gkxh * Dh[a] + gkxb * Db[a]);
+        acc[4 + a] += -wt2 * (gkyh * Dh[a] + gkyb * Db[a]);
+    }
+    const double xh = gkxh * v.qh, xb = gkxb * v.qb, yh = gkyh * v.qh, yb = gkyb * v.qb;
+    acc[8] += wt2 * (cx * (xh * shh + xb * shb) + cy * (yh * shh + yb * shb));
+    acc[9] += wt2 * M.coeff * 2.0 * c2 * (cx * (xh + xb) + cy * (yh + yb));
+    acc[10] += wt2 * M.coeff * (xh * (-shh - 4.0 * M.lam * cx * cx) + xb * (-shb - 4.0 * M.lam * cx * cx) +
+                                (yh + yb) * (-4.0 * M.lam * cx * cy));
+    acc[11] += wt2 * M.coeff * (yh * (-shh - 4.0 * M.lam * cy * cy) + yb * (-shb - 4.0 * M.lam * cy * cy) +
+                                (xh + xb) * (-4.0 * M.lam * cx * cy));
+    const double Ah = wt2 * (gmh + M.coeff * shh * (cx * gkxh + cy * gkyh));
+    const double Ab = wt2 * (gmb + M.coeff * shb * (cx * gkxb + cy * gkyb));
+    double Bh[4], Bb[4], hh[4], hb[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        Bh[a] = -wt2 * (gkxh * M.tdx[a] + gkyh * M.tdy[a]);
+        Bb[a] = -wt2 * (gkxb * M.tdx[a] + gkyb * M.tdy[a]);
+    }
+    vhess(th, v, 0, Bh, hh);
+    vhess(th, v, 1, Bb, hb);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) acc[12 + a] += Ah * Dh[a] + Ab * Db[a] + hh[a] + hb[a];
+}
+
 // ---------------------------------------------------------------------------------------------
 // build_targets of a state, transposed: one warp per (cell, volume node).  gT: cotangents of the six
 // target arrays; the node's scalars (tscal) and state (wq) come from the forward targets of that state.
-// Writes gwq[(cell * 9 + node) * 4 + m].
-__global__ void __launch_bounds__(256, 2) k_adj_targets(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A,
-                                                         const double* gT0, const double* gT1, const double* gT2,
-                                                         const double* gT3, const double* gT4, const double* gT5) {
+// Writes gwq[(cell * 9 + node) * 4 + m].  TENSOR: the sums by polynomial nodes, 6 evaluations of the first pass's
+// expression a column and 2 a lane of the second's in place of one a velocity; three warps a CTA, so that a cell is three CTAs and their shared
+// memory admits four an SM.  At 8x64x32^2 (4608 nodes) 177 us before, 100 with the nodes and 86 with the scalars in shared
+// memory; 3, 5 and 6 CTAs an SM 107, 111 and 141 us (ncu, cold).
+struct AdjTargetShared {   // a warp's: the node, the closure's Jacobian and its cotangent, two right-hand sides J^T x = b
+    S2Th th;
+    WMke M;
+    double jac[16], gJ[16], b[2][4];
+};
+struct PnTargets {   // a warp's row basis (then node weights) and its columns' nodes
+    double row[64][6], a[6][6][32];
+};
+template <bool TENSOR>
+__global__ void __launch_bounds__(TENSOR ? 96 : 256, TENSOR ? 4 : 2) k_adj_targets(
+    LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A, const double* gT0, const double* gT1, const double* gT2,
+    const double* gT3, const double* gT4, const double* gT5) {
     const int nc = P.nx * P.ny, nv = P.nvel, ck = P.ck, nr = (nv + 31) >> 5, lane = threadIdx.x & 31;
     const int wid = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (wid >= nc * 9) return;
@@ -482,92 +646,117 @@ __global__ void __launch_bounds__(256, 2) k_adj_targets(LoParams P, LoBuffers B,
     const double gw3[3] = {5.0 / 18.0, 4.0 / 9.0, 5.0 / 18.0};
     const double wt2 = gw3[p % 3] * gw3[p / 3];
     const double* o = S.tscal + (size_t)wid * kS2TScal;
-    double thv[4], jac[16];
-    WMke M;
-    w_load_scalars(o, thv, M);
-#pragma unroll
-    for (int m = 0; m < 16; ++m) jac[m] = o[16 + m];
-    const S2Th th = s2_th(thv, ck);
+    __shared__ AdjTargetShared Ns[TENSOR ? 3 : 8];
+    AdjTargetShared& N = Ns[threadIdx.x >> 5];
+    const S2Th& th = N.th;
+    const WMke& M = N.M;
+    double* const jac = N.jac;
+    if (lane < 16) jac[lane] = o[16 + lane];
+    if (lane == 0) {
+        double thv[4];
+        w_load_scalars(o, thv, N.M);
+        N.th = s2_th(thv, ck);
+    }
+    __syncwarp();
     const double shb_add = 2.0 / (double)ck;
+    __shared__ PnTargets Xs[TENSOR ? 3 : 1];
+    PnTargets& X = Xs[TENSOR ? threadIdx.x >> 5 : 0];
     // pass A: d/d(tdx, tdy, coeff, lam, ux, vy, theta) of the Gauss-weighted sums
     double acc[16];
 #pragma unroll
     for (int m = 0; m < 16; ++m) acc[m] = 0.0;
-    for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
-        if (!s.ok) continue;
-        const size_t q = (size_t)cc * nv + s.k;
-        const double gmh = gT0[q], gmb = gT1[q], gkxh = gT2[q], gkxb = gT3[q], gkyh = gT4[q], gkyb = gT5[q];
-        const QV v = qv_at(th, s.u, s.v);
-        const double cx = s.u - M.ux, cy = s.v - M.vy, c2 = cx * cx + cy * cy;
-        const double shh = 2.0 * M.lam * c2 - 4.0, shb = shh + shb_add;
-        double Dh[4], Db[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) { Dh[a] = v.qh * v.ld[a]; Db[a] = v.qb * v.ldb[a]; }
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            acc[a] += -wt2 * (gkxh * Dh[a] + gkxb * Db[a]);
-            acc[4 + a] += -wt2 * (gkyh * Dh[a] + gkyb * Db[a]);
+    if constexpr (TENSOR) {   // the rows' polynomial nodes of each column (the sums' polynomials: degree 5 along an axis)
+        const int nu = P.tnu, nw = P.tnv;
+        const double* tab = B.tab;
+        const double width = sqrt(th.tw), iw = 1.0 / width;
+        for (int j = lane; j < nw; j += 32) {
+            const double d = tab[128 + j] - th.v;
+            pn_basis<6>(d * iw, exp(-(d * d) * th.itw), X.row[j]);
         }
-        const double xh = gkxh * v.qh, xb = gkxb * v.qb, yh = gkyh * v.qh, yb = gkyb * v.qb;
-        acc[8] += wt2 * (cx * (xh * shh + xb * shb) + cy * (yh * shh + yb * shb));
-        acc[9] += wt2 * M.coeff * 2.0 * c2 * (cx * (xh + xb) + cy * (yh + yb));
-        acc[10] += wt2 * M.coeff * (xh * (-shh - 4.0 * M.lam * cx * cx) + xb * (-shb - 4.0 * M.lam * cx * cx) +
-                                    (yh + yb) * (-4.0 * M.lam * cx * cy));
-        acc[11] += wt2 * M.coeff * (yh * (-shh - 4.0 * M.lam * cy * cy) + yb * (-shb - 4.0 * M.lam * cy * cy) +
-                                    (xh + xb) * (-4.0 * M.lam * cx * cy));
-        const double Ah = wt2 * (gmh + M.coeff * shh * (cx * gkxh + cy * gkyh));
-        const double Ab = wt2 * (gmb + M.coeff * shb * (cx * gkxb + cy * gkyb));
-        double Bh[4], Bb[4], hh[4], hb[4];
+        __syncwarp();
+        const PnCols L(nu);
+        for (int c0 = 0; c0 < nu; c0 += 32) {
+            const bool act = L.act && c0 + L.c < nu;
+            const int c = min(c0 + L.c, nu - 1);
+            double a[6][6];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            Bh[a] = -wt2 * (gkxh * M.tdx[a] + gkyh * M.tdy[a]);
-            Bb[a] = -wt2 * (gkxb * M.tdx[a] + gkyb * M.tdy[a]);
+            for (int t = 0; t < 6; ++t)
+#pragma unroll
+                for (int m = 0; m < 6; ++m) a[t][m] = 0.0;
+            if (act) {
+#pragma unroll 2
+                for (int j = L.g; j < nw; j += L.G) {
+                    const size_t q = (size_t)cc * nv + j * nu + c;
+                    const double d[6] = {gT0[q], gT1[q], gT2[q], gT3[q], gT4[q], gT5[q]};
+#pragma unroll
+                    for (int m = 0; m < 6; ++m) {
+                        const double l = X.row[j][m];
+#pragma unroll
+                        for (int t = 0; t < 6; ++t) a[t][m] += d[t] * l;
+                    }
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 6; ++t)
+#pragma unroll
+                for (int m = 0; m < 6; ++m) X.a[t][m][lane] = a[t][m];
+            const double u = tab[c], du = u - th.u, qx = th.pref * exp(-(du * du) * th.itw);
+#pragma unroll 1
+            for (int m = 0; m < 6; ++m) {
+                pn_reload();
+                const double vv = th.v + c_pn6[m] * width;
+                target_vjp(th, qv_of(th, s2_q_at(th, u, vv, qx), u, vv), M, u, vv, wt2, shb_add, X.a[0][m][lane],
+                           X.a[1][m][lane], X.a[2][m][lane], X.a[3][m][lane], X.a[4][m][lane], X.a[5][m][lane], acc);
+            }
         }
-        vhess(th, v, 0, Bh, hh);
-        vhess(th, v, 1, Bb, hb);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) acc[12 + a] += Ah * Dh[a] + Ab * Db[a] + hh[a] + hb[a];
+    } else {
+        for (int r = 0; r < nr; ++r) {
+            const WVel s = wvel(B, nv, r);
+            if (!s.ok) continue;
+            const size_t q = (size_t)cc * nv + s.k;
+            const double gmh = gT0[q], gmb = gT1[q], gkxh = gT2[q], gkxb = gT3[q], gkyh = gT4[q], gkyb = gT5[q];
+            const QV v = qv_at(th, s.u, s.v);
+            target_vjp(th, v, M, s.u, s.v, wt2, shb_add, gmh, gmb, gkxh, gkxb, gkyh, gkyb, acc);
+        }
     }
     warp_sum_all<16>(acc);
     // make_mke's directions: tdx = J^-1 accx(theta, ux, vy, lam, coeff) with accx the moments of the raw
     // Shakhov terms
-    double gax[4], gay[4], gJ[16];
-    solve_t4(jac, acc, gax);
-    solve_t4(jac, acc + 4, gay);
+    if (lane < 2) {
+        double b[4], x[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+        for (int a = 0; a < 4; ++a) b[a] = lane == 0 ? acc[a] : acc[4 + a];
+        solve_t4(jac, b, x);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) gJ[r * 4 + a] = -(gax[r] * M.tdx[a] + gay[r] * M.tdy[a]);
+        for (int a = 0; a < 4; ++a) N.b[lane][a] = x[a];
+    }
+    __syncwarp();
+    const double *gax = N.b[0], *gay = N.b[1], *gJ = N.gJ;
+    if (lane < 16) N.gJ[lane] = -(gax[lane >> 2] * M.tdx[lane & 3] + gay[lane >> 2] * M.tdy[lane & 3]);
+    __syncwarp();
     double g[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) g[m] = 0.0;   // coeff, lam, ux, vy, theta[4]
-    for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
-        if (!s.ok) continue;
-        const QV v = qv_at(th, s.u, s.v);
-        const double cx = s.u - M.ux, cy = s.v - M.vy, c2 = cx * cx + cy * cy;
-        const double shh = 2.0 * M.lam * c2 - 4.0, shb = shh + shb_add;
-        const double kxh = psi_h(s.w, s.u, s.v, gax), kxb = psi_b(s.w, gax), kyh = psi_h(s.w, s.u, s.v, gay),
-                     kyb = psi_b(s.w, gay);
-        const double xh = kxh * v.qh, xb = kxb * v.qb, yh = kyh * v.qh, yb = kyb * v.qb;
-        g[0] += cx * (xh * shh + xb * shb) + cy * (yh * shh + yb * shb);
-        g[1] += M.coeff * 2.0 * c2 * (cx * (xh + xb) + cy * (yh + yb));
-        g[2] += M.coeff * (xh * (-shh - 4.0 * M.lam * cx * cx) + xb * (-shb - 4.0 * M.lam * cx * cx) +
-                           (yh + yb) * (-4.0 * M.lam * cx * cy));
-        g[3] += M.coeff * (yh * (-shh - 4.0 * M.lam * cy * cy) + yb * (-shb - 4.0 * M.lam * cy * cy) +
-                           (xh + xb) * (-4.0 * M.lam * cx * cy));
-        const double Ah = M.coeff * shh * (cx * kxh + cy * kyh), Ab = M.coeff * shb * (cx * kxb + cy * kyb);
-        double Vh[4], Vb[4], hh[4], hb[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            Vh[a] = s.w * (gJ[a] + s.u * gJ[4 + a] + s.v * gJ[8 + a] + 0.5 * (s.u * s.u + s.v * s.v) * gJ[12 + a]);
-            Vb[a] = 0.5 * s.w * gJ[12 + a];
+    if constexpr (TENSOR) {   // both axes by nodes (degree 7)
+        const double width = sqrt(th.tw), iw = 1.0 / width;
+        double* wn = &X.row[0][0];
+        __syncwarp();
+        pn_weights<false>(B.tab, B.tab + 64, P.tnu, th.u, th.itw, iw, wn);
+        pn_weights<false>(B.tab + 128, B.tab + 192, P.tnv, th.v, th.itw, iw, wn + 8);
+#pragma unroll 1
+        for (int t = lane; t < 64; t += 32) {
+            pn_reload();
+            const double u = th.u + c_pn8[t & 7] * width, vv = th.v + c_pn8[t >> 3] * width;
+            mke_vjp(th, qv_of(th, s2_q_at(th, u, vv, th.pref), u, vv), M, wn[t & 7] * wn[8 + (t >> 3)], u, vv, shb_add, gax,
+                    gay, gJ, g);
         }
-        vhess(th, v, 0, Vh, hh);
-        vhess(th, v, 1, Vb, hb);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) g[4 + a] += Ah * v.qh * v.ld[a] + Ab * v.qb * v.ldb[a] + hh[a] + hb[a];
+    } else {
+        for (int r = 0; r < nr; ++r) {
+            const WVel s = wvel(B, nv, r);
+            if (!s.ok) continue;
+            const QV v = qv_at(th, s.u, s.v);
+            mke_vjp(th, v, M, s.w, s.u, s.v, shb_add, gax, gay, gJ, g);
+        }
     }
     warp_sum_all<8>(g);
     const double gprim[4] = {acc[10] + g[2], acc[11] + g[3], acc[9] + g[1], acc[8] + g[0]};   // ux, vy, lam, coeff
@@ -742,14 +931,126 @@ __global__ void __launch_bounds__(NT) k_adj_stream(LoParams P, LoBuffers B, S2Bu
 }
 
 // ---------------------------------------------------------------------------------------------
+// a face node's scalars
+struct AdjFaceNode {
+    S2Th th;
+    WMke M;
+    double tdl[4], tdr[4], tdt[4], tdm[4], mt[5], q0x, q0y, shb_add;
+};
+struct AdjFaceShared {   // a warp's: the node, the closure's Jacobian and its cotangent, five right-hand sides J^T x = b
+    AdjFaceNode n;
+    double jac[16], gJ[16], b[5][4];
+};
+// the node's flux transposed at one velocity (or polynomial node), but for the face values' terms: cotangents ah, ab of
+// its distributions; acc: [0..2] Mt, [5, 6] q0, [7..22] the directions, [23..26] coeff, lam, ux, vy, [27..30] theta
+__device__ __forceinline__ void face_flux_vjp(const AdjFaceNode& n, const QV& v, double u, double vv, double vn, double vt,
+                                              bool left, double ah, double ab, double acc[32]) {
+    double Dh[4], Db[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) { Dh[a] = v.qh * v.ld[a]; Db[a] = v.qb * v.ldb[a]; }
+    const double cx = u - n.M.ux, cy = vv - n.M.vy, c2 = cx * cx + cy * cy;
+    const double shh = 2.0 * n.M.lam * c2 - 4.0, shb = shh + n.shb_add;
+    double dx_h = 0.0, dx_b = 0.0, dy_h = 0.0, dy_b = 0.0, lr_h = 0.0, lr_b = 0.0, t_h = 0.0, t_b = 0.0, m_h = 0.0,
+           m_b = 0.0;
+    const double* tlr = left ? n.tdl : n.tdr;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        dx_h += Dh[a] * n.M.tdx[a]; dx_b += Db[a] * n.M.tdx[a];
+        dy_h += Dh[a] * n.M.tdy[a]; dy_b += Db[a] * n.M.tdy[a];
+        lr_h += Dh[a] * tlr[a]; lr_b += Db[a] * tlr[a];
+        t_h += Dh[a] * n.tdt[a]; t_b += Db[a] * n.tdt[a];
+        m_h += Dh[a] * n.tdm[a]; m_b += Db[a] * n.tdm[a];
+    }
+    const double kxh = n.M.coeff * cx * shh * v.qh - dx_h, kxb = n.M.coeff * cx * shb * v.qb - dx_b;
+    const double kyh = n.M.coeff * cy * shh * v.qh - dy_h, kyb = n.M.coeff * cy * shb * v.qb - dy_b;
+    const double s0h = v.qh + kxh * n.q0x + kyh * n.q0y, s0b = v.qb + kxb * n.q0x + kyb * n.q0y;
+    const double sh = vn * lr_h + vt * t_h, sb = vn * lr_b + vt * t_b;
+    acc[0] += ah * s0h + ab * s0b;
+    acc[1] += ah * sh + ab * sb;
+    acc[2] += ah * m_h + ab * m_b;
+    acc[5] += n.mt[0] * (ah * kxh + ab * kxb);
+    acc[6] += n.mt[0] * (ah * kyh + ab * kyb);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const double e = ah * Dh[a] + ab * Db[a];
+        acc[7 + a] += left ? vn * e : 0.0;
+        acc[11 + a] += left ? 0.0 : vn * e;
+        acc[15 + a] += vt * e;
+        acc[19 + a] += e;
+    }
+    const double qd = n.q0x * cx + n.q0y * cy, hq = ah * v.qh, bq = ab * v.qb;
+    acc[23] += n.mt[0] * qd * (hq * shh + bq * shb);
+    acc[24] += n.mt[0] * n.M.coeff * 2.0 * c2 * qd * (hq + bq);
+    acc[25] += n.mt[0] * n.M.coeff * (hq * (n.q0x * (-shh - 4.0 * n.M.lam * cx * cx) + n.q0y * (-4.0 * n.M.lam * cx * cy)) +
+                                 bq * (n.q0x * (-shb - 4.0 * n.M.lam * cx * cx) + n.q0y * (-4.0 * n.M.lam * cx * cy)));
+    acc[26] += n.mt[0] * n.M.coeff * (hq * (n.q0y * (-shh - 4.0 * n.M.lam * cy * cy) + n.q0x * (-4.0 * n.M.lam * cx * cy)) +
+                                 bq * (n.q0y * (-shb - 4.0 * n.M.lam * cy * cy) + n.q0x * (-4.0 * n.M.lam * cx * cy)));
+    const double ch = n.mt[0] * (1.0 + n.M.coeff * shh * qd), cb = n.mt[0] * (1.0 + n.M.coeff * shb * qd);
+    double V[4], hh[4], hb[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+        V[a] = -n.mt[0] * (n.M.tdx[a] * n.q0x + n.M.tdy[a] * n.q0y) + n.mt[1] * (vn * tlr[a] + vt * n.tdt[a]) + n.mt[2] * n.tdm[a];
+    vhess(n.th, v, 0, V, hh);
+    vhess(n.th, v, 1, V, hb);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) acc[27 + a] += ah * (ch * Dh[a] + hh[a]) + ab * (cb * Db[a] + hb[a]);
+}
+// the time direction's moments (of the flux directions) transposed at one velocity of weight w, cotangents gwt of the
+// moments; acc: [0..11] the slope directions, [12..15] theta
+__device__ __forceinline__ void face_time_vjp(const AdjFaceNode& n, const QV& v, double w, double u, double vv, double vn,
+                                              double vt, bool left, const double gwt[4], double acc[16]) {
+    const double* tlr = left ? n.tdl : n.tdr;
+    const double gfh = -psi_h(w, u, vv, gwt), gfb = -psi_b(w, gwt);
+    double U[4], hh[4], hb[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const double e = gfh * v.qh * v.ld[a] + gfb * v.qb * v.ldb[a];
+        acc[a] += left ? vn * e : 0.0;
+        acc[4 + a] += left ? 0.0 : vn * e;
+        acc[8 + a] += vt * e;
+        U[a] = vn * tlr[a] + vt * n.tdt[a];
+    }
+    vhess(n.th, v, 0, U, hh);
+    vhess(n.th, v, 1, U, hb);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) acc[12 + a] += gfh * hh[a] + gfb * hb[a];
+}
+// E(W0), the Maxwellian of q0's heat flux, transposed at one velocity of weight w (W0: density, velocity (eu, ev),
+// temperature temp = 1 / lamn; ex: its exponential): g[0..3] += W0's; returns E's values
+__device__ __forceinline__ void face_q0_vjp(const AdjFaceNode& n, int ck, double nrho, double eu, double ev, double lamn,
+                                            double temp, double ex, double w, double u, double vv, double gq0x, double gq0y,
+                                            double g[4], double& eah, double& eab) {
+    const double cx = u - n.M.ux, cy = vv - n.M.vy, c2 = cx * cx + cy * cy;
+    const double du = u - eu, dv = vv - ev, cn2 = du * du + dv * dv;
+    eah = nrho * lamn / kPi * ex;
+    eab = 0.5 * (double)ck * temp * eah;
+    const double geah = -0.5 * w * c2 * (cx * gq0x + cy * gq0y), geab = -0.5 * w * (cx * gq0x + cy * gq0y);
+    const double ge = geah + 0.5 * (double)ck * temp * geab;
+    g[0] += ge * eah / nrho;
+    g[1] += ge * eah * 2.0 * lamn * du;
+    g[2] += ge * eah * 2.0 * lamn * dv;
+    g[3] += ge * (-eah * lamn * (1.0 - lamn * cn2)) + geab * 0.5 * (double)ck * eah;
+}
+
+struct PnFace {   // a warp's row basis, its columns' nodes, node weights and the order of the rows
+    double row[64][6], a[4][12][32], wn[32];
+    unsigned char ord[64];
+};
+
+// ---------------------------------------------------------------------------------------------
 // ugks_node at one interior face Gauss node, transposed: flux (k_s2_face_flux) and node scalars
 // (k_s2_face_nodes) together, one warp per (face, node).  Cotangents in: the face fluxes' through
 // the stream rates of the two cells (grh, grb, gws), folded with the Gauss weight and face length.
 // Cotangents out: the face cache at the upwind side of every velocity (grec, written; the other side's
 // entry is set to zero), the macro slopes of the node (gmac) and mu_ref.
-// Three CTAs per SM (168 registers with spills instead of 254 without): measured 2.5 % faster over the
-// backward, the extra resident warps hiding the spills' latency.
-__global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
+// The node's scalars and its 4x4 systems are the warp's in shared memory: held by every lane they were 110 registers
+// and 2.6 KB of spills a thread at three CTAs an SM.  TENSOR: the sums by polynomial nodes.  At 8x64x32^2 (3048 nodes)
+// 408 us without, 257 with them, 169 with the scalars in shared memory and the columns' nodes stored before the long
+// expression runs, so that its 31 sums are not live beside the reads, 158 with the last pass's reads ahead of its
+// stores (ncu, cold).  What bounds it now is the latency of its reads at 12 warps an SM in 1.7 waves: 4 CTAs of two
+// warps, without the last change, took 197 us, 5 with it 161.
+template <bool TENSOR>
+__global__ void __launch_bounds__(TENSOR ? 64 : 128, TENSOR ? 6 : 3) k_adj_face_nodes(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
     const int nv = P.nvel, nx = P.nx, ny = P.ny, ck = P.ck, nr = (nv + 31) >> 5, lane = threadIdx.x & 31;
     const int nfx = nx * ny, nf = nfx + nx * (ny - 1);
     const int wid = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -761,21 +1062,26 @@ __global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers
     const double dt = B.dt[0];
     const double* sc = S.fscal + (size_t)wid * kS2FScal;
     if (sc[0] == 0.0) return;   // the forward node failed (its status is set)
-    double thv[4], tdl[4], tdr[4], tdt[4], tdm[4], mt[5], jac[16];
-    WMke M;
+    __shared__ AdjFaceShared Ns[TENSOR ? 2 : 4];
+    AdjFaceShared& N = Ns[threadIdx.x >> 5];
+    AdjFaceNode& n = N.n;
+    double* const jac = N.jac;
+    if (lane < 16) jac[lane] = sc[44 + lane];
+    if (lane == 0) {
+        double thv[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        thv[m] = sc[1 + m]; M.tdx[m] = sc[5 + m]; M.tdy[m] = sc[9 + m];
-        tdl[m] = sc[19 + m]; tdr[m] = sc[23 + m]; tdt[m] = sc[27 + m]; tdm[m] = sc[31 + m];
+        for (int m = 0; m < 4; ++m) {
+            thv[m] = sc[1 + m]; n.M.tdx[m] = sc[5 + m]; n.M.tdy[m] = sc[9 + m];
+            n.tdl[m] = sc[19 + m]; n.tdr[m] = sc[23 + m]; n.tdt[m] = sc[27 + m]; n.tdm[m] = sc[31 + m];
+        }
+        n.M.ux = sc[13]; n.M.vy = sc[14]; n.M.lam = sc[15]; n.M.coeff = sc[16];
+        n.q0x = sc[17]; n.q0y = sc[18];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) n.mt[m] = sc[35 + m];
+        n.th = s2_th(thv, ck);
+        n.shb_add = 2.0 / (double)ck;
     }
-    M.ux = sc[13]; M.vy = sc[14]; M.lam = sc[15]; M.coeff = sc[16];
-    const double q0x = sc[17], q0y = sc[18];
-#pragma unroll
-    for (int m = 0; m < 5; ++m) mt[m] = sc[35 + m];
-#pragma unroll
-    for (int m = 0; m < 16; ++m) jac[m] = sc[44 + m];
-    const S2Th th = s2_th(thv, ck);
-    const double shb_add = 2.0 / (double)ck;
+    __syncwarp();
     const double gw3[3] = {5.0 / 18.0, 4.0 / 9.0, 5.0 / 18.0};
     const double ia = 1.0 / P.area, fold = (axis == 0 ? P.dy : P.dx) * gw3[g] * ia;
     double gnw[4];   // cotangent of the node's macro flux
@@ -789,72 +1095,116 @@ __global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers
         ah = vn * Gh;
         ab = vn * Gb;
     };
+    __shared__ PnFace Xs[TENSOR ? 2 : 1];
+    PnFace& X = Xs[TENSOR ? threadIdx.x >> 5 : 0];
     // pass 1: the flux transposed -> Mt, q0, the directions, make_mke's scalars and theta
     double acc[32];
-#pragma unroll
-    for (int m = 0; m < 32; ++m) acc[m] = 0.0;
-    for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
-        if (!s.ok) continue;
-        const double vn = axis == 0 ? s.u : s.v, vt = axis == 0 ? s.v : s.u;
-        const bool left = vn >= 0.0;
-        const int cell = left ? cl : cr;
-        double ah, ab;
-        flux_cot(s, vn, ah, ab);
-        const QV v = qv_at(th, s.u, s.v);
-        double Dh[4], Db[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) { Dh[a] = v.qh * v.ld[a]; Db[a] = v.qb * v.ldb[a]; }
-        const double cx = s.u - M.ux, cy = s.v - M.vy, c2 = cx * cx + cy * cy;
-        const double shh = 2.0 * M.lam * c2 - 4.0, shb = shh + shb_add;
-        double dx_h = 0.0, dx_b = 0.0, dy_h = 0.0, dy_b = 0.0, lr_h = 0.0, lr_b = 0.0, t_h = 0.0, t_b = 0.0, m_h = 0.0,
-               m_b = 0.0;
-        const double* tlr = left ? tdl : tdr;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            dx_h += Dh[a] * M.tdx[a]; dx_b += Db[a] * M.tdx[a];
-            dy_h += Dh[a] * M.tdy[a]; dy_b += Db[a] * M.tdy[a];
-            lr_h += Dh[a] * tlr[a]; lr_b += Db[a] * tlr[a];
-            t_h += Dh[a] * tdt[a]; t_b += Db[a] * tdt[a];
-            m_h += Dh[a] * tdm[a]; m_b += Db[a] * tdm[a];
+    double W0[4] = {0.0, 0.0, 0.0, 0.0};   // moments of the upwind face values (not stored)
+    double hs[4] = {0.0, 0.0, 0.0, 0.0};   // and sums of theirs about make_mke's velocity: c^2 h + b, cx^2 h, cx cy h, cy^2 h
+    const double width = sqrt(n.th.tw), iw = 1.0 / width;
+    if constexpr (TENSOR) {   // polynomial nodes of each column, degree 5; one read of the cotangents and the face cache
+        const int nu = P.tnu, nw = P.tnv;
+        const double *tu = B.tab, *tv = B.tab + 128;
+        double e3 = 0.0, e4 = 0.0;
+        int n0 = 0;   // the rows in order, those a velocity leaves the left cell through first (y faces)
+        if (axis == 1) {
+            for (int c = 0; c < nw; c += 32) n0 += __popc(__ballot_sync(0xffffffffu, c + lane < nw && tv[c + lane] >= 0.0));
+            int pos = 0, neg = n0;
+            for (int c = 0; c < nw; c += 32) {
+                const bool in = c + lane < nw, up = in && tv[c + lane] >= 0.0;
+                const unsigned mu = __ballot_sync(0xffffffffu, up), mi = __ballot_sync(0xffffffffu, in && !up);
+                const unsigned below = (1u << lane) - 1u;
+                if (up) X.ord[pos + __popc(mu & below)] = c + lane;
+                else if (in) X.ord[neg + __popc(mi & below)] = c + lane;
+                pos += __popc(mu);
+                neg += __popc(mi);
+            }
+        } else {
+            for (int c = lane; c < nw; c += 32) X.ord[c] = c;
+            n0 = nw;
         }
-        const double kxh = M.coeff * cx * shh * v.qh - dx_h, kxb = M.coeff * cx * shb * v.qb - dx_b;
-        const double kyh = M.coeff * cy * shh * v.qh - dy_h, kyb = M.coeff * cy * shb * v.qb - dy_b;
-        const double s0h = v.qh + kxh * q0x + kyh * q0y, s0b = v.qb + kxb * q0x + kyb * q0y;
-        const double sh = vn * lr_h + vt * t_h, sb = vn * lr_b + vt * t_b;
-        const double f0h = rec_at(cell, 0, s.k), f0b = rec_at(cell, 1, s.k);
-        const double ph = rec_at(cell, 2, s.k), pb = rec_at(cell, 3, s.k);
-        acc[0] += ah * s0h + ab * s0b;
-        acc[1] += ah * sh + ab * sb;
-        acc[2] += ah * m_h + ab * m_b;
-        acc[3] += ah * f0h + ab * f0b;
-        acc[4] += -(ah * ph + ab * pb);
-        acc[5] += mt[0] * (ah * kxh + ab * kxb);
-        acc[6] += mt[0] * (ah * kyh + ab * kyb);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const double e = ah * Dh[a] + ab * Db[a];
-            acc[7 + a] += left ? vn * e : 0.0;
-            acc[11 + a] += left ? 0.0 : vn * e;
-            acc[15 + a] += vt * e;
-            acc[19 + a] += e;
+        __syncwarp();
+        for (int r = lane; r < nw; r += 32) {
+            const double d = tv[X.ord[r]] - n.th.v;
+            pn_basis<6>(d * iw, exp(-(d * d) * n.th.itw), X.row[r]);
         }
-        const double qd = q0x * cx + q0y * cy, hq = ah * v.qh, bq = ab * v.qb;
-        acc[23] += mt[0] * qd * (hq * shh + bq * shb);
-        acc[24] += mt[0] * M.coeff * 2.0 * c2 * qd * (hq + bq);
-        acc[25] += mt[0] * M.coeff * (hq * (q0x * (-shh - 4.0 * M.lam * cx * cx) + q0y * (-4.0 * M.lam * cx * cy)) +
-                                     bq * (q0x * (-shb - 4.0 * M.lam * cx * cx) + q0y * (-4.0 * M.lam * cx * cy)));
-        acc[26] += mt[0] * M.coeff * (hq * (q0y * (-shh - 4.0 * M.lam * cy * cy) + q0x * (-4.0 * M.lam * cx * cy)) +
-                                     bq * (q0y * (-shb - 4.0 * M.lam * cy * cy) + q0x * (-4.0 * M.lam * cx * cy)));
-        const double ch = mt[0] * (1.0 + M.coeff * shh * qd), cb = mt[0] * (1.0 + M.coeff * shb * qd);
-        double V[4], hh[4], hb[4];
+        __syncwarp();
+        const PnCols L(nu);
+        for (int c0 = 0; c0 < nu; c0 += 32) {
+            const bool act = L.act && c0 + L.c < nu;
+            const int c = min(c0 + L.c, nu - 1);
+            const double u = tu[c];
+            for (int half = 0; half <= axis; ++half) {
+                const int r1 = act ? (half ? nw : n0) : 0;
+                const bool left = axis == 0 ? u >= 0.0 : half == 0;
+                const int cell = left ? cl : cr;
+                double a[12];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-            V[a] = -mt[0] * (M.tdx[a] * q0x + M.tdy[a] * q0y) + mt[1] * (vn * tlr[a] + vt * tdt[a]) + mt[2] * tdm[a];
-        vhess(th, v, 0, V, hh);
-        vhess(th, v, 1, V, hb);
+                for (int m = 0; m < 12; ++m) a[m] = 0.0;
+#pragma unroll 2
+                for (int r = (half ? n0 : 0) + L.g; r < r1; r += L.G) {
+                    WVel s;
+                    s.k = X.ord[r] * nu + c;
+                    s.u = u;
+                    s.v = tv[X.ord[r]];
+                    s.w = __ldg(B.w + s.k);
+                    const double vn = axis == 0 ? s.u : s.v;
+                    double ah, ab;
+                    flux_cot(s, vn, ah, ab);
+                    const double f0h = rec_at(cell, 0, s.k), f0b = rec_at(cell, 1, s.k);
+                    const double ph = rec_at(cell, 2, s.k), pb = rec_at(cell, 3, s.k);
+                    e3 += ah * f0h + ab * f0b;
+                    e4 += -(ah * ph + ab * pb);
+                    moment_add(s.w, s.u, s.v, f0h, f0b, W0);
+                    const double cx = s.u - n.M.ux, cy = s.v - n.M.vy, wh = s.w * f0h;
+                    hs[0] += (cx * cx + cy * cy) * wh + s.w * f0b;
+                    hs[1] += cx * cx * wh;
+                    hs[2] += cx * cy * wh;
+                    hs[3] += cy * cy * wh;
 #pragma unroll
-        for (int a = 0; a < 4; ++a) acc[27 + a] += ah * (ch * Dh[a] + hh[a]) + ab * (cb * Db[a] + hb[a]);
+                    for (int m = 0; m < 6; ++m) {
+                        const double l = X.row[r][m];
+                        a[m] += ah * l;
+                        a[6 + m] += ab * l;
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < 12; ++m) X.a[c0 / 16 + half][m][lane] = a[m];
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < 32; ++m) acc[m] = 0.0;
+        acc[3] = e3;
+        acc[4] = e4;
+        for (int c0 = 0; c0 < nu; c0 += 32) {
+            const double u = tu[min(c0 + L.c, nu - 1)], du = u - n.th.u, qx = n.th.pref * exp(-(du * du) * n.th.itw);
+#pragma unroll 1
+            for (int t = 0; t < 6 * (axis + 1); ++t) {
+                pn_reload();
+                const int half = t >= 6, m = t - 6 * half;
+                const double v = n.th.v + c_pn6[m] * width;
+                face_flux_vjp(n, qv_of(n.th, s2_q_at(n.th, u, v, qx), u, v), u, v, axis == 0 ? u : v, axis == 0 ? v : u,
+                              axis == 0 ? u >= 0.0 : half == 0, X.a[c0 / 16 + half][m][lane], X.a[c0 / 16 + half][6 + m][lane],
+                              acc);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < 32; ++m) acc[m] = 0.0;
+        for (int r = 0; r < nr; ++r) {
+            const WVel s = wvel(B, nv, r);
+            if (!s.ok) continue;
+            const double vn = axis == 0 ? s.u : s.v, vt = axis == 0 ? s.v : s.u;
+            const bool left = vn >= 0.0;
+            const int cell = left ? cl : cr;
+            double ah, ab;
+            flux_cot(s, vn, ah, ab);
+            const double f0h = rec_at(cell, 0, s.k), f0b = rec_at(cell, 1, s.k);
+            const double ph = rec_at(cell, 2, s.k), pb = rec_at(cell, 3, s.k);
+            acc[3] += ah * f0h + ab * f0b;
+            acc[4] += -(ah * ph + ab * pb);
+            face_flux_vjp(n, qv_at(n.th, s.u, s.v), s.u, s.v, vn, vt, left, ah, ab, acc);
+        }
     }
     warp_sum_all<31>(acc);
     double gmt[5], gtdl[4], gtdr[4], gtdt[4], gtdm[4], gtdx[4], gtdy[4];
@@ -863,47 +1213,43 @@ __global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers
     const double gq0x = acc[5], gq0y = acc[6];
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        gtdl[a] = mt[1] * acc[7 + a];
-        gtdr[a] = mt[1] * acc[11 + a];
-        gtdt[a] = mt[1] * acc[15 + a];
-        gtdm[a] = mt[2] * acc[19 + a];
-        gtdx[a] = -mt[0] * q0x * acc[19 + a];
-        gtdy[a] = -mt[0] * q0y * acc[19 + a];
+        gtdl[a] = n.mt[1] * acc[7 + a];
+        gtdr[a] = n.mt[1] * acc[11 + a];
+        gtdt[a] = n.mt[1] * acc[15 + a];
+        gtdm[a] = n.mt[2] * acc[19 + a];
+        gtdx[a] = -n.mt[0] * n.q0x * acc[19 + a];
+        gtdy[a] = -n.mt[0] * n.q0y * acc[19 + a];
     }
     double gcoeff = acc[23], glam = acc[24], gux = acc[25], gvy = acc[26], gth[4];
 #pragma unroll
     for (int a = 0; a < 4; ++a) gth[a] = acc[27 + a];
     // the time direction: tdm = J^-1 wt, wt = -moments of the flux directions
-    double gwt[4], gJ[16];
+    double gwt[4];
     solve_t4(jac, gtdm, gwt);
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int a = 0; a < 4; ++a) gJ[r * 4 + a] = -gwt[r] * tdm[a];
     double acc3[16];
 #pragma unroll
     for (int m = 0; m < 16; ++m) acc3[m] = 0.0;
-    for (int r = 0; r < nr; ++r) {   // pass 3: wt transposed -> the slope directions and theta
-        const WVel s = wvel(B, nv, r);
-        if (!s.ok) continue;
-        const double vn = axis == 0 ? s.u : s.v, vt = axis == 0 ? s.v : s.u;
-        const bool left = vn >= 0.0;
-        const double* tlr = left ? tdl : tdr;
-        const QV v = qv_at(th, s.u, s.v);
-        const double gfh = -psi_h(s.w, s.u, s.v, gwt), gfb = -psi_b(s.w, gwt);
-        double U[4], hh[4], hb[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const double e = gfh * v.qh * v.ld[a] + gfb * v.qb * v.ldb[a];
-            acc3[a] += left ? vn * e : 0.0;
-            acc3[4 + a] += left ? 0.0 : vn * e;
-            acc3[8 + a] += vt * e;
-            U[a] = vn * tlr[a] + vt * tdt[a];
+    if constexpr (TENSOR) {   // both axes by nodes, degree 7; wn: normal axis left, right, tangential axis
+        const int an = axis == 0 ? 0 : 128, at = 128 - an;
+        const double mn = axis == 0 ? n.th.u : n.th.v, mt_ = axis == 0 ? n.th.v : n.th.u;
+        pn_weights<true>(B.tab + an, B.tab + an + 64, axis == 0 ? P.tnu : P.tnv, mn, n.th.itw, iw, X.wn);
+        pn_weights<false>(B.tab + at, B.tab + at + 64, axis == 0 ? P.tnv : P.tnu, mt_, n.th.itw, iw, X.wn + 16);
+#pragma unroll 1
+        for (int t = lane; t < 128; t += 32) {
+            pn_reload();
+            const double vn = mn + c_pn8[t & 7] * width, vt = mt_ + c_pn8[(t >> 3) & 7] * width;
+            const double u = axis == 0 ? vn : vt, v = axis == 0 ? vt : vn;
+            face_time_vjp(n, qv_of(n.th, s2_q_at(n.th, u, v, n.th.pref), u, v),
+                          X.wn[(t >> 6) * 8 + (t & 7)] * X.wn[16 + ((t >> 3) & 7)], u, v, vn, vt, t < 64, gwt, acc3);
         }
-        vhess(th, v, 0, U, hh);
-        vhess(th, v, 1, U, hb);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) acc3[12 + a] += gfh * hh[a] + gfb * hb[a];
+    } else {
+        for (int r = 0; r < nr; ++r) {   // pass 3: wt transposed -> the slope directions and theta
+            const WVel s = wvel(B, nv, r);
+            if (!s.ok) continue;
+            const double vn = axis == 0 ? s.u : s.v, vt = axis == 0 ? s.v : s.u;
+            const bool left = vn >= 0.0;
+            face_time_vjp(n, qv_at(n.th, s.u, s.v), s.w, s.u, s.v, vn, vt, left, gwt, acc3);
+        }
     }
     warp_sum_all<16>(acc3);
 #pragma unroll
@@ -914,29 +1260,38 @@ __global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers
         gth[a] += acc3[12 + a];
     }
     // the macro slopes: tdl = J^-1 mac_l (and r, t); make_mke's directions tdx = J^-1 accx
-    double gml[4], gmr[4], gmtg[4], gax[4], gay[4];
-    solve_t4(jac, gtdl, gml);
-    solve_t4(jac, gtdr, gmr);
-    solve_t4(jac, gtdt, gmtg);
-    solve_t4(jac, gtdx, gax);
-    solve_t4(jac, gtdy, gay);
-    if (lane == 0) {
-        double* o = A.gmac + (size_t)wid * 12;
+    // (one lane each)
+    if (lane == 0)
 #pragma unroll
-        for (int m = 0; m < 4; ++m) { o[m] = gml[m]; o[4 + m] = gmr[m]; o[8 + m] = gmtg[m]; }
+        for (int a = 0; a < 4; ++a) {
+            N.b[0][a] = gtdl[a]; N.b[1][a] = gtdr[a]; N.b[2][a] = gtdt[a]; N.b[3][a] = gtdx[a]; N.b[4][a] = gtdy[a];
+        }
+    __syncwarp();
+    if (lane < 5) {
+        double x[4];
+        solve_t4(jac, N.b[lane], x);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) N.b[lane][a] = x[a];
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-            gJ[r * 4 + a] += -(gml[r] * tdl[a] + gmr[r] * tdr[a] + gmtg[r] * tdt[a] + gax[r] * M.tdx[a] + gay[r] * M.tdy[a]);
+    __syncwarp();
+    const double *gml = N.b[0], *gmr = N.b[1], *gmtg = N.b[2], *gax = N.b[3], *gay = N.b[4], *gJ = N.gJ;
+    if (lane < 12) A.gmac[(size_t)wid * 12 + lane] = N.b[lane >> 2][lane & 3];
+    if (lane < 16) {
+        const int r = lane >> 2, a = lane & 3;
+        double wr = gwt[0];
+        if (r == 1) wr = gwt[1]; else if (r == 2) wr = gwt[2]; else if (r == 3) wr = gwt[3];
+        N.gJ[lane] = -(wr * n.tdm[a] + gml[r] * n.tdl[a] + gmr[r] * n.tdr[a] + gmtg[r] * n.tdt[a] + gax[r] * n.M.tdx[a] +
+                       gay[r] * n.M.tdy[a]);
+    }
+    __syncwarp();
     // pass 4: accx / accy, the Jacobian and q0's analytic Maxwellian transposed
-    double W0[4] = {0.0, 0.0, 0.0, 0.0};   // W0, the moments of the upwind face values (not stored)
-    for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
-        const double vn = axis == 0 ? s.u : s.v;
-        const bool left = vn >= 0.0;
-        moment_add(s.w, s.u, s.v, rec_at(left ? cl : cr, 0, s.k), rec_at(left ? cl : cr, 1, s.k), W0);
+    if constexpr (!TENSOR) {
+        for (int r = 0; r < nr; ++r) {
+            const WVel s = wvel(B, nv, r);
+            const double vn = axis == 0 ? s.u : s.v;
+            const bool left = vn >= 0.0;
+            moment_add(s.w, s.u, s.v, rec_at(left ? cl : cr, 0, s.k), rec_at(left ? cl : cr, 1, s.k), W0);
+        }
     }
     warp_sum_all<4>(W0);
     const double nrho = W0[0], nu = W0[1] / W0[0], nvv = W0[2] / W0[0];
@@ -945,46 +1300,48 @@ __global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers
     double acc4[12];
 #pragma unroll
     for (int m = 0; m < 12; ++m) acc4[m] = 0.0;
-    for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
-        if (!s.ok) continue;
-        const double vn = axis == 0 ? s.u : s.v;
-        const bool left = vn >= 0.0;
-        const int cell = left ? cl : cr;
-        const QV v = qv_at(th, s.u, s.v);
-        const double cx = s.u - M.ux, cy = s.v - M.vy, c2 = cx * cx + cy * cy;
-        const double shh = 2.0 * M.lam * c2 - 4.0, shb = shh + shb_add;
-        const double kxh = psi_h(s.w, s.u, s.v, gax), kxb = psi_b(s.w, gax), kyh = psi_h(s.w, s.u, s.v, gay),
-                     kyb = psi_b(s.w, gay);
-        const double xh = kxh * v.qh, xb = kxb * v.qb, yh = kyh * v.qh, yb = kyb * v.qb;
-        acc4[0] += cx * (xh * shh + xb * shb) + cy * (yh * shh + yb * shb);
-        acc4[1] += M.coeff * 2.0 * c2 * (cx * (xh + xb) + cy * (yh + yb));
-        acc4[2] += M.coeff * (xh * (-shh - 4.0 * M.lam * cx * cx) + xb * (-shb - 4.0 * M.lam * cx * cx) +
-                              (yh + yb) * (-4.0 * M.lam * cx * cy));
-        acc4[3] += M.coeff * (yh * (-shh - 4.0 * M.lam * cy * cy) + yb * (-shb - 4.0 * M.lam * cy * cy) +
-                              (xh + xb) * (-4.0 * M.lam * cx * cy));
-        const double Ah = M.coeff * shh * (cx * kxh + cy * kyh), Ab = M.coeff * shb * (cx * kxb + cy * kyb);
-        double Vh[4], Vb[4], hh[4], hb[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            Vh[a] = s.w * (gJ[a] + s.u * gJ[4 + a] + s.v * gJ[8 + a] + 0.5 * (s.u * s.u + s.v * s.v) * gJ[12 + a]);
-            Vb[a] = 0.5 * s.w * gJ[12 + a];
+    if constexpr (TENSOR) {
+        __syncwarp();
+        if (lane < 8) X.wn[24 + lane] = X.wn[lane] + X.wn[8 + lane];
+        __syncwarp();
+        const double *wx = axis == 0 ? X.wn + 24 : X.wn + 16, *wy = axis == 0 ? X.wn + 16 : X.wn + 24;
+#pragma unroll 1
+        for (int t = lane; t < 64; t += 32) {
+            pn_reload();
+            const double u = n.th.u + c_pn8[t & 7] * width, v = n.th.v + c_pn8[t >> 3] * width;
+            mke_vjp(n.th, qv_of(n.th, s2_q_at(n.th, u, v, n.th.pref), u, v), n.M, wx[t & 7] * wy[t >> 3], u, v, n.shb_add, gax,
+                    gay, gJ, acc4);
         }
-        vhess(th, v, 0, Vh, hh);
-        vhess(th, v, 1, Vb, hb);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) acc4[4 + a] += Ah * v.qh * v.ld[a] + Ab * v.qb * v.ldb[a] + hh[a] + hb[a];
-        // q0 = heat(w0, f0 - E(W0)) with (cx, cy) about make_mke's (ux, vy)
-        const double du = s.u - nu, dv = s.v - nvv, cn2 = du * du + dv * dv;
-        const double eah = nrho * lamn / kPi * exp(-lamn * cn2), eab = 0.5 * (double)ck * temp * eah;
-        const double dh = rec_at(cell, 0, s.k) - eah, db = rec_at(cell, 1, s.k) - eab;
-        heat_shift_adj(s.w, cx, cy, dh, db, gq0x, gq0y, acc4[2], acc4[3]);
-        const double geah = -0.5 * s.w * c2 * (cx * gq0x + cy * gq0y), geab = -0.5 * s.w * (cx * gq0x + cy * gq0y);
-        const double ge = geah + 0.5 * (double)ck * temp * geab;
-        acc4[8] += ge * eah / nrho;
-        acc4[9] += ge * eah * 2.0 * lamn * du;
-        acc4[10] += ge * eah * 2.0 * lamn * dv;
-        acc4[11] += ge * (-eah * lamn * (1.0 - lamn * cn2)) + geab * 0.5 * (double)ck * eah;
+        // q0 = heat(w0, f0 - E(W0)) with (cx, cy) about make_mke's (ux, vy): E(W0) by its own nodes, f0 by its sums
+        const double we = sqrt(temp), iwe = 1.0 / we;
+        pn_weights<false>(B.tab, B.tab + 64, P.tnu, nu, lamn, iwe, X.wn);
+        pn_weights<false>(B.tab + 128, B.tab + 192, P.tnv, nvv, lamn, iwe, X.wn + 8);
+#pragma unroll 1
+        for (int t = lane; t < 64; t += 32) {
+            pn_reload();
+            const double u = nu + c_pn8[t & 7] * we, v = nvv + c_pn8[t >> 3] * we, w = X.wn[t & 7] * X.wn[8 + (t >> 3)];
+            double eah, eab;
+            face_q0_vjp(n, ck, nrho, nu, nvv, lamn, temp, 1.0, w, u, v, gq0x, gq0y, acc4 + 8, eah, eab);
+            heat_shift_adj(w, u - n.M.ux, v - n.M.vy, -eah, -eab, gq0x, gq0y, acc4[2], acc4[3]);
+        }
+        acc4[2] += gq0x * (-0.5 * hs[0] - hs[1]) - gq0y * hs[2];
+        acc4[3] += gq0y * (-0.5 * hs[0] - hs[3]) - gq0x * hs[2];
+    } else {
+        for (int r = 0; r < nr; ++r) {
+            const WVel s = wvel(B, nv, r);
+            if (!s.ok) continue;
+            const double vn = axis == 0 ? s.u : s.v;
+            const bool left = vn >= 0.0;
+            const int cell = left ? cl : cr;
+            mke_vjp(n.th, qv_at(n.th, s.u, s.v), n.M, s.w, s.u, s.v, n.shb_add, gax, gay, gJ, acc4);
+            // q0 = heat(w0, f0 - E(W0)) with (cx, cy) about make_mke's (ux, vy)
+            const double du = s.u - nu, dv = s.v - nvv;
+            double eah, eab;
+            face_q0_vjp(n, ck, nrho, nu, nvv, lamn, temp, exp(-lamn * (du * du + dv * dv)), s.w, s.u, s.v, gq0x, gq0y, acc4 + 8,
+                        eah, eab);
+            heat_shift_adj(s.w, s.u - n.M.ux, s.v - n.M.vy, rec_at(cell, 0, s.k) - eah, rec_at(cell, 1, s.k) - eab, gq0x, gq0y,
+                           acc4[2], acc4[3]);
+        }
     }
     warp_sum_all<12>(acc4);
     gcoeff += acc4[0];
@@ -1007,21 +1364,28 @@ __global__ void __launch_bounds__(128, 3) k_adj_face_nodes(LoParams P, LoBuffers
 #pragma unroll
     for (int m = 0; m < 4; ++m) gW0[m] = gin[m] + gwc[m];
     if (lane == 0) atomic_add(A.gpar + GP_MU, gin[4]);
-    // pass 2: the face cache at the upwind side (the other side's entry of this node is zero)
-    for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
-        if (!s.ok) continue;
-        const double vn = axis == 0 ? s.u : s.v;
-        const bool left = vn >= 0.0;
-        double ah, ab;
-        flux_cot(s, vn, ah, ab);
-        const double cx = s.u - M.ux, cy = s.v - M.vy, c2 = cx * cx + cy * cy;
-        const double gh0 = ah * mt[3] + psi_h(s.w, s.u, s.v, gW0) + 0.5 * s.w * c2 * (cx * gq0x + cy * gq0y);
-        const double gb0 = ab * mt[3] + psi_b(s.w, gW0) + 0.5 * s.w * (cx * gq0x + cy * gq0y);
-        const double gv[kRecFields] = {gh0, gb0, -ah * mt[4], -ab * mt[4]};
-        double* up = A.grec + rec_cell(left ? cl : cr, axis, 0, g, nv) + s.k;
+    // pass 2: the face cache at the upwind side (the other side's entry of this node is zero); the reads of RB rounds
+    // ahead of their stores
+    constexpr int RB = 4;
+    for (int r0 = 0; r0 < nr; r0 += RB) {
+        WVel s[RB];
+        double ah[RB], ab[RB];
 #pragma unroll
-        for (int fld = 0; fld < kRecFields; ++fld) up[(size_t)fld * 3 * nv] = gv[fld];
+        for (int q = 0; q < RB; ++q) {
+            s[q] = wvel(B, nv, r0 + q);
+            flux_cot(s[q], axis == 0 ? s[q].u : s[q].v, ah[q], ab[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < RB; ++q) {
+            if (!s[q].ok) continue;
+            const double u = s[q].u, v = s[q].v, w = s[q].w, cx = u - n.M.ux, cy = v - n.M.vy, c2 = cx * cx + cy * cy;
+            const double gh0 = ah[q] * n.mt[3] + psi_h(w, u, v, gW0) + 0.5 * w * c2 * (cx * gq0x + cy * gq0y);
+            const double gb0 = ab[q] * n.mt[3] + psi_b(w, gW0) + 0.5 * w * (cx * gq0x + cy * gq0y);
+            const double gv[kRecFields] = {gh0, gb0, -ah[q] * n.mt[4], -ab[q] * n.mt[4]};
+            double* up = A.grec + rec_cell((axis == 0 ? u : v) >= 0.0 ? cl : cr, axis, 0, g, nv) + s[q].k;
+#pragma unroll
+            for (int fld = 0; fld < kRecFields; ++fld) up[(size_t)fld * 3 * nv] = gv[fld];
+        }
     }
 }
 
@@ -1881,6 +2245,16 @@ void adj_bind_work(AdjBuffers& A, double* base, int nx, int ny, int nv) {
 
 cudaError_t prepare_s2_adjoint() { return s2_upload_tables(); }
 
+// the node kernels' warps: the polynomial-node forms on tensor-product tables (they need the table's structure)
+static void launch_targets(const LoParams& P, const LoBuffers& B, const S2Buffers& S, const AdjBuffers& A, double* const* gT,
+                           cudaStream_t s) {
+    const unsigned n = (unsigned)(P.nx * P.ny * 9);
+    if (P.tnu > 0)
+        k_adj_targets<true><<<n / 3, 96, 0, s>>>(P, B, S, A, gT[0], gT[1], gT[2], gT[3], gT[4], gT[5]);
+    else
+        k_adj_targets<false><<<(n + 7) / 8, 256, 0, s>>>(P, B, S, A, gT[0], gT[1], gT[2], gT[3], gT[4], gT[5]);
+}
+
 template <int VPT>
 static cudaError_t adj_launch(const LoParams& P, const LoBuffers& B, const S2Buffers& S, const S2Buffers& T,
                               const S2Buffers& To, const CnBuffers& C, const AdjBuffers& A, cudaStream_t s,
@@ -1891,8 +2265,7 @@ static cudaError_t adj_launch(const LoParams& P, const LoBuffers& B, const S2Buf
     const cudaStream_t sw = side ? s2 : s;
     cudaError_t e = cudaSuccess;
     k_adj_collide<VPT, 256><<<nc, 256, 0, s>>>(P, B, To, C, A);
-    k_adj_targets<<<warps((long long)nc * 9, 256), 256, 0, s>>>(P, B, S, A, A.gTo[0], A.gTo[1], A.gTo[2], A.gTo[3],
-                                                                A.gTo[4], A.gTo[5]);
+    launch_targets(P, B, S, A, A.gTo, s);
     k_adj_macro_cells<<<(unsigned)((nc * 4 + 255) / 256), 256, 0, s>>>(P, C.ws, A.gwq, A.gws);
     k_adj_stream<VPT, 256><<<nc, 256, 0, s>>>(P, B, T, A);
     // the wall nodes (2 nx x 3 warps) beside the interior face nodes: they write disjoint sides of the face
@@ -1905,7 +2278,8 @@ static cudaError_t adj_launch(const LoParams& P, const LoBuffers& B, const S2Buf
         k_adj_wall_nodes<<<warps(2LL * nx * 3, 256), 256, 0, sw>>>(P, B, S, A);
     }
     if (e == cudaSuccess) {
-        k_adj_face_nodes<<<warps((long long)nf * 3, 128), 128, 0, s>>>(P, B, S, A);
+        if (P.tnu > 0) k_adj_face_nodes<true><<<warps((long long)nf * 3, 64), 64, 0, s>>>(P, B, S, A);
+        else k_adj_face_nodes<false><<<warps((long long)nf * 3, 128), 128, 0, s>>>(P, B, S, A);
         if (side) e = cudaEventRecord(ev[2], s);
     }
     if (e == cudaSuccess && side) e = cudaStreamWaitEvent(s2, ev[2], 0);
@@ -1947,8 +2321,7 @@ cudaError_t enqueue_s2cn2_adjoint(const LoParams& P, const LoBuffers& B, const S
 cudaError_t enqueue_targets_adjoint(const LoParams& P, const LoBuffers& B, const S2Buffers& S, double* const gT[6],
                                     double* gW, const AdjBuffers& A, cudaStream_t s) {
     const int nc = P.nx * P.ny;
-    k_adj_targets<<<(unsigned)(((long long)nc * 9 * 32 + 255) / 256), 256, 0, s>>>(P, B, S, A, gT[0], gT[1], gT[2],
-                                                                                 gT[3], gT[4], gT[5]);
+    launch_targets(P, B, S, A, gT, s);
     k_adj_macro_cells<<<(unsigned)((nc * 4 + 255) / 256), 256, 0, s>>>(P, B.W, A.gwq, gW);
     return cudaGetLastError();
 }
