@@ -26,7 +26,7 @@
 // and transposed; every per-velocity expression is transposed by hand.  Scatter-adjoints into the
 // state, the first layer and W accumulate with atomicAdd (one ulp of ordering noise run to run).
 #include "ugks_s2_adjoint.cuh"
-#include "ugks_s2_math.cuh"
+#include "ugks_s2_tensor.cuh"
 
 #include <utility>
 
@@ -1389,6 +1389,29 @@ __global__ void __launch_bounds__(TENSOR ? 64 : 128, TENSOR ? 6 : 3) k_adj_face_
     }
 }
 
+
+// sums over a wall node's CTA: every thread returns the same totals (two barriers; s of N values a warp and N)
+constexpr int kAdjWall = 128;
+template <int N>
+__device__ __forceinline__ void cta_sum_all(double* v, double* s) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    warp_sum_all<N>(v);
+    if (lane == 0)
+#pragma unroll
+        for (int m = 0; m < N; ++m) s[warp * N + m] = v[m];
+    __syncthreads();
+    if ((int)threadIdx.x < N) {
+        double t = s[threadIdx.x];
+#pragma unroll
+        for (int w = 1; w < kAdjWall / 32; ++w) t += s[w * N + threadIdx.x];
+        s[kAdjWall / 32 * N + threadIdx.x] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < N; ++m) v[m] = s[kAdjWall / 32 * N + m];
+    __syncthreads();
+}
+
 // ---------------------------------------------------------------------------------------------
 // the multiscale wall's scalar chain (s2w2_wall_node, mod_S2MultiscaleWall.f90:45-184), generic over
 // double / Dl: inputs the wall cell's W, the wall speed and temperature, mu_ref and the tangential
@@ -1493,17 +1516,19 @@ __device__ void wall_chain(const LoParams& P, double dt, double side, const T in
     out[24] = Mxi[2];
 }
 
-// the wall node transposed: one warp per (wall face, Gauss node).  The node's forward quantities are
+// the wall node transposed: one CTA per (wall face, Gauss node).  The node's forward quantities are
 // recomputed here (closure of the wall state, the tangential and incident moments, the wall density);
 // cotangents in: the wall face flux's (from the wall cell's stream rates) and the wall outputs' seed.
 // Out: the wall cell's face cache at its wall side (written), its W, the wall speed and temperature and
-// mu_ref (added).
-__global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
-    const int nv = P.nvel, nx = P.nx, ny = P.ny, ck = P.ck, lane = threadIdx.x & 31, nr = (nv + 31) >> 5;
+// mu_ref (added).  R > 0: the closure by 1-D sums (tensor-product tables of up to 8 R abscissae an axis).
+// It runs beside the interior nodes, and a domain has few wall nodes, so the chain of one node's passes is what it costs:
+// at 8x64x32^2 (48 nodes) 256 us by a warp a node, 75 by 4 warps, 68 by 8 and 79 by 16; beside the interior nodes the 4
+// leave them the most room (backward and forward 1174 us a step, 1182 with 8, 1187 with 16, 1239 by a warp a node).
+template <int R>
+__global__ void __launch_bounds__(kAdjWall, 1) k_adj_wall_nodes(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
+    const int nv = P.nvel, nx = P.nx, ny = P.ny, ck = P.ck, lane = threadIdx.x & 31, nr = (nv + kAdjWall - 1) / kAdjWall;
     const int nf = nx * ny + nx * (ny - 1);
-    const int wid = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (wid >= 2 * nx * 3) return;
-    const int wf = wid / 3, g = wid % 3;
+    const int wf = blockIdx.x / 3, g = blockIdx.x % 3;
     const int top = wf >= nx ? 1 : 0, i = wf - top * nx;
     const int cc = top ? (ny - 1) * nx + i : i;
     const size_t node = (size_t)(nf + wf) * 3 + g;
@@ -1515,16 +1540,38 @@ __global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers
     const double lambda = 0.5 / theta;
     const double prim_g[4] = {pp / theta, 0.0, -ux, lambda};
     const double wwall[4] = {prim_g[0], prim_g[0] * ux, 0.0, prim_g[0] * ((double)(ck + 2) * theta / 2.0 + ux * ux / 2.0)};
-    __shared__ double s_jac[8][16];
-    WClosure C;
-    C.jac = s_jac[threadIdx.x >> 5];
-    if (!(pp > 0.0 && w_closure(P, B, wwall, C))) return;   // the forward node failed (its status is set)
+    __shared__ double s_th[4], s_jac[R > 0 ? 4 : 1][16], s_red[(kAdjWall / 32 + 1) * 28];
+    __shared__ int s_ok;
+    if (threadIdx.x < 32) {   // the wall closure by one warp (on a tensor-product table its four node groups work alike)
+        bool ok = pp > 0.0;
+        double th[4] = {1.0, 0.0, 0.0, 1.0};
+        if constexpr (R > 0) {
+            TClosure C;
+            C.jac = s_jac[lane / kTG];
+            ok = t_closure<R>(P, B, wwall, ok, C) && ok;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) th[m] = C.th[m];
+        } else if (ok) {
+            WClosure C;
+            C.jac = s_jac[0];
+            ok = w_closure(P, B, wwall, C);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) th[m] = C.th[m];
+        }
+        if (lane == 0) {
+            s_ok = ok;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) s_th[m] = th[m];
+        }
+    }
+    __syncthreads();
+    if (!s_ok) return;   // the forward node failed (its status is set)
     auto rec = [&](int k, int field) { return S.rec[rec_wall(nx, ny, top, i, field, g, nv) + k]; };
     double acc[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) acc[m] = 0.0;
     for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
+        const WVel s = wvel<kAdjWall>(B, nv, r);
         const double hin = rec(s.k, 0), bin = rec(s.k, 1), ht = rec(s.k, 3), bt = rec(s.k, 5);
         const double vn = s.v, vt = -s.u, v2 = vn * vn + vt * vt;
         acc[0] += s.w * (-ht);
@@ -1538,7 +1585,7 @@ __global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers
         acc[6] += s.w * vn * vt2 * hin;
         acc[7] += 0.5 * s.w * (w2 * hin + bin) + s.w * vt2 * vt2 * hin;
     }
-    warp_sum_all<8>(acc);
+    cta_sum_all<8>(acc, s_red);
     const double hlx = acc[4], hly = acc[5], dhlx_dux = acc[6], dhly_dux = acc[7];
     // the scalar chain's values and, one input per lane, its Jacobian
     const double win[kWallIn] = {wcell[0], wcell[1], wcell[2], wcell[3], ux, 1.0 / P.wall_lam[top], P.mu_ref,
@@ -1553,7 +1600,7 @@ __global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers
 #pragma unroll
     for (int m = 0; m < 5; ++m) mt[m] = xo[18 + m].v;
     const double rhog = xo[0].v, lam = xo[1].v, coeff = xo[23].v, mxi2 = xo[24].v;
-    const S2Th tt = s2_th(C.th, ck);
+    const S2Th tt = s2_th(s_th, ck);
     const bool shak = P.pr != 1.0;
     const double shb_add = 2.0 / (double)ck;
     // the incident micro flux of one velocity, as the forward kernel
@@ -1580,14 +1627,14 @@ __global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers
     };
     acc[0] = acc[1] = 0.0;
     for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
+        const WVel s = wvel<kAdjWall>(B, nv, r);
         const QV q = qv_at(tt, s.u, s.v);
         double gh, gb;
         gin(s, q, gh, gb);
         if (side * s.v > 0.0) acc[0] += s.w * s.v * gh;
         else acc[1] += dt * s.w * s.v * (q.qh / rhog);
     }
-    warp_sum_all<2>(acc);
+    cta_sum_all<2>(acc, s_red);
     const double inc = acc[0], refl = acc[1], rhow = -inc / refl;
     // cotangents of the node's micro and macro flux: the wall cell's stream rates (the bottom wall is the
     // cell's lower face, the top wall its upper face) and the wall outputs' seed
@@ -1610,14 +1657,14 @@ __global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers
     // W1: the wall density's cotangent
     acc[0] = 0.0;
     for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
+        const WVel s = wvel<kAdjWall>(B, nv, r);
         if (!s.ok || side * s.v > 0.0) continue;
         const QV q = qv_at(tt, s.u, s.v);
         double Gh, Gb;
         Gcot(s, Gh, Gb);
         acc[0] += dt * s.v * (q.qh / rhog * Gh + q.qb / rhog * Gb);
     }
-    warp_sum_all<1>(acc);
+    cta_sum_all<1>(acc, s_red);
     const double grhow = acc[0], ginc = -grhow / refl, grefl = -grhow * rhow / refl;
     // per-velocity cotangents of (ginh, ginb) and of the wall Maxwellian (wallh, wallb)
     auto cots = [&](const WVel& s, double& gh, double& gb, double& gwh, double& gwb) {
@@ -1633,7 +1680,7 @@ __global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers
     // [0..4] Mt, [5..8] an, [9..12] at, [13..16] atime, [17] Mxi2, [18] coeff, [19] hlx, [20] hly, [21] lambda,
     // [22] wall speed, [23..26] theta of the wall closure, [27] rho_g
     for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
+        const WVel s = wvel<kAdjWall>(B, nv, r);
         if (!s.ok) continue;
         const QV q = qv_at(tt, s.u, s.v);
         double gh, gb, gwh, gwb;
@@ -1694,16 +1741,16 @@ __global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers
         for (int a = 0; a < 4; ++a) a2[23 + a] += gmh * q.qh * q.ld[a] + gmb * q.qb * q.ldb[a];
         a2[27] += -(gwh * mh + gwb * mb) / (rhog * rhog);
     }
-    warp_sum_all<28>(a2);
+    cta_sum_all<28>(a2, s_red);
     // the wall closure (theta = closure(wwall)) and the scalar chain, transposed
     double gww[4];
-    solve_t4(C.jac, a2 + 23, gww);
+    solve_t4(s_jac[0], a2 + 23, gww);
     const double gout[kWallOut] = {a2[27], a2[21], gww[0], gww[1], gww[2], gww[3],
                                    a2[5], a2[6], a2[7], a2[8], a2[9], a2[10], a2[11], a2[12],
                                    a2[13], a2[14], a2[15], a2[16], a2[0], a2[1], a2[2], a2[3], a2[4], a2[18], a2[17]};
     double gI[kWallIn];
     transpose_lanes<kWallOut, kWallIn>(xo, gout, gI);
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
 #pragma unroll
         for (int m = 0; m < 4; ++m) atomic_add(A.gWi + cc * 4 + m, gI[m]);
         atomic_add(A.gpar + (top ? GP_UX1 : GP_UX0), gI[4] + a2[22] + gux_direct + a2[19] * dhlx_dux + a2[20] * dhly_dux);
@@ -1713,7 +1760,7 @@ __global__ void __launch_bounds__(256, 2) k_adj_wall_nodes(LoParams P, LoBuffers
     const double ghlx = a2[19], ghly = a2[20];
     // W3: the wall cell's face cache at the wall side
     for (int r = 0; r < nr; ++r) {
-        const WVel s = wvel(B, nv, r);
+        const WVel s = wvel<kAdjWall>(B, nv, r);
         if (!s.ok) continue;
         double gh, gb, gwh, gwb;
         cots(s, gh, gb, gwh, gwb);
@@ -2275,7 +2322,11 @@ static cudaError_t adj_launch(const LoParams& P, const LoBuffers& B, const S2Buf
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s2, ev[0], 0);
     }
     if (e == cudaSuccess) {
-        k_adj_wall_nodes<<<warps(2LL * nx * 3, 256), 256, 0, sw>>>(P, B, S, A);
+        const unsigned n = (unsigned)(2 * nx * 3);
+        const int nab = P.tnu > P.tnv ? P.tnu : P.tnv;
+        if (P.tnu <= 0) k_adj_wall_nodes<0><<<n, kAdjWall, 0, sw>>>(P, B, S, A);
+        else if (nab <= 32) k_adj_wall_nodes<4><<<n, kAdjWall, 0, sw>>>(P, B, S, A);
+        else k_adj_wall_nodes<8><<<n, kAdjWall, 0, sw>>>(P, B, S, A);
     }
     if (e == cudaSuccess) {
         if (P.tnu > 0) k_adj_face_nodes<true><<<warps((long long)nf * 3, 64), 64, 0, s>>>(P, B, S, A);

@@ -532,9 +532,10 @@ struct WVel {
     bool ok;     // a real velocity of this lane
     double u, v, w;
 };
+template <int NT = 32>   // threads over the velocities: a warp, or a CTA of NT
 __device__ __forceinline__ WVel wvel(const LoBuffers& B, int nv, int r) {
     WVel s;
-    const int k = (threadIdx.x & 31) + 32 * r;
+    const int k = (int)(threadIdx.x & (NT - 1)) + NT * r;
     s.ok = k < nv;
     s.k = s.ok ? k : nv - 1;
     s.u = __ldg(B.u + s.k);
