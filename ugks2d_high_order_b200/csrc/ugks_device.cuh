@@ -235,8 +235,8 @@ __device__ __forceinline__ void moment_add(double wl, double un, double ut, doub
 // the other half, so N values cost about N shuffles instead of 5N.  Then one lane per value and
 // warp writes a partial, and a serial sum over the warps finishes.  Every thread returns with the
 // block totals in v[0..NS+NM).  red needs (blockDim/32)*(pow2(NS)+pow2(NM)) doubles, out NS+NM.
-constexpr int pow2_ceil(int n) { return n <= 1 ? 1 : 2 * pow2_ceil((n + 1) / 2); }
-constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n / 2); }
+__host__ __device__ constexpr int pow2_ceil(int n) { return n <= 1 ? 1 : 2 * pow2_ceil((n + 1) / 2); }
+__host__ __device__ constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n / 2); }
 
 template <int N, bool MAX>
 __device__ __forceinline__ double warp_halving(const double* v) {
