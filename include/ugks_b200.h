@@ -139,8 +139,8 @@ int ugks_compute_residual(ugks_ctx* ctx, int with_collision);
 int ugks_apply_explicit_update(ugks_ctx* ctx, double* res_out);
 
 /* nsteps full Explicit steps (TimeStep, Interpolation, Evolution, ComputeResidual,
- * ApplyExplicitUpdate; src/mod_Solve.f90:84-186) fused into two kernels per step and replayed
- * from a CUDA graph.  dt_out / res_out (optional) report the last step. */
+ * ApplyExplicitUpdate; src/mod_Solve.f90:84-186) as two kernels per step on tensor-product velocity
+ * tables, four on others, replayed from a CUDA graph.  dt_out / res_out (optional) report the last step. */
 int ugks_step_explicit(ugks_ctx* ctx, int nsteps, double* dt_out, double* res_out);
 
 /* The Explicit step of ugks_step_explicit for callers that cannot allocate device memory.  No
@@ -156,7 +156,7 @@ int ugks_step_explicit(ugks_ctx* ctx, int nsteps, double* dt_out, double* res_ou
  * loaded on a device, and its 36 MiB taken there, at the first call on that device (CUDA loads modules
  * lazily), so callers that size their own device pool or run under a memory cap make one call per
  * device before they do; the array then stays until the process exits.  Each call synchronises
- * `stream` twice (it reads the velocity table's extent, which sets dt, and then the status), so it
+ * `stream` twice (it reads the velocity table's extent, which sets dt, and structure, then the status), so it
  * cannot be captured in a CUDA graph.  All calls on one device share the array: calls that overlap on
  * that GPU (other streams, other host threads) race and must be serialised by the caller; host threads
  * driving different devices share nothing. */

@@ -5,20 +5,25 @@
 //   k_s2_macro        : macro WENO of W: the normal / tangential slopes of every interior face at its 3
 //                       Gauss nodes (compute_flux :803-808,849-854) and the 9 mean-shifted volume node
 //                       states of every cell (build_targets, mod_S2D1.f90:1246-1300).
-//   k_s2_target_nodes : build_targets' closures: one warp per (cell, volume node) -> node scalars.
-//   k_s2_target_sum   : the Gauss-weighted targets M, K_x, K_y per (cell, velocity) from those scalars.
 //   k_s2_recon1/2     : tensor WENO-AO(5,3) reconstruction with one-sided wall quartics and the
 //                       positivity limiter (mod_S2D1Reconstruction.f90, limit_cell_outputs
 //                       mod_S2D1.f90:315-345): the shared first layer, then per cell the second-layer
 //                       templates and the limiter; writes the face cache.
-//   k_s2_face_nodes   : ugks_node (mod_S2D1.f90:421-521) at one Gauss node of one interior face per warp:
-//                       closure, directions and time coefficients -> node scalars.
-//   k_s2_face_flux    : the node's micro flux from those scalars, one CTA per face node.
-//   k_s2_wall_nodes   : the multiscale diffuse wall node (s2w2_wall_node, mod_S2MultiscaleWall.f90:45-184)
-//                       per warp.
+// then, on tensor-product velocity tables (LoParams::tnu > 0; ugks_s2_tensor.cuh),
+//   k_s2_target_nodes_t : build_targets' closures by 1-D sums: eight lanes per (cell, volume node) -> node scalars.
+//   k_s2_target_sum_t   : the Gauss-weighted targets M, K_x, K_y per (cell, velocity) from those scalars
+//                         (S2CN2's collision forms them itself).
+//   k_s2_face_moments   : the velocity sums of a face's three nodes over the upwind face values, one CTA a face.
+//   k_s2_face_nodes_t   : ugks_node (mod_S2D1.f90:421-521) at one Gauss node by eight lanes: closure, directions and time
+//                         coefficients -> node scalars.
+//   k_s2_face_flux_t    : the three nodes' micro fluxes, Gauss-weighted, into the face arrays, one CTA a face.
+//   k_s2_walls_t        : the multiscale diffuse wall (s2w2_wall_node, mod_S2MultiscaleWall.f90:45-184), one CTA a wall
+//                         face: its three nodes, their flux and the wall diagnostics.
+// and on other tables, and where a wall variant wants the nodes' fluxes or coefficients,
+//   k_s2_target_nodes, k_s2_target_sum, k_s2_face_nodes, k_s2_face_flux (one CTA per face node), k_s2_wall_nodes, and
 //   k_s2_combine      : the Gauss-weighted node fluxes times the face length into the face arrays.
 //
-// The discrete closure (solve_q_first, mod_CorrectedWF2DClosure.f90:331-426) runs on one warp: its
+// In the latter the discrete closure (solve_q_first, mod_CorrectedWF2DClosure.f90:331-426) runs on one warp: its
 // lanes stride over the velocities, every moment sum is a per-lane sum and a fixed butterfly whose
 // totals every lane receives, and every lane runs the reference's accept / backtrack / stop logic on
 // those identical totals.  Per-velocity closure quantities (the Maxwellian, the Shakhov directions,

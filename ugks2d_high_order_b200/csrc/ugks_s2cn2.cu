@@ -2,7 +2,7 @@
 //
 // One step (TimeStep; S2NativeEvolution with the volume targets kept between steps,
 // mod_S2NativeAdapter.f90:469-490; ComputeResidual; S2NativeApplyUpdate, :867-940, whose
-// advance_step, mod_S2D1.f90:1302-1435, runs on the stream state) is 13 launches:
+// advance_step, mod_S2D1.f90:1302-1435, runs on the stream state) is:
 //   k_lo_timestep  : dt of the accepted state.
 //   S2 evolution   : reconstruction, interior faces and (side stream) walls of ugks_s2.cu, with the
 //                    accepted state's targets.
@@ -10,13 +10,15 @@
 //                    AssembleSteadyRateResiduals and S2NativePhysicalCollision (mod_Residual.f90,
 //                    mod_S2NativeAdapter.f90:735-759), q_old = heat(W, h - M) and the CN right-hand
 //                    side rh = hs + beta_old (M + K q_old - h), hs = h + res_h.
-//   k_s2_targets   : build_targets of wn into the other target set.
+//   targets        : build_targets of wn into the other target set: macro slopes and node scalars (on
+//                    tensor-product velocity tables k_cn_collide forms M, K_x, K_y from those).
 //   k_cn_collide   : the 2x2 solve for the new heat flux and h_new = (rh + beta eq) / (1 + beta),
 //                    written into the other state set; the cnres / mmerr gates; a last-CTA epilogue
 //                    that takes the global conservation drift against the wall ledger and accepts
 //                    (ledger advanced, accepted counter incremented, and the next step's dt taken from
 //                    the accepted state's per-cell dt_local, so the steps of a ugks_s2cn2_steps sequence
-//                    after its first launch no k_lo_timestep: 12 launches) or rejects (halt flag set:
+//                    after its first launch no k_lo_timestep: 11 launches on a tensor-product table, 12
+//                    on another) or rejects (halt flag set:
 //                    every later kernel of the launch sequence returns at entry and the accepted state
 //                    stays in its set).
 // The state and the targets are double-buffered: a step reads set p and writes set 1-p, so a
