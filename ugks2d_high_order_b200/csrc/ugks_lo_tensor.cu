@@ -526,9 +526,29 @@ struct LoCellC {
         F = bf * H * (sh + qd * c2ck);
     }
 };
+// The stream projection's Gram sums again, into rout[4..13], for a cell (hc, bc) whose maximum of |h| or |b| passes 1, and its
+// floors.  Out of line and on the stored distribution, so that the kernel holds nothing for it: a state near the
+// reference's units (density 1, T = 2: h up to 0.16) never comes here.
+__device__ __noinline__ void lo_dense_stream(const double* __restrict__ hc, const double* __restrict__ bc,
+                                             const double* __restrict__ u, const double* __restrict__ v,
+                                             const double* __restrict__ w, int nv, double* red, double* rout, double* floors) {
+    __shared__ double s_max[2], s_gram[10];
+    double acc[10], mx[2] = {0.0, 0.0};
+    for (int k = threadIdx.x; k < nv; k += blockDim.x) { mx[0] = fmax(mx[0], fabs(hc[k])); mx[1] = fmax(mx[1], fabs(bc[k])); }
+    block_reduce_smem<0, 2>(mx, red, s_max);
+    const double fh = kEps * fmax(s_max[0], 1.0), fb = kEps * fmax(s_max[1], 1.0);
+#pragma unroll
+    for (int m = 0; m < 10; ++m) acc[m] = 0.0;
+    for (int k = threadIdx.x; k < nv; k += blockDim.x) gram_add(w[k], fmax(fabs(hc[k]), fh), fmax(fabs(bc[k]), fb), u[k], v[k], acc);
+    block_reduce_smem<10, 0>(acc, red, s_gram);
+    if (threadIdx.x < 10) rout[4 + threadIdx.x] = s_gram[threadIdx.x];
+    if (threadIdx.x == 0) { floors[0] = fh; floors[1] = fb; }
+    __syncthreads();
+}
+
 template <int VPT, int NTMAX, int MODE>
 __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, LoBuffers B) {
-    __shared__ double red[16 * 32], rout[kRedSlots], ex[2][64], ey[2][64], s_lam[4], s_tau[2], s_mx[16][4];
+    __shared__ double red[16 * 32], rout[kRedSlots], ex[2][64], ey[2][64], s_lam[4], s_tau[2], s_mx[16][4], s_floor[2];
     __shared__ LoCellC sc[2];
     const int nv = P.nvel, nu = P.tnu, tid = threadIdx.x, nx = P.nx, lane = tid & 31;
     const int c = blockIdx.x, i = c % nx, j = c / nx;
@@ -537,9 +557,9 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, L
     const size_t fl = (size_t)(j * nx + i), fr = (size_t)(j * nx + wrapx(i + 1, nx)), gr = (size_t)((j + 1) * nx + i);
     const double uo = Wo[1] / Wo[0], vo = Wo[2] / Wo[0], scale = 1.0 / (P.area * dt);
     const float inu = 1.0f / (float)nu;
-    double h[VPT], b[VPT], rh[VPT], rb[VPT], acc[16];
+    double h[VPT], b[VPT], rh[VPT], rb[VPT], acc[17];
 #pragma unroll
-    for (int m = 0; m < 16; ++m) acc[m] = 0.0;
+    for (int m = 0; m < 17; ++m) acc[m] = 0.0;
 #pragma unroll
     for (int r = 0; r < VPT; ++r) {
         const Slot s = slot(r, nv);
@@ -562,6 +582,7 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, L
         if (MODE & MODE_RESIDUAL) {
             moment_add(w, u, v, rh[r], rb[r], acc);
             gram_add(w, fmax(fabs(h[r]), kEps), fmax(fabs(b[r]), kEps), u, v, acc + 4);
+            acc[16] = fmax(acc[16], fmax(fabs(h[r]), fabs(b[r])));   // a slot past the table repeats its last velocity
         }
         if (MODE & MODE_UPDATE) {   // GetHeatFlux_Vec of the old state
             const double cx = u - uo, cy = v - vo, t = 0.5 * w * ((cx * cx + cy * cy) * h[r] + b[r]);
@@ -569,7 +590,11 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, L
             acc[15] += t * cy;
         }
     }
-    block_reduce_smem<16, 0>(acc, red, rout);
+    block_reduce_smem<16, 1>(acc, red, rout);
+    // the stream projection's weights are max(|h|, eps max(1, max |h|)): those above stand unless a maximum passes 1
+    if ((MODE & MODE_RESIDUAL) && rout[16] > 1.0)
+        lo_dense_stream(B.h + (size_t)c * nv, B.b + (size_t)c * nv, B.u, B.v, B.w, nv, red, rout, s_floor);
+    else if (tid == 0) s_floor[0] = s_floor[1] = kEps;
     double resw[4], Wn[4];   // AssembleMacroResidual (mod_Residual.f90:30-54)
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
@@ -701,8 +726,8 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, L
         for (int r = 0; r < VPT; ++r) {
             const Slot s = slot(r, nv);
             const double u = B.u[s.kk], v = B.v[s.kk];
-            rh[r] = dt * (rh[r] + fmax(fabs(h[r]), kEps) * (s_lam[0] + u * s_lam[1] + v * s_lam[2] + 0.5 * (u * u + v * v) * s_lam[3]));
-            rb[r] = dt * (rb[r] + 0.5 * fmax(fabs(b[r]), kEps) * s_lam[3]);
+            rh[r] = dt * (rh[r] + fmax(fabs(h[r]), s_floor[0]) * (s_lam[0] + u * s_lam[1] + v * s_lam[2] + 0.5 * (u * u + v * v) * s_lam[3]));
+            rb[r] = dt * (rb[r] + 0.5 * fmax(fabs(b[r]), s_floor[1]) * s_lam[3]);
             if (MODE == MODE_RESIDUAL && s.ok) {
                 B.res_h[(size_t)c * nv + s.k] = rh[r];
                 B.res_b[(size_t)c * nv + s.k] = rb[r];
