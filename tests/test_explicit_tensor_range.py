@@ -1,5 +1,6 @@
 """Explicit steps on a tensor-product velocity table against the same table in another order, which takes the general kernels,
-outside the reference's units: dense and cold states, where the projections' weight floors pass 1e-16."""
+outside the reference's units: dense and cold states, where the projections' weight floors pass 1e-16, and densities at which
+the product of the slopes' four denominators overflows."""
 import numpy as np
 import pytest
 
@@ -97,3 +98,17 @@ def test_stream_floor(shape):
     assert h.max() > 5e5 and far.sum() > 8
     g, w = (np.median(np.abs(a[0][2:-2, :, far])) for a in (got, want))
     assert w > 0 and 1 / 30 < g / w < 30
+
+
+# Tolerance: EXPLICIT_TOL, relative roundings of the largest value as in any units.  One step: its slopes are the ones at stake.
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(8, 4), (16, 16), (50, 50)])
+@pytest.mark.parametrize("rho", [1e76, 1e80, 1e140])
+def test_slopes_of_large_values(shape, rho):
+    t, (nx, ny) = rectangle(*shape), (4, 5)
+
+    def run(s):
+        s.step_explicit(1)
+        return s.download() + (s.wall_aero(),)
+
+    close(*both(case(nx, ny, rho), t, run, *state(t, nx, ny, rho, 2.0)))
