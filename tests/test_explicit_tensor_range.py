@@ -1,6 +1,6 @@
 """Explicit steps on a tensor-product velocity table against the same table in another order, which takes the general kernels,
-outside the reference's units: dense and cold states, where the projections' weight floors pass 1e-16, and densities at which
-the product of the slopes' four denominators overflows."""
+outside the reference's units: dense and cold states, where the projections' weight floors pass 1e-16, densities at which
+the product of the slopes' four denominators overflows, and states that the projections' gates refuse."""
 import numpy as np
 import pytest
 
@@ -112,3 +112,64 @@ def test_slopes_of_large_values(shape, rho):
         return s.download() + (s.wall_aero(),)
 
     close(*both(case(nx, ny, rho), t, run, *state(t, nx, ny, rho, 2.0)))
+
+
+def codes(s, *steps):
+    """The reference's abort code of each operator, 0 for none."""
+    from ugks2d_high_order_b200.capi import UgksError
+    out = []
+    for f in steps:
+        try:
+            f(s)
+            out.append(0)
+        except UgksError as e:
+            out.append(e.reference_code)
+    return out
+
+
+OPERATORS = [lambda s: s.time_step(), lambda s: s.evolution(), lambda s: s.compute_residual(), lambda s: s.apply_explicit_update()]
+
+
+# The smallest pivot of the equilibrium's Gram matrix falls as the mean's fourth power: 1e-11 of its largest entry at 100
+# and 1e-17 at 1000, on either side of the rule's 2.2e-13.
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(16, 16), (50, 50)])
+@pytest.mark.parametrize("mean,refused", [(100.0, [0, 0, 0, 0]), (1000.0, [0, 446, 444, 444])])
+def test_pivots_of_a_fast_mean(shape, mean, refused):
+    """A gas whose mean velocity is far above its thermal width, on a table moved with it."""
+    (u, v, w), (nx, ny) = rectangle(*shape), (3, 4)
+    t = (u + mean, v, w)
+    c = case(nx, ny).with_(wall_ux=(mean, mean), wall_tnative=(2.0, 2.0))
+    h = np.broadcast_to(np.exp(-(u ** 2 + v ** 2) / 2) / (2 * np.pi), (ny, nx, len(u))).copy()
+    W = np.stack([h @ w, h @ (w * t[0]), h @ (w * v), 0.5 * (h @ (w * (t[0] ** 2 + v ** 2)) + h @ w)], -1)
+    got, want = both(c, t, lambda s: codes(s, *OPERATORS), h, h, W)
+    assert want == refused and got == refused
+
+
+# A distribution whose density, momentum and energy are the state's and whose heat flux is A: its Shakhov equilibria are of
+# size 0.02 A, and their moments, which the projection's gate takes from W to 1e-10, carry rounding errors of 1e-16 of that and
+# more: far below the gate at A = 1, above it at 1e10.
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(16, 16), (50, 50)])
+@pytest.mark.parametrize("A,refused", [(1.0, [0]), (1e10, [444])])
+def test_moments_of_the_projected_equilibria(shape, A, refused):
+    t, (nx, ny) = rectangle(*shape), (3, 4)
+    M = np.exp(-(t[0] ** 2 + t[1] ** 2) / 2) / (2 * np.pi)
+    psi = np.stack([np.ones_like(t[0]), t[0], t[1], 0.5 * (t[0] ** 2 + t[1] ** 2)])
+    g = t[0] * (t[0] ** 2 + t[1] ** 2 - 4)
+    g = g - psi.T @ np.linalg.solve((psi * (t[2] * M)) @ psi.T, psi @ (t[2] * M * g))
+    full = lambda a: np.broadcast_to(a, (ny, nx, len(M))).copy()
+    W = np.broadcast_to([M @ t[2], 0.0, 0.0, 0.5 * (M @ (t[2] * (t[0] ** 2 + t[1] ** 2)) + M @ t[2])], (ny, nx, 4)).copy()
+    c = case(nx, ny).with_(wall_ux=(0.0, 0.0), wall_tnative=(2.0, 2.0))
+
+    from ugks2d_high_order_b200.solver import Solver
+    order = np.random.default_rng(1).permutation(len(M))
+    for q in (np.arange(len(M)), order):
+        s = Solver(c, *(np.ascontiguousarray(a[q]) for a in t))
+        try:
+            s.upload(full(M[q]), full(M[q]), W)
+            assert codes(s, *OPERATORS[:3]) == [0, 0, 0]   # the Maxwellian: no residual
+            s.upload(full((M * (1 + A * g))[q]), full(M[q]), W)
+            assert codes(s, OPERATORS[3]) == refused
+        finally:
+            s.close()

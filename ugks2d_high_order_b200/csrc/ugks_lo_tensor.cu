@@ -10,13 +10,16 @@
 // taken in one reduction, about a mean known beforehand.  Then one warp runs the scalar chain while the others take the
 // equilibria's sums, whose exponentials are products of two rows on a tensor table.  The equilibria are projected
 // (mod_ImplicitCommon.f90:42-82) in the basis 1, cx, cy, c^2 / 2 about their mean, which spans the same corrections with
-// the same weights, max(|E|, eps max(1, max |E|)); whether a projection met its moments is read off its linear system.
+// the same weights, max(|E|, eps max(1, max |E|)), and gated as there: by the pivots of the Gram matrix in the
+// basis 1, u, v, |v|^2 / 2 and by the moments of the projected distribution summed over the velocities.
 // ImplicitSteady keeps the kernels of ugks_lo.cu: its gate step is decided by their rounding.
 //
-// Bound by the latency of its phases (barriers, the scalar chain) and by issue: about 22 million warp instructions the
-// fluxes, 13 million the cells at 8x64x32^2.  Explicit step there 116.7 -> 89.9 us, 13x51x48^2 387 -> 275 us.  128 threads
-// a CTA with the table's velocities spread over them: 256 threads took 112 us, 64 143, six CTAs an SM (80 registers) 148;
-// above 1024 velocities 256 threads with 10 each: 512 with 5 took 299 us.
+// Bound by the latency of its phases (barriers, the scalar chain), by issue, and by spills: the long unrolled loops read
+// their scalars from shared memory anew for each velocity (lo_reread), and the cells the old distribution from L2 (13x51x48^2:
+// faces 176 -> 163 us, cells 153 -> 136).  The step takes 83 us at 8x64x32^2 and 287 at 13x51x48^2 (the kernels of ugks_lo.cu 117
+// and 387).  128 threads a CTA with the table's velocities spread over them, four CTAs an SM; above 1024 velocities 256 threads
+// with 10 each, two CTAs an SM (faces 512 with 5: 190 us instead of 175, 320 with 8: 174; cells 512 with 5: 135, 320 with 8:
+// 135, 384 with 7: 132 instead of 133).
 #include "ugks_s2_tensor.cuh"
 
 namespace ugks {
@@ -68,23 +71,62 @@ __device__ __forceinline__ double lo_peak(const LoParams& P, const double* ex, c
     return v[0] * v[1];
 }
 
-// G lam = rhs of a projection in the basis 1, cx, cy, c^2/2; false when singular or not met to 1e-10 of `scale`
-__device__ __forceinline__ bool lo_project(const double G[16], const double rhs[4], double scale, double lam[4]) {
-    const bool ok = t_solve(G, rhs, lam);
-    return ok && t_left(G, lam, rhs) <= 1.0e-10 * scale;
-}
+// the scalars in shared memory are read again after it: held in registers across an unrolled loop they spilled its state
+__device__ __forceinline__ void lo_reread() { asm volatile("" ::: "memory"); }
+
+// Projections (ProjectToConservedMoments, mod_ImplicitCommon.f90:42-82).  Two gates, as the kernels of ugks_lo.cu have them:
+// the pivots of the Gram matrix in the basis 1, u, v, |v|^2 / 2 (solve_dense4's rule, which refuses a mean far
+// outside the thermal width however well the centred system can be solved), and, in the kernels' last pass, the moments of the
+// projected distribution summed over the velocities.
+constexpr double kGate = 1.0e-10;
 __device__ __forceinline__ double lo_scale(const double w[4]) {
     return fmax(fmax(fmax(fabs(w[0]), fabs(w[1])), fmax(fabs(w[2]), fabs(w[3]))), 1.0);
 }
-
-// lam of a projection from its 14 sums f (moments of the equilibrium and Gram matrix in the basis about (U, V)) onto the
-// conserved moments tg
-__device__ __forceinline__ bool lo_lambda(const double f[14], double U, double V, const double tg[4], double lam[4]) {
-    double G[16];
+// a projection's targets and what its moments may miss each of them by; a lane a moment compares
+struct LoTarget {
+    double w[4], tol;
+    __device__ __forceinline__ void set(const double t[4]) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) w[m] = t[m];
+        tol = kGate * lo_scale(t);
+    }
+    __device__ __forceinline__ bool missed(int m, double moment) const { return !(fabs(moment - w[m]) <= tol); }
+};
+__device__ __forceinline__ double lo_least(const double G[16]) {
+    double ps = DBL_MIN;
+#pragma unroll
+    for (int m = 0; m < 16; ++m) ps = fmax(ps, fabs(G[m]));
+    return 1000.0 * kEps * ps;
+}
+// lam of a projection from its 14 sums f (moments of the equilibrium and Gram matrix in the basis 1, cx, cy, c^2 / 2 about
+// (U, V)) onto the conserved moments tg.  `plain`: the lane takes the system in the basis 1, u, v, |v|^2 / 2 instead, for its
+// pivots; a warp's lanes of both kinds run through one solve.
+__device__ __forceinline__ bool lo_lambda(const double f[14], double U, double V, const double tg[4], bool plain, double lam[4]) {
+    const double K = 0.5 * (U * U + V * V);
+    double G[16], least = 100.0 * DBL_MIN;
     gram_expand(f + 4, G);
-    const double rhs[4] = {tg[0] - f[0], (tg[1] - U * tg[0]) - f[1], (tg[2] - V * tg[0]) - f[2],
-                           (tg[3] - U * tg[1] - V * tg[2] + 0.5 * (U * U + V * V) * tg[0]) - f[3]};
-    return lo_project(G, rhs, lo_scale(tg), lam);
+    double rhs[4] = {tg[0] - f[0], (tg[1] - U * tg[0]) - f[1], (tg[2] - V * tg[0]) - f[2],
+                     (tg[3] - U * tg[1] - V * tg[2] + K * tg[0]) - f[3]};
+    if (plain) {   // rows, then columns: u = cx + U, v = cy + V, |v|^2 / 2 = c^2 / 2 + U cx + V cy + K
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            G[12 + c] += U * G[4 + c] + V * G[8 + c] + K * G[c];
+            G[4 + c] += U * G[c];
+            G[8 + c] += V * G[c];
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            double* g = G + 4 * r;
+            g[3] += U * g[1] + V * g[2] + K * g[0];
+            g[1] += U * g[0];
+            g[2] += V * g[0];
+        }
+        rhs[3] += U * rhs[1] + V * rhs[2] + K * rhs[0];
+        rhs[1] += U * rhs[0];
+        rhs[2] += V * rhs[0];
+        least = lo_least(G);
+    }
+    return t_solve(G, rhs, lam, least);
 }
 
 // a microscopic slope (1, vn, vt, |v|^2/2) of a face (dir 0: vn = u, vt = v; 1: vn = v, vt = -u) as a polynomial in the
@@ -100,6 +142,7 @@ __device__ __forceinline__ void lo_centred(int dir, const double X[4], double U,
 struct LoFluxC {
     double U, V, l2, kq, qx, qy, lam[4], bf, fh, fb, mxi2, mt[5];   // mean, 2 L, Shakhov factor, heat, lam, ck/(2L), floors
     double a[2][4], b[4], T[4];   // slopes along the normal (left / right, or a wall's), tangential, in time
+    LoTarget tg[2];               // the projection's, and a wall's unit shape's
 };
 
 // values and slopes of h and b at cell c, velocity k (Interpolation, mod_Interpolation.f90:26-170).  The four limiters
@@ -147,9 +190,8 @@ __device__ __forceinline__ void lo_equilibrium(const LoFluxC& c, double H0, doub
     Bq = b0 + 0.5 * fmax(b0, c.fb) * c.lam[3];
 }
 __device__ __forceinline__ void lo_poly(const LoFluxC& c, const double* d, double H0, double cx, double cy, double vn, double vt,
-                                        double c2ck, double& gh, double& gb) {
+                                        double c2ck, double& H, double& Bq, double& gh, double& gb) {
     const double c2 = cx * cx + cy * cy, qd = c.kq * (cx * c.qx + cy * c.qy), sh = 1.0 + qd * (c.l2 * c2 - 4.0);
-    double H, Bq;
     lo_equilibrium(c, H0, cx, cy, c2, H, Bq);
     const double pn = d[0] + d[1] * cx + d[2] * cy + d[3] * c2, pt = c.b[0] + c.b[1] * cx + c.b[2] * cy + c.b[3] * c2;
     const double pT = c.T[0] + c.T[1] * cx + c.T[2] * cy + c.T[3] * c2;
@@ -157,6 +199,13 @@ __device__ __forceinline__ void lo_poly(const LoFluxC& c, const double* d, doubl
     const double z3 = c.mt[1] * (vn * d[3] + vt * c.b[3]) + c.mt[2] * c.T[3];
     gh = H * (c.mt[0] * sh + Z) + Bq * z3;
     gb = Bq * (c.mt[0] * (sh + qd * c2ck) + Z) + c.mxi2 * H * z3;
+}
+
+// the projected unit-density wall Maxwellian of the value Hw (s_w: lam, floors)
+__device__ __forceinline__ void lo_shape(double Hw, double bfac, const double* s_w, double cx, double cy, double& h, double& b) {
+    const double bw = Hw * bfac;
+    h = Hw + fmax(Hw, s_w[4]) * (s_w[0] + s_w[1] * cx + s_w[2] * cy + s_w[3] * (0.5 * (cx * cx + cy * cy)));
+    b = bw + 0.5 * fmax(bw, s_w[5]) * s_w[3];
 }
 
 template <int VPT>
@@ -256,20 +305,21 @@ __device__ __forceinline__ void lo_wall_t(const LoParams& P, const LoBuffers& B,
         }
     }
     __syncthreads();
-    if (tid < 32) {   // lane 0: the equilibrium's projection, lane 1: the shape's
+    if (tid < 32) {   // lane 0: the equilibrium's projection, lane 1: the shape's, lanes 2 and 3: their pivots
         double f[14], tg[4], lam[4];
-        const int o = lane == 1 ? 14 : 0;
+        const int o = lane & 1 ? 14 : 0;
 #pragma unroll
         for (int m = 0; m < 14; ++m) f[m] = C.total(red, o + m);
-        const Prim pq{lane == 1 ? 1.0 : pg.r, ux, 0.0, L};
+        const Prim pq{lane & 1 ? 1.0 : pg.r, ux, 0.0, L};
         get_conserved(P.gm1, pq, tg);
-        const bool pok = lo_lambda(f, ux, 0.0, tg, lam);
+        const bool pok = lo_lambda(f, ux, 0.0, tg, lane & 2, lam);
         if (lane < 2) {
             double* q = lane == 0 ? sc.lam : s_w;
 #pragma unroll
             for (int m = 0; m < 4; ++m) q[m] = lam[m];
-            if (!pok) set_status(B.status, ST_FACE_PROJECTION);
+            sc.tg[lane].set(tg);
         }
+        if (!pok && lane < 4) set_status(B.status, ST_FACE_PROJECTION);
     }
     __syncthreads();
     // toward the wall: the incident flux; away from it: the unit wall Maxwellian, its density from zero net mass (:2166)
@@ -282,20 +332,30 @@ __device__ __forceinline__ void lo_wall_t(const LoParams& P, const LoBuffers& B,
         const double u = B.u[s.kk], v = B.v[s.kk], wv = (s.ok ? B.w[s.kk] : 0.0) * v, H0 = ex[s.kk - jv * nu] * ey[jv];
         const double cx = u - ux;
         if ((copysign(1.0, v) > 0.0) == (iw == 1)) {
-            double gh, gb;
-            lo_poly(sc, sc.a[0], H0, cx, v, v, -u, c2ck, gh, gb);
+            double H, Bq, gh, gb;
+            lo_poly(sc, sc.a[0], H0, cx, v, v, -u, c2ck, H, Bq, gh, gb);
             hv[r] = gh + sc.mt[3] * hv[r] - sc.mt[4] * ph[r];
             bv[r] = gb + sc.mt[3] * bv[r] - sc.mt[4] * pb[r];
             acc[0] += wv * hv[r];
         } else {
-            const double c2 = cx * cx + v * v, Hw = H0 * irho, bw = Hw * bfac;
-            hv[r] = Hw + fmax(Hw, s_w[4]) * (s_w[0] + s_w[1] * cx + s_w[2] * v + s_w[3] * (0.5 * c2));
-            bv[r] = bw + 0.5 * fmax(bw, s_w[5]) * s_w[3];
+            lo_shape(H0 * irho, bfac, s_w, cx, v, hv[r], bv[r]);
             acc[1] += wv * hv[r];
         }
     }
-    block_reduce<2, 0>(acc, red, rout);
-    const double rhow = -acc[0] / (dt * acc[1]), flen = P.dx;
+    // the gates of both projections, over all velocities, in a loop of their own: a domain has few wall faces
+    double mom[10] = {acc[0], acc[1], 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int k = tid; k < nv; k += (int)blockDim.x) {
+        const int jv = lo_row(k, inu);
+        const double w = B.w[k], u = B.u[k], v = B.v[k], cx = u - ux, H0 = ex[k - jv * nu] * ey[jv];
+        double h, b;
+        lo_equilibrium(sc, H0, cx, v, cx * cx + v * v, h, b);
+        moment_add(w, u, v, h, b, mom + 2);
+        lo_shape(H0 * irho, bfac, s_w, cx, v, h, b);
+        moment_add(w, u, v, h, b, mom + 6);
+    }
+    block_reduce_smem<10, 0>(mom, red, rout);
+    if (tid >= 2 && tid < 10 && sc.tg[(tid - 2) >> 2].missed((tid - 2) & 3, rout[tid])) set_status(B.status, ST_FACE_PROJECTION);
+    const double rhow = -rout[0] / (dt * rout[1]), flen = P.dx;
     const size_t o = (size_t)((iw ? P.ny : 0) * nx + i);
 #pragma unroll
     for (int m = 0; m < 4; ++m) acc[m] = 0.0;
@@ -464,18 +524,18 @@ __device__ __forceinline__ void lo_face_t(const LoParams& P, const LoBuffers& B,
         }
     }
     __syncthreads();
-    if (tid < 32) {
+    if (tid < 32) {   // lane 0: the projection, lane 1: its pivots
         double t[14], tg[4], lam[4];
 #pragma unroll
         for (int m = 0; m < 14; ++m) t[m] = C.total(red, m);
         const Prim pq{pf.r, U, V, pf.L};
         get_conserved(P.gm1, pq, tg);
-        const bool pok = lo_lambda(t, U, V, tg, lam);
-        if (lane == 0) {
+        const bool pok = lo_lambda(t, U, V, tg, lane & 1, lam);
+        if (lane == 0)
 #pragma unroll
             for (int m = 0; m < 4; ++m) sc.lam[m] = lam[m];
-            if (!pok) set_status(B.status, ST_FACE_PROJECTION);
-        }
+        if (lane == 0) sc.tg[0].set(tg);
+        if (!pok && lane < 2) set_status(B.status, ST_FACE_PROJECTION);
     }
     __syncthreads();
     // the micro flux (mod_Evolution.f90:396-453) times the face length
@@ -484,25 +544,28 @@ __device__ __forceinline__ void lo_face_t(const LoParams& P, const LoBuffers& B,
     double* Fh = (dir == 0 ? B.fxh : B.fyh) + o * nv;
     double* Fb = (dir == 0 ? B.fxb : B.fyb) + o * nv;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) acc[m] = 0.0;
+    for (int m = 0; m < 8; ++m) acc[m] = 0.0;   // the flux's moments, the projected equilibrium's
 #pragma unroll
     for (int r = 0; r < VPT; ++r) {
         const Slot s = slot(r, nv);
         const int jv = lo_row(s.kk, inu);
         const double u = B.u[s.kk], v = B.v[s.kk], w = s.ok ? B.w[s.kk] : 0.0, H0 = ex[s.kk - jv * nu] * ey[jv];
-        const double vn = dir == 0 ? u : v, vt = dir == 0 ? v : -u;
-        double gh, gb;
-        lo_poly(sc, sc.a[copysign(1.0, vn) > 0.0 ? 0 : 1], H0, u - sc.U, v - sc.V, vn, vt, c2ck, gh, gb);
+        lo_reread();
+        const double vn = dir == 0 ? u : v, vt = dir == 0 ? v : -u, cx = u - sc.U, cy = v - sc.V;
+        double H, Bq, gh, gb;
+        lo_poly(sc, sc.a[copysign(1.0, vn) > 0.0 ? 0 : 1], H0, cx, cy, vn, vt, c2ck, H, Bq, gh, gb);
+        moment_add(w, u, v, H, Bq, acc + 4);
         const double fh = flen * (vn * (gh + sc.mt[3] * hv[r] - sc.mt[4] * ph[r]));
         const double fb = flen * (vn * (gb + sc.mt[3] * bv[r] - sc.mt[4] * pb[r]));
         if (s.ok) { Fh[s.k] = fh; Fb[s.k] = fb; }
         moment_add(w, u, v, fh, fb, acc);   // MomentConserved in the global frame (:470-473)
     }
-    block_reduce_smem<4, 0>(acc, red, rout);
+    block_reduce_smem<8, 0>(acc, red, rout);
     if (tid < 4) {
         ((dir == 0 ? B.fxw : B.fyw) + o * 4)[tid] = rout[tid];
         if (!isfinite(rout[tid])) set_status(B.status, ST_NONFINITE_FLUX);
     }
+    if (tid >= 4 && tid < 8 && sc.tg[0].missed(tid - 4, rout[tid])) set_status(B.status, ST_FACE_PROJECTION);
 }
 
 template <int VPT, int NTMAX>
@@ -522,6 +585,7 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_fluxes_t(LoParams P, 
 enum { MODE_RESIDUAL = 1, MODE_UPDATE = 2 };
 struct LoCellC {
     double U, V, l2, kx, ky, bf, fh, fb, lam[4];   // mean, 2 L, coeff q, ck/(2L), floors, lam
+    LoTarget tg;
     // equilibrium + Shakhov of the Maxwellian value H
     __device__ __forceinline__ void at(double H, double cx, double cy, double c2, double c2ck, double& E, double& F) const {
         const double qd = kx * cx + ky * cy, sh = 1.0 + qd * (l2 * c2 - 4.0);
@@ -553,6 +617,7 @@ template <int VPT, int NTMAX, int MODE>
 __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, LoBuffers B) {
     __shared__ double red[16 * 32], rout[kRedSlots], ex[2][64], ey[2][64], s_lam[4], s_tau[2], s_mx[16][4], s_floor[2];
     __shared__ LoCellC sc[2];
+    __shared__ LoTarget s_rate;
     const int nv = P.nvel, nu = P.tnu, tid = threadIdx.x, nx = P.nx, lane = tid & 31;
     const int c = blockIdx.x, i = c % nx, j = c / nx;
     const double dt = B.dt[0], dti = 1.0 / dt, c2ck = 2.0 / (double)P.ck;
@@ -560,35 +625,33 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, L
     const size_t fl = (size_t)(j * nx + i), fr = (size_t)(j * nx + wrapx(i + 1, nx)), gr = (size_t)((j + 1) * nx + i);
     const double uo = Wo[1] / Wo[0], vo = Wo[2] / Wo[0], scale = 1.0 / (P.area * dt);
     const float inu = 1.0f / (float)nu;
-    double h[VPT], b[VPT], rh[VPT], rb[VPT], acc[17];
+    double *hc = B.h + (size_t)c * nv, *bc = B.b + (size_t)c * nv;
+    double rh[VPT], rb[VPT], acc[17];
 #pragma unroll
     for (int m = 0; m < 17; ++m) acc[m] = 0.0;
 #pragma unroll
     for (int r = 0; r < VPT; ++r) {
         const Slot s = slot(r, nv);
-        const size_t q = (size_t)c * nv + s.kk;
-        h[r] = B.h[q];
-        b[r] = B.b[q];
+        const int k = s.kk;
         if (MODE & MODE_RESIDUAL) {   // AssembleMicroFluxResidual (mod_Residual.f90:60-95)
-            const int k = s.kk;
             rh[r] = (B.fxh[fl * nv + k] - B.fxh[fr * nv + k] + B.fyh[fl * nv + k] - B.fyh[gr * nv + k]) * scale;
             rb[r] = (B.fxb[fl * nv + k] - B.fxb[fr * nv + k] + B.fyb[fl * nv + k] - B.fyb[gr * nv + k]) * scale;
         } else {
-            rh[r] = B.res_h[q];
-            rb[r] = B.res_b[q];
+            rh[r] = B.res_h[(size_t)c * nv + k];
+            rb[r] = B.res_b[(size_t)c * nv + k];
         }
     }
 #pragma unroll
     for (int r = 0; r < VPT; ++r) {
         const Slot s = slot(r, nv);
-        const double u = B.u[s.kk], v = B.v[s.kk], w = s.ok ? B.w[s.kk] : 0.0;
+        const double u = B.u[s.kk], v = B.v[s.kk], w = s.ok ? B.w[s.kk] : 0.0, hr = hc[s.kk], br = bc[s.kk];
         if (MODE & MODE_RESIDUAL) {
             moment_add(w, u, v, rh[r], rb[r], acc);
-            gram_add(w, fmax(fabs(h[r]), kEps), fmax(fabs(b[r]), kEps), u, v, acc + 4);
-            acc[16] = fmax(acc[16], fmax(fabs(h[r]), fabs(b[r])));   // a slot past the table repeats its last velocity
+            gram_add(w, fmax(fabs(hr), kEps), fmax(fabs(br), kEps), u, v, acc + 4);
+            acc[16] = fmax(acc[16], fmax(fabs(hr), fabs(br)));   // a slot past the table repeats its last velocity
         }
         if (MODE & MODE_UPDATE) {   // GetHeatFlux_Vec of the old state
-            const double cx = u - uo, cy = v - vo, t = 0.5 * w * ((cx * cx + cy * cy) * h[r] + b[r]);
+            const double cx = u - uo, cy = v - vo, t = 0.5 * w * ((cx * cx + cy * cy) * hr + br);
             acc[14] += t * cx;
             acc[15] += t * cy;
         }
@@ -596,7 +659,7 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, L
     block_reduce_smem<16, 1>(acc, red, rout);
     // the stream projection's weights are max(|h|, eps max(1, max |h|)): those above stand unless a maximum passes 1
     if ((MODE & MODE_RESIDUAL) && rout[16] > 1.0)
-        lo_dense_stream(B.h + (size_t)c * nv, B.b + (size_t)c * nv, B.u, B.v, B.w, nv, red, rout, s_floor);
+        lo_dense_stream(hc, bc, B.u, B.v, B.w, nv, red, rout, s_floor);
     else if (tid == 0) s_floor[0] = s_floor[1] = kEps;
     double resw[4], Wn[4];   // AssembleMacroResidual (mod_Residual.f90:30-54)
 #pragma unroll
@@ -692,12 +755,14 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, L
             }
         }
         if (MODE & MODE_RESIDUAL) {   // EnforceStreamingMomentCompatibility (mod_ImplicitMicro.f90:293-306)
-            double G[16], rhs[4], lam[4], sr = 1.0;
+            double G[16], rhs[4], lam[4];
             gram_expand(rout + 4, G);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) { rhs[m] = resw[m] * dti - rout[m]; sr = fmax(sr, fabs(resw[m] * dti)); }
-            const bool ok = lo_project(G, rhs, sr, lam);
+            for (int m = 0; m < 4; ++m) rhs[m] = resw[m] * dti - rout[m];
+            const bool ok = t_solve(G, rhs, lam, lo_least(G));
             if (lane == 0) {
+                const double rate[4] = {resw[0] * dti, resw[1] * dti, resw[2] * dti, resw[3] * dti};
+                s_rate.set(rate);
 #pragma unroll
                 for (int m = 0; m < 4; ++m) s_lam[m] = lam[m];
                 if (!ok) set_status(B.status, ST_PROJECTION);
@@ -706,63 +771,94 @@ __global__ void __launch_bounds__(NTMAX, 512 / NTMAX) k_lo_cells_t(LoParams P, L
     }
     __syncthreads();
     if (MODE & MODE_UPDATE) {
-        if (tid < 32) {   // lane 0: the old equilibrium onto W_old's moments, lane 1: the new one onto W_new
+        if (tid < 32) {   // lane 0: the old equilibrium onto W_old's moments, lane 1: the new one onto W_new, lanes 2, 3: pivots
+            const bool nw = lane & 1;
             double f[14], tg[4], lam[4];
-            const int o = lane == 1 ? 14 : 0;
+            const int o = nw ? 14 : 0;
 #pragma unroll
             for (int m = 0; m < 14; ++m) f[m] = C.total(red, o + m);
             get_conserved(P.gm1, po, tg);
-            if (lane == 1)
+            if (nw)
 #pragma unroll
                 for (int m = 0; m < 4; ++m) tg[m] = Wn[m];
-            const bool ok = lo_lambda(f, lane == 1 ? pn.U : po.U, lane == 1 ? pn.V : po.V, tg, lam);
-            if (lane < 2) {
+            const bool ok = lo_lambda(f, nw ? pn.U : po.U, nw ? pn.V : po.V, tg, lane & 2, lam);
+            if (lane < 2)
 #pragma unroll
                 for (int m = 0; m < 4; ++m) sc[lane].lam[m] = lam[m];
-                if (!ok) set_status(B.status, ST_PROJECTION);
-            }
+            if (lane < 2) sc[lane].tg.set(tg);
+            if (!ok && lane < 4) set_status(B.status, ST_PROJECTION);
         }
         __syncthreads();
     }
+    // the moments of the projected stream and equilibria, for the gates: a warp's totals, then a lane of the second warp each,
+    // beside the first thread's norms
+    auto put = [&](int g, const double* m) {
+        const double t = warp_halving<4, false>(m);
+        if ((lane & 7) == 0) red[(tid >> 5) * 12 + 4 * g + (lane >> 3)] = t;
+    };
     if (MODE & MODE_RESIDUAL) {   // res_h_flux_store = stream_h * dt (mod_Residual.f90:114-115)
+        double mom[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
         for (int r = 0; r < VPT; ++r) {
             const Slot s = slot(r, nv);
-            const double u = B.u[s.kk], v = B.v[s.kk];
-            rh[r] = dt * (rh[r] + fmax(fabs(h[r]), s_floor[0]) * (s_lam[0] + u * s_lam[1] + v * s_lam[2] + 0.5 * (u * u + v * v) * s_lam[3]));
-            rb[r] = dt * (rb[r] + 0.5 * fmax(fabs(b[r]), s_floor[1]) * s_lam[3]);
+            lo_reread();
+            const double u = B.u[s.kk], v = B.v[s.kk], c2 = u * u + v * v;
+            // (no read past the table's end of an element that its own thread may have updated)
+            const double hr = s.ok ? hc[s.kk] : 0.0, br = s.ok ? bc[s.kk] : 0.0;
+            const double sh = rh[r] + fmax(fabs(hr), s_floor[0]) * (s_lam[0] + u * s_lam[1] + v * s_lam[2] + 0.5 * c2 * s_lam[3]);
+            const double sb = rb[r] + 0.5 * fmax(fabs(br), s_floor[1]) * s_lam[3];
+            moment_add(s.ok ? B.w[s.kk] : 0.0, u, v, sh, sb, mom);
+            rh[r] = dt * sh;
+            rb[r] = dt * sb;
             if (MODE == MODE_RESIDUAL && s.ok) {
                 B.res_h[(size_t)c * nv + s.k] = rh[r];
                 B.res_b[(size_t)c * nv + s.k] = rb[r];
             }
         }
-        if (MODE == MODE_RESIDUAL) {
-            if (tid == 0)
+        put(2, mom);
+    }
+    if (MODE & MODE_UPDATE) {   // ApplyExplicitUpdate (mod_TimeIntegrator.f90:16-134, 235-293)
+        const double ito = 0.5 * dt / s_tau[0], itn = 0.5 * dt / s_tau[1], inv = 1.0 / (1.0 + itn);
+        double mq[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
 #pragma unroll
-                for (int m = 0; m < 4; ++m) B.res_w[c * 4 + m] = resw[m];
-            return;
+        for (int r = 0; r < VPT; ++r) {
+            const Slot s = slot(r, nv);
+            const int jv = lo_row(s.kk, inu), iv = s.kk - jv * nu;
+            const double u = B.u[s.kk], v = B.v[s.kk], w = s.ok ? B.w[s.kk] : 0.0;
+            const double hr = s.ok ? hc[s.kk] : 0.0, br = s.ok ? bc[s.kk] : 0.0;
+            lo_reread();
+            double E[2], F[2];
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const LoCellC& q = sc[t];
+                const double cx = u - q.U, cy = v - q.V, c2 = cx * cx + cy * cy;
+                q.at(ex[t][iv] * ey[t][jv], cx, cy, c2, c2ck, E[t], F[t]);
+                E[t] = E[t] + fmax(fabs(E[t]), q.fh) * (q.lam[0] + q.lam[1] * cx + q.lam[2] * cy + q.lam[3] * (0.5 * c2));
+                F[t] = F[t] + 0.5 * fmax(fabs(F[t]), q.fb) * q.lam[3];
+                moment_add(w, u, v, E[t], F[t], mq[t]);
+            }
+            if (s.ok) {
+                hc[s.k] = (hr + rh[r] + (itn * E[1] + ito * (E[0] - hr))) * inv;
+                bc[s.k] = (br + rb[r] + (itn * F[1] + ito * (F[0] - br))) * inv;
+            }
+        }
+        put(0, mq[0]);
+        put(1, mq[1]);
+    }
+    __syncthreads();
+    {
+        const int m = tid - 32, first = MODE & MODE_UPDATE ? 0 : 8, last = MODE & MODE_RESIDUAL ? 12 : 8;
+        if (m >= first && m < last) {
+            double t = red[m];
+            for (int q = 1; q < (int)blockDim.x / 32; ++q) t += red[q * 12 + m];
+            if ((m < 8 ? sc[m >> 2].tg : s_rate).missed(m & 3, t)) set_status(B.status, ST_PROJECTION);
         }
     }
-    // ApplyExplicitUpdate (mod_TimeIntegrator.f90:16-134, 235-293)
-    const double ito = 0.5 * dt / s_tau[0], itn = 0.5 * dt / s_tau[1], inv = 1.0 / (1.0 + itn);
+    if (MODE == MODE_RESIDUAL) {
+        if (tid == 0)
 #pragma unroll
-    for (int r = 0; r < VPT; ++r) {
-        const Slot s = slot(r, nv);
-        const int jv = lo_row(s.kk, inu), iv = s.kk - jv * nu;
-        const double u = B.u[s.kk], v = B.v[s.kk];
-        double E[2], F[2];
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const LoCellC& q = sc[t];
-            const double cx = u - q.U, cy = v - q.V, c2 = cx * cx + cy * cy;
-            q.at(ex[t][iv] * ey[t][jv], cx, cy, c2, c2ck, E[t], F[t]);
-            E[t] = E[t] + fmax(fabs(E[t]), q.fh) * (q.lam[0] + q.lam[1] * cx + q.lam[2] * cy + q.lam[3] * (0.5 * c2));
-            F[t] = F[t] + 0.5 * fmax(fabs(F[t]), q.fb) * q.lam[3];
-        }
-        if (s.ok) {
-            B.h[(size_t)c * nv + s.k] = (h[r] + rh[r] + (itn * E[1] + ito * (E[0] - h[r]))) * inv;
-            B.b[(size_t)c * nv + s.k] = (b[r] + rb[r] + (itn * F[1] + ito * (F[0] - b[r]))) * inv;
-        }
+            for (int m = 0; m < 4; ++m) B.res_w[c * 4 + m] = resw[m];
+        return;
     }
     if (tid == 0) {
         bool fin = true, dok;

@@ -71,8 +71,9 @@ __device__ __noinline__ void t_sums(const double* __restrict__ tu, const double*
     out->ey = t_min(ey);
 }
 
-// solve_dense_4x4 (mod_CorrectedWF2DClosure.f90:631-661) as s2_solve4, the pivots' divisions taken as one reciprocal each
-__device__ __noinline__ bool t_solve(const double* m, const double* rhs, double* out) {
+// solve_dense_4x4 (mod_CorrectedWF2DClosure.f90:631-661) as s2_solve4, the pivots' divisions taken as one reciprocal each;
+// `least`: the largest pivot that counts as none
+__device__ __noinline__ bool t_solve(const double* m, const double* rhs, double* out, double least = 100.0 * DBL_MIN) {
     double a[4][5], x[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -88,7 +89,7 @@ __device__ __noinline__ bool t_solve(const double* m, const double* rhs, double*
         double best = fabs(a[p][p]);
 #pragma unroll
         for (int i = p + 1; i < 4; ++i) if (fabs(a[i][p]) > best) { best = fabs(a[i][p]); row = i; }
-        ok = ok && best > 100.0 * DBL_MIN && isfinite(best);
+        ok = ok && best > least && isfinite(best);
 #pragma unroll
         for (int i = p + 1; i < 4; ++i) {
             const bool sw = row == i;
