@@ -448,24 +448,34 @@ __global__ void __launch_bounds__(128, 3) k_s2_target_nodes_t(LoParams P, LoBuff
     o[24 + gl] = C.jac[8 + gl];
 }
 
-// build_targets, sum part, on a tensor table: one CTA per cell and 1024 velocities (STargets, ugks_s2_tensor.cuh)
-__global__ void __launch_bounds__(256) k_s2_target_sum_t(LoParams P, LoBuffers B, S2Buffers SB) {
+// build_targets, sum part, on a tensor table: one CTA per cell (STargets, ugks_s2_tensor.cuh)
+__global__ void __launch_bounds__(256, 2) k_s2_target_sum_t(LoParams P, LoBuffers B, S2Buffers SB) {
     if (eval_cached(B)) return;
     __shared__ STargets st;
-    const int nv = P.nvel, cc = blockIdx.y;
+    __shared__ double red[8 * 8], rout[kRedSlots];
+    const int nv = P.nvel, cc = blockIdx.x, tid = threadIdx.x, nt = (int)blockDim.x;
     st.fill(P, B, SB, cc);
     __syncthreads();
-    double a[4][6];
-    const int k0 = blockIdx.x * 1024 + threadIdx.x;
-    st.at<4>(P, B, k0, blockDim.x, a);
     double* out[6] = {SB.mh, SB.mb, SB.kxh, SB.kxb, SB.kyh, SB.kyb};
+    double mom[8];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int k = k0 + r * (int)blockDim.x;
-        if (k < nv && k < (int)(blockIdx.x + 1) * 1024)
+    for (int m = 0; m < 8; ++m) mom[m] = 0.0;
+    for (int k0 = tid; k0 < nv; k0 += 4 * nt) {
+        double a[4][6];
+        st.at<4>(P, B, k0, nt, a);
 #pragma unroll
-            for (int m = 0; m < 6; ++m) out[m][(size_t)cc * nv + k] = a[r][m];
+        for (int r = 0; r < 4; ++r) {
+            const int k = k0 + r * nt;
+            if (k < nv) {
+                moment_add(B.w[k], B.u[k], B.v[k], a[r][2], a[r][3], mom);
+                moment_add(B.w[k], B.u[k], B.v[k], a[r][4], a[r][5], mom + 4);
+#pragma unroll
+                for (int m = 0; m < 6; ++m) out[m][(size_t)cc * nv + k] = a[r][m];
+            }
+        }
     }
+    block_reduce_smem<8, 0>(mom, red, rout);
+    if (tid < 8 && !(fabs(rout[tid]) <= kTGate)) set_status(B.status, ST_PROJECTION);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -816,11 +826,7 @@ __global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffer
                        t.pref * (0.5 * (un * un + uo * uo) * m0 + un * mn + uo * mo + 0.5 * m2 + 0.5 * t.ckh * mb)};
 #pragma unroll
         for (int m = 0; m < 4; ++m) wt[m] = -(t_get(c[m], 2) + t_get(c[m], 3) + t_get(c[m], 4));
-        ok = t_solve(C.jac, wt, tdm) && ok;
-        double sc = 1.0;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) sc = fmax(sc, fabs(wt[m]));
-        ok = ok && t_left(C.jac, tdm, wt) / sc <= 2.0e-12;
+        ok = t_solve(C.jac, wt, tdm) && ok;   // its moments are gated in k_s2_face_flux_t
     }
     double tau = 0.0, mt[5];
     ok = ok && s2_tau(P, w0, tau) && isfinite(q0x) && isfinite(q0y);
@@ -857,17 +863,19 @@ __global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffer
 // shared memory) times a cubic in the velocity, whose coefficients join s0, the slope and the time directions
 // with their Mt, plus the face values' part (ugks_node, mod_S2D1.f90:486-507).  The three nodes' Gauss sum
 // goes straight to the face arrays and its velocity moments are the face's macro flux, so no node flux is
-// stored.  Bound by the latency of the face cache's 12 values a (face, velocity), 100 MB at 8x64x32^2.  Nodes unrolled
+// stored.  The moments of each node's time direction are summed on the way and gated as in k_s2_face_flux (about 6 us a
+// step).  Bound by the latency of the face cache's 12 values a (face, velocity), 100 MB at 8x64x32^2.  Nodes unrolled
 // took 379 to 410 us a step instead of 347 (instruction fetch), 2 velocities a thread at four CTAs an SM 350.
 struct S2FluxC {
     double u, v, ux, vy, ckh, l2, kq, kb, qx, qy, mt0, mt3, mt4;   // means, ck T / 2, 2 lam, mt0 coeff, kq 2 / ck, q0, Mt
     double e[5], t[5], d[2][5];   // polynomials 1, cx, cy, c^2 and b part: mt2 dm - mt0 K dirs; mt1 tangential; mt1 left, right
+    double m[5];                  // dm, the time direction
 };
 __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers B, S2Buffers SB) {
     if (eval_cached(B)) return;
     __shared__ double ex[3][64], ey[3][64];
     __shared__ S2FluxC sc[3];
-    __shared__ double red[8 * 8], rout[kRedSlots];
+    __shared__ double red[8 * 8], rout[kRedSlots], s_time[8][12];   // s_time: the warps' moments of the nodes' time directions
     const int nv = P.nvel, nu = P.tnu, nw = P.tnv, nx = P.nx, ny = P.ny, nfx = nx * ny, tid = threadIdx.x;
     const int fi = blockIdx.x, axis = fi < nfx ? 0 : 1, cl = axis == 0 ? fi : fi - nfx, i = cl % nx, j = cl / nx;
     const int cr = axis == 0 ? j * nx + (i + 1) % nx : (j + 1) * nx + i;
@@ -881,7 +889,7 @@ __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers
         c.u = t.u; c.v = t.v; c.ux = o[13]; c.vy = o[14]; c.ckh = t.ckh; c.l2 = 2.0 * o[15];
         c.qx = o[17]; c.qy = o[18]; c.mt0 = o[35]; c.mt3 = o[38]; c.mt4 = o[39];
         c.kq = o[35] * o[16]; c.kb = c.kq * (2.0 / (double)P.ck);
-        auto poly = [&](const double td[4], double* p) {
+        auto poly = [&](const double* td, double* p) {
             p[0] = td[0] * t.ir - td[3] * t.itw;
             p[1] = 2.0 * t.itw * td[1];
             p[2] = 2.0 * t.itw * td[2];
@@ -901,7 +909,9 @@ __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers
 #pragma unroll
         for (int m = 0; m < 4; ++m) x[m] = o[36] * o[23 + m];
         poly(x, c.d[1]);
+        poly(o + 31, c.m);
     }
+    if (tid < 96) s_time[tid / 12][tid % 12] = 0.0;
     for (int q = tid; q < 3 * (nu + nw); q += blockDim.x) {
         const int g = q / (nu + nw), a = q - g * (nu + nw);
         const double* o = fs + g * kS2FScal + 1;
@@ -923,7 +933,8 @@ __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers
     double* Fw = (axis == 0 ? B.fxw : B.fyw) + out * 4;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     int bad = 0;
-    for (int k0 = tid; k0 < nv; k0 += 4 * (int)blockDim.x) {
+    for (int kb = 0; kb < nv; kb += 4 * (int)blockDim.x) {   // every lane, for the warps' sums
+        const int k0 = kb + tid;
         double fh[4], fb[4], uk[4], vk[4];
         int iu[4], iv[4];
 #pragma unroll
@@ -938,6 +949,7 @@ __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers
 #pragma unroll 1
         for (int g = 0; g < 3; ++g) {
             const S2FluxC& c = sc[g];
+            double mt[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const double vn = axis == 0 ? uk[r] : vk[r], vt = axis == 0 ? vk[r] : uk[r];
@@ -956,7 +968,13 @@ __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers
                 const double wn = gw[g] * vn;
                 fh[r] += wn * (q * vh + c.mt3 * f0h - c.mt4 * ph);
                 fb[r] += wn * (c.ckh * q * vb + c.mt3 * f0b - c.mt4 * pb);
+                asm volatile("" ::: "memory");   // the node's scalars are read again: held across the velocities they spilled
+                const int k = k0 + r * (int)blockDim.x;
+                const double pm = c.m[0] + c.m[1] * cx + c.m[2] * cy + c.m[3] * c2;
+                moment_add(k < nv ? B.w[k] : 0.0, uk[r], vk[r], q * pm, c.ckh * q * (pm + c.m[4]), mt);
             }
+            const double t = warp_halving<4, false>(mt);
+            if ((tid & 7) == 0) s_time[tid >> 5][4 * g + ((tid & 31) >> 3)] += t;
         }
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -972,6 +990,13 @@ __global__ void __launch_bounds__(256, 2) k_s2_face_flux_t(LoParams P, LoBuffers
         }
     }
     block_reduce_smem<4, 0>(acc, red, rout);
+    if (tid < 12) {   // the time directions' gate, as in k_s2_face_flux
+        const double* wt = fs + (tid >> 2) * kS2FScal + 40;
+        double t = s_time[0][tid];
+        for (int w = 1; w < (int)blockDim.x / 32; ++w) t += s_time[w][tid];
+        const double scl = fmax(fmax(fmax(fabs(wt[0]), fabs(wt[1])), fmax(fabs(wt[2]), fabs(wt[3]))), 1.0);
+        if (!(fabs(t - wt[tid & 3]) / scl <= 2.0e-12)) bad = 1;
+    }
     bad = __syncthreads_or(bad);
     if (tid < 4) Fw[tid] = rout[tid];
     if (tid == 0 && bad) set_status(B.status, ST_NONFINITE_FLUX);
@@ -1493,7 +1518,7 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
             else if (n <= 48) k_s2_target_nodes_t<6><<<g, 128, 0, ts>>>(P, B, S);
             else k_s2_target_nodes_t<8><<<g, 128, 0, ts>>>(P, B, S);
             const int nt = std::min(256, (nv + 127) / 128 * 32);
-            if (which != 5) k_s2_target_sum_t<<<dim3((unsigned)((nv + 1023) / 1024), (unsigned)nc), nt, 0, ts>>>(P, B, S);
+            if (which != 5) k_s2_target_sum_t<<<(unsigned)nc, nt, 0, ts>>>(P, B, S);
             e = cudaGetLastError();
         } else {
             const int qb = qrec_bytes(S, nv, 256, kQRecCap256x2);

@@ -248,24 +248,30 @@ __device__ bool t_closure(const LoParams& P, const LoBuffers& B, const double w[
     return ok;
 }
 
-// J x - rhs in the largest component (the moments left by a direction of the closure)
-__device__ __forceinline__ double t_left(const double* jac, const double x[4], const double rhs[4]) {
-    double mx = 0.0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        double s = -rhs[r];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) s = s + jac[r * 4 + a] * x[a];
-        mx = fmax(mx, fabs(s));
-    }
-    return mx;
+// moments of a closure direction td (s2_dq over the velocities) by the 1-D sums about (ux, vy): a sum of its own, about
+// another centre than the Jacobian's, so a gate on it tests the Jacobian and the solve
+__device__ __noinline__ void t_direction(const TAxes* ax, const S2Th* th, double ux, double vy, const double* td, double* m) {
+    const S2Th& t = *th;
+    const double dx = ux - t.u, dy = vy - t.v, ab = td[3] * t.itw, p3 = ab * t.itw;
+    const double a1 = 2.0 * t.itw * td[1], a2 = 2.0 * t.itw * td[2];
+    const double p0 = td[0] * t.ir - ab + a1 * dx + a2 * dy + p3 * (dx * dx + dy * dy), p1 = a1 + 2.0 * p3 * dx, p2 = a2 + 2.0 * p3 * dy;
+    auto S = [&](int a, int b) { return ax->x[a] * ax->y[b]; };
+    const double s00 = S(0, 0), s10 = S(1, 0), s01 = S(0, 1), s11 = S(1, 1), s20 = S(2, 0), s02 = S(0, 2);
+    const double c20 = s20 + s02, c30 = S(3, 0) + S(1, 2), c03 = S(2, 1) + S(0, 3), c40 = S(4, 0) + 2.0 * S(2, 2) + S(0, 4);
+    const double m0 = p0 * s00 + p1 * s10 + p2 * s01 + p3 * c20, mx = p0 * s10 + p1 * s20 + p2 * s11 + p3 * c30;
+    const double my = p0 * s01 + p1 * s11 + p2 * s02 + p3 * c03, m2 = p0 * c20 + p1 * c30 + p2 * c03 + p3 * c40;
+    m[0] = t.pref * m0;
+    m[1] = t.pref * (ux * m0 + mx);
+    m[2] = t.pref * (vy * m0 + my);
+    m[3] = t.pref * (0.5 * (ux * ux + vy * vy) * m0 + ux * mx + vy * my + 0.5 * m2 + 0.5 * t.ckh * (m0 + ab * s00));
 }
 
 // make_mke_prepared (mod_S2D1.f90:111-151) at the closure C of w: the primitive scalars and the closure
 // directions of the raw Shakhov terms, whose moments come from 1-D sums about the state's mean.  Lane 0
 // of the group solves for K_x, lane 1 (the axes exchanged) for K_y; lanes 2..4 solve for three further
 // right-hand sides extra[0..11] when given (the macro slopes of a face node) and return their own solution
-// in td.  Returns the gates: M's moments equal w, every direction's moments are met to 2e-12, all finite.
+// in td.  Returns the gates: M's moments equal w, the moments that every direction leaves, summed anew, are below 2e-12
+// (K's as they stand, the others relative to theirs), all finite.
 template <int R>
 __device__ bool t_mke(const LoParams& P, const LoBuffers& B, const double w[4], const TClosure& C, WMke& M,
                       const double* extra, double td[4]) {
@@ -304,7 +310,11 @@ __device__ bool t_mke(const LoParams& P, const LoBuffers& B, const double w[4], 
     if (mine)
 #pragma unroll
         for (int m = 0; m < 4; ++m) sc = fmax(sc, fabs(rhs[m]));
-    ok = ok && t_left(C.jac, td, rhs) / sc <= 2.0e-12;
+    double mom[4], left = 0.0;
+    t_direction(&ax, &t, M.ux, M.vy, td, mom);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) { left = fmax(left, fabs(rhs[m] - mom[m])); ok = ok && isfinite(mom[m]); }
+    ok = ok && left / sc <= 2.0e-12;
 #pragma unroll
     for (int m = 0; m < 4; ++m) { M.tdx[m] = t_get(td[m], 0); M.tdy[m] = t_get(td[m], 1); }
     const unsigned grp = 0xffu << ((threadIdx.x & 31) & ~(kTG - 1));
@@ -315,6 +325,9 @@ __device__ bool t_mke(const LoParams& P, const LoBuffers& B, const double w[4], 
 // build_targets' sums (mod_S2D1.f90:1246-1300) of one cell in shared memory: its 9 nodes' Maxwellians as products of two
 // rows of exponentials (the Gauss weight and rho / (pi T) folded into the x row), and M, K_x, K_y the product times a
 // cubic in the velocity whose coefficients are the node's.
+// make_mke's gate on the moments of K_x and K_y (2e-12) is taken here on the sums over the nodes, by the kernels that form
+// them, with every velocity's own rounding; each node's is t_mke's, by 1-D sums.  Per node and velocity it cost 4 % of a step.
+constexpr double kTGate = 2.0e-12;
 struct STargetNode {   // mean of theta, mean of the state, ck T / 2, the cubic's coefficients
     double u, v, ux, vy, ckh, sl, s0, kb;   // Shakhov factor sl c^2 - s0; kb = 2 coeff / ck
     double x[5], y[5];                      // direction polynomial 1, cx, cy, c^2 of K_x and K_y, and its b part

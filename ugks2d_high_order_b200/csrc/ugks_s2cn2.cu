@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_cn_collide(LoParams P, LoBuffe
     }
     const double beta = sc[0], ux = sc[1], vy = sc[2];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) acc[m] = 0.0;
+    for (int m = 0; m < 16; ++m) acc[m] = 0.0;
 #pragma unroll
     for (int r = 0; r < VPT; ++r) {
         const Slot s = slot(r, nv);
@@ -189,8 +189,13 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_cn_collide(LoParams P, LoBuffe
         heat_add(wk, cx, cy, T[r][0], T[r][1], acc + 2);
         heat_add(wk, cx, cy, T[r][2], T[r][3], acc + 4);   // kappa(:,1) of build_targets
         heat_add(wk, cx, cy, T[r][4], T[r][5], acc + 6);   // kappa(:,2)
+        if (TENSOR) {   // the moments of K_x and K_y, for their gate
+            moment_add(wk, uk, vk, T[r][2], T[r][3], acc + 8);
+            moment_add(wk, uk, vk, T[r][4], T[r][5], acc + 12);
+        }
     }
-    block_reduce_smem<8, 0>(acc, red, rout);
+    block_reduce_smem<TENSOR ? 16 : 8, 0>(acc, red, rout);
+    if (TENSOR && tid >= 8 && tid < 16 && !(fabs(rout[tid]) <= kTGate)) set_status(B.status, ST_PROJECTION);
     if (tid == 0) {
         const double rhs0 = rout[0] - rout[2], rhs1 = rout[1] - rout[3];
         double a11 = -beta * rout[4], a21 = -beta * rout[5], a12 = -beta * rout[6], a22 = -beta * rout[7];
