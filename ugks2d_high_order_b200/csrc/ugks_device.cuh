@@ -286,12 +286,12 @@ __device__ __forceinline__ void warp_max_all(double* v) {
 // Compensated summation.  two_sum (Knuth, TAOCP vol. 2, 4.2.2): s = fl(a + b) and the exact rounding error
 // e = a + b - s, in either argument order.  A compensated sum carries (s, c): every term enters s through
 // two_sum and its error into c (Neumaier's form of Kahan summation); the sum is s + c.
-__device__ __forceinline__ void two_sum(double a, double b, double& s, double& e) {
+__host__ __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e) {
     s = a + b;
     const double bb = s - a;
     e = (a - (s - bb)) + (b - bb);
 }
-__device__ __forceinline__ void comp_add(double& s, double& c, double x) {
+__host__ __device__ __forceinline__ void comp_add(double& s, double& c, double x) {
     double t, e;
     two_sum(s, x, t, e);
     s = t;

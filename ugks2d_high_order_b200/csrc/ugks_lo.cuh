@@ -106,8 +106,26 @@ __device__ __forceinline__ Slot slot(int r, int nv) {
 // w[k] = wx_i wy_j to within 4 units in the last place, the rounding of a product whose factors are
 // themselves recovered from the products (the S2 closures use the factors: a table of rounded decimal weights that
 // misses this keeps the general kernels).  On success tab holds u, wx, v, wy, each padded to 64 with its last
-// abscissa and weight 0, and the weights of the axes' halves (LoBuffers::tab).  Host only.
+// abscissa and weight 0, and the weights of the axes' halves (LoBuffers::tab).  tensor_table on the host and the scan of
+// the allocation-free entry point on the device apply one rule with one arithmetic, so that a table takes the same
+// kernels through both: the factors, up to their common scale, are two alternations of means of the ratios, each
+// weight's rounding averaged out, the sums compensated so that a factor is right to about an ulp.
 constexpr int kTensorTab = 8 * 64;
+// the factor of one abscissa: the mean of its n weights (stride apart) over the other axis's factors
+__host__ __device__ inline double tensor_factor(const double* w, int n, int stride, const double* other) {
+    double t = 0.0, c = 0.0;
+    for (int k = 0; k < n; ++k) comp_add(t, c, w[(size_t)k * stride] / other[k]);
+    return (t + c) / (double)n;
+}
+// whether the weight is its factors' product, rounded (never a fused product and difference), to 4 units in the last place
+__host__ __device__ inline bool tensor_weight(double fx, double fy, double w) {
+#ifdef __CUDA_ARCH__
+    const double p = __dmul_rn(fx, fy), d = __dsub_rn(p, w);
+#else
+    const double p = fx * fy, d = p - w;
+#endif
+    return fabs(d) <= 4.0 * 2.220446049250313e-16 * w;
+}
 inline bool tensor_table(int nv, const double* u, const double* v, const double* w, int* nu_out, int* nv_out,
                          double tab[kTensorTab]) {
     int nu = 1;
@@ -119,36 +137,24 @@ inline bool tensor_table(int nv, const double* u, const double* v, const double*
         if (!(u[k] == u[k % nu] && v[k] == v[k - k % nu])) return false;
         if (!(w[k] > 0.0) || !std::isfinite(w[k]) || !std::isfinite(u[k]) || !std::isfinite(v[k])) return false;
     }
-    // factors up to their common scale: alternating weighted means of the ratios, each weight's rounding averaged out
-    long double fx[64], fy[64];
-    for (int j = 0; j < nj; ++j) fy[j] = (long double)w[j * nu] / (long double)w[0];
+    double fx[64], fy[64];
+    for (int j = 0; j < nj; ++j) fy[j] = w[(size_t)j * nu] / w[0];
     for (int it = 0; it < 2; ++it) {
-        for (int i = 0; i < nu; ++i) {
-            fx[i] = 0.0L;
-            for (int j = 0; j < nj; ++j) fx[i] += (long double)w[j * nu + i] / fy[j];
-            fx[i] /= (long double)nj;
-        }
-        for (int j = 0; j < nj; ++j) {
-            fy[j] = 0.0L;
-            for (int i = 0; i < nu; ++i) fy[j] += (long double)w[j * nu + i] / fx[i];
-            fy[j] /= (long double)nu;
-        }
+        for (int i = 0; i < nu; ++i) fx[i] = tensor_factor(w + i, nj, nu, fy);
+        for (int j = 0; j < nj; ++j) fy[j] = tensor_factor(w + (size_t)j * nu, nu, 1, fx);
     }
     for (int a = 0; a < 64; ++a) {
         tab[a] = u[std::min(a, nu - 1)];
-        tab[64 + a] = a < nu ? (double)fx[a] : 0.0;
+        tab[64 + a] = a < nu ? fx[a] : 0.0;
         tab[128 + a] = v[(size_t)std::min(a, nj - 1) * nu];
-        tab[192 + a] = a < nj ? (double)fy[a] : 0.0;
+        tab[192 + a] = a < nj ? fy[a] : 0.0;
         tab[256 + a] = tab[a] >= 0.0 ? tab[64 + a] : 0.0;
         tab[320 + a] = tab[a] >= 0.0 ? 0.0 : tab[64 + a];
         tab[384 + a] = tab[128 + a] >= 0.0 ? tab[192 + a] : 0.0;
         tab[448 + a] = tab[128 + a] >= 0.0 ? 0.0 : tab[192 + a];
     }
-    for (int j = 0; j < nj; ++j)
-        for (int i = 0; i < nu; ++i) {
-            const double x = w[j * nu + i];
-            if (!(std::fabs(tab[64 + i] * tab[192 + j] - x) <= 4.0 * 2.220446049250313e-16 * x)) return false;
-        }
+    for (int k = 0; k < nv; ++k)
+        if (!tensor_weight(fx[k % nu], fy[k / nu], w[k])) return false;
     *nu_out = nu;
     *nv_out = nj;
     return true;

@@ -86,8 +86,8 @@ Plan plan_for(int nx, int ny, int nv) {
 }
 
 // One CTA over the velocity table: U_MAX and V_MAX (InitVelocityFromStructuredFile, mod_InitializeFlow.f90:508), and
-// whether it is a tensor product, by tensor_table's rule (the factors as means of the ratios, two alternations): then
-// out[2], out[3] are its abscissae per axis and tab its axes.  One launch and one small copy instead of two copies of the table.
+// whether it is a tensor product, by tensor_table's rule and arithmetic: then out[2], out[3] are its abscissae per axis and
+// tab its axes.  One launch and one small copy instead of two copies of the table.
 constexpr int kScanThreads = 256;
 __global__ void __launch_bounds__(kScanThreads) k_table_scan(const double* u, const double* v, const double* w, int nv, double* out,
                                                              double* tab) {
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kScanThreads) k_table_scan(const double* u, co
     for (int k = tid; k < nv; k += kScanThreads) {
         m[0] = fmax(m[0], u[k]);
         m[1] = fmax(m[1], v[k]);
-        if (v[k] != v[0]) atomicMin(&s_nu, k);
+        if (k > 0 && !(v[k] == v[0])) atomicMin(&s_nu, k);   // (v[0] itself may compare unequal: not a number)
     }
     warp_max_all<2>(m);
     if ((tid & 31) == 0) { mx[0][tid >> 5] = m[0]; mx[1][tid >> 5] = m[1]; }
@@ -113,26 +113,15 @@ __global__ void __launch_bounds__(kScanThreads) k_table_scan(const double* u, co
             if (!(u[k] == u[i] && v[k] == v[k - i] && w[k] > 0.0 && isfinite(w[k]) && isfinite(u[k]) && isfinite(v[k]))) s_bad = 1;
         }
         if (tid < nj) fy[tid] = w[tid * nu] / w[0];
-        // compensated means: the factors to an ulp, as the rule's 4 ulp for their product needs
         for (int it = 0; it < 2; ++it) {
             __syncthreads();
-            if (tid < nu) {
-                double t = 0.0, c = 0.0;
-                for (int j = 0; j < nj; ++j) comp_add(t, c, w[j * nu + tid] / fy[j]);
-                fx[tid] = (t + c) / (double)nj;
-            }
+            if (tid < nu) fx[tid] = tensor_factor(w + tid, nj, nu, fy);
             __syncthreads();
-            if (tid < nj) {
-                double t = 0.0, c = 0.0;
-                for (int i = 0; i < nu; ++i) comp_add(t, c, w[tid * nu + i] / fx[i]);
-                fy[tid] = (t + c) / (double)nu;
-            }
+            if (tid < nj) fy[tid] = tensor_factor(w + tid * nu, nu, 1, fx);
         }
         __syncthreads();
-        for (int k = tid; k < nv; k += kScanThreads) {
-            const int i = k % nu, j = k / nu;
-            if (!(fabs(fx[i] * fy[j] - w[k]) <= 4.0 * kEps * w[k])) s_bad = 1;
-        }
+        for (int k = tid; k < nv; k += kScanThreads)
+            if (!tensor_weight(fx[k % nu], fy[k / nu], w[k])) s_bad = 1;
         if (tid < 64) {
             const double xu = u[min(tid, nu - 1)], xv = v[min(tid, nj - 1) * nu], a = tid < nu ? fx[tid] : 0.0, b = tid < nj ? fy[tid] : 0.0;
             tab[tid] = xu; tab[64 + tid] = a; tab[128 + tid] = xv; tab[192 + tid] = b;
