@@ -408,20 +408,6 @@ __device__ __forceinline__ void weno_points_vjp(const double q[5], const int pts
     weno_points_vjp<NP>(w, x, pts, gval, gder, gq);
 }
 
-// s2_companion3 with the weights' intermediates kept for companion3_vjp (the same values bit for bit)
-__device__ __forceinline__ bool companion3_fwd(const double q[5], const double comp[5], double val[3], double der[3],
-                                               double cval[3], S2Weno& w, S2WenoX& x) {
-    if (!s2_weno_x<true>(q, w, &x)) return false;
-    bool ok = true;
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {
-        s2_at(w, S2_G0 + s, val[s], der[s]);
-        cval[s] = s2_cand_sum(w.fw, comp, c_s2p.E[S2_G0 + s]);
-        ok = ok && isfinite(val[s]) && isfinite(der[s]) && isfinite(cval[s]);
-    }
-    return ok;
-}
-
 // transpose of companion_eval3 (s2_companion3): val[s], der[s] of the interpolant of q and cval[s] of the
 // companion samples with q's weights, at the 3 Gauss nodes
 __device__ __forceinline__ void companion3_vjp(const S2Weno& w, const S2WenoX& x, const double comp[5],
@@ -1881,7 +1867,7 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffer
     if (p < 2) {
 #pragma unroll
         for (int r = 0; r < 5; ++r) { a5[r] = X(r, 2 * p); b5[r] = X(r, 2 * p + 1); }
-        if (!nw) companion3_fwd(a5, b5, face, dt, dn, wf, xf);
+        if (!nw) s2_companion3_x(a5, b5, face, dt, dn, wf, xf);
         else {
             double dummy;
 #pragma unroll
@@ -1908,16 +1894,13 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffer
                 s2_wall_eval(q, j, ny, s == 0 ? -0.5 : 0.5, a5[r + 2], b5[r + 2]);
             }
         }
-        companion3_fwd(a5, b5, face, dt, dn, wf, xf);
+        s2_companion3_x(a5, b5, face, dt, dn, wf, xf);
     }
     if (p < 3) {
 #pragma unroll
         for (int r = 0; r < 5; ++r) c5[r] = X(r, 4 + p);
         if (!nw) {
-            S2Weno ww;
-            s2_weno(c5, ww);
-#pragma unroll
-            for (int b = 0; b < 3; ++b) vol[b] = s2_at_v(ww, S2_G0 + b);
+            s2_power_values3(c5, vol);
         } else {
             double dummy;
 #pragma unroll
@@ -2067,7 +2050,7 @@ __global__ void __launch_bounds__(128, 5) k_adj_recon2(LoParams P, LoBuffers B, 
             b5[r] = l[(size_t)(q0 + 1) * nv];
             o5[r] = l[(size_t)q1 * nv];
         }
-        companion3_fwd(a5, b5, face, dt, dn, wf, xf);
+        s2_companion3_x(a5, b5, face, dt, dn, wf, xf);
         s2_power_values3(o5, v3);
 #pragma unroll
         for (int a = 0; a < 3; ++a) { sample(face[a], a); sample(v3[a], 3 + a); }

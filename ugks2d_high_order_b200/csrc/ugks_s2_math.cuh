@@ -231,6 +231,15 @@ __device__ __forceinline__ void s2_power_values3(const double q[5], double val[3
     s2_gauss_values(c, val);
 }
 
+// s2_power_companion3 for the adjoint, which needs the weights and their intermediates for the transpose as well.  The values
+// are the forward's, in its form: the positivity limiter takes its smallest sample from them, and where a cell's mean is
+// as small as its neighbours' roundings another form's values would pick another sample or none.
+__device__ __forceinline__ void s2_companion3_x(const double q[5], const double comp[5], double val[3], double der[3],
+                                                double cval[3], S2Weno& w, S2WenoX& x) {
+    s2_weno_x<true>(q, w, &x);
+    s2_power_companion3(q, comp, val, der, cval);
+}
+
 // companion_eval3 (:287-318): the weights of q applied to the companion samples comp as well
 __device__ __forceinline__ bool s2_companion3(const double q[5], const double comp[5], double val[3], double der[3],
                                               double cval[3]) {
