@@ -1574,7 +1574,7 @@ extern "C" int ugks_s2cn2_backward(ugks_ctx* c, const double* seed, double* grad
                 const S2Buffers Sm = with_record(c, slot_targets(c, a), m);
                 UGKS_CK(enqueue_s2cn2_adjoint(c->P, slot_lo(c, a), Sm, Sm, with_record(c, slot_targets(c, b), m),
                                               record_cn(c, Cr, m), A, c->stream, c->stream2, c->adj_ev));
-                c->launches += kAdjStepKernels;
+                c->launches += adj_step_kernels(c->P);
                 cur = 1 - cur;
             }
         } else {
@@ -1593,7 +1593,7 @@ extern "C" int ugks_s2cn2_backward(ugks_ctx* c, const double* seed, double* grad
                 const bool last = q == nckpt - 1 && m == len - 1;
                 const AdjBuffers A = adj_bind(c, cur, last ? c->adj_seed : nullptr);
                 UGKS_CK(enqueue_s2cn2_adjoint(c->P, Ba, c->T[0], Ta, c->T[1], Cr, A, c->stream, c->stream2, c->adj_ev));
-                c->launches += kAdjStepKernels;
+                c->launches += adj_step_kernels(c->P);
                 cur = 1 - cur;
             }
         }
@@ -1636,7 +1636,7 @@ extern "C" int ugks_s2cn2_step_vjp(ugks_ctx* c, const double* gh, const double* 
     UGKS_CK(enqueue_s2cn2_adjoint(c->P, B0, c->T[0], c->T[0], c->T[1], rerun_cn(c), A, c->stream, c->stream2, c->adj_ev));
     UGKS_CK(s2_enqueue(3, c->P, B0, c->T[1], c->stream, c->stream, nullptr, nullptr));   // W's targets, for their adjoint
     UGKS_CK(enqueue_targets_adjoint(c->P, B0, c->T[0], in.T, in.W, A, c->stream));
-    c->launches += kAdjStepKernels + s2_enqueue_kernels(3, c->P, c->T[1]) + 2;
+    c->launches += adj_step_kernels(c->P) + s2_enqueue_kernels(3, c->P, c->T[1]) + 2;
     if (int r = adj_status(c)) return r;
     return adj_download(c, in, gh_in, gb_in, gW_in, grad);
 }

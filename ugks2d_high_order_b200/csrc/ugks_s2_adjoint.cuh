@@ -58,6 +58,7 @@ cudaError_t enqueue_s2cn2_adjoint(const LoParams& P, const LoBuffers& B, const S
 // s2_enqueue(3)) added to gW.
 cudaError_t enqueue_targets_adjoint(const LoParams& P, const LoBuffers& B, const S2Buffers& S, double* const gT[6],
                                     double* gW, const AdjBuffers& A, cudaStream_t s);
-constexpr int kAdjStepKernels = 10;
+// kernels of enqueue_s2cn2_adjoint: the inner cells' second-layer transpose is there from seven rows on
+inline int adj_step_kernels(const LoParams& P) { return 10 + (P.ny > 6 ? 1 : 0); }
 
 }  // namespace ugks
