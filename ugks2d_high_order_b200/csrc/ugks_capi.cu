@@ -100,7 +100,7 @@ struct ugks_ctx {
     double* rmem = nullptr;        // per-step records of one segment: the scratch each step's adjoint reads
     unsigned* aflags = nullptr;    // [0..2] halt, counter, accepted of the re-runs, [3] adjoint status
     int adj_capacity_ckpt = 0, adj_capacity_seg = 0, adj_capacity_rec = 0;
-    cudaEvent_t adj_ev[4] = {nullptr, nullptr, nullptr, nullptr};   // the adjoint's fork / join points
+    cudaEvent_t adj_ev[3] = {nullptr, nullptr, nullptr};   // the adjoint's fork / join points
     double* ckpt = nullptr;        // [ckpt][h | b | W | ledger]
     double* seg = nullptr;         // [slot][h | b | W | 6 targets | ledger]
     double* cot[2] = {nullptr, nullptr};   // [h | b | W | 6 targets] cotangent sets
@@ -391,7 +391,7 @@ extern "C" int ugks_ctx_destroy(ugks_ctx* c) {
     if (c->amem) cudaFree(c->amem);
     if (c->bmem) cudaFree(c->bmem);
     if (c->rmem) cudaFree(c->rmem);
-    for (int q = 0; q < 4; ++q) if (c->adj_ev[q]) cudaEventDestroy(c->adj_ev[q]);
+    for (int q = 0; q < 3; ++q) if (c->adj_ev[q]) cudaEventDestroy(c->adj_ev[q]);
     if (c->aflags) cudaFree(c->aflags);
     if (c->cmem) cudaFree(c->cmem);
     if (c->cflags) cudaFree(c->cflags);
@@ -1367,7 +1367,7 @@ int adj_reserve_ckpt(ugks_ctx* c, int nckpt) {
 
 // the reverse sweep's work: nseg segment slots, the two cotangent sets and the adjoint's arrays
 int adj_reserve_bwd(ugks_ctx* c, int nseg) {
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < 3; ++q)
         if (!c->adj_ev[q]) UGKS_CK(cudaEventCreateWithFlags(&c->adj_ev[q], cudaEventDisableTiming));
     if (!c->aflags) {
         UGKS_CK(cudaMalloc(&c->aflags, 4 * sizeof(unsigned)));

@@ -1845,7 +1845,7 @@ __global__ void __launch_bounds__(256) k_adj_macro_faces(LoParams P, const doubl
 // of the rows / columns the templates read, and the state (the limiter's cell means, the wall rows' direct samples).
 //
 // k_adj_recon2_wall: the cells in the three rows next to a wall; CTA = 8 warps (field, part) over 32 velocities of one
-// cell.  Three CTAs per SM (80 registers with spills): measured 2.3 % faster over the backward than two at 128.
+// cell.  Three CTAs per SM (80 registers, 740 / 916 bytes of spills a thread): 2.3 % faster over the backward than two at 128.
 __global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
     __shared__ double s_th[8][32];
     __shared__ double s_gth[8][32];
@@ -1855,8 +1855,7 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffer
     const bool kok = k0 < nv;
     const int k = kok ? k0 : nv - 1;
     const int wrows = min(ny, 6), row = blockIdx.y / nx, i = blockIdx.y % nx, j = row < 3 ? row : ny - wrows + row, cc = j * nx + i;
-    const bool nw = s2_near_wall(j, ny);
-    const int first = nw ? s2_wall_first(j, ny) : j - 2;
+    const int first = s2_wall_first(j, ny);   // rows of the one-sided quartics across y
     const double* L1 = S.l1 + (size_t)f * 11 * nv + k;
     auto X = [&](int r, int q) { return L1[((size_t)((first + r) * nx + i) * 22 + q) * nv]; };
     const S2Field F{(f == 0 ? B.h : B.b) + k, nv, nx, ny};
@@ -1867,45 +1866,29 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffer
     if (p < 2) {
 #pragma unroll
         for (int r = 0; r < 5; ++r) { a5[r] = X(r, 2 * p); b5[r] = X(r, 2 * p + 1); }
-        if (!nw) s2_companion3_x(a5, b5, face, dt, dn, wf, xf);
-        else {
-            double dummy;
+        double dummy;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                s2_wall_eval(a5, j, ny, c_s2.gnode[a], face[a], dt[a]);
-                s2_wall_eval(b5, j, ny, c_s2.gnode[a], dn[a], dummy);
-            }
+        for (int a = 0; a < 3; ++a) {
+            s2_wall_eval(a5, j, ny, c_s2.gnode[a], face[a], dt[a]);
+            s2_wall_eval(b5, j, ny, c_s2.gnode[a], dn[a], dummy);
         }
     } else {
         const int s = p - 2;
-        if (!nw) {
 #pragma unroll
-            for (int r = 0; r < 5; ++r) {
-                const double* y = L1 + ((size_t)(j * nx + wrapx(i + r - 2, nx)) * 22 + 7 + 2 * s) * nv;
-                a5[r] = y[0];
-                b5[r] = y[(size_t)nv];
-            }
-        } else {
+        for (int r = -2; r <= 2; ++r) {
+            double q[5];
 #pragma unroll
-            for (int r = -2; r <= 2; ++r) {
-                double q[5];
-#pragma unroll
-                for (int t = 0; t < 5; ++t) q[t] = F.at(i + r, first + t);
-                s2_wall_eval(q, j, ny, s == 0 ? -0.5 : 0.5, a5[r + 2], b5[r + 2]);
-            }
+            for (int t = 0; t < 5; ++t) q[t] = F.at(i + r, first + t);
+            s2_wall_eval(q, j, ny, s == 0 ? -0.5 : 0.5, a5[r + 2], b5[r + 2]);
         }
         s2_companion3_x(a5, b5, face, dt, dn, wf, xf);
     }
     if (p < 3) {
 #pragma unroll
         for (int r = 0; r < 5; ++r) c5[r] = X(r, 4 + p);
-        if (!nw) {
-            s2_power_values3(c5, vol);
-        } else {
-            double dummy;
+        double dummy;
 #pragma unroll
-            for (int b = 0; b < 3; ++b) s2_wall_eval(c5, j, ny, c_s2.gnode[b], vol[b], dummy);
-        }
+        for (int b = 0; b < 3; ++b) s2_wall_eval(c5, j, ny, c_s2.gnode[b], vol[b], dummy);
     }
     const double hm = B.h[(size_t)cc * nv + k], bm = B.b[(size_t)cc * nv + k];
     const double mf = f == 0 ? hm : bm;
@@ -1968,45 +1951,28 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffer
     atomic_add(gS + (size_t)cc * nv, gmf);
     double ga5[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, gb5[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (p < 2) {
-        if (!nw) companion3_vjp(wf, xf, b5, gface, gdt, gdn, ga5, gb5);
-        else
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                wall_eval_vjp(j, ny, c_s2.gnode[a], gface[a], gdt[a], ga5);
-                wall_eval_vjp(j, ny, c_s2.gnode[a], gdn[a], 0.0, gb5);
-            }
+        for (int a = 0; a < 3; ++a) {
+            wall_eval_vjp(j, ny, c_s2.gnode[a], gface[a], gdt[a], ga5);
+            wall_eval_vjp(j, ny, c_s2.gnode[a], gdn[a], 0.0, gb5);
+        }
 #pragma unroll
         for (int r = 0; r < 5; ++r) { atomic_add(gX(r, 2 * p), ga5[r]); atomic_add(gX(r, 2 * p + 1), gb5[r]); }
     } else {
         const int s = p - 2;
         companion3_vjp(wf, xf, b5, gface, gdt, gdn, ga5, gb5);
-        if (!nw) {
 #pragma unroll
-            for (int r = 0; r < 5; ++r) {
-                double* y = gL1 + ((size_t)(j * nx + wrapx(i + r - 2, nx)) * 22 + 7 + 2 * s) * nv;
-                atomic_add(y, ga5[r]);
-                atomic_add(y + nv, gb5[r]);
-            }
-        } else {
+        for (int r = -2; r <= 2; ++r) {
+            double gq[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+            wall_eval_vjp(j, ny, s == 0 ? -0.5 : 0.5, ga5[r + 2], gb5[r + 2], gq);
 #pragma unroll
-            for (int r = -2; r <= 2; ++r) {
-                double gq[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-                wall_eval_vjp(j, ny, s == 0 ? -0.5 : 0.5, ga5[r + 2], gb5[r + 2], gq);
-#pragma unroll
-                for (int t = 0; t < 5; ++t) atomic_add(gS + (size_t)((first + t) * nx + wrapx(i + r, nx)) * nv, gq[t]);
-            }
+            for (int t = 0; t < 5; ++t) atomic_add(gS + (size_t)((first + t) * nx + wrapx(i + r, nx)) * nv, gq[t]);
         }
     }
     if (p < 3 && (gvol[0] != 0.0 || gvol[1] != 0.0 || gvol[2] != 0.0)) {
         double gc5[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        if (!nw) {
-            const int pts[3] = {S2_G0, S2_G0 + 1, S2_G0 + 2};
-            const double zero3[3] = {0.0, 0.0, 0.0};
-            weno_points_vjp<3>(c5, pts, gvol, zero3, gc5);
-        } else {
 #pragma unroll
-            for (int b = 0; b < 3; ++b) wall_eval_vjp(j, ny, c_s2.gnode[b], gvol[b], 0.0, gc5);
-        }
+        for (int b = 0; b < 3; ++b) wall_eval_vjp(j, ny, c_s2.gnode[b], gvol[b], 0.0, gc5);
 #pragma unroll
         for (int r = 0; r < 5; ++r) atomic_add(gX(r, 4 + p), gc5[r]);
     }
@@ -2314,19 +2280,19 @@ static cudaError_t adj_launch(const LoParams& P, const LoBuffers& B, const S2Buf
     if (e == cudaSuccess) {
         if (P.tnu > 0) k_adj_face_nodes<true><<<warps((long long)nf * 3, 64), 64, 0, s>>>(P, B, S, A);
         else k_adj_face_nodes<false><<<warps((long long)nf * 3, 128), 128, 0, s>>>(P, B, S, A);
-        if (side) e = cudaEventRecord(ev[2], s);
+        if (side) e = cudaEventRecord(ev[1], s);
     }
-    if (e == cudaSuccess && side) e = cudaStreamWaitEvent(s2, ev[2], 0);
+    if (e == cudaSuccess && side) e = cudaStreamWaitEvent(s2, ev[1], 0);
     const dim3 grid((unsigned)((nv + 31) / 32), (unsigned)nc);
     if (e == cudaSuccess) {
         k_adj_macro_faces<<<(unsigned)((nf * 8 + 255) / 256), 256, 0, sw>>>(P, B.W, A.gmac, A.gWi);
         // the wall rows' cells after the wall nodes, whose sides they read, beside the others
         k_adj_recon2_wall<<<dim3(grid.x, (unsigned)((ny < 6 ? ny : 6) * nx)), 256, 0, sw>>>(P, B, S, A);
-        if (side) e = cudaEventRecord(ev[3], s2);
+        if (side) e = cudaEventRecord(ev[2], s2);
     }
     if (e == cudaSuccess) {
         if (ny > 6) k_adj_recon2<<<dim3(grid.x, (unsigned)((ny - 6) * nx)), 128, 0, s>>>(P, B, S, A);
-        if (side) e = cudaStreamWaitEvent(s, ev[3], 0);   // the wall rows; and gWi complete before the next step
+        if (side) e = cudaStreamWaitEvent(s, ev[2], 0);   // the wall rows; and gWi complete before the next step
     }
     if (e == cudaSuccess) {
         const unsigned kb = (unsigned)((nv + 31) / 32);
