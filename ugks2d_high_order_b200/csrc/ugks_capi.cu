@@ -180,6 +180,9 @@ static int check_wall_variant(const ugks_params* p) {
     return UGKS_OK;
 }
 
+// the second-order kernels of tensor-product velocity tables (ugks_lo_tensor.cu), on Explicit contexts
+static bool lo_tensor(const ugks_ctx* c) { return c->P.tnu > 0 && c->prm.method == UGKS_METHOD_EXPLICIT; }
+
 extern "C" int ugks_ctx_create(const ugks_params* p, const double* u, const double* v, const double* w, int device,
                                ugks_ctx** out) {
     if (!p || !u || !v || !w || !out) return UGKS_EINVAL;
@@ -199,6 +202,8 @@ extern "C" int ugks_ctx_create(const ugks_params* p, const double* u, const doub
     double umax = -INFINITY, vmax = -INFINITY;
     for (int k = 0; k < nv; ++k) { umax = std::fmax(umax, u[k]); vmax = std::fmax(vmax, v[k]); }
     c->P = make_lo_params(*p, umax, vmax);
+    double tab[kTensorTab];
+    if (!tensor_table(nv, u, v, w, &c->P.tnu, &c->P.tnv, tab)) c->P.tnu = c->P.tnv = 0;
 
     // buffer plan (doubles)
     const size_t S = (size_t)nc * nv, SY = (size_t)(ny + 1) * nx * nv;
@@ -206,7 +211,8 @@ extern "C" int ugks_ctx_create(const ugks_params* p, const double* u, const doub
     auto take = [&](size_t n) { size_t o = off; off += (n + 31) / 32 * 32; return o; };
     const size_t o_u = take(nv), o_v = take(nv), o_w = take(nv), o_tab = take(kTensorTab);
     const size_t o_h = take(S), o_b = take(S), o_W = take((size_t)nc * 4);
-    const size_t o_sxh = take(S), o_syh = take(S), o_sxb = take(S), o_syb = take(S);
+    const size_t SL = lo_tensor(c) ? 0 : S;   // the tensor kernels form the slopes on the way
+    const size_t o_sxh = take(SL), o_syh = take(SL), o_sxb = take(SL), o_syb = take(SL);
     const size_t o_fxh = take(S), o_fxb = take(S), o_fxw = take((size_t)nc * 4);
     const size_t o_fyh = take(SY), o_fyb = take(SY), o_fyw = take((size_t)(ny + 1) * nx * 4);
     const size_t o_rw = take((size_t)nc * 4), o_rh = take(S), o_rb = take(S);
@@ -234,11 +240,7 @@ extern "C" int ugks_ctx_create(const ugks_params* p, const double* u, const doub
     B.peq_h = d + o_eh; B.peq_b = d + o_eb; B.pcol_h = d + o_ch; B.pcol_b = d + o_cb;
     B.dtl = d + o_dtl; B.dt = d + o_dt; B.cell_diag = d + o_cd; B.diag = d + o_dg; B.wall_aero = d + o_wa;
     B.counter = c->dflags; B.status = c->dflags + 1;
-    double tab[kTensorTab];
-    if (tensor_table(nv, u, v, w, &c->P.tnu, &c->P.tnv, tab))
-        e = cudaMemcpyAsync(d + o_tab, tab, sizeof tab, cudaMemcpyHostToDevice, c->stream);
-    else
-        c->P.tnu = c->P.tnv = 0;
+    if (c->P.tnu > 0) e = cudaMemcpyAsync(d + o_tab, tab, sizeof tab, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d + o_u, u, nv * sizeof(double), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d + o_v, v, nv * sizeof(double), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d + o_w, w, nv * sizeof(double), cudaMemcpyHostToDevice, c->stream);
@@ -562,9 +564,6 @@ static int s2_evolution(ugks_ctx* c, bool rebuild_targets) {
 static bool is_s2(const ugks_ctx* c) {
     return c->prm.method == UGKS_METHOD_S2CN2 || c->prm.method == UGKS_METHOD_HIGH_ORDER_IMPLICIT;
 }
-
-// the second-order kernels of tensor-product velocity tables (ugks_lo_tensor.cu), on Explicit contexts
-static bool lo_tensor(const ugks_ctx* c) { return c->P.tnu > 0 && c->prm.method == UGKS_METHOD_EXPLICIT; }
 
 extern "C" int ugks_evolution(ugks_ctx* c) {
     if (!c) return UGKS_EINVAL;
