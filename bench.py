@@ -14,11 +14,11 @@ itself prescribes), no dataset is involved.
                  from pinned host memory, runs to the gate and downloads the final state.
   roofline       the dominant stage of the pseudo-step (per-stage CUDA events in a separate
                  profiling pass, same stream) against its algorithmic bytes.
-  fp64           (in roofline and in each method's object) algorithmic FP64 operations per update
-                 (counted by oracle/count_flops.py) x updates/s, against a cuBLAS float64 GEMM
-                 measured in the same run.  The count is the reference's formulation's: on tensor-product
-                 velocity tables the kernels need fewer operations for the same update, so the fraction
-                 compares the rate of finished work with the GEMM and may pass 1.
+  fp64           algorithmic FP64 operations per update (counted by oracle/count_flops.py: the reference's
+                 formulation's) x updates/s, beside a cuBLAS float64 GEMM measured in the same run.  In the
+                 roofline, whose kernels do those operations, also as a fraction of it; in the other
+                 methods' objects the kernels need fewer for the same update (tensor-product velocity
+                 tables), so there it is a rate of finished work and no fraction is formed.
   cpu_baseline   the C oracle (a restatement of the reference's Fortran; the Fortran itself does not
                  build on this image) timed on a bounded number of pseudo-steps of the same case.
   explicit_plain the plain second-order Explicit step (1000 steps, CFL 0.5, omega 0.81) for context.
@@ -114,7 +114,7 @@ def peaks():
 
 def fp64_peak(device):
     """FP64 throughput of this GPU in TFLOP/s: a cuBLAS float64 GEMM (8192^3) through torch, the
-    denominator of the FP64 fractions (B200's nominal FP64 and FP64 tensor peaks are both 37 TFLOP/s)."""
+    denominator of the FP64 fraction (B200's nominal FP64 and FP64 tensor peaks are both 37 TFLOP/s)."""
     import torch
     n = 8192
     a = torch.randn(n, n, dtype=torch.float64, device=device)
@@ -134,10 +134,18 @@ def fp64_peak(device):
 
 
 def fp64_fraction(flops_per_update, updates_per_s, peak_tflops):
+    """For kernels that do the counted operations."""
     achieved = flops_per_update * updates_per_s / 1e12
     return {"flops_per_update": flops_per_update, "achieved_tflops": achieved, "peak_tflops": peak_tflops,
-            "frac": achieved / peak_tflops, "peak_source": "cuBLAS float64 GEMM 8192^3 measured in this run",
-            "counted": "the reference formulation's operations; the kernels need fewer on tensor-product tables"}
+            "frac": achieved / peak_tflops, "peak_source": "cuBLAS float64 GEMM 8192^3 measured in this run"}
+
+
+def fp64_reference_work(flops_per_update, updates_per_s, gemm_tflops):
+    """For kernels that finish the same update with fewer operations: the reference formulation's operations in the
+    time taken, which is no rate of the hardware and no fraction of its peak."""
+    return {"reference_flops_per_update": flops_per_update, "reference_work_tflops": flops_per_update * updates_per_s / 1e12,
+            "gemm_tflops": gemm_tflops, "gemm_source": "cuBLAS float64 GEMM 8192^3 measured in this run",
+            "counted": "the reference formulation's operations; the kernels do fewer on tensor-product tables"}
 
 
 class ClockSampler:
@@ -674,7 +682,7 @@ def main():
                 "config": "Explicit 8x64x1024, CFL 0.5, omega 0.81, 1000 steps from the cold start, CUDA graphs",
                 "kernel_avg_us": {k: 1e3 * t / max(n, 1) for k, (t, n) in kt.items()},
                 "faces_roofline_frac": (BYTES_PER_UPDATE_EXPLICIT * nc * nv / (kt["faces"][0] / kt["faces"][1] * 1e-3) / 1e9) / peak}
-    explicit["fp64"] = fp64_fraction(FLOPS_PER_UPDATE["explicit"], explicit["value"], fpk)
+    explicit["fp64"] = fp64_reference_work(FLOPS_PER_UPDATE["explicit"], explicit["value"], fpk)
 
     # ---------------- HighOrderImplicit: the cold start to the 3000 pseudo-step cap (the reference run
     # also stops at its iteration limit, analysis.json high_implicit status)
@@ -698,7 +706,7 @@ def main():
                   "c_minus_1": float(rep_h[52]), "science_1_4": [float(x) for x in rep_h[12:16]],
                   "Rh_Rb": [float(rep_h[24]), float(rep_h[25])],
                   "hbm_roofline_frac": BYTES_PER_UPDATE_PSEUDO_STEP * ho_value / 1e9 / peak,
-                  "fp64": fp64_fraction(FLOPS_PER_UPDATE["high_order_implicit"], ho_value, fpk),
+                  "fp64": fp64_reference_work(FLOPS_PER_UPDATE["high_order_implicit"], ho_value, fpk),
                   "config": "HighOrderImplicit 8x64x1024 (WENO5-AO S2 evolution, PR2 + LU-SGS, 8 slabs), CFL 0.1, "
                             "nCFL 1000, mass rescale on, cold start, 3000 pseudo-step cap; FP64-bound (the "
                             "closures and WENO templates), so the HBM fraction is small by construction"}
@@ -747,7 +755,7 @@ def main():
     s2cn2 = {"value": cn_value, "unit": UNIT, "steps": int(done_c2), "ms_per_step": cms / max(done_c2, 1),
              "cnres": float(rep_c2[1]), "mmerr": float(rep_c2[2]), "drift": float(rep_c2[9]),
              "hbm_roofline_frac": BYTES_PER_UPDATE_EXPLICIT * cn_value / 1e9 / peak,
-             "fp64": fp64_fraction(FLOPS_PER_UPDATE["s2cn2"], cn_value, fpk),
+             "fp64": fp64_reference_work(FLOPS_PER_UPDATE["s2cn2"], cn_value, fpk),
              "config": "S2CN2 8x64x1024, CFL 0.1, 8 steps warm-up then 400 steps, two steps per CUDA graph; "
                        "FP64-bound"}
     # the research wall variants of the same step (FluxWall_type 0; W1T; W1T + W1D; W2R at Pr 1)
@@ -804,7 +812,7 @@ def main():
                "steps": BATCH_STEPS, "ms_per_batched_step": bms / BATCH_STEPS, "streams": int(k_tuned),
                "all_accepted": bool((bdone == BATCH_STEPS).all() and not bst.any()),
                "vs_plain_s2cn2": b_value / (world * s2cn2["value"]),
-               "fp64": dict(fp64_fraction(b_flops / bcv, b_value / world, fpk),
+               "fp64": dict(fp64_reference_work(b_flops / bcv, b_value / world, fpk),
                             note="flops per update counted per velocity set (24^2: %.0f, 32^2: %.0f, 48^2: %.0f) "
                                  "and weighted by each instance's cell-velocities" %
                                  (S2CN2_FLOPS_BY_TABLE[24], S2CN2_FLOPS_BY_TABLE[32], S2CN2_FLOPS_BY_TABLE[48])),
