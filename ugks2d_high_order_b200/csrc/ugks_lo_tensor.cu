@@ -6,8 +6,8 @@
 //
 // The kernels of ugks_lo.cu take every velocity sum as a block reduction, five to seven a CTA, each with its barriers
 // and a scalar phase behind it, take an exponential a velocity and equilibrium, and read the distribution and its stored
-// slopes twice.  Here the distribution is read once into registers (the slopes formed on the way) and all its own sums
-// taken in one reduction, about a mean known beforehand.  Then one warp runs the scalar chain while the others take the
+// slopes twice.  Here all sums of the distribution's own are taken in one reduction over one reading of it (the slopes formed
+// on the way), about a mean known beforehand.  Then one warp runs the scalar chain while the others take the
 // equilibria's sums, whose exponentials are products of two rows on a tensor table.  The equilibria are projected
 // (mod_ImplicitCommon.f90:42-82) in the basis 1, cx, cy, c^2 / 2 about their mean, which spans the same corrections with
 // the same weights, max(|E|, eps max(1, max |E|)), and gated as there: by the pivots of the Gram matrix in the

@@ -88,10 +88,8 @@ __global__ void __launch_bounds__(128) k_s2_recon1(LoParams P, LoBuffers B, S2Bu
 // Cells in the three rows next to a wall (one-sided quartics across y; the wall sides for every velocity): CTA = 4
 // warps (field, axis) over 32 velocities, both sides of the axis held until theta is known.
 // Bound by FP64 arithmetic and issue slots (about 930 FP64 operations a thread, two threads a cell-velocity;
-// 56 % and 63 % busy).  Residency pays: at 8x64x32^2 the S2CN2 step took 392, 384, 382 and 380 us with 5, 6, 7 and 8
-// CTAs an SM (94 to 64 registers).  All four sides in the tables' form took 220 us here and this form 110 (ncu,
-// cold), k_s2_recon1 42 and 33; the step went from 500 to 380 us, at 48^2 velocities from 1011 to 748 us, and the
-// 16-instance batch from 9.24 to 6.63 ms a step.
+// 56 % and 63 % busy).  Residency pays: eight CTAs an SM, although 64 registers spill 412 / 388 bytes a thread, beat five to
+// seven.  104 us at 8x64x32^2 against 214 for all four sides in the tables' form, k_s2_recon1 34 against 42 (ncu, cold).
 // The limiter's candidate of a sample x < 0, (1 - margin) m / (m - x), falls with x (m > 0; theta is 0 otherwise): the
 // smallest sample gives the smallest candidate.
 __device__ __forceinline__ double s2_limit(double xmin, double mf) {
@@ -415,8 +413,8 @@ __global__ void __launch_bounds__(256) k_s2_target_sum(LoParams P, LoBuffers B, 
 
 // build_targets on a tensor-product velocity table (LoParams::tnu > 0): the closures by 1-D sums, eight lanes a
 // (cell, volume node), four nodes a warp -> the same node scalars.  Bound by the latency of the Newton
-// chain (two exponentials, a butterfly, a 4x4 solve an evaluation).  With the sums below it took the S2CN2 step at
-// 8x64x32^2 from 0.869 to 0.704 ms and the 16-instance batch from 17.5 to 14.0 ms a step.  Eight lanes a
+// chain (two exponentials, a butterfly, a 4x4 solve an evaluation): 16 us at 8x64x32^2 and 27 for the sums below, against 165
+// and 49 for the kernels above (ncu, cold).  Eight lanes a
 // node share the uniform scalar work four ways a warp and still fill the chip with 1152 warps at that size.
 // A table that is no tensor product (tensor_table) takes the kernels above.
 template <int R>
@@ -698,14 +696,13 @@ __global__ void __launch_bounds__(256, 3) k_s2_face_flux(LoParams P, LoBuffers B
 //   k_s2_face_moments : one CTA a face, the sums of the upwind face values that W0 and q0 of its three nodes need,
 //                       taken about the lower cell's velocity -> fscal[1..9] (the only pass over the velocities
 //                       that the node's scalars need; bound by the latency of the face cache's values, 48 KB
-//                       a face at 32^2: 12 loads in flight a thread.  One warp a node took the S2CN2 step to 357 us
-//                       instead of 347, 6 loads in flight to 363, 24 to 348)
+//                       a face at 32^2: 12 loads in flight a thread, 20 us; 6 in flight or one warp a node cost the step
+//                       10 to 16 us more)
 //   k_s2_face_nodes_t : eight lanes a node, W0's closure, make_mke, q0, the directions and Mt by 1-D sums
 //                       -> the node scalars of k_s2_face_nodes
 //   k_s2_face_flux_t  : one CTA a face, its three nodes' micro fluxes and their Gauss sum -> the face arrays
-// Against k_s2_face_nodes, k_s2_face_flux and k_s2_combine, which other tables and the wall variants' coefficient
-// outputs keep, the S2CN2 step at 8x64x32^2 went from 0.704 to 0.565 ms and the 16-instance batch from
-// 14.0 to 10.6 ms a step.
+// 20 + 26 + 69 us at 8x64x32^2 against 220 + 63 + 13 for k_s2_face_nodes, k_s2_face_flux and k_s2_combine (ncu, cold), which
+// other tables and the wall variants' coefficient outputs keep.
 __global__ void __launch_bounds__(128) k_s2_face_moments(LoParams P, LoBuffers B, S2Buffers SB) {
     if (eval_cached(B)) return;
     __shared__ double red[4][32];
@@ -863,9 +860,9 @@ __global__ void __launch_bounds__(128, 3) k_s2_face_nodes_t(LoParams P, LoBuffer
 // shared memory) times a cubic in the velocity, whose coefficients join s0, the slope and the time directions
 // with their Mt, plus the face values' part (ugks_node, mod_S2D1.f90:486-507).  The three nodes' Gauss sum
 // goes straight to the face arrays and its velocity moments are the face's macro flux, so no node flux is
-// stored.  The moments of each node's time direction are summed on the way and gated as in k_s2_face_flux (about 6 us a
-// step).  Bound by the latency of the face cache's 12 values a (face, velocity), 100 MB at 8x64x32^2.  Nodes unrolled
-// took 379 to 410 us a step instead of 347 (instruction fetch), 2 velocities a thread at four CTAs an SM 350.
+// stored.  The moments of each node's time direction are summed on the way and gated as in k_s2_face_flux (6 us of 69).
+// Bound by the latency of the face cache's 12 values a (face, velocity), 100 MB at 8x64x32^2.  The nodes unrolled wait on
+// instruction fetch (30 to 60 us more a step).
 struct S2FluxC {
     double u, v, ux, vy, ckh, l2, kq, kb, qx, qy, mt0, mt3, mt4;   // means, ck T / 2, 2 lam, mt0 coeff, kq 2 / ck, q0, Mt
     double e[5], t[5], d[2][5];   // polynomials 1, cx, cy, c^2 and b part: mt2 dm - mt0 K dirs; mt1 tangential; mt1 left, right
@@ -1200,9 +1197,10 @@ __global__ void __launch_bounds__(256, 2) k_s2_wall_nodes(LoParams P, LoBuffers 
 // sum the incident state's moments; three lanes then form the nodes' slopes, and each velocity's
 // incident flux is taken once, kept in registers until the wall density is known, and summed over the nodes
 // into the face arrays (no node flux is stored; nodew keeps the nodes' macro fluxes).  16 CTAs at nx = 8, beside
-// the interior faces on the side stream: bound by the chain closure -> slopes -> two block reductions (54 us alone,
-// 136 us for k_s2_wall_nodes, one warp a node).  S2CN2 step 8x64x32^2 527 -> 500 us, 7x21x20^2 166 -> 138 us,
-// HighOrderImplicit pseudo-step 701 -> 644 us; the batch, whose other instances hid it, 9.18 -> 9.24 ms.
+// the interior faces on the side stream: bound by the chain closure -> slopes -> two block reductions (50 us at 8x64x32^2,
+// 136 us for k_s2_wall_nodes, one warp a node; ncu, cold).  254 registers a thread keep an SM to itself, which costs a batch, whose
+// other instances hid the walls, 0.6 %.  Above 1024 velocities 512 threads with 5 each spill 776 / 916 bytes a thread,
+// in 2 nx CTAs.
 struct S2WallC {
     double n[4], t[4], m[4], hx, hy;   // normal, tangential, time slopes (half of the energy slope last); heat of the incident state
 };
@@ -1495,8 +1493,7 @@ cudaError_t s2_enqueue(int which, const LoParams& P, const LoBuffers& B, const S
     const int faces = which < 3, targets = which != 2;
     const long long nmacw = (faces ? (long long)nf * 2 : 0) + (targets ? (long long)nc : 0);   // warps
     // The macro pass feeds the targets and the face nodes, the reconstruction neither of them: with an evolution it runs on
-    // the side stream beside the reconstruction (S2CN2 step 381 -> 378 us, HighOrderImplicit pseudo-step 519 -> 510
-    // at 8x64x32^2), followed there by the targets of which 1 (first read after the face
+    // the side stream beside the reconstruction (9 us), followed there by the targets of which 1 (first read after the face
     // arrays) and, after the reconstruction, the wall nodes; which 3 and 5: everything on the main stream
     cudaStream_t ts = faces ? s2 : s;
     cudaError_t e = cudaSuccess;

@@ -610,9 +610,9 @@ __device__ __forceinline__ void target_vjp(const S2Th& th, const QV& v, const WM
 // build_targets of a state, transposed: one warp per (cell, volume node).  gT: cotangents of the six
 // target arrays; the node's scalars (tscal) and state (wq) come from the forward targets of that state.
 // Writes gwq[(cell * 9 + node) * 4 + m].  TENSOR: the sums by polynomial nodes, 6 evaluations of the first pass's
-// expression a column and 2 a lane of the second's in place of one a velocity; three warps a CTA, so that a cell is three CTAs and their shared
-// memory admits four an SM.  At 8x64x32^2 (4608 nodes) 177 us before, 100 with the nodes and 86 with the scalars in shared
-// memory; 3, 5 and 6 CTAs an SM 107, 111 and 141 us (ncu, cold).
+// expression a column and 2 a lane of the second's in place of one a velocity; three warps a CTA, so that a cell is three
+// CTAs and their shared memory admits four an SM.  At 8x64x32^2 (4608 nodes) 87 us, 177 by velocities with the scalars in every
+// lane; 3, 5 and 6 CTAs an SM 107, 111 and 141 (ncu, cold).
 struct AdjTargetShared {   // a warp's: the node, the closure's Jacobian and its cotangent, two right-hand sides J^T x = b
     S2Th th;
     WMke M;
@@ -1030,11 +1030,10 @@ struct PnFace {   // a warp's row basis, its columns' nodes, node weights and th
 // Cotangents out: the face cache at the upwind side of every velocity (grec, written; the other side's
 // entry is set to zero), the macro slopes of the node (gmac) and mu_ref.
 // The node's scalars and its 4x4 systems are the warp's in shared memory: held by every lane they were 110 registers
-// and 2.6 KB of spills a thread at three CTAs an SM.  TENSOR: the sums by polynomial nodes.  At 8x64x32^2 (3048 nodes)
-// 408 us without, 257 with them, 169 with the scalars in shared memory and the columns' nodes stored before the long
-// expression runs, so that its 31 sums are not live beside the reads, 158 with the last pass's reads ahead of its
-// stores (ncu, cold).  What bounds it now is the latency of its reads at 12 warps an SM in 1.7 waves: 4 CTAs of two
-// warps, without the last change, took 197 us, 5 with it 161.
+// and 2.6 KB of spills a thread at three CTAs an SM.  TENSOR: the sums by polynomial nodes, the columns' nodes stored before
+// the long expression runs, so that its 31 sums are not live beside the reads, and the last pass's reads ahead of its
+// stores.  At 8x64x32^2 (3048 nodes) 157 us, 408 by velocities (ncu, cold); 456 / 548 bytes of spills a thread.  Bound by the
+// latency of its reads at 12 warps an SM in 1.7 waves; 4 and 5 CTAs an SM 197 and 161 us.
 template <bool TENSOR>
 __global__ void __launch_bounds__(TENSOR ? 64 : 128, TENSOR ? 6 : 3) k_adj_face_nodes(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
     const int nv = P.nvel, nx = P.nx, ny = P.ny, ck = P.ck, nr = (nv + 31) >> 5, lane = threadIdx.x & 31;
@@ -1508,8 +1507,8 @@ __device__ void wall_chain(const LoParams& P, double dt, double side, const T in
 // Out: the wall cell's face cache at its wall side (written), its W, the wall speed and temperature and
 // mu_ref (added).  R > 0: the closure by 1-D sums (tensor-product tables of up to 8 R abscissae an axis).
 // It runs beside the interior nodes, and a domain has few wall nodes, so the chain of one node's passes is what it costs:
-// at 8x64x32^2 (48 nodes) 256 us by a warp a node, 75 by 4 warps, 68 by 8 and 79 by 16; beside the interior nodes the 4
-// leave them the most room (backward and forward 1174 us a step, 1182 with 8, 1187 with 16, 1239 by a warp a node).
+// at 8x64x32^2 (48 nodes) 256 us by a warp a node, 77 by 4 warps, 68 by 8 and 79 by 16 (ncu, cold); beside the interior
+// nodes the 4 leave them the most room (1 % of a step over 8 or 16).
 template <int R>
 __global__ void __launch_bounds__(kAdjWall, 1) k_adj_wall_nodes(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
     const int nv = P.nvel, nx = P.nx, ny = P.ny, ck = P.ck, lane = threadIdx.x & 31, nr = (nv + kAdjWall - 1) / kAdjWall;
@@ -1982,7 +1981,7 @@ __global__ void __launch_bounds__(256, 3) k_adj_recon2_wall(LoParams P, LoBuffer
 // leaves through carries cotangents (the face cache keeps no other), so a thread runs that side's template and its
 // transpose; the other side and the volume rows enter the limiter's minimum with their values, and a transpose of theirs
 // runs only where one of them is the smallest sample of a limited cell.
-// At 8x64x32^2 188 us and 62 for the wall rows, which run beside it, against 482 for all cells in the wall rows' form
+// At 8x64x32^2 188 us and 55 for the wall rows, which run beside it, against 482 for all cells in the wall rows' form
 // (ncu, cold); 3, 4 and 6 CTAs an SM took 216, 191 and 195.
 __global__ void __launch_bounds__(128, 5) k_adj_recon2(LoParams P, LoBuffers B, S2Buffers S, AdjBuffers A) {
     __shared__ double s_th[4][32], s_gth[4][32];

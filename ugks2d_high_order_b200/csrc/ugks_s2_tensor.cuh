@@ -38,8 +38,7 @@ __device__ __forceinline__ double t_get(double v, int src) {
 // abscissae (pos) and weights (wt) of an axis of the table (LoBuffers::tab: rows of 64, padded with weight 0), and
 // the smallest exponential of each.  R >= abscissae / 8.  A function of its own, as is t_solve: a node runs through it
 // six to eight times, and in line the nodes' kernels spent more time fetching instructions than waiting on them
-// (stalls 3.0 against 2.1 an issue).  S2CN2 step 8x64x32^2 347 -> 344.5 us, HighOrderImplicit pseudo-step 490 -> 486,
-// 16-instance batch 6.23 -> 6.14 ms a step.
+// (stalls 3.0 against 2.1 an issue; 1 % of an S2CN2 step).
 struct TAxes {
     double x[6], y[6], ex, ey;
 };
@@ -326,7 +325,8 @@ __device__ bool t_mke(const LoParams& P, const LoBuffers& B, const double w[4], 
 // rows of exponentials (the Gauss weight and rho / (pi T) folded into the x row), and M, K_x, K_y the product times a
 // cubic in the velocity whose coefficients are the node's.
 // make_mke's gate on the moments of K_x and K_y (2e-12) is taken here on the sums over the nodes, by the kernels that form
-// them, with every velocity's own rounding; each node's is t_mke's, by 1-D sums.  Per node and velocity it cost 4 % of a step.
+// them, with every velocity's own rounding; each node's is t_mke's, by 1-D sums.  Per node and velocity it cost 4 % of an S2CN2
+// step more.
 constexpr double kTGate = 2.0e-12;
 struct STargetNode {   // mean of theta, mean of the state, ck T / 2, the cubic's coefficients
     double u, v, ux, vy, ckh, sl, s0, kb;   // Shakhov factor sl c^2 - s0; kb = 2 coeff / ck

@@ -128,10 +128,9 @@ __global__ void __launch_bounds__(NT) k_cn_stream(LoParams P, LoBuffers B, S2Buf
 // the CN collision of advance_step (mod_S2D1.f90:1376-1421): one CTA per cell, then the step's
 // acceptance in the last CTA.  The targets of the stream state stay in registers through both passes; on a tensor
 // velocity table the CTA also forms them from the node scalars (STargets) and writes them for the next step, instead of
-// reading what a kernel of its own stored.  Bound by the barriers around its three reductions at 16 warps an SM; with
-// 6 maxima instead of 11 in the last one the S2CN2 step at 8x64x32^2 went from 378 to 372 us and the 16-instance
-// batch from 6.6 to 6.5 ms a step.  512 threads (2 velocities each, 64 registers) took 390 us, 128 threads (8) 387,
-// three CTAs an SM (80 registers) 404.
+// reading what a kernel of its own stored.  Bound by the barriers around its three reductions at 16 warps an SM: 68 us at
+// 8x64x32^2 (ncu, cold), 53 + 49 with the targets' kernel apart.  512 threads with 2 velocities, 128 with 8, and three
+// CTAs an SM were 4 to 8 % slower over a step.
 template <int VPT, int NT, bool TENSOR>
 __global__ void __launch_bounds__(NT, 512 / NT) k_cn_collide(LoParams P, LoBuffers B, S2Buffers Tn, CnBuffers C, LoBuffers Bo) {
     if (halted(B)) return;
